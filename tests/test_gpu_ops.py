@@ -291,3 +291,15 @@ def test_attention_bf16_prefill_tcgen05(rb, orc, B, nh, kvh, S, L, mode):
     # one query tile per CTA (the default at these sizes) and two query tiles per CTA (forced from 256 query rows
     # up) do the same arithmetic per row
     assert np.array_equal(got, two_tiles)
+
+
+@pytest.mark.parametrize("M,K,N", [(1, 1, 1), (2, 3, 7), (3, 4, 8), (5, 511, 9), (8, 512, 33), (9, 513, 31), (16, 1025, 100), (17, 515, 1376),
+                                   (64, 96, 1024), (512, 70, 65), (513, 70, 65)])
+def test_f32_linear_row_groups_and_strips(rb, M, K, N):
+    """Edges of the row groups (1, 2, 4, 8, 16), column strips (8, 32), staged parts of K (512) and the step to 64x64 tiles.
+    Any order of K products and the bias is within (K + 1) roundings of 2^-24 of the absolute sum."""
+    rng = np.random.default_rng(M * 7 + K)
+    x, w, b = rng.normal(size=(M, K)).astype(np.float32), rng.normal(size=(K, N)).astype(np.float32), rng.normal(size=N).astype(np.float32)
+    y = rb.Linear(T(rb, w), T(rb, b)).forward(T(rb, x)).to_host()
+    want = x.astype(np.float64) @ w + b
+    assert np.all(np.abs(y - want) <= (K + 1) * 2.0 ** -24 * (np.abs(x).astype(np.float64) @ np.abs(w) + np.abs(b)))
