@@ -790,7 +790,10 @@ int layered_plans(rewb200_model* m) {
       D.g.m.talk_wide = std::any_of(D.g.talk_host.begin(), D.g.talk_host.end(), [](float t) { return !(std::fabs(t) < 65504.f); });
     }
   if (m->cfg.dtype != REWB200_BF16) return REWB200_OK;
-  auto plan = [&](LinW& w) { return linear_bf16_plan(&w.plan, (const bf16*)w.w, w.K, w.N, 0); };
+  auto plan = [&](LinW& w) {
+    w.plan.early_w = true;
+    return linear_bf16_plan(&w.plan, (const bf16*)w.w, w.K, w.N, 0);
+  };
   if (m->loop_in.w) RB_TRY(plan(m->loop_in));
   for (LayerDev& D : m->layers) {
     for (LinW* w : mixer_linears(D)) RB_TRY(plan(*w));

@@ -1544,6 +1544,9 @@ int rewb200_model_finalize(rewb200_model* m) {
       }
     }
     RB_TRY(linear_bf16_plan(&m->lm.plan, (const bf16*)m->lm.w, m->lm.K, m->lm.N, 0));
+    for (LayerDev& L : m->layers)  // a quantised Linear's matrix is scratch, expanded right ahead of the launch that reads it
+      for (LinW* w : {&L.qkv, &L.o, &L.gu, &L.down, &L.x.router}) w->plan.early_w = !w->quant;
+    m->lm.plan.early_w = true;
   }
   for (LayerDev& L : m->layers)  // shared experts' down biases were summed on the host
     if (!m->layered && L.moe && L.ffn_local > 0)

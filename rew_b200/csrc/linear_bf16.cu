@@ -293,9 +293,20 @@ int linear_bf16_pick_ksplit(Ctx* c, int64_t M, int64_t K, int64_t N) {
   const int tiles = (int)((N + BN - 1) / BN);
   const int nkb = (int)((K + BK - 1) / BK);
   const int target = 2 * c->sm_count;
+  int split = 1;
+  if (M > 64 && c->linear_impl != 0) {
+    // Above 64 rows every slab costs its M rows twice through L2 (4 bytes an element there and back, about 4 TB/s), and an SM
+    // spends 0.29 us on a 128 x 64 block of weights whatever the step's rows: the count that makes both together least.
+    // 135 rows of 4096 x 6144 (48 tiles) take 3 slabs, of 4096 x 4096 and 14336 x 4096 (32 tiles) 4.
+    double best = 0;
+    for (int k = 1; k <= 4 && (k == 1 || nkb / k >= c->splitk_min_blocks); ++k) {
+      const double us = 0.29 * ((tiles * k + c->sm_count - 1) / c->sm_count) * ((nkb + k - 1) / k) + 8e-6 * k * M * N / 4;
+      if (k == 1 || us < best) best = us, split = k;
+    }
+    return split;
+  }
   // every split is another f32 slab of M rows that the consumer kernel reads back: fewer of them as the step grows
   const int cap = M <= 64 ? 16 : (M <= 128 ? 4 : 2);
-  int split = 1;
   // stop doubling once the CTA count would overshoot the resident slots by more than a quarter
   while (tiles * split * 2 <= target + target / 4 && nkb / (split * 2) >= c->splitk_min_blocks && split < cap) split *= 2;
   // a launch that still leaves SMs empty (narrow layers of a tensor-parallel shard) may cut K finer

@@ -8,7 +8,7 @@
 // accumulator D[feature][token] lives in TMEM: lane = output feature, column =
 // token.
 //
-// Roles inside the CTA (192 threads):
+// Roles inside the CTA (320 threads):
 //   warp 0   TMA producer: cp.async.bulk.tensor boxes of W (64 k x 64 features,
 //            two per stage) and x (64 k x TN tokens), 128-byte swizzle, into a
 //            multi-stage mbarrier ring; W loads are issued before
@@ -16,7 +16,7 @@
 //   warp 1   allocates TMEM, then one elected thread issues four
 //            tcgen05.mma.kind::f16 (K = 16 each) per stage from shared-memory
 //            descriptors and releases the stage with tcgen05.commit.
-//   warps 2-5 epilogue: tcgen05.ld the accumulator (each warp owns 32 lanes),
+//   warps 2-9 epilogue: tcgen05.ld the accumulator (a warp owns 32 lanes),
 //            apply bias / SwiGLU, store.
 // All waits are bounded; on a timeout the roles fall through to the common
 // exit, where TMEM is released.
@@ -34,17 +34,6 @@ constexpr int BM = 128;  // output features per CTA
 constexpr int BK = 64;
 constexpr int A_BYTES = 2 * BK * 64 * 2;  // two 64x64 boxes
 
-template <int TN>
-struct TcCfg {
-  // 32 tokens: 5 x 20 KB, 64: 4 x 24 KB, 128: 3 x 32 KB, so that two CTAs share an SM (these tiles serve steps
-  // with a single token tile, where a launch has only as many CTAs as feature tiles x splits); 256: 4 x 48 KB
-  static constexpr int STAGES = TN <= 32 ? 5 : (TN <= 64 ? 4 : (TN <= 128 ? 3 : 4));
-  static constexpr int B_BYTES = TN * 128;
-  static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 + 256;
-  static constexpr int TMEM_COLS = TN < 32 ? 32 : TN;
-};
-
 struct TcArgs {
   int64_t M, N, K;
   int kb_per_split;
@@ -56,8 +45,36 @@ struct TcArgs {
   int* status;
   const int* row_offsets;  // grouped launches (persistent kernel): rows of group g = [row_offsets[g], row_offsets[g+1])
   int groups;
+  int tn, stages;          // launches that choose their tile and ring
+  int ksplit;              // persistent kernel: pieces of a tile along K
+  int early_w;             // ... the weights are final before any step: they may be requested ahead of the stream dependency
   int fuse_qkv;       // cluster kernel: finish q|k|v in the epilogue (bias, RoPE, cache write) instead of one f32 slab
   QkvPostArgs qp;     // what qkv_post_kernel would have been given (partial / nsplit unused)
+};
+
+template <int TN>
+struct TcCfg {
+  // 32 tokens: 5 x 20 KB, 64: 4 x 24 KB, so that two CTAs share an SM (these tiles serve steps with a single token
+  // tile, where a launch has only as many CTAs as feature tiles x splits)
+  static constexpr int STAGES = TN <= 32 ? 5 : 4;
+  static constexpr int B_BYTES = TN * 128;
+  static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
+  static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 + 256;
+  static constexpr int TMEM_COLS = TN < 32 ? 32 : TN;
+  __device__ __forceinline__ static int tn(const TcArgs&) { return TN; }
+  __device__ __forceinline__ static int stages(const TcArgs&) { return STAGES; }
+  __device__ __forceinline__ static uint32_t tmem_cols(const TcArgs&) { return TMEM_COLS; }
+};
+// TN = 0: steps of more than 64 tokens, whose tile (a multiple of 16 tokens) and ring are the launch's choice.  Up to 160
+// tokens two CTAs share an SM, with three stages or more each; larger tiles have the SM to themselves.
+template <>
+struct TcCfg<0> {
+  static constexpr int MAX_STAGES = 8;
+  static constexpr int FIXED = 1024 + 256;
+  static constexpr int stage_bytes(int tn) { return A_BYTES + tn * 128; }
+  __device__ __forceinline__ static int tn(const TcArgs& a) { return a.tn; }
+  __device__ __forceinline__ static int stages(const TcArgs& a) { return a.stages; }
+  __device__ __forceinline__ static uint32_t tmem_cols(const TcArgs& a) { return a.tn <= 128 ? 128u : 256u; }
 };
 
 // ---- thread-block cluster pieces of the split-K kernel
@@ -88,6 +105,81 @@ __device__ __forceinline__ float act_f(float v, int epi) {
   if (epi != EPI_RELU2_BF16) return v;
   v = fmaxf(v, 0.f);
   return v * v;
+}
+
+// The way out of an accumulator.  Eight warps share a tile: warp w owns the tensor-memory lanes 32 (w % 4) .. + 31, one feature
+// a lane, and every other run of 16 tokens, so that each scheduler has two warps to hide the tensor-memory loads and the
+// shuffles of one another.  Values leave straight from the registers: for bf16, two neighbouring lanes trade a token, so that a
+// store holds two neighbouring features and a warp writes whole 32-byte sectors.  SwiGLU: gates sit in lanes with
+// (lane & 8) == 0, their up partners eight lanes higher; such a pair trades a token the same way, so that both compute.
+// With four warps and rows staged through shared memory for 16-byte stores, 32 tokens took 1.2 us of a tile's exposed tail.
+constexpr int EPI_WARPS = 8;
+constexpr int TC_THREADS = 64 + 32 * EPI_WARPS;
+
+template <int EPI>
+__device__ __forceinline__ void store_tokens(const TcArgs& a, uint32_t tmem, void* out, int64_t feat0, int lane, int half, float bias_v, int64_t row0,
+                                             int rows, bool any) {
+  const bool feat_ok = feat0 + lane < a.N;
+  const int64_t ldo = a.ldo;
+#pragma unroll 1
+  for (int c0 = 16 * half; c0 < rows; c0 += 32) {
+    uint32_t r[16];
+    if (any) {
+      tc::ld16(tmem + (uint32_t)c0, r);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) r[j] = 0u;
+    }
+    const int here = feat_ok ? min(16, rows - c0) : 0;
+    float v[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]) + bias_v;
+    if constexpr (EPI == EPI_PARTIAL_F32 || EPI == EPI_BIAS_F32) {
+      float* o = reinterpret_cast<float*>(out) + (row0 + c0) * ldo + feat0 + lane;
+#pragma unroll
+      for (int j = 0; j < 16; ++j, o += ldo)
+        if (j < here) *o = v[j];
+    } else if constexpr (EPI == EPI_SWIGLU_BF16) {
+      const bool up = (lane & 8) != 0, odd = (lane & 1) != 0;
+      const int first = (odd ? 2 : 0) + (up ? 1 : 0);   // of every four tokens
+      bf16* o = reinterpret_cast<bf16*>(out) + (row0 + c0 + first) * ldo + feat0 / 2 + (lane >> 4) * 8 + (lane & 6);
+#pragma unroll
+      for (int j = 0; j < 16; j += 4, o += 4 * ldo) {
+        float h[2];   // of tokens j + up and j + 2 + up
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const float keep = up ? v[j + 2 * i + 1] : v[j + 2 * i];
+          const float got = __shfl_xor_sync(0xffffffffu, up ? v[j + 2 * i] : v[j + 2 * i + 1], 8);
+          h[i] = silu_f(up ? got : keep) * (up ? keep : got);
+        }
+        const float got = __shfl_xor_sync(0xffffffffu, odd ? h[0] : h[1], 1);
+        if (j + first < here) *reinterpret_cast<uint32_t*>(o) = odd ? pack_bf16(got, h[1]) : pack_bf16(h[0], got);
+      }
+    } else {
+      const bool odd = (lane & 1) != 0;
+      const int first = odd ? 1 : 0;                    // of every two tokens
+      bf16* o = reinterpret_cast<bf16*>(out) + (row0 + c0 + first) * ldo + feat0 + (lane & 30);
+#pragma unroll
+      for (int j = 0; j < 16; j += 2, o += 2 * ldo) {
+        const float v0 = act_f(v[j], EPI), v1 = act_f(v[j + 1], EPI);
+        const float got = __shfl_xor_sync(0xffffffffu, odd ? v0 : v1, 1);
+        if (j + first < here) *reinterpret_cast<uint32_t*>(o) = odd ? pack_bf16(got, v1) : pack_bf16(v0, got);
+      }
+    }
+  }
+}
+// tmem: the accumulator's first column at this warp's lanes; row0, rows: the tile's tokens; any: whether anything was accumulated
+__device__ __forceinline__ void store_tile(const TcArgs& a, uint32_t tmem, void* out, int64_t feat0, int lane, int half, const float* bias, int64_t row0,
+                                           int rows, bool any) {
+  const float b = (bias && feat0 + lane < a.N && a.epi != EPI_PARTIAL_F32) ? bias[feat0 + lane] : 0.f;
+  switch (a.epi) {
+    case EPI_PARTIAL_F32:
+    case EPI_BIAS_F32: return store_tokens<EPI_BIAS_F32>(a, tmem, out, feat0, lane, half, b, row0, rows, any);
+    case EPI_SWIGLU_BF16: return store_tokens<EPI_SWIGLU_BF16>(a, tmem, out, feat0, lane, half, b, row0, rows, any);
+    case EPI_RELU2_BF16: return store_tokens<EPI_RELU2_BF16>(a, tmem, out, feat0, lane, half, b, row0, rows, any);
+    case EPI_GELU_BF16: return store_tokens<EPI_GELU_BF16>(a, tmem, out, feat0, lane, half, b, row0, rows, any);
+    default: return store_tokens<EPI_BIAS_BF16>(a, tmem, out, feat0, lane, half, b, row0, rows, any);
+  }
 }
 
 // Second half of the cluster split-K epilogue, run by the four epilogue warps of every CTA after the
@@ -199,15 +291,16 @@ __device__ __forceinline__ void cluster_finish(const TcArgs& a, uint8_t* smem, i
 // of the tile's tokens, so the launch leaves one finished slab (or finished q / k / v) instead of
 // ksplit partial slabs for the next kernel to add up.
 template <int TN, int CL>
-__global__ void __launch_bounds__(192) linear_tc_kernel(const __grid_constant__ CUtensorMap tmW,
+__global__ void __launch_bounds__(TC_THREADS) linear_tc_kernel(const __grid_constant__ CUtensorMap tmW,
                                                          const __grid_constant__ CUtensorMap tmX, TcArgs a) {
   static_assert(CL == 0 || TN == 32, "the cluster reduction is written for the decode tile");
   using C = TcCfg<TN>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + C::STAGES * C::STAGE_BYTES);
-  uint64_t* empty = full + C::STAGES;
-  uint64_t* tmem_full = empty + C::STAGES;
+  const int tn = C::tn(a), stages = C::stages(a), stage_bytes = A_BYTES + tn * 128;
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + stages * stage_bytes);
+  uint64_t* empty = full + stages;
+  uint64_t* tmem_full = empty + stages;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_full + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -227,15 +320,15 @@ __global__ void __launch_bounds__(192) linear_tc_kernel(const __grid_constant__ 
     tile_n = in_group / group_rows;
   }
   const int col0 = tile_n * BM;              // first output feature of the tile
-  const int row0 = tile_m * TN;              // first token of the tile
+  const int row0 = tile_m * tn;              // first token of the tile
   const int split = blockIdx.z;
-  const int rows_valid = (int)min((int64_t)TN, a.M - row0);
+  const int rows_valid = (int)min((int64_t)tn, a.M - row0);
   const int nkb_total = (int)((a.K + BK - 1) / BK);
   const int kb0 = split * a.kb_per_split;
   const int nkb = max(0, min(a.kb_per_split, nkb_total - kb0));
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < C::STAGES; ++s) {
+    for (int s = 0; s < stages; ++s) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
@@ -243,13 +336,25 @@ __global__ void __launch_bounds__(192) linear_tc_kernel(const __grid_constant__ 
     fence_barrier_init();
     pdl_launch_dependents();
   }
-  if (warp == 1) {
-    tc::alloc(tmem_slot, (uint32_t)C::TMEM_COLS);
+  // Large accumulators take their tensor memory after the stream dependency: a launch that held it while it waits could
+  // keep it from a CTA of the launch it waits for.
+  constexpr bool LATE = TN == 0;
+  if (LATE) {
+    __syncthreads();
+    if (warp != 0) {
+      pdl_wait();
+      if (warp == 1) tc::alloc(tmem_slot, C::tmem_cols(a));
+      tc::fence_before();
+      asm volatile("bar.sync 2, %0;" ::"n"(TC_THREADS - 32) : "memory");
+      tc::fence_after();
+    }
+  } else {
+    if (warp == 1) tc::alloc(tmem_slot, C::tmem_cols(a));
+    tc::fence_before();
+    __syncthreads();
+    tc::fence_after();
   }
-  tc::fence_before();
-  __syncthreads();
-  tc::fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = LATE && warp == 0 ? 0u : *tmem_slot;
 
   bool epi_ok = true;
   if (warp == 0) {
@@ -258,41 +363,40 @@ __global__ void __launch_bounds__(192) linear_tc_kernel(const __grid_constant__ 
       tma_prefetch_desc(&tmX);
       const uint64_t pol_w = policy_evict_first();
       const uint64_t pol_x = policy_evict_last();
-      const int pre = min(C::STAGES, nkb);
+      const int pre = min(stages, nkb);
       for (int kb = 0; kb < pre; ++kb) {
-        uint8_t* st = smem + kb * C::STAGE_BYTES;
-        mbar_expect_tx(&full[kb], C::STAGE_BYTES);
+        uint8_t* st = smem + kb * stage_bytes;
+        mbar_expect_tx(&full[kb], stage_bytes);
         const int k = (kb0 + kb) * BK;
         tma_load_2d_hint(st, &tmW, &full[kb], col0, k, pol_w);
         tma_load_2d_hint(st + A_BYTES / 2, &tmW, &full[kb], col0 + 64, k, pol_w);
       }
       pdl_wait();
       for (int kb = 0; kb < pre; ++kb)
-        tma_load_2d_hint(smem + kb * C::STAGE_BYTES + A_BYTES, &tmX, &full[kb], (kb0 + kb) * BK, row0, pol_x);
-      for (int kb = pre; kb < nkb; ++kb) {
-        const int s = kb % C::STAGES;
-        if (!mbar_wait(&empty[s], ((kb / C::STAGES) - 1) & 1, a.status)) break;
-        uint8_t* st = smem + s * C::STAGE_BYTES;
-        mbar_expect_tx(&full[s], C::STAGE_BYTES);
+        tma_load_2d_hint(smem + kb * stage_bytes + A_BYTES, &tmX, &full[kb], (kb0 + kb) * BK, row0, pol_x);
+      for (int kb = pre, s = 0, lap = 0; kb < nkb; ++kb) {
+        if (!mbar_wait(&empty[s], lap & 1, a.status)) break;
+        uint8_t* st = smem + s * stage_bytes;
+        mbar_expect_tx(&full[s], stage_bytes);
         const int k = (kb0 + kb) * BK;
         tma_load_2d_hint(st, &tmW, &full[s], col0, k, pol_w);
         tma_load_2d_hint(st + A_BYTES / 2, &tmW, &full[s], col0 + 64, k, pol_w);
         tma_load_2d_hint(st + A_BYTES, &tmX, &full[s], k, row0, pol_x);
+        if (++s == stages) s = 0, ++lap;
       }
     }
   } else if (warp == 1) {
     if (lane == 0 && nkb > 0) {
-      // instruction descriptor: D f32, A/B bf16, A MN-major, B K-major, N = TN, M = 128
-      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | ((uint32_t)(TN >> 3) << 17) |
+      // instruction descriptor: D f32, A/B bf16, A MN-major, B K-major, N = tn, M = 128
+      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | ((uint32_t)(tn >> 3) << 17) |
                              ((uint32_t)(BM >> 4) << 24);
       const uint32_t smem_base = smem_u32(smem);
       bool ok = true;
-      for (int kb = 0; kb < nkb && ok; ++kb) {
-        const int s = kb % C::STAGES;
-        ok = mbar_wait(&full[s], (kb / C::STAGES) & 1, a.status);
+      for (int kb = 0, s = 0, lap = 0; kb < nkb && ok; ++kb) {
+        ok = mbar_wait(&full[s], lap & 1, a.status);
         if (!ok) break;
         tc::fence_after();
-        const uint32_t sa = smem_base + s * C::STAGE_BYTES;
+        const uint32_t sa = smem_base + s * stage_bytes;
         const uint32_t sb = sa + A_BYTES;
 #pragma unroll
         for (int kk = 0; kk < BK / 16; ++kk) {
@@ -303,16 +407,13 @@ __global__ void __launch_bounds__(192) linear_tc_kernel(const __grid_constant__ 
           tc::umma_bf16_ss(tmem_base, da, db, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
         }
         tc::commit(&empty[s]);  // stage is free once these MMAs have read it
+        if (++s == stages) s = 0, ++lap;
       }
       if (ok) tc::commit(tmem_full);
     }
   } else {
-    // ---------------- epilogue warps 2..5; TMEM lanes 32*(warp%4) .. +31
-    // The accumulator is D[feature][token]; the output is [token][feature].  Each thread owns one
-    // feature, so the tile is transposed through shared memory (the pipeline stages are free once
-    // tmem_full fires) and then written with 16-byte, fully coalesced stores.
-    const int q = warp & 3;
-    const int et = threadIdx.x - 64;  // 0..127 among the epilogue threads
+    // ---------------- epilogue warps 2..9; TMEM lanes 32*(warp%4) .. +31
+    const int q = warp & 3, half = (warp - 2) >> 2;
     bool ok = true;
     if (nkb > 0) {
       ok = mbar_wait(tmem_full, 0, a.status);
@@ -321,115 +422,23 @@ __global__ void __launch_bounds__(192) linear_tc_kernel(const __grid_constant__ 
     pdl_wait();
     if constexpr (CL == 1) {
       // own partial tile -> shared memory as [token][feature] f32 (the pipeline stages are free by now)
-      uint32_t r[32];
       ok = __all_sync(0xffffffffu, ok);  // the tensor-memory load below is warp-collective
-      if (ok && nkb > 0) {
-        tc::ld32(tmem_base + ((uint32_t)(q * 32) << 16), r);
-      } else {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) r[j] = 0u;
-      }
-      float* stg = reinterpret_cast<float*>(smem);
-#pragma unroll
-      for (int j = 0; j < 32; ++j) stg[j * BM + q * 32 + lane] = __uint_as_float(r[j]);
-      epi_ok = ok;
-    } else if constexpr (TN == 32) {
-      // decode-size tile: the output is a few KB, direct stores (32 lanes = 32 consecutive features)
-      if (ok) {
-        const int64_t feat = (int64_t)col0 + q * 32 + lane;
-        const bool feat_ok = feat < a.N;
-        const float bias_v = (a.bias && feat_ok && a.epi != EPI_PARTIAL_F32) ? a.bias[feat] : 0.f;
+      if (half == 0) {
         uint32_t r[32];
-        if (nkb > 0) {
+        if (ok && nkb > 0) {
           tc::ld32(tmem_base + ((uint32_t)(q * 32) << 16), r);
         } else {
 #pragma unroll
           for (int j = 0; j < 32; ++j) r[j] = 0u;
         }
-        if (a.epi == EPI_SWIGLU_BF16) {
-          const bool is_gate = (lane & 15) < 8;
-          const int64_t oc = ((int64_t)col0 + q * 32) / 2 + (lane >> 4) * 8 + (lane & 7);
+        float* stg = reinterpret_cast<float*>(smem);
 #pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const float v = __uint_as_float(r[j]) + bias_v;
-            const float up = __shfl_down_sync(0xffffffffu, v, 8);
-            if (is_gate && feat_ok && j < rows_valid)
-              reinterpret_cast<bf16*>(a.out)[(int64_t)(row0 + j) * a.ldo + oc] = __float2bfloat16_rn(silu_f(v) * up);
-          }
-        } else if (feat_ok) {
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            if (j >= rows_valid) break;
-            const float v = __uint_as_float(r[j]) + bias_v;
-            const int64_t grow = row0 + j;
-            if (a.epi == EPI_PARTIAL_F32)
-              reinterpret_cast<float*>(a.out)[split * a.split_stride + grow * a.ldo + feat] = v;
-            else if (a.epi == EPI_BIAS_F32)
-              reinterpret_cast<float*>(a.out)[grow * a.ldo + feat] = v;
-            else
-              reinterpret_cast<bf16*>(a.out)[grow * a.ldo + feat] = __float2bfloat16_rn(act_f(v, a.epi));
-          }
-        }
+        for (int j = 0; j < 32; ++j) stg[j * BM + q * 32 + lane] = __uint_as_float(r[j]);
       }
-    } else {
-      const bool swiglu = a.epi == EPI_SWIGLU_BF16;
-      const bool out_f32 = a.epi == EPI_PARTIAL_F32 || a.epi == EPI_BIAS_F32;
-      const int tile_cols = swiglu ? 64 : 128;
-      const int row_bytes = tile_cols * (out_f32 ? 4 : 2);
-      uint8_t* stg = smem;
-      if (ok) {
-        const int64_t feat = (int64_t)col0 + q * 32 + lane;
-        const bool feat_ok = feat < a.N;
-        const float bias_v = (a.bias && feat_ok && a.epi != EPI_PARTIAL_F32) ? a.bias[feat] : 0.f;
-        // gate features sit in lanes with (lane % 16) < 8, their up partners 8 lanes higher
-        const bool is_gate = (lane & 15) < 8;
-        const int hcol = q * 16 + (lane >> 4) * 8 + (lane & 7);
-  #pragma unroll 1
-        for (int c0 = 0; c0 < TN; c0 += 32) {
-          if (c0 >= rows_valid) break;
-          uint32_t r[32];
-          if (nkb > 0) {
-            tc::ld32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, r);
-          } else {
-  #pragma unroll
-            for (int j = 0; j < 32; ++j) r[j] = 0u;
-          }
-          if (swiglu) {
-  #pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              const float v = __uint_as_float(r[j]) + bias_v;
-              const float up = __shfl_down_sync(0xffffffffu, v, 8);
-              if (is_gate) reinterpret_cast<bf16*>(stg + (c0 + j) * row_bytes)[hcol] = __float2bfloat16_rn(silu_f(v) * up);
-            }
-          } else if (out_f32) {
-  #pragma unroll
-            for (int j = 0; j < 32; ++j)
-              reinterpret_cast<float*>(stg + (c0 + j) * row_bytes)[q * 32 + lane] = __uint_as_float(r[j]) + bias_v;
-          } else {
-  #pragma unroll
-            for (int j = 0; j < 32; ++j)
-              reinterpret_cast<bf16*>(stg + (c0 + j) * row_bytes)[q * 32 + lane] = __float2bfloat16_rn(act_f(__uint_as_float(r[j]) + bias_v, a.epi));
-          }
-        }
-      }
-      asm volatile("bar.sync 1, 128;" ::: "memory");  // the four epilogue warps only
-      if (ok) {
-        const int chunks_per_row = row_bytes / 16;           // 32 (f32), 16 (bf16), 8 (SwiGLU)
-        const int elems_per_chunk = out_f32 ? 4 : 8;
-        const int64_t out_col0 = swiglu ? col0 / 2 : col0;
-        const int64_t out_cols = swiglu ? a.N / 2 : a.N;
-        const size_t esz = out_f32 ? 4 : 2;
-        uint8_t* obase = reinterpret_cast<uint8_t*>(a.out) + (a.epi == EPI_PARTIAL_F32 ? (size_t)split * a.split_stride * 4 : 0);
-        const int total = rows_valid * chunks_per_row;
-        for (int i = et; i < total; i += 128) {
-          const int row = i / chunks_per_row, ch = i % chunks_per_row;
-          const int64_t col = out_col0 + (int64_t)ch * elems_per_chunk;
-          if (col >= out_cols) continue;
-          const uint4 v = *reinterpret_cast<const uint4*>(stg + row * row_bytes + ch * 16);
-          *reinterpret_cast<uint4*>(obase + ((size_t)(row0 + row) * a.ldo + col) * esz) = v;
-        }
-      }
-
+      epi_ok = ok;
+    } else if (ok) {
+      void* out = reinterpret_cast<uint8_t*>(a.out) + (a.epi == EPI_PARTIAL_F32 ? (size_t)split * a.split_stride * 4 : 0);
+      store_tile(a, tmem_base + ((uint32_t)(q * 32) << 16), out, (int64_t)col0 + q * 32, lane, half, a.bias, row0, rows_valid, nkb > 0);
     }
   }
   (void)epi_ok;
@@ -437,7 +446,7 @@ __global__ void __launch_bounds__(192) linear_tc_kernel(const __grid_constant__ 
     (void)rows_valid;
     __syncwarp();
     cluster_sync_all();  // every CTA of the cluster has staged its partial tile
-    if (warp >= 2) {
+    if (warp >= 2 && warp < 6) {
       const int q = warp & 3;
       switch (gridDim.z) {
         case 2: cluster_finish<2>(a, smem, q, lane, col0, row0, epi_ok); break;
@@ -447,29 +456,36 @@ __global__ void __launch_bounds__(192) linear_tc_kernel(const __grid_constant__ 
     }
     cluster_sync_all();  // nobody leaves while a peer may still read its tile
   }
+  __syncwarp();  // the lanes of a role come back together: what follows is warp-collective
   tc::fence_before();
   __syncthreads();
   if (warp == 1) {
     tc::fence_after();
-    tc::dealloc(tmem_base, (uint32_t)C::TMEM_COLS);
+    tc::dealloc(tmem_base, C::tmem_cols(a));
   }
 }
 
-// ---- persistent variant for prefill-size launches (256-token tiles, no split-K) -------------------
-// One CTA per SM walks its share of the output tiles.  The accumulator is double-buffered in TMEM
-// (2 x 256 columns), so the epilogue warps drain tile j while the MMA warp already accumulates tile
-// j + 1 and the TMA ring keeps running across tile boundaries; the per-tile cost becomes
-// max(main loop, epilogue) instead of their sum.  The epilogue transposes 32 tokens at a time through
-// two small staging buffers, which leaves room for the same four pipeline stages.
+// ---- persistent variant for steps of more than 64 tokens ------------------------------------------
+// One CTA per SM walks its share of the output tiles (or of their pieces along K).  The accumulator is
+// double-buffered in TMEM (2 x 256 columns), so the epilogue warps drain tile j while the MMA warp
+// already accumulates tile j + 1 and the TMA ring keeps running across tile boundaries; the per-tile
+// cost becomes max(main loop, epilogue) instead of their sum.  What bounds it: the tensor core takes
+// 0.27 us for the 128 x 64 block of weights of a stage whatever the tokens of the tile (the weights are
+// an MN-major operand), so a step of up to 256 tokens is fast when every SM has equal work and slow
+// when 32 of them do: hence the pieces along K, and tiles of the step's own size (a multiple of 16
+// tokens), which leave room for a deep ring.  135 tokens of 4096 x 28672: 42 us (67 us in one-tile CTAs
+// of 256 tokens), of which 35 us are the weights' time out of HBM.
 struct PersistCfg {
-  static constexpr int TN = 256;
-  static constexpr int STAGES = 4;
-  static constexpr int B_BYTES = TN * 128;
-  static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;   // 48 KB
-  static constexpr int STG_LD = 528;                      // bytes per staged token row (512 + 16: no bank conflicts)
-  static constexpr int STG_BYTES = 32 * STG_LD;           // 32 tokens x 128 features x 4 bytes
-  static constexpr int SMEM = STAGES * STAGE_BYTES + 2 * STG_BYTES + 1024 + 256;
+  static constexpr int TN = 256;                          // most tokens of a tile
+  static constexpr int MAX_STAGES = 8;
+  static constexpr int FIXED = 1024 + 256;
   static constexpr int TMEM_COLS = 512;
+  static constexpr int stage_bytes(int tn) { return A_BYTES + tn * 128; }
+  static constexpr int stages(int tn) {
+    const int n = (227 * 1024 - FIXED) / stage_bytes(tn);
+    return n < MAX_STAGES ? n : MAX_STAGES;
+  }
+  static constexpr int smem(int tn) { return stages(tn) * stage_bytes(tn) + FIXED; }
 };
 
 // GROUPED: the weights are `groups` stacked matrices (3-D tensor map, third coordinate = group, e.g. the
@@ -480,27 +496,26 @@ struct PersistCfg {
 constexpr int kMaxGroups = 256;
 constexpr int kMaxPersistCtas = 256;
 // Per-CTA list "token tiles ahead of each group" of the grouped launches.  The kernel's shared memory is full
-// (four 48 KB stages, two staging buffers), so each CTA keeps its copy in global memory, where it stays in L1.
+// (the stages of its ring), so each CTA keeps its copy in global memory, where it stays in L1.
 static __device__ int g_first_tile[kMaxPersistCtas][kMaxGroups + 1];
 
 template <bool GROUPED>
-__global__ void __launch_bounds__(192) linear_tc_persist_kernel(const __grid_constant__ CUtensorMap tmW,
+__global__ void __launch_bounds__(TC_THREADS) linear_tc_persist_kernel(const __grid_constant__ CUtensorMap tmW,
                                                                  const __grid_constant__ CUtensorMap tmX, TcArgs a,
                                                                  int tiles_n, int tiles_m) {
   using C = PersistCfg;
-  constexpr int TN = C::TN;
+  const int TN = GROUPED ? C::TN : a.tn, STAGES = C::stages(TN), stage_bytes = C::stage_bytes(TN);
   int* const s_first_tile = g_first_tile[blockIdx.x % kMaxPersistCtas];  // this CTA's copy (grouped launches only)
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* stg_base = smem + C::STAGES * C::STAGE_BYTES;
-  uint64_t* full = reinterpret_cast<uint64_t*>(stg_base + 2 * C::STG_BYTES);
-  uint64_t* empty = full + C::STAGES;
-  uint64_t* tmem_full = empty + C::STAGES;   // [2]
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES * stage_bytes);
+  uint64_t* empty = full + STAGES;
+  uint64_t* tmem_full = empty + STAGES;   // [2]
   uint64_t* tmem_empty = tmem_full + 2;      // [2]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nkb = (int)((a.K + BK - 1) / BK);
+  const int nkb_total = (int)((a.K + BK - 1) / BK);
   if constexpr (GROUPED) {
     pdl_wait();  // the row offsets come from an earlier kernel of the step
     if (threadIdx.x == 0) {
@@ -515,7 +530,12 @@ __global__ void __launch_bounds__(192) linear_tc_persist_kernel(const __grid_con
     __syncthreads();
     tiles_m = s_first_tile[a.groups];
   }
-  const int total_tiles = tiles_n * tiles_m;
+  // a tile is cut into a.ksplit pieces along K, whose sums go to slabs of their own; a whole output tile is one piece
+  const int plane = tiles_n * tiles_m, total_tiles = GROUPED ? plane : plane * a.ksplit;
+  auto k_range = [&](int lin, int& kb0, int& nkb) {
+    kb0 = GROUPED ? 0 : lin / plane * a.kb_per_split;
+    nkb = GROUPED ? nkb_total : max(0, min(a.kb_per_split, nkb_total - kb0));
+  };
   // Dense: same tile order as the one-tile kernel, groups of 8 token tiles per feature tile.  Grouped:
   // feature tiles fastest, so the CTAs of a wave work on a few token tiles of one or two experts.
   // row0 = first row of the tile, rows_valid = rows of it that belong to the output, grp = weight matrix.
@@ -535,6 +555,7 @@ __global__ void __launch_bounds__(192) linear_tc_persist_kernel(const __grid_con
     } else {
       constexpr int GROUP_M = 8;
       const int per_group = GROUP_M * tiles_n;
+      lin %= plane;
       const int group = lin / per_group;
       const int first_m = group * GROUP_M;
       const int group_rows = min(GROUP_M, tiles_m - first_m);
@@ -548,7 +569,7 @@ __global__ void __launch_bounds__(192) linear_tc_persist_kernel(const __grid_con
   };
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < C::STAGES; ++s) {
+    for (int s = 0; s < STAGES; ++s) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
@@ -573,30 +594,48 @@ __global__ void __launch_bounds__(192) linear_tc_persist_kernel(const __grid_con
       tma_prefetch_desc(&tmX);
       const uint64_t pol_w = policy_evict_first();
       const uint64_t pol_x = policy_evict_last();
+      int early = 0;   // stages whose weights were requested ahead of the stream dependency (no kernel of a step writes them)
+      if constexpr (!GROUPED) {
+        int tile_n, row0, rows_valid, grp, kb0, nkb;
+        tile_coords(blockIdx.x, tile_n, row0, rows_valid, grp);
+        k_range(blockIdx.x, kb0, nkb);
+        early = a.early_w ? min(STAGES, nkb) : 0;
+        for (int i = 0; i < early; ++i) {
+          uint8_t* st = smem + i * stage_bytes;
+          mbar_expect_tx(&full[i], stage_bytes);
+          tma_load_2d_hint(st, &tmW, &full[i], tile_n * BM, (kb0 + i) * BK, pol_w);
+          tma_load_2d_hint(st + A_BYTES / 2, &tmW, &full[i], tile_n * BM + 64, (kb0 + i) * BK, pol_w);
+        }
+      }
       pdl_wait();  // the activations come from the previous kernel
-      int it = 0;
+      int s = 0, lap = 0;
       bool ok = true;
       for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
-        int tile_n, row0, rows_valid, grp;
+        int tile_n, row0, rows_valid, grp, kb0, nkb;
         tile_coords(t, tile_n, row0, rows_valid, grp);
+        k_range(t, kb0, nkb);
         const int col0 = tile_n * BM;
-        for (int kb = 0; kb < nkb; ++kb, ++it) {
-          const int s = it % C::STAGES;
-          if (it >= C::STAGES && !mbar_wait(&empty[s], ((it / C::STAGES) - 1) & 1, a.status)) {
+        for (int kb = 0; kb < nkb; ++kb) {
+          if (lap > 0 && !mbar_wait(&empty[s], (lap - 1) & 1, a.status)) {
             ok = false;
             break;
           }
-          uint8_t* st = smem + s * C::STAGE_BYTES;
-          mbar_expect_tx(&full[s], C::STAGE_BYTES);
-          const int k = kb * BK;
-          if constexpr (GROUPED) {
-            tma_load_3d_hint(st, &tmW, &full[s], col0, k, grp, pol_x);  // an expert's weights serve several token tiles: keep them in L2
-            tma_load_3d_hint(st + A_BYTES / 2, &tmW, &full[s], col0 + 64, k, grp, pol_x);
+          uint8_t* st = smem + s * stage_bytes;
+          const int k = (kb0 + kb) * BK;
+          if (early > 0) {
+            --early;
           } else {
-            tma_load_2d_hint(st, &tmW, &full[s], col0, k, pol_w);
-            tma_load_2d_hint(st + A_BYTES / 2, &tmW, &full[s], col0 + 64, k, pol_w);
+            mbar_expect_tx(&full[s], stage_bytes);
+            if constexpr (GROUPED) {
+              tma_load_3d_hint(st, &tmW, &full[s], col0, k, grp, pol_x);  // an expert's weights serve several token tiles: keep them in L2
+              tma_load_3d_hint(st + A_BYTES / 2, &tmW, &full[s], col0 + 64, k, grp, pol_x);
+            } else {
+              tma_load_2d_hint(st, &tmW, &full[s], col0, k, pol_w);
+              tma_load_2d_hint(st + A_BYTES / 2, &tmW, &full[s], col0 + 64, k, pol_w);
+            }
           }
           tma_load_2d_hint(st + A_BYTES, &tmX, &full[s], k, row0, pol_x);
+          if (++s == STAGES) s = 0, ++lap;
         }
       }
     }
@@ -605,22 +644,23 @@ __global__ void __launch_bounds__(192) linear_tc_persist_kernel(const __grid_con
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | ((uint32_t)(TN >> 3) << 17) |
                              ((uint32_t)(BM >> 4) << 24);
       const uint32_t smem_base = smem_u32(smem);
-      int it = 0, j = 0;
+      int s = 0, lap = 0, j = 0;
       bool ok = true;
       for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x, ++j) {
+        int kb0, nkb;
+        k_range(t, kb0, nkb);
         const int buf = j & 1;
         if (j >= 2) {  // the epilogue must have drained this accumulator (tile j - 2)
           ok = mbar_wait(&tmem_empty[buf], ((j >> 1) - 1) & 1, a.status);
           if (!ok) break;
           tc::fence_after();
         }
-        const uint32_t d_tmem = tmem_base + (uint32_t)(buf * TN);
-        for (int kb = 0; kb < nkb; ++kb, ++it) {
-          const int s = it % C::STAGES;
-          ok = mbar_wait(&full[s], (it / C::STAGES) & 1, a.status);
+        const uint32_t d_tmem = tmem_base + (uint32_t)(buf * C::TN);
+        for (int kb = 0; kb < nkb; ++kb) {
+          ok = mbar_wait(&full[s], lap & 1, a.status);
           if (!ok) break;
           tc::fence_after();
-          const uint32_t sa = smem_base + s * C::STAGE_BYTES;
+          const uint32_t sa = smem_base + s * stage_bytes;
           const uint32_t sb = sa + A_BYTES;
 #pragma unroll
           for (int kk = 0; kk < BK / 16; ++kk) {
@@ -629,86 +669,37 @@ __global__ void __launch_bounds__(192) linear_tc_persist_kernel(const __grid_con
             tc::umma_bf16_ss(d_tmem, da, db, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
           }
           tc::commit(&empty[s]);
+          if (++s == STAGES) s = 0, ++lap;
         }
         if (ok) tc::commit(&tmem_full[buf]);
       }
     }
   } else {
-    // ---------------- epilogue warps 2..5; TMEM lanes 32*(warp%4) .. +31
-    const int q = warp & 3;
-    const int et = threadIdx.x - 64;
-    const bool swiglu = a.epi == EPI_SWIGLU_BF16;
-    const bool out_f32 = a.epi == EPI_PARTIAL_F32 || a.epi == EPI_BIAS_F32;
-    const int tile_cols = swiglu ? 64 : 128;
-    const int row_bytes = tile_cols * (out_f32 ? 4 : 2);
-    const int chunks_per_row = row_bytes / 16;
-    const int elems_per_chunk = out_f32 ? 4 : 8;
-    const size_t esz = out_f32 ? 4 : 2;
-    const int64_t out_cols = swiglu ? a.N / 2 : a.N;
+    // ---------------- epilogue warps 2..9; TMEM lanes 32*(warp%4) .. +31
+    const int q = warp & 3, half = (warp - 2) >> 2;
     pdl_wait();  // the output buffer may still be read by the previous kernel
     int j = 0;
     bool ok = true;
     for (int t = blockIdx.x; t < total_tiles; t += gridDim.x, ++j) {
-      int tile_n, row0, rows_valid, grp;
+      int tile_n, row0, rows_valid, grp, kb0, nkb;
       tile_coords(t, tile_n, row0, rows_valid, grp);
+      k_range(t, kb0, nkb);
       const int col0 = tile_n * BM;
       const int buf = j & 1;
       if (ok) ok = mbar_wait(&tmem_full[buf], (j >> 1) & 1, a.status);
       tc::fence_after();
-      const int64_t feat = (int64_t)col0 + q * 32 + lane;
-      const bool feat_ok = feat < a.N;
       // grouped launches keep one bias row per group: [groups][N]
-      const float bias_v = (a.bias && feat_ok && a.epi != EPI_PARTIAL_F32) ? a.bias[(int64_t)grp * a.N + feat] : 0.f;
-      const int64_t out_col0 = swiglu ? col0 / 2 : col0;
-#pragma unroll 1
-      for (int c0 = 0; c0 < TN; c0 += 32) {
-        if (c0 >= rows_valid) break;  // uniform over the four warps
-        uint8_t* stg = stg_base + ((c0 >> 5) & 1) * C::STG_BYTES;
-        if (ok) {
-          uint32_t r[32];
-          tc::ld32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * TN + c0), r);
-          if (swiglu || out_f32) {
-            // f32 [token][feature]; SwiGLU is applied on the way out, by all 128 threads
-#pragma unroll
-            for (int jj = 0; jj < 32; ++jj)
-              reinterpret_cast<float*>(stg + jj * C::STG_LD)[q * 32 + lane] = __uint_as_float(r[jj]) + bias_v;
-          } else {
-#pragma unroll
-            for (int jj = 0; jj < 32; ++jj)
-              reinterpret_cast<bf16*>(stg + jj * C::STG_LD)[q * 32 + lane] = __float2bfloat16_rn(act_f(__uint_as_float(r[jj]) + bias_v, a.epi));
-          }
-        }
-        asm volatile("bar.sync 1, 128;" ::: "memory");  // the four epilogue warps only
-        if (ok) {
-          const int rows_here = min(32, rows_valid - c0);
-          const int total = rows_here * chunks_per_row;
-          uint8_t* obase = reinterpret_cast<uint8_t*>(a.out);
-          for (int i = et; i < total; i += 128) {
-            const int row = i / chunks_per_row, ch = i % chunks_per_row;
-            const int64_t col = out_col0 + (int64_t)ch * elems_per_chunk;
-            if (col >= out_cols) continue;
-            uint4 v;
-            if (swiglu) {
-              // features ch*16 .. +7 are gates, +8 .. +15 their up partners (the engine's interleave)
-              const float4* gp = reinterpret_cast<const float4*>(stg + row * C::STG_LD + ch * 64);
-              const float4 g0 = gp[0], g1 = gp[1], u0 = gp[2], u1 = gp[3];
-              v.x = pack_bf16(silu_f(g0.x) * u0.x, silu_f(g0.y) * u0.y);
-              v.y = pack_bf16(silu_f(g0.z) * u0.z, silu_f(g0.w) * u0.w);
-              v.z = pack_bf16(silu_f(g1.x) * u1.x, silu_f(g1.y) * u1.y);
-              v.w = pack_bf16(silu_f(g1.z) * u1.z, silu_f(g1.w) * u1.w);
-            } else {
-              v = *reinterpret_cast<const uint4*>(stg + row * C::STG_LD + ch * 16);
-            }
-            *reinterpret_cast<uint4*>(obase + ((size_t)(row0 + c0 + row) * a.ldo + col) * esz) = v;
-          }
-        }
-      }
+      void* const out = reinterpret_cast<uint8_t*>(a.out) + (GROUPED || a.epi != EPI_PARTIAL_F32 ? 0 : (size_t)(t / plane) * a.split_stride * 4);
+      if (ok)
+        store_tile(a, tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * C::TN), out, (int64_t)col0 + q * 32, lane, half,
+                   a.bias ? a.bias + (int64_t)grp * a.N : nullptr, row0, rows_valid, nkb > 0);
       // every epilogue warp has read its part of the accumulator: hand the buffer back
       tc::fence_before();
-      asm volatile("bar.sync 1, 128;" ::: "memory");
-      if (et == 0) mbar_arrive(&tmem_empty[buf]);
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      if (warp == 2 && lane == 0) mbar_arrive(&tmem_empty[buf]);
     }
   }
+  __syncwarp();  // the lanes of a role come back together: what follows is warp-collective
   tc::fence_before();
   __syncthreads();
   if (warp == 1) {
@@ -734,9 +725,7 @@ struct PairCfg {
   static constexpr int STAGES = 6;
   static constexpr int B_BYTES = (TN / 2) * 128;          // this CTA's 128 tokens x 64 k
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;   // 32 KB
-  static constexpr int STG_LD = 528;
-  static constexpr int STG_BYTES = 32 * STG_LD;
-  static constexpr int SMEM = STAGES * STAGE_BYTES + 2 * STG_BYTES + 1024 + 256;
+  static constexpr int SMEM = 227 * 1024;                 // all of it: no CTA of another launch beside a pair's
   static constexpr int TMEM_COLS = 512;
 };
 
@@ -767,15 +756,14 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster_addr) : "memory");
 }
 
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192) linear_tc_pair_kernel(const __grid_constant__ CUtensorMap tmW,
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS) linear_tc_pair_kernel(const __grid_constant__ CUtensorMap tmW,
                                                                                         const __grid_constant__ CUtensorMap tmX,
                                                                                         TcArgs a, int tiles_n, int tiles_m) {
   using C = PairCfg;
   constexpr int TN = C::TN;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* stg_base = smem + C::STAGES * C::STAGE_BYTES;
-  uint64_t* full = reinterpret_cast<uint64_t*>(stg_base + 2 * C::STG_BYTES);
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + C::STAGES * C::STAGE_BYTES);
   uint64_t* empty = full + C::STAGES;
   uint64_t* tmem_full = empty + C::STAGES;   // [2]
   uint64_t* tmem_empty = tmem_full + 2;      // [2]
@@ -885,17 +873,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192) linear_tc_pair_
       }
     }
   } else {
-    // ---------------- epilogue warps 2..5 of each CTA; TMEM lanes 32*(warp%4) .. +31 = this CTA's 128 features
-    const int q = warp & 3;
-    const int et = threadIdx.x - 64;
-    const bool swiglu = a.epi == EPI_SWIGLU_BF16;
-    const bool out_f32 = a.epi == EPI_PARTIAL_F32 || a.epi == EPI_BIAS_F32;
-    const int tile_cols = swiglu ? 64 : 128;
-    const int row_bytes = tile_cols * (out_f32 ? 4 : 2);
-    const int chunks_per_row = row_bytes / 16;
-    const int elems_per_chunk = out_f32 ? 4 : 8;
-    const size_t esz = out_f32 ? 4 : 2;
-    const int64_t out_cols = swiglu ? a.N / 2 : a.N;
+    // ---------------- epilogue warps 2..9 of each CTA; TMEM lanes 32*(warp%4) .. +31 = this CTA's 128 features
+    const int q = warp & 3, half = (warp - 2) >> 2;
     const uint32_t leader_tmem_empty0 = dsmem_addr(smem_u32(&tmem_empty[0]), 0);
     pdl_wait();  // the output buffer may still be read by the previous kernel
     int j = 0;
@@ -908,57 +887,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192) linear_tc_pair_
       const int buf = j & 1;
       if (ok) ok = mbar_wait(&tmem_full[buf], (j >> 1) & 1, a.status);
       tc::fence_after();
-      const int64_t feat = (int64_t)col0 + q * 32 + lane;
-      const bool feat_ok = feat < a.N;
-      const float bias_v = (a.bias && feat_ok && a.epi != EPI_PARTIAL_F32) ? a.bias[feat] : 0.f;
-      const int64_t out_col0 = swiglu ? col0 / 2 : col0;
-#pragma unroll 1
-      for (int c0 = 0; c0 < TN; c0 += 32) {
-        if (c0 >= rows_valid) break;  // uniform over the four warps
-        uint8_t* stg = stg_base + ((c0 >> 5) & 1) * C::STG_BYTES;
-        if (ok) {
-          uint32_t r[32];
-          tc::ld32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * TN + c0), r);
-          if (swiglu || out_f32) {
-#pragma unroll
-            for (int jj = 0; jj < 32; ++jj)
-              reinterpret_cast<float*>(stg + jj * C::STG_LD)[q * 32 + lane] = __uint_as_float(r[jj]) + bias_v;
-          } else {
-#pragma unroll
-            for (int jj = 0; jj < 32; ++jj)
-              reinterpret_cast<bf16*>(stg + jj * C::STG_LD)[q * 32 + lane] = __float2bfloat16_rn(act_f(__uint_as_float(r[jj]) + bias_v, a.epi));
-          }
-        }
-        asm volatile("bar.sync 1, 128;" ::: "memory");  // the four epilogue warps only
-        if (ok) {
-          const int rows_here = min(32, rows_valid - c0);
-          const int total = rows_here * chunks_per_row;
-          uint8_t* obase = reinterpret_cast<uint8_t*>(a.out);
-          for (int i = et; i < total; i += 128) {
-            const int row = i / chunks_per_row, ch = i % chunks_per_row;
-            const int64_t col = out_col0 + (int64_t)ch * elems_per_chunk;
-            if (col >= out_cols) continue;
-            uint4 v;
-            if (swiglu) {
-              const float4* gp = reinterpret_cast<const float4*>(stg + row * C::STG_LD + ch * 64);
-              const float4 g0 = gp[0], g1 = gp[1], u0 = gp[2], u1 = gp[3];
-              v.x = pack_bf16(silu_f(g0.x) * u0.x, silu_f(g0.y) * u0.y);
-              v.y = pack_bf16(silu_f(g0.z) * u0.z, silu_f(g0.w) * u0.w);
-              v.z = pack_bf16(silu_f(g1.x) * u1.x, silu_f(g1.y) * u1.y);
-              v.w = pack_bf16(silu_f(g1.z) * u1.z, silu_f(g1.w) * u1.w);
-            } else {
-              v = *reinterpret_cast<const uint4*>(stg + row * C::STG_LD + ch * 16);
-            }
-            *reinterpret_cast<uint4*>(obase + ((size_t)(row0 + c0 + row) * a.ldo + col) * esz) = v;
-          }
-        }
-      }
+      if (ok)
+        store_tile(a, tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * TN), a.out, (int64_t)col0 + q * 32, lane, half,
+                   a.bias, row0, rows_valid, true);
       // every epilogue warp of this CTA has read its part of the accumulator: tell the leader
       tc::fence_before();
-      asm volatile("bar.sync 1, 128;" ::: "memory");
-      if (et == 0) mbar_arrive_cluster(leader_tmem_empty0 + (uint32_t)buf * 8u);
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      if (warp == 2 && lane == 0) mbar_arrive_cluster(leader_tmem_empty0 + (uint32_t)buf * 8u);
     }
   }
+  __syncwarp();
   tc::fence_before();
   __syncthreads();
   cluster_sync_all();  // nobody leaves (or frees tensor memory) while the peer may still use this CTA's memory or barriers
@@ -976,7 +914,7 @@ int launch_tn(Ctx* c, const LinearBf16Plan& plan, const CUtensorMap& tmX, const 
     RB_CUDA(cudaFuncSetAttribute(linear_tc_kernel<TN, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
     attr_set = true;
   }
-  RB_CUDA(launch_k(linear_tc_kernel<TN, 0>, grid, dim3(192), (size_t)C::SMEM, c->stream, c->use_pdl, plan.tmW, tmX, a));
+  RB_CUDA(launch_k(linear_tc_kernel<TN, 0>, grid, dim3(TC_THREADS), (size_t)C::SMEM, c->stream, c->use_pdl, plan.tmW, tmX, a));
   ++g_launch_total;
   return REWB200_OK;
 }
@@ -1021,7 +959,7 @@ int linear_tc_cluster_launch(Ctx* c, const LinearBf16Plan& plan, const bf16* x, 
     attr_set = true;
   }
   dim3 grid((unsigned)((plan.N + BM - 1) / BM), 1u, (unsigned)ksplit);
-  RB_CUDA(launch_k_cluster(linear_tc_kernel<32, 1>, grid, dim3(192), (size_t)C::SMEM, c->stream, c->use_pdl,
+  RB_CUDA(launch_k_cluster(linear_tc_kernel<32, 1>, grid, dim3(TC_THREADS), (size_t)C::SMEM, c->stream, c->use_pdl,
                            dim3(1, 1, (unsigned)ksplit), plan.tmW, tmX, a));
   ++g_launch_total;
   return REWB200_OK;
@@ -1054,16 +992,17 @@ int linear_tc_grouped_launch(Ctx* c, const LinearBf16Plan& plan, const bf16* x, 
   a.status = c->d_status;
   a.row_offsets = row_offsets;
   a.groups = plan.groups;
+  a.tn = PersistCfg::TN;
   static bool attr_set = false;
   if (!attr_set) {
-    RB_CUDA(cudaFuncSetAttribute(linear_tc_persist_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PersistCfg::SMEM));
+    RB_CUDA(cudaFuncSetAttribute(linear_tc_persist_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     attr_set = true;
   }
   const int tiles_n = (int)((plan.N + BM - 1) / BM);
   // at most ceil(M / TN) + groups token tiles exist; one CTA per SM walks them
   const int64_t max_tiles = (int64_t)tiles_n * ((M + PersistCfg::TN - 1) / PersistCfg::TN + plan.groups);
   const int ctas = (int)std::min<int64_t>(std::min<int64_t>(max_tiles, c->sm_count), kMaxPersistCtas);
-  RB_CUDA(launch_k(linear_tc_persist_kernel<true>, dim3((unsigned)ctas), dim3(192), (size_t)PersistCfg::SMEM, c->stream, c->use_pdl,
+  RB_CUDA(launch_k(linear_tc_persist_kernel<true>, dim3((unsigned)ctas), dim3(TC_THREADS), (size_t)PersistCfg::smem(a.tn), c->stream, c->use_pdl,
                    plan.tmW, tmX, a, tiles_n, 0));
   ++g_launch_total;
   return REWB200_OK;
@@ -1086,9 +1025,8 @@ int linear_tc_launch(Ctx* c, const LinearBf16Plan& plan, const bf16* x, int64_t 
   RB_REQUIRE(ksplit >= 1 && (ksplit == 1 || epi == EPI_PARTIAL_F32), "split-K needs the partial epilogue");
   RB_REQUIRE(epi != EPI_SWIGLU_BF16 || plan.N % 16 == 0, "SwiGLU epilogue needs interleaved width % 16 == 0");
   if (M == 0) return REWB200_OK;
-  const int TN = M <= 32 ? 32 : (M <= 64 ? 64 : (M <= 128 ? 128 : 256));
-  CUtensorMap tmX;
-  RB_TRY(make_tmap_2d_bf16(&tmX, x, (uint64_t)plan.K, (uint64_t)M, (uint64_t)ldx * 2, 64, TN));
+  const int64_t token_tiles = M <= 64 ? 1 : (M + 255) / 256;
+  const int TN = M <= 32 ? 32 : M <= 64 ? 64 : (int)(((M + token_tiles - 1) / token_tiles + 15) / 16 * 16);
   TcArgs a;
   memset(&a, 0, sizeof(a));
   a.M = M;
@@ -1102,9 +1040,13 @@ int linear_tc_launch(Ctx* c, const LinearBf16Plan& plan, const bf16* x, int64_t 
   a.split_stride = M * ldo;
   a.bias = bias;
   a.status = c->d_status;
+  a.ksplit = ksplit;
+  a.tn = TN;
   dim3 grid((unsigned)((plan.N + BM - 1) / BM), (unsigned)((M + TN - 1) / TN), (unsigned)ksplit);
-  if (TN == 256 && ksplit == 1 && c->prefill_persistent && c->prefill_pair && plan.N % 256 == 0 && c->sm_count % 2 == 0 &&
-      (int64_t)grid.x * grid.y >= 2 * (int64_t)c->sm_count) {
+  // Pairs of CTAs where a launch runs long enough for the power cap to set the pace (six layers of the 8B shape, 16 384 tokens:
+  // 42.6 against 45.0 ms); below that one CTA a tile is ahead (4096 x 28672: 4096 tokens 638 against 674 us, 512 97 against 103).
+  if (M >= 8192 && ksplit == 1 && c->prefill_persistent && c->prefill_pair && plan.N % 256 == 0 && c->sm_count % 2 == 0 &&
+      (int64_t)grid.x * token_tiles >= 2 * (int64_t)c->sm_count) {
     // two-CTA tiles: 256 features x 256 tokens per pair of SMs
     CUtensorMap tmXh;
     RB_TRY(make_tmap_2d_bf16(&tmXh, x, (uint64_t)plan.K, (uint64_t)M, (uint64_t)ldx * 2, 64, PairCfg::TN / 2));
@@ -1113,31 +1055,43 @@ int linear_tc_launch(Ctx* c, const LinearBf16Plan& plan, const bf16* x, int64_t 
       RB_CUDA(cudaFuncSetAttribute(linear_tc_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg::SMEM));
       pair_attr = true;
     }
-    const int tiles_n = (int)(plan.N / 256), tiles_m = (int)grid.y;
+    const int tiles_n = (int)(plan.N / 256), tiles_m = (int)token_tiles;
     const int ctas = (int)std::min<int64_t>(2 * (int64_t)tiles_n * tiles_m, c->sm_count);
-    RB_CUDA(launch_k(linear_tc_pair_kernel, dim3((unsigned)(ctas & ~1)), dim3(192), (size_t)PairCfg::SMEM, c->stream, c->use_pdl,
+    RB_CUDA(launch_k(linear_tc_pair_kernel, dim3((unsigned)(ctas & ~1)), dim3(TC_THREADS), (size_t)PairCfg::SMEM, c->stream, c->use_pdl,
                      plan.tmW, tmXh, a, tiles_n, tiles_m));
     ++g_launch_total;
     return REWB200_OK;
   }
-  if (TN == 256 && ksplit == 1 && c->prefill_persistent && (int64_t)grid.x * grid.y >= 2 * (int64_t)c->sm_count) {
+  CUtensorMap tmX;
+  RB_TRY(make_tmap_2d_bf16(&tmX, x, (uint64_t)plan.K, (uint64_t)M, (uint64_t)ldx * 2, 64, TN));
+  if (M <= 32) return launch_tn<32>(c, plan, tmX, a, grid);
+  if (M <= 64) return launch_tn<64>(c, plan, tmX, a, grid);
+  // More tiles of up to 160 tokens than SMs: two CTAs an SM, since those of a second wave start as the first ones leave
+  // (4096 x 28672: 135 tokens 42 us, 48 in the persistent kernel, 300 tokens 70 and 92).  Otherwise the persistent kernel.
+  const bool two = TN <= 160 && (int64_t)grid.x * grid.y * grid.z > c->sm_count;
+  if (c->prefill_persistent && !two) {
+    a.early_w = plan.early_w;
     static bool attr_set = false;
     if (!attr_set) {
-      RB_CUDA(cudaFuncSetAttribute(linear_tc_persist_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, PersistCfg::SMEM));
+      RB_CUDA(cudaFuncSetAttribute(linear_tc_persist_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
       attr_set = true;
     }
-    const int ctas = (int)std::min<int64_t>((int64_t)grid.x * grid.y, c->sm_count);
-    RB_CUDA(launch_k(linear_tc_persist_kernel<false>, dim3((unsigned)ctas), dim3(192), (size_t)PersistCfg::SMEM, c->stream, c->use_pdl,
-                     plan.tmW, tmX, a, (int)grid.x, (int)grid.y));
+    const int ctas = (int)std::min<int64_t>((int64_t)grid.x * grid.y * grid.z, c->sm_count);
+    RB_CUDA(launch_k(linear_tc_persist_kernel<false>, dim3((unsigned)ctas), dim3(TC_THREADS), (size_t)PersistCfg::smem(a.tn), c->stream, c->use_pdl, plan.tmW,
+                     tmX, a, (int)grid.x, (int)grid.y));
     ++g_launch_total;
     return REWB200_OK;
   }
-  switch (TN) {
-    case 32: return launch_tn<32>(c, plan, tmX, a, grid);
-    case 64: return launch_tn<64>(c, plan, tmX, a, grid);
-    case 128: return launch_tn<128>(c, plan, tmX, a, grid);
-    default: return launch_tn<256>(c, plan, tmX, a, grid);
+  using C = TcCfg<0>;
+  a.stages = std::min((int)C::MAX_STAGES, ((TN <= 160 ? 113 : 227) * 1024 - C::FIXED) / C::stage_bytes(TN));
+  static bool attr_set = false;
+  if (!attr_set) {
+    RB_CUDA(cudaFuncSetAttribute(linear_tc_kernel<0, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    attr_set = true;
   }
+  RB_CUDA(launch_k(linear_tc_kernel<0, 0>, grid, dim3(TC_THREADS), (size_t)(a.stages * C::stage_bytes(TN) + C::FIXED), c->stream, c->use_pdl, plan.tmW, tmX, a));
+  ++g_launch_total;
+  return REWB200_OK;
 }
 
 }  // namespace rewb

@@ -57,6 +57,36 @@ def test_tc_model_matches_oracle_and_mma_path(rb_tc, orc):
         assert rel_l2(logits, logits_mma) <= 1e-2
 
 
+@pytest.mark.parametrize("M", [65, 80, 81, 129, 160, 161, 257, 300, 321, 513])
+@pytest.mark.parametrize("K,N", [(200, 18968), (1032, 264)])
+def test_linear_tiles_of_the_steps_own_size(rb_tc, M, K, N):
+    """Tiles of 16-token steps around their edges: more tiles than SMs (two CTAs an SM up to 160 tokens, persistent above) and
+    fewer (persistent), a last feature tile that is only partly there, K that is no multiple of a block.  bf16 operands are
+    exact in f32, so the only roundings are K + 1 of f32 sums and the bf16 output's half ulp."""
+    from rew_b200 import _lib
+    rng = np.random.default_rng(M + N)
+    x, w = W.bf16_round(rng.normal(size=(M, K))), W.bf16_round(rng.normal(size=(K, N)))
+    b = rng.normal(size=N).astype(np.float32)
+    T = rb_tc.Tensor.from_host
+    lin = rb_tc.Linear(T(w, _lib.BF16), T(b))
+    got = lin.forward(T(x, _lib.BF16)).to_host()
+    want = x.astype(np.float64) @ w + b
+    bound = (K + 1) * 2.0 ** -24 * (np.abs(x).astype(np.float64) @ np.abs(w) + np.abs(b)) + 2.0 ** -8 * np.abs(want)
+    assert np.all(np.abs(got - want) <= bound)
+
+
+@pytest.mark.parametrize("B,S", [(13, 5), (2, 80), (1, 250)])
+def test_split_steps_match_the_oracle(rb_tc, orc, B, S):
+    """Steps of 65 to 256 rows whose Linears are cut along K into the count of slabs that costs least (here 2 to 4 of 18 blocks)."""
+    from rew_b200 import _lib
+    cfg = W.ModelConfig(vocab=256, d_model=1152, n_layers=1, n_heads=9, n_kv_heads=3, head_dim=128, ffn=1536, max_seq=256,
+                        theta=500000.0, dtype=_lib.BF16, mask_kind=1)
+    t = [orc.bf16_round(a) if a.ndim == 2 else a for a in W.init_weights(cfg, seed=6, std=0.03, trivial_affine=False)]
+    prompt = np.random.default_rng(S).integers(0, cfg.vocab, size=(B, S)).astype(np.int32)
+    _, logits = rb_tc.CausalLM(cfg).load(t).session(B, S).forward(prompt, want_logits=True)
+    assert rel_l2(logits, orc.model_forward(cfg, t, prompt, 0, True)[:, -1]) <= 2e-2
+
+
 def test_persistent_prefill_linear_matches_oracle(rb_tc, orc):
     """Enough 256-token tiles (17 x 20 >= 2 per SM) for the persistent kernel with the double-buffered
     accumulator; a ragged last token tile and a last feature tile that is only half there."""
