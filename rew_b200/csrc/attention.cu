@@ -43,6 +43,7 @@ struct AttnDev {
   const int* block_table;
   int max_pages;
   int kvh, nh, group, S, hd;
+  const int2* seq;  // see AttnArgs::seq
   int64_t kv_len_fixed;
   int64_t contiguous_len;
   int causal, mask_kind;
@@ -68,6 +69,18 @@ struct AttnDev {
 
 __device__ __forceinline__ int kv_len_of(const AttnDev& a, int b) {
   return a.kv_len_fixed >= 0 ? (int)a.kv_len_fixed : a.pos0[b] + a.S;
+}
+// Sequences of unequal lengths share a launch sized for the longest: narrows `a` to the CTA's own sequence and says whether it
+// has a query q0.  The table predates the step's first launch, so it is read ahead of the stream dependency.
+template <typename T>
+__device__ __forceinline__ bool take_sequence(AttnDev& a, int b, int q0) {
+  if (a.seq) {
+    const int2 s = a.seq[b];
+    a.S = s.y;
+    a.q = reinterpret_cast<const T*>(a.q) + s.x * a.q_ss;
+    a.out = reinterpret_cast<T*>(a.out) + s.x * a.o_ss;
+  }
+  return q0 < a.S;
 }
 __device__ __forceinline__ bool visible(const AttnDev& a, int i, int j, int ctx) {
   if (!a.causal) return true;
@@ -101,6 +114,7 @@ __global__ void __launch_bounds__(128) attn_f32_kernel(AttnDev a) {
   pdl_launch_dependents();
   pdl_wait();
   const int i = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+  if (!take_sequence<float>(a, b, i)) return;
   const int kv_len = kv_len_of(a, b), ctx = kv_len - a.S;
   const int hd = a.hd, hk = h / a.group;
   float* scores = sm;
@@ -515,6 +529,7 @@ __global__ void __launch_bounds__(128) attn_prefill_kernel(const __grid_constant
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3, l8 = lane & 7, lq = lane >> 3;
 
+  if (!take_sequence<bf16>(a, b, qb * 64)) return;
   if (threadIdx.x == 0) {
     for (int s = 0; s < ATT_STAGES; ++s) mbar_init(&full[s], 1);
     fence_barrier_init();
@@ -861,6 +876,7 @@ __global__ void __launch_bounds__(fa::THREADS, 2) attn_prefill_tc_kernel(const _
   const int head = blockIdx.y, b = blockIdx.z;
   const int kvh_idx = head / a.group;
   const int q0 = qt * BQ;
+  if (!take_sequence<bf16>(a, b, q0)) return;
   if (threadIdx.x == 0) {
     mbar_init(k_full, 1);
     mbar_init(k_empty, 1);
@@ -1012,6 +1028,7 @@ __global__ void __launch_bounds__(fa2::THREADS, 1) attn_prefill_tc2_kernel(const
   const int head = blockIdx.y, b = blockIdx.z;
   const int kvh_idx = head / a.group;
   const int q0 = qt * BQ;
+  if (!take_sequence<bf16>(a, b, q0)) return;
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2; ++i) {
       mbar_init(k_full + i, 1);
@@ -1196,7 +1213,7 @@ int attn_launch(Ctx* c, const AttnArgs& h) {
   a.pos0 = h.pos0;
   a.block_table = h.kv.block_table;
   a.max_pages = h.kv.max_pages;
-  a.kvh = h.kv.kvh; a.nh = h.nh; a.group = h.nh / h.kv.kvh; a.S = h.S; a.hd = h.kv.hd;
+  a.kvh = h.kv.kvh; a.nh = h.nh; a.group = h.nh / h.kv.kvh; a.S = h.S; a.seq = h.seq; a.hd = h.kv.hd;
   a.kv_len_fixed = h.kv_len_fixed;
   a.contiguous_len = h.kv.contiguous_len;
   a.causal = h.causal; a.mask_kind = h.mask_kind;

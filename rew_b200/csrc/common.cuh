@@ -352,6 +352,8 @@ struct QkvPostArgs {
   int act_dtype;
   KvLayout kv;
   int* status;
+  const int* row_seq;     // steps of unequal portions: [rows] sequence of a row, whose first row is seq[sequence].x; nullptr:
+  const int2* seq;        // row / S and row % S
   int early_lookup;       // positions, block tables and RoPE tables predate every kernel that may still be in flight
                           // (a captured decode step): they may be read before the stream dependency resolves
 };
@@ -366,6 +368,7 @@ struct AttnArgs {
   const int* pos0;        // [B] device: context length before these S queries, or nullptr
   int64_t B;
   int S;
+  const int2* seq;        // sequences of unequal lengths: [B] first row of q / out and queries (at most S); q_sb and o_sb are 0
   int nh;
   int causal;             // 0: every key visible
   int mask_kind;          // 0 as written (key j visible to query i iff i <= j), 1 conventional causal

@@ -706,7 +706,7 @@ __global__ void __launch_bounds__(256) qkv_post_vec_kernel(QkvPostArgs a) {
   pdl_launch_dependents();
   pdl_wait();
   const int64_t row = blockIdx.x;
-  const int b = (int)(row / a.S), s = (int)(row % a.S);
+  const int b = a.row_seq ? a.row_seq[row] : (int)(row / a.S), s = a.row_seq ? (int)row - a.seq[b].x : (int)(row % a.S);
   const int pos = a.pos0[b] + s;
   const int hd = a.hd;
   const int nq = a.nh * hd, nkv = a.kvh * hd, ntot = nq + 2 * nkv;
@@ -775,7 +775,7 @@ __global__ void __launch_bounds__(256) qkv_post_kernel(QkvPostArgs a) {
   // as its predecessor has STARTED, so "several launches back" proves nothing): wait first.
   if (!a.early_lookup) pdl_wait();
   const int64_t row = blockIdx.x;
-  const int b = (int)(row / a.S), s = (int)(row % a.S);
+  const int b = a.row_seq ? a.row_seq[row] : (int)(row / a.S), s = a.row_seq ? (int)row - a.seq[b].x : (int)(row % a.S);
   const int pos = a.pos0[b] + s;
   const int hd = a.hd, half = hd / 2;
   const int nq = a.nh * hd, nkv = a.kvh * hd, ntot = nq + 2 * nkv;

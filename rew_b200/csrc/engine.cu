@@ -169,6 +169,18 @@ __global__ void advance_kernel(const int* next, int* ids, int* pos, int* out_ids
   if (threadIdx.x == 0) *step = st + 1;
 }
 
+// The tables of the lanes of a step, one CTA per portion {lane, first position, tokens, -}: ahead of the step the lane is active
+// at its first position with these pages, behind it (pages null) the lane has moved on.
+__global__ void feed_lanes_kernel(const int4* portions, const int* pages, int max_pages, int* pos, int* active, int* block_table) {
+  const int4 p = portions[blockIdx.x];
+  if (threadIdx.x == 0) {
+    pos[p.x] = pages ? p.y : p.y + p.z;
+    active[p.x] = 1;
+  }
+  if (pages)
+    for (int i = threadIdx.x; i < max_pages; i += blockDim.x) block_table[(int64_t)p.x * max_pages + i] = pages[(int64_t)blockIdx.x * max_pages + i];
+}
+
 }  // namespace
 }  // namespace rewb
 
@@ -661,6 +673,11 @@ int fetch_logits(rewb200_session* s, int64_t rows, float* host) {
   return REWB200_OK;
 }
 
+// Portions that share an attention launch: the choice of kernel follows a portion's own length, as if it stood alone
+// (128 tokens and more: tcgen05; fewer: mma.sync; one: split-KV decode), so its numbers do not depend on its neighbours.
+enum PortionKind : int { PORTION_LONG = 0, PORTION_SHORT, PORTION_SINGLE };
+PortionKind portion_kind(int n) { return n >= 128 ? PORTION_LONG : n > 1 ? PORTION_SHORT : PORTION_SINGLE; }
+
 // The decoder blocks of a grouped-query model (llama.nim:106-129, deepseek.nim:198-220) over rows = nb*S tokens: embedding
 // and first norm, then every layer; leaves the final norm's output in s->xn.
 int gqa_blocks(rewb200_session* s, const FwdOpts& o, const NormArgs& na, int64_t rows, bool in_graph) {
@@ -669,8 +686,9 @@ int gqa_blocks(rewb200_session* s, const FwdOpts& o, const NormArgs& na, int64_t
   const rewb200_config& cf = m->cfg;
   const int b0 = o.b0, nb = o.nb < 0 ? s->B : o.nb;
   const int64_t d = cf.d_model;
-  int* const pos = s->d_pos + b0;
-  const int* const block_table = s->block_table + (size_t)b0 * s->max_pages;
+  const bool portions = o.seq != nullptr;   // unequal ones: the tables of the step in place of the session's
+  const int* const pos = portions ? o.seq_pos : s->d_pos + b0;
+  const int* const block_table = portions ? o.seq_pages : s->block_table + (size_t)b0 * s->max_pages;
   const int dt = cf.dtype;
   // embedding gather + first norm
   {
@@ -773,7 +791,9 @@ int gqa_blocks(rewb200_session* s, const FwdOpts& o, const NormArgs& na, int64_t
     qa.cosT = m->cosT;
     qa.sinT = m->sinT;
     qa.pos0 = pos;
-    qa.S = o.S;
+    qa.S = portions ? 1 : o.S;
+    qa.seq = o.seq;
+    qa.row_seq = o.row_seq;
     qa.rope_shift = o.rope_shift;
     qa.nh = m->nh_l;
     qa.kvh = m->kvh_l;
@@ -792,16 +812,16 @@ int gqa_blocks(rewb200_session* s, const FwdOpts& o, const NormArgs& na, int64_t
     qa.kv_capacity = s->max_len;
     qa.status = c->d_status;
     qa.early_lookup = in_graph ? 1 : 0;
-    RB_TRY(run_linear(s, L.qkv, s->xn, d, rows, true, 0, s->part, m->nqkv, &ks, dt == REWB200_BF16 ? &qa : nullptr, &qkv_done));
+    RB_TRY(run_linear(s, L.qkv, s->xn, d, rows, true, 0, s->part, m->nqkv, &ks, dt == REWB200_BF16 && !portions ? &qa : nullptr, &qkv_done));
     if (o.trace) RB_TRY(o.trace->mark(TC_QKV));
     // decode steps: the attention kernel finishes q / k / v of the new token from the slabs itself
     // ... when its grid is at most one wave of two CTAs per SM (measured: with several waves the prologue in front of
     // every CTA costs more than the launch it saves: l8 batch 128 5.69 -> 6.08 ms, the MoE model 7.07 -> 7.28 ms)
-    const bool fuse_into_attn = !qkv_done && o.S == 1 && dt == REWB200_BF16 && c->attn_fuse_qkv && m->nh_l / m->kvh_l <= 16 &&
+    const bool fuse_into_attn = !qkv_done && o.S == 1 && !portions && dt == REWB200_BF16 && c->attn_fuse_qkv && m->nh_l / m->kvh_l <= 16 &&
                                 (c->attn_fuse_qkv_always ||
                                  (int64_t)nb * m->kvh_l * decode_splits(c, nb, m->kvh_l) <= 2 * (int64_t)c->sm_count);
     qa.nsplit = ks;
-    if (!qkv_done && !fuse_into_attn) RB_TRY(qkv_post_launch(c, qa, nb));
+    if (!qkv_done && !fuse_into_attn) RB_TRY(qkv_post_launch(c, qa, portions ? rows : nb));
     if (o.trace) RB_TRY(o.trace->mark(TC_QKV_POST));
 
     AttnArgs aa;
@@ -833,7 +853,33 @@ int gqa_blocks(rewb200_session* s, const FwdOpts& o, const NormArgs& na, int64_t
       aa.tmV = &s->tmV[l];
     }
     if (fuse_into_attn) aa.fuse_qkv = &qa;
-    RB_TRY(attn_launch(c, aa));
+    if (portions) {
+      // one launch per kind of portion: the longest ones first, each kind sized for its longest; single tokens decode.
+      // The rows of all portions share the Linears, so the weights stream once a step and not once a portion: eleven
+      // prompts of about 150 tokens, then six steps of 100 tokens beside eleven single ones, six layers of the 8B
+      // shape: 10.1 ms, 62.4 ms portion by portion.
+      const std::vector<StepEntry>& es = *o.entries;
+      for (size_t e0 = 0, e1; e0 < es.size(); e0 = e1) {
+        const PortionKind kind = portion_kind(es[e0].n);
+        AttnArgs g = aa;
+        g.S = 0;
+        for (e1 = e0; e1 < es.size() && portion_kind(es[e1].n) == kind; ++e1) g.S = std::max(g.S, es[e1].n);
+        g.B = (int64_t)(e1 - e0);
+        g.pos0 = pos + e0;
+        g.kv.block_table = block_table + e0 * s->max_pages;
+        if (kind == PORTION_SINGLE) {
+          g.q = (const char*)s->q + (size_t)es[e0].row0 * m->nq * dtype_size(dt);
+          g.out = (char*)s->attn + (size_t)es[e0].row0 * m->nq * dtype_size(dt);
+          g.q_sb = g.o_sb = m->nq;
+        } else {
+          g.seq = o.seq + e0;
+          g.q_sb = g.o_sb = 0;
+        }
+        RB_TRY(attn_launch(c, g));
+      }
+    } else {
+      RB_TRY(attn_launch(c, aa));
+    }
     if (o.trace) RB_TRY(o.trace->mark(TC_ATTN));
 
     RB_TRY(run_row_parallel(L.o, s->attn, m->nq, &ks));
@@ -955,7 +1001,7 @@ int ensure_head_rows(rewb200_session* s, int64_t rows) {
 std::vector<StepEntry> uniform_entries(const rewb200_session* s, int b0, int nb, int S, int pos0) {
   (void)s;
   std::vector<StepEntry> e;
-  for (int b = 0; b < nb; ++b) e.push_back({b0 + b, b * S, S, pos0});
+  for (int b = 0; b < nb; ++b) e.push_back({b0 + b, b * S, S, pos0, b * S});
   return e;
 }
 
@@ -1692,12 +1738,23 @@ void rewb200_session_free(rewb200_session* s) {
   delete s;
 }
 
+// Takes a lane's blocks back on the host.
+static void lane_drop(rewb200_session* s, int lane) {
+  for (int pg : s->lane_pages[lane]) s->free_blocks.push_back(pg);
+  s->lane_pages[lane].clear();
+  s->lane_active[lane] = 0;
+  s->lane_len[lane] = 0;
+}
+
 int rewb200_session_reset(rewb200_session* s) {
   RB_REQUIRE(s, "rewb200_session_reset: NULL session");
   Ctx* c = s->m->c;
   RB_CUDA(cudaSetDevice(c->device));
-  if (s->paged)
-    for (int b = 0; b < s->B; ++b) RB_TRY(rewb200_lane_release(s, b));
+  if (s->paged) {  // every lane back on the scratch block at once
+    for (int b = 0; b < s->B; ++b) lane_drop(s, b);
+    RB_CUDA(cudaMemsetAsync(s->d_active, 0, s->B * sizeof(int), c->stream));
+    RB_CUDA(cudaMemsetAsync(s->block_table, 0, (size_t)s->B * s->max_pages * sizeof(int), c->stream));
+  }
   RB_CUDA(cudaMemsetAsync(s->d_pos, 0, s->B * sizeof(int), c->stream));
   RB_CUDA(cudaMemsetAsync(s->d_step, 0, sizeof(int), c->stream));
   s->host_pos = 0;
@@ -1893,6 +1950,15 @@ int rewb200_generate(rewb200_session* s, const int32_t* prompt, int S, int n_new
 
 namespace {
 
+// Gives `lane` blocks for `new_len` tokens on the host (the caller has checked that they are free).
+void lane_take(rewb200_session* s, int lane, int new_len) {
+  std::vector<int>& pages = s->lane_pages[lane];
+  while ((int)pages.size() < (new_len + PAGE - 1) / PAGE) {
+    pages.push_back(s->free_blocks.back());
+    s->free_blocks.pop_back();
+  }
+}
+
 // Makes sure `lane` owns blocks for `new_len` tokens and uploads its block-table row when it grew.
 int lane_reserve(rewb200_session* s, int lane, int new_len) {
   Ctx* c = s->m->c;
@@ -1902,10 +1968,7 @@ int lane_reserve(rewb200_session* s, int lane, int new_len) {
   RB_REQUIRE((int)s->free_blocks.size() >= need - (int)pages.size(),
              "PagedKvCache: out of free blocks (lane " + std::to_string(lane) + " needs " +
                  std::to_string(need - (int)pages.size()) + ", " + std::to_string(s->free_blocks.size()) + " free)");
-  while ((int)pages.size() < need) {
-    pages.push_back(s->free_blocks.back());
-    s->free_blocks.pop_back();
-  }
+  lane_take(s, lane, new_len);
   std::vector<int> row((size_t)s->max_pages, 0);
   for (size_t i = 0; i < pages.size(); ++i) row[i] = pages[i];
   RB_CUDA(cudaStreamSynchronize(c->stream));
@@ -2028,7 +2091,7 @@ int rewb200_lanes_feed(rewb200_session* s, int n_entries, const int32_t* lanes, 
     const int pos0 = s->lane_active[l] ? s->lane_len[l] : 0;
     RB_REQUIRE((int64_t)pos0 + counts[e] <= s->max_len, "KvCache.append: total length " + std::to_string((int64_t)pos0 + counts[e]) +
                                                             " of lane " + std::to_string(l) + " exceeds maxLen " + std::to_string(s->max_len));
-    entries.push_back({l, (int)rows, counts[e], pos0});
+    entries.push_back({l, (int)rows, counts[e], pos0, (int)rows});
     rows += counts[e];
     need += std::max(0, (pos0 + counts[e] + PAGE - 1) / PAGE - (int)s->lane_pages[l].size());
   }
@@ -2048,16 +2111,58 @@ int rewb200_lanes_feed(rewb200_session* s, int n_entries, const int32_t* lanes, 
       act[lanes[e]] = 1;
       any_sample = true;
     }
-  RB_CUDA(cudaStreamSynchronize(c->stream));  // the host-side tables below are read by no kernel in flight
+  // A grouped-query step runs its portions in the order of their kinds; a layered one in the caller's.
+  if (!m->layered) {
+    std::stable_sort(entries.begin(), entries.end(), [](const StepEntry& x, const StepEntry& y) { return portion_kind(x.n) < portion_kind(y.n); });
+    int row = 0;
+    for (StepEntry& e : entries) {
+      e.src = e.row0;
+      e.row0 = row;
+      row += e.n;
+    }
+  }
+  // one upload: ids | rows of the lm_head (wanted places, then every lane's last row) | sampled lanes | portions and their pages |
+  // and for grouped-query models the rows and positions of the portions
+  const size_t at_rows = (size_t)rows, at_act = at_rows + n_want + s->B, at_port = (at_act + s->B + 3) / 4 * 4,
+               at_seq = at_port + 4 * (size_t)n_entries, at_pos = at_seq + 2 * (size_t)n_entries, at_pages = at_pos + n_entries,
+               at_row_seq = at_pages + (size_t)n_entries * s->max_pages, total = at_row_seq + (m->layered ? 0 : (size_t)rows);
+  std::vector<int> up(total, 0);
+  for (size_t k = 0; k < entries.size(); ++k) {
+    const StepEntry& e = entries[k];
+    lane_take(s, e.lane, e.pos0 + e.n);
+    memcpy(up.data() + e.row0, ids + e.src, (size_t)e.n * sizeof(int));
+    for (int i = 0; i < n_want; ++i)
+      if (want[i] >= e.src && want[i] < e.src + e.n) up[at_rows + i] = e.row0 + want[i] - e.src;
+    up[at_rows + n_want + e.lane] = e.row0 + e.n - 1;
+    const int port[4] = {e.lane, e.pos0, e.n, 0}, seq[2] = {e.row0, e.n};
+    memcpy(up.data() + at_port + 4 * k, port, sizeof(port));
+    memcpy(up.data() + at_seq + 2 * k, seq, sizeof(seq));
+    up[at_pos + k] = e.pos0;
+    std::copy(s->lane_pages[e.lane].begin(), s->lane_pages[e.lane].end(), up.begin() + at_pages + k * s->max_pages);
+    if (!m->layered) std::fill_n(up.begin() + at_row_seq + e.row0, e.n, (int)k);
+  }
+  for (int b = 0; b < s->B; ++b) up[at_act + b] = act[b];
+  if (up.size() > s->feed_cap) {
+    RB_CUDA(cudaStreamSynchronize(c->stream));
+    if (s->feed_dev) RB_CUDA(cudaFree(s->feed_dev));
+    s->feed_dev = nullptr;
+    s->feed_cap = 0;
+    RB_CUDA(cudaMalloc((void**)&s->feed_dev, up.size() * sizeof(int)));
+    s->feed_cap = up.size();
+  }
+  RB_CUDA(cudaMemcpyAsync(s->feed_dev, up.data(), up.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream));
+  const int4* d_port = reinterpret_cast<const int4*>(s->feed_dev + at_port);
+  feed_lanes_kernel<<<(unsigned)n_entries, 64, 0, c->stream>>>(d_port, s->feed_dev + at_pages, s->max_pages, s->d_pos, s->d_active, s->block_table);
+  RB_CUDA(cudaGetLastError());
+  ++g_launch_total;
   for (const StepEntry& e : entries) {
-    RB_TRY(lane_reserve(s, e.lane, e.pos0 + e.n));
     if (!s->lane_active[e.lane]) {
-      const int one = 1;
-      RB_CUDA(cudaMemcpyAsync(s->d_active + e.lane, &one, sizeof(int), cudaMemcpyHostToDevice, c->stream));
       s->lane_active[e.lane] = 1;
       s->lane_len[e.lane] = 0;
       if (s->samp_on) {
-        const uint64_t seed = seeds ? seeds[&e - &entries[0]] : 0;
+        uint64_t seed = 0;
+        for (int k = 0; k < n_entries && seeds; ++k)
+          if (lanes[k] == e.lane) seed = seeds[k];
         s->samp_seeds[e.lane] = seed;
         const uint32_t k[2] = {(uint32_t)(seed & 0xFFFFFFFFull), (uint32_t)(seed >> 32)};
         const int zero = 0;
@@ -2067,78 +2172,40 @@ int rewb200_lanes_feed(rewb200_session* s, int n_entries, const int32_t* lanes, 
     }
     if (s->samp_on) {  // tokens seen so far = everything fed to the model
       const int n = e.pos0 + e.n;
-      RB_CUDA(cudaMemcpyAsync(s->samp_hist + (size_t)e.lane * s->max_len + e.pos0, ids + e.row0, (size_t)e.n * sizeof(int), cudaMemcpyHostToDevice, c->stream));
+      RB_CUDA(cudaMemcpyAsync(s->samp_hist + (size_t)e.lane * s->max_len + e.pos0, ids + e.src, (size_t)e.n * sizeof(int), cudaMemcpyHostToDevice, c->stream));
       RB_CUDA(cudaMemcpyAsync(s->samp_hist_len + e.lane, &n, sizeof(int), cudaMemcpyHostToDevice, c->stream));
     }
-    RB_CUDA(cudaMemcpyAsync(s->d_pos + e.lane, &e.pos0, sizeof(int), cudaMemcpyHostToDevice, c->stream));
   }
-  // one upload: ids | rows of the lm_head (wanted places, then every lane's last row) | sampled lanes
-  std::vector<int> up((size_t)rows + n_want + s->B + s->B, 0);
-  memcpy(up.data(), ids, (size_t)rows * sizeof(int));
-  for (int i = 0; i < n_want; ++i) up[(size_t)rows + i] = want[i];
-  for (const StepEntry& e : entries) up[(size_t)rows + n_want + e.lane] = e.row0 + e.n - 1;
-  for (int b = 0; b < s->B; ++b) up[(size_t)rows + n_want + s->B + b] = act[b];
-  if (up.size() > s->feed_cap) {
-    if (s->feed_dev) RB_CUDA(cudaFree(s->feed_dev));
-    s->feed_dev = nullptr;
-    s->feed_cap = 0;
-    RB_CUDA(cudaMalloc((void**)&s->feed_dev, up.size() * sizeof(int)));
-    s->feed_cap = up.size();
-  }
-  RB_CUDA(cudaMemcpyAsync(s->feed_dev, up.data(), up.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream));
-  const int* d_rows = s->feed_dev + rows;
-  const int* d_act = s->feed_dev + rows + n_want + s->B;
   RB_CUDA(cudaEventRecord(s->ev0, c->stream));
+  FwdOpts o;
+  o.entries = &entries;
+  o.ids_src = s->feed_dev;
+  o.record_out = false;
+  o.out_rows = s->feed_dev + at_rows;
+  o.n_want = n_want;
+  o.sample = any_sample;
+  o.sample_active = s->feed_dev + at_act;
+  o.advance = 0;
   if (m->layered) {
-    FwdOpts o;
-    o.entries = &entries;
-    o.ids_src = s->feed_dev;
-    o.record_out = false;
-    o.out_rows = d_rows;
-    o.n_want = n_want;
-    o.sample = any_sample;
-    o.sample_active = d_act;
-    o.advance = 0;
     RB_TRY(layered_prepare(s, o, rows));
-    RB_TRY(enqueue_forward(s, o));
-    if (n_want > 0)
-      RB_CUDA(cudaMemcpyAsync(logits_out, s->logits, (size_t)n_want * m->cfg.vocab * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
   } else {
-    int w0 = 0;
-    for (const StepEntry& e : entries) {
-      // this portion's wanted places, relative to its first row, then its last row
-      int w1 = w0;
-      std::vector<int> list;
-      while (w1 < n_want && want[w1] < e.row0 + e.n) list.push_back(want[w1++] - e.row0);
-      list.push_back(e.n - 1);
-      RB_CUDA(cudaMemcpyAsync(s->feed_dev + rows, list.data(), list.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream));
-      FwdOpts o;
-      o.S = e.n;
-      o.b0 = e.lane;
-      o.nb = 1;
-      o.ids_src = s->feed_dev + e.row0;
-      o.record_out = false;
-      o.out_rows = d_rows;
-      o.n_want = w1 - w0;
-      o.sample = act[e.lane] != 0;
-      o.advance = 0;
-      RB_TRY(enqueue_forward(s, o));
-      if (w1 > w0)
-        RB_CUDA(cudaMemcpyAsync(logits_out + (size_t)w0 * m->cfg.vocab, s->logits, (size_t)(w1 - w0) * m->cfg.vocab * sizeof(float),
-                                cudaMemcpyDeviceToHost, c->stream));
-      RB_CUDA(cudaStreamSynchronize(c->stream));  // `list` and the shared row list are reused by the next portion
-      w0 = w1;
-    }
+    o.seq = reinterpret_cast<const int2*>(s->feed_dev + at_seq);
+    o.seq_pos = s->feed_dev + at_pos;
+    o.seq_pages = s->feed_dev + at_pages;
+    o.row_seq = s->feed_dev + at_row_seq;
   }
+  RB_TRY(enqueue_forward(s, o));
+  if (n_want > 0)
+    RB_CUDA(cudaMemcpyAsync(logits_out, s->logits, (size_t)n_want * m->cfg.vocab * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
+  feed_lanes_kernel<<<(unsigned)n_entries, 64, 0, c->stream>>>(d_port, nullptr, s->max_pages, s->d_pos, s->d_active, s->block_table);
+  RB_CUDA(cudaGetLastError());
+  ++g_launch_total;
   RB_CUDA(cudaEventRecord(s->ev1, c->stream));
   std::vector<int> next(s->B, -1);
   if (any_sample) RB_CUDA(cudaMemcpyAsync(next.data(), s->d_next, s->B * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   RB_CUDA(cudaStreamSynchronize(c->stream));
   RB_CUDA(cudaEventElapsedTime(&s->prefill_ms, s->ev0, s->ev1));
-  for (const StepEntry& e : entries) {
-    s->lane_len[e.lane] = e.pos0 + e.n;
-    RB_CUDA(cudaMemcpyAsync(s->d_pos + e.lane, &s->lane_len[e.lane], sizeof(int), cudaMemcpyHostToDevice, c->stream));
-  }
+  for (const StepEntry& e : entries) s->lane_len[e.lane] = e.pos0 + e.n;
   if (next_ids)
     for (int e = 0; e < n_entries; ++e) next_ids[e] = act[lanes[e]] ? next[lanes[e]] : -1;
   return ctx_check_status(c);
@@ -2149,16 +2216,10 @@ int rewb200_lane_release(rewb200_session* s, int lane) {
   if (!s->lane_active[lane] && s->lane_pages[lane].empty()) return REWB200_OK;  // idempotent
   Ctx* c = s->m->c;
   RB_CUDA(cudaSetDevice(c->device));
-  RB_CUDA(cudaStreamSynchronize(c->stream));
-  const int zero = 0;
-  RB_CUDA(cudaMemcpyAsync(s->d_active + lane, &zero, sizeof(int), cudaMemcpyHostToDevice, c->stream));
-  RB_CUDA(cudaMemcpyAsync(s->d_pos + lane, &zero, sizeof(int), cudaMemcpyHostToDevice, c->stream));
-  std::vector<int> row((size_t)s->max_pages, 0);  // back on the scratch block
-  RB_CUDA(cudaMemcpyAsync(s->block_table + (size_t)lane * s->max_pages, row.data(), row.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream));
-  for (int pg : s->lane_pages[lane]) s->free_blocks.push_back(pg);
-  s->lane_pages[lane].clear();
-  s->lane_active[lane] = 0;
-  s->lane_len[lane] = 0;
+  RB_CUDA(cudaMemsetAsync(s->d_active + lane, 0, sizeof(int), c->stream));
+  RB_CUDA(cudaMemsetAsync(s->d_pos + lane, 0, sizeof(int), c->stream));
+  RB_CUDA(cudaMemsetAsync(s->block_table + (size_t)lane * s->max_pages, 0, (size_t)s->max_pages * sizeof(int), c->stream));  // back on the scratch block
+  lane_drop(s, lane);
   return REWB200_OK;
 }
 

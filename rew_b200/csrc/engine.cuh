@@ -336,6 +336,7 @@ struct Trace {
 // A portion of a step: rows row0 .. row0 + n - 1 are the tokens at positions pos0 .. of `lane`.
 struct StepEntry {
   int lane, row0, n, pos0;
+  int src;               // place of its first token among the ids the caller gave
 };
 
 struct FwdOpts {
@@ -353,6 +354,10 @@ struct FwdOpts {
   bool record_out = true;    // append the new ids to the session's [step][B] output buffer
   // Steps of unequal portions (rewb200_lanes_feed) and layered steps of more than one token: the portions, in row order
   const std::vector<StepEntry>* entries = nullptr;
+  // ... and for grouped-query models, whose portions stand in the order of their kinds (PortionKind): device tables of the
+  // portions' rows {first, count}, positions and pages, and every row's portion
+  const int2* seq = nullptr;
+  const int *row_seq = nullptr, *seq_pos = nullptr, *seq_pages = nullptr;
   // lm_head on these rows (device list) instead of the last row of every lane: n_want rows whose logits are only
   // read back, then the last rows of lanes [b0, b0 + nb) if `sample`
   const int* out_rows = nullptr;

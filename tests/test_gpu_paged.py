@@ -106,3 +106,44 @@ def test_pool_exhaustion_and_lane_errors(rb):
         sess.generate(p[None, :].repeat(2, 0), 4)
     with pytest.raises(RuntimeError):
         rb.CausalLM(cfg).load(W.init_weights(cfg, seed=0)).paged_session(2, 128, 1)
+
+
+@pytest.mark.parametrize("dtype,hd,mask,tol", [("f32", 32, 0, 1e-5), ("f32", 32, 1, 1e-5), ("bf16", 64, 1, 2e-2), ("bf16", 128, 1, 2e-2), ("bf16", 128, 0, 2e-2)])
+def test_feed_of_unequal_portions_in_any_order(rb, orc, dtype, hd, mask, tol):
+    """Every kind of portion (one token, below 128, 128 and more) in one step, several of each, in scrambled order and on lanes
+    whose contexts differ: wanted rows equal the oracle's forward of each lane's whole text.  A conventional mask only lets
+    later portions see earlier ones; the mask as written is checked on first portions, where it needs no context."""
+    from rew_b200 import _lib
+    bf = dtype == "bf16"
+    cfg = W.ModelConfig(vocab=128, d_model=128, n_layers=2, n_heads=4, n_kv_heads=2, head_dim=hd, ffn=192, max_seq=512, theta=10000.0,
+                        dtype=_lib.BF16 if bf else _lib.F32, mask_kind=mask)
+    t = [orc.bf16_round(a) if bf and a.ndim == 2 else a for a in W.init_weights(cfg, seed=3, std=0.08, trivial_affine=False)]
+    model = rb.CausalLM(cfg).load(t)
+    lanes, rng = 7, np.random.default_rng(hd + mask)
+    sess = model.paged_session(lanes, 400, 60)
+    texts = [np.zeros(0, np.int32) for _ in range(lanes)]
+    steps = [[(3, 130), (0, 1), (5, 2), (6, 300), (1, 127), (2, 128)]]
+    if mask == 1:
+        steps += [[(0, 129), (6, 1), (4, 64), (1, 1), (2, 65), (5, 128)], [(4, 1), (0, 1), (1, 1), (3, 1), (5, 1), (2, 2), (6, 1)]]
+    for portions in steps:
+        fed = [(l, rng.integers(0, cfg.vocab, n).astype(np.int32)) for l, n in portions]
+        start = [len(texts[l]) for l, _ in fed]
+        for l, ids in fed:
+            texts[l] = np.concatenate([texts[l], ids])
+        total = sum(n for _, n in portions)
+        want = sorted(set(rng.integers(0, total, 40).tolist()) | set(np.cumsum([n for _, n in portions]) - 1))
+        logits, nxt = sess.feed(fed, want=want, sample=[i % 2 == 0 for i in range(len(fed))])
+        whole = [orc.model_forward(cfg, t, texts[l][None], 0, True)[0] for l, _ in fed]
+        rows = np.concatenate([w[s:] for w, s in zip(whole, start)])
+        exp = rows[want]
+        err = np.linalg.norm(logits - exp, axis=1) / np.linalg.norm(exp, axis=1)
+        assert err.max() <= (1.5 * tol if bf else tol), (portions, err.argmax(), err.max())
+        ends = np.cumsum([n for _, n in portions]) - 1
+        for i, (l, _) in enumerate(fed):
+            assert sess.lane_length(l) == len(texts[l])
+            if i % 2:
+                assert nxt[i] == -1
+            else:
+                assert nxt[i] == int(np.argmax(logits[want.index(ends[i])]))
+    sess.reset()
+    assert sess.free_blocks() == 59 and all(sess.lane_length(l) == -1 for l in range(lanes))
