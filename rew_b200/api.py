@@ -28,12 +28,27 @@ class Tensor:
 
     def __init__(self, handle):
         self._h = C.c_void_p(handle) if not isinstance(handle, C.c_void_p) else handle
-        dt = C.c_int32()
-        nd = C.c_int32()
-        dims = (C.c_int64 * 8)()
-        check(lib().rewb200_buffer_info(self._h, C.byref(dt), dims, C.byref(nd)))
-        self.dtype = dt.value
-        self.shape = tuple(dims[i] for i in range(nd.value))
+        self._meta = None
+        if not self._h.value:
+            self._info()
+
+    def _info(self):
+        """(dtype, shape), asked for when first needed: most intermediate tensors are only passed on."""
+        if self._meta is None:
+            dt = C.c_int32()
+            nd = C.c_int32()
+            dims = (C.c_int64 * 8)()
+            check(lib().rewb200_buffer_info(self._h, C.byref(dt), dims, C.byref(nd)))
+            self._meta = dt.value, tuple(dims[:nd.value])
+        return self._meta
+
+    @property
+    def dtype(self):
+        return self._info()[0]
+
+    @property
+    def shape(self):
+        return self._info()[1]
 
     @staticmethod
     def from_host(array, dtype=None, slot=0):
@@ -65,12 +80,15 @@ class Tensor:
 
     def release(self):
         if self._h is not None and self._h.value:
+            self._info()    # a released tensor still says what it was
             lib().rewb200_buffer_release(self._h)
         self._h = None
 
     def __del__(self):
         try:
-            self.release()
+            if self._h is not None and self._h.value:
+                lib().rewb200_buffer_release(self._h)
+                self._h = None
         except Exception:
             pass
 

@@ -87,6 +87,7 @@ struct Ctx {
 Ctx* ctx_get(int slot);       // nullptr + error when not initialised
 Ctx* ctx_current();           // slot 0
 int ctx_check_status(Ctx* c); // reads d_status after a sync; non-zero -> error
+int ctx_status(Ctx* c);       // the same for a status whose copy to h_status the caller has waited for
 
 size_t dtype_size(int dtype);
 
@@ -186,6 +187,9 @@ struct rewb200_buffer {
 namespace rewb {
 
 int buffer_new(Ctx* c, int dtype, const int64_t* dims, int ndims, rewb200_buffer** out);
+// Linear.forward's checks, and the product into rows of its own stride, f32 or the operands' type (bias added).
+int linear_check(const rewb200_buffer* x, const rewb200_buffer* w, const rewb200_buffer* b);
+int linear_into(Ctx* c, const rewb200_buffer* x, const rewb200_buffer* w, const rewb200_buffer* b, void* out, int64_t ldo, int out_dtype);
 
 // ---------------------------------------------------------------- launchers
 enum Epilogue : int {

@@ -67,6 +67,11 @@ int place_cols(Ctx* c, const rewb200_buffer* src, int64_t rows, int64_t cols, vo
   return REWB200_OK;
 }
 
+__global__ void set_positions_kernel(int* pos, int n, int v) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) pos[i] = v;
+}
+
 // f32 parity path of the experts: out[t] (+)= w_e(t) * y[t] with w_e(t) = sum_j topw[t][j] * (topi[t][j] == e)
 // (routedWeightForExpert, src/rew/models/deepseek.nim:114-120,140-144)
 __global__ void expert_acc_kernel(const float* y, const float* topw, const int* topi, int k, int e, int64_t rows, int64_t d,
@@ -200,27 +205,22 @@ int rewb200_qkv_rope_kvappend(const rewb200_buffer* x, const rewb200_buffer* wq,
   Pool pool(c);
   float* fused = nullptr;  // [rows][nq | nkv | nkv] f32, biases added
   RB_TRY(pool.get(&fused, (size_t)rows * ntot * sizeof(float)));
-  // the three projections through the same entry point the Linear layer uses, then side by side in one row
+  // the three projections as the Linear layer computes them, side by side in one row and unrounded
   const rewb200_buffer* ws[3] = {wq, wk, wv};
   const rewb200_buffer* bs[3] = {bq, bk, bv};
-  const int64_t widths[3] = {nq, nkv, nkv}, offs[3] = {0, nq, nq + nkv};
+  const int64_t offs[3] = {0, nq, nq + nkv};
   rewb200_buffer x2 = *x;  // [rows, d] view
   x2.ndims = 2;
   x2.dims[0] = rows;
   x2.dims[1] = d;
   x2.owned = false;
-  for (int i = 0; i < 3; ++i) {
-    rewb200_buffer* y = nullptr;
-    RB_TRY(rewb200_linear(&x2, ws[i], bs[i], &y));
-    const int st = place_cols(c, y, rows, widths[i], fused, REWB200_F32, ntot, widths[i], widths[i], offs[i]);
-    rewb200_buffer_release(y);
-    RB_TRY(st);
-  }
+  for (int i = 0; i < 3; ++i) RB_TRY(linear_check(&x2, ws[i], bs[i]));
+  for (int i = 0; i < 3; ++i) RB_TRY(linear_into(c, &x2, ws[i], bs[i], fused + offs[i], ntot, REWB200_F32));
   const int64_t qd[3] = {B, S, nq};
   RB_TRY(buffer_new(c, dt, qd, 3, q_out));
-  std::vector<int> pos((size_t)B, kv->len);
-  RB_CUDA(cudaMemcpyAsync(kv->d_pos, pos.data(), B * sizeof(int), cudaMemcpyHostToDevice, c->stream));
-  RB_CUDA(cudaStreamSynchronize(c->stream));  // `pos` is pageable host memory
+  set_positions_kernel<<<(unsigned)((B + 255) / 256), 256, 0, c->stream>>>(kv->d_pos, (int)B, kv->len);
+  RB_CUDA(cudaGetLastError());
+  ++g_launch_total;
   QkvPostArgs qa;
   memset(&qa, 0, sizeof(qa));
   qa.partial = fused;

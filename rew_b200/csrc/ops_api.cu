@@ -81,13 +81,31 @@ int norm_common(const rewb200_buffer* x, const rewb200_buffer* gamma, const rewb
   return residual_norm_launch(c, a, d ? x->numel() / d : 0);
 }
 
+// bf16 SwiGLU of two projections: silu(gate) * up in f32, rounded once; eight elements a thread, the last thread fewer.  Bound by
+// launch and memory latency at decode sizes, by 6 bytes an element above; casts to f32 and back around an f32 kernel were four
+// launches of 20 bytes an element.
+__global__ void __launch_bounds__(256) swiglu_bf16_kernel(const bf16* gate, const bf16* up, bf16* out, int64_t n) {
+  const int64_t i = 8 * ((int64_t)blockIdx.x * 256 + threadIdx.x);
+  if (i >= n) return;
+  auto one = [](float g, float u) { return (g * (1.0f / (1.0f + expf(-g)))) * u; };
+  if (i + 8 > n) {
+    for (int64_t j = i; j < n; ++j) out[j] = __float2bfloat16_rn(one(__bfloat162float(gate[j]), __bfloat162float(up[j])));
+    return;
+  }
+  const uint4 g4 = *reinterpret_cast<const uint4*>(gate + i), u4 = *reinterpret_cast<const uint4*>(up + i);
+  const uint32_t g[4] = {g4.x, g4.y, g4.z, g4.w}, u[4] = {u4.x, u4.y, u4.z, u4.w};
+  uint32_t o[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    o[j] = pack_bf16(one(__uint_as_float(g[j] << 16), __uint_as_float(u[j] << 16)),
+                     one(__uint_as_float(g[j] & 0xFFFF0000u), __uint_as_float(u[j] & 0xFFFF0000u)));
+  *reinterpret_cast<uint4*>(out + i) = make_uint4(o[0], o[1], o[2], o[3]);
+}
+
 }  // namespace
-}  // namespace rewb
 
-extern "C" {
-
-int rewb200_linear(const rewb200_buffer* x, const rewb200_buffer* w, const rewb200_buffer* b, rewb200_buffer** y) {
-  RB_REQUIRE(x && w && y, "Linear.forward: NULL argument");
+int linear_check(const rewb200_buffer* x, const rewb200_buffer* w, const rewb200_buffer* b) {
+  RB_REQUIRE(x && w, "Linear.forward: NULL argument");
   RB_REQUIRE(x->ndims == 2 && w->ndims == 2,
              "matmul: expected rank-2 operands, got ranks " + std::to_string(x->ndims) + " and " + std::to_string(w->ndims));
   RB_REQUIRE(x->dims[1] == w->dims[0], "matmul: inner dim mismatch: [" + std::to_string(x->dims[0]) + "," +
@@ -96,19 +114,33 @@ int rewb200_linear(const rewb200_buffer* x, const rewb200_buffer* w, const rewb2
   RB_REQUIRE(x->dtype == w->dtype, "Linear.forward: x and weight dtypes differ");
   RB_TRY(same_slot(x, w));
   RB_REQUIRE(!b || (b->dtype == REWB200_F32 && b->numel() == w->dims[1]), "Linear.forward: bias must be f32 [out]");
-  Ctx* c = ctx_get(x->slot);
-  if (!c) return REWB200_ERR;
-  RB_CUDA(cudaSetDevice(c->device));
+  return REWB200_OK;
+}
+
+int linear_into(Ctx* c, const rewb200_buffer* x, const rewb200_buffer* w, const rewb200_buffer* b, void* out, int64_t ldo, int out_dtype) {
   const int64_t M = x->dims[0], K = x->dims[1], N = w->dims[1];
-  const int64_t od[2] = {M, N};
-  RB_TRY(buffer_new(c, x->dtype, od, 2, y));
   const float* bias = b ? (const float*)b->ptr : nullptr;
   if (x->dtype == REWB200_F32)
-    return gemm_f32_launch(c, (const float*)x->ptr, (const float*)w->ptr, bias, (float*)(*y)->ptr, M, K, N);
+    return gemm_f32_ld_launch(c, (const float*)x->ptr, K, (const float*)w->ptr, N, bias, (float*)out, ldo, M, K, N);
   RB_REQUIRE(x->dtype == REWB200_BF16, "Linear.forward: dtype must be f32 or bf16");
   LinearBf16Plan plan;
   RB_TRY(linear_bf16_plan(&plan, (const bf16*)w->ptr, K, N, 0));
-  return linear_bf16_launch(c, plan, (const bf16*)x->ptr, K, M, EPI_BIAS_BF16, 1, (*y)->ptr, N, bias, nullptr, 0);
+  return linear_bf16_launch(c, plan, (const bf16*)x->ptr, K, M, out_dtype == REWB200_F32 ? EPI_BIAS_F32 : EPI_BIAS_BF16, 1, out, ldo, bias, nullptr, 0);
+}
+
+}  // namespace rewb
+
+extern "C" {
+
+int rewb200_linear(const rewb200_buffer* x, const rewb200_buffer* w, const rewb200_buffer* b, rewb200_buffer** y) {
+  RB_REQUIRE(y, "Linear.forward: NULL argument");
+  RB_TRY(linear_check(x, w, b));
+  Ctx* c = ctx_get(x->slot);
+  if (!c) return REWB200_ERR;
+  RB_CUDA(cudaSetDevice(c->device));
+  const int64_t od[2] = {x->dims[0], w->dims[1]};
+  RB_TRY(buffer_new(c, x->dtype, od, 2, y));
+  return linear_into(c, x, w, b, (*y)->ptr, od[1], x->dtype);
 }
 
 int rewb200_rmsnorm(const rewb200_buffer* x, const rewb200_buffer* gamma, float eps, rewb200_buffer** y) {
@@ -271,18 +303,12 @@ int rewb200_swiglu_ffn(const rewb200_buffer* x, const rewb200_buffer* gate_w, co
   if (st == REWB200_OK) {
     if (x->dtype == REWB200_F32) {
       st = swiglu_f32_launch(c, (const float*)g->ptr, (const float*)u->ptr, (float*)h->ptr, M * f);
-    } else {
+    } else if (M * f > 0) {
       // bf16 Tier-B call: activation in f32 on the rounded projections, rounded once more
-      float *gf = nullptr, *uf = nullptr;
-      if (cudaMallocAsync((void**)&gf, (size_t)M * f * 8 + 256, c->stream) != cudaSuccess) st = fail("allocation failed");
-      if (st == REWB200_OK) {
-        uf = gf + M * f;
-        st = cast_launch(c, g->ptr, REWB200_BF16, gf, REWB200_F32, M * f);
-        if (st == REWB200_OK) st = cast_launch(c, u->ptr, REWB200_BF16, uf, REWB200_F32, M * f);
-        if (st == REWB200_OK) st = swiglu_f32_launch(c, gf, uf, gf, M * f);
-        if (st == REWB200_OK) st = cast_launch(c, gf, REWB200_F32, h->ptr, REWB200_BF16, M * f);
-        cudaFreeAsync(gf, c->stream);
-      }
+      const int64_t n = M * f;
+      swiglu_bf16_kernel<<<(unsigned)((n + 2047) / 2048), 256, 0, c->stream>>>((const bf16*)g->ptr, (const bf16*)u->ptr, (bf16*)h->ptr, n);
+      if (cudaGetLastError() != cudaSuccess) st = fail("SwiGLU launch failed");
+      ++g_launch_total;
     }
   }
   if (st == REWB200_OK) st = rewb200_linear(h, down_w, down_b, y);

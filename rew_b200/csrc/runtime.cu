@@ -44,10 +44,13 @@ size_t dtype_size(int dtype) {
 }
 
 int ctx_check_status(Ctx* c) {
-  int st = 0;
   RB_CUDA(cudaMemcpyAsync(c->h_status, c->d_status, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   RB_CUDA(cudaStreamSynchronize(c->stream));
-  st = *c->h_status;
+  return ctx_status(c);
+}
+
+int ctx_status(Ctx* c) {
+  const int st = *c->h_status;
   if (st != 0) {
     RB_CUDA(cudaMemsetAsync(c->d_status, 0, sizeof(int), c->stream));
     RB_CUDA(cudaMemsetAsync(c->d_tickets, 0, Ctx::kTickets * sizeof(int), c->stream));  // a kernel that gave up may have left counts behind
@@ -388,12 +391,13 @@ int rewb200_buffer_to_host(const rewb200_buffer* buf, void* dst, size_t nbytes) 
   while (off < nbytes) {
     const size_t n = std::min(c->pinned_bytes, nbytes - off);
     RB_CUDA(cudaMemcpyAsync(c->pinned, (const char*)buf->ptr + off, n, cudaMemcpyDeviceToHost, c->stream));
+    // the status of what made the data comes along with its last part: one wait
+    if (off + n == nbytes) RB_CUDA(cudaMemcpyAsync(c->h_status, c->d_status, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     RB_CUDA(cudaStreamSynchronize(c->stream));
     memcpy((char*)dst + off, c->pinned, n);
     off += n;
   }
-  if (nbytes == 0) RB_CUDA(cudaStreamSynchronize(c->stream));
-  return ctx_check_status(c);
+  return nbytes == 0 ? ctx_check_status(c) : ctx_status(c);
 }
 
 int rewb200_buffer_info(const rewb200_buffer* buf, int* dtype, int64_t* dims, int* ndims) {

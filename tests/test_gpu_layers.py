@@ -152,3 +152,22 @@ def test_generate_stops_at_stop_token_ids(rb, orc):
     # eos and stopTokenIds combine (generate.nim:263)
     got2 = sess.generate(prompt, 12, eos=stop_a, stop_ids=[stop_b])
     assert np.array_equal(got, got2)
+
+
+@pytest.mark.parametrize("M,f", [(1, 8), (3, 24), (5, 1000), (257, 264)])
+def test_bf16_ffn_activation_edges(rb, orc, M, f):
+    """SwiGLU of eight elements a thread: single threads, part-filled CTAs and several of them.  The projections are rounded to
+    bf16 once each and the product once more, 2^-9 relative apiece, before the down projection adds its own."""
+    from rew_b200 import _lib
+    rng = np.random.default_rng(M + f)
+    bf = lambda *s, std: orc.bf16_round(rng.normal(0, std, s).astype(np.float32))
+    x, wg, wu, wd = bf(M, 64, std=1.0), bf(64, f, std=0.2), bf(64, f, std=0.2), bf(f, 40, std=0.1)
+    T = rb.Tensor.from_host
+    lin = lambda w: rb.Linear(T(w, _lib.BF16), T(np.zeros(w.shape[1], np.float32)))
+    got = rb.GatedFeedForward(lin(wg), lin(wu), lin(wd)).forward(T(x, _lib.BF16)).to_host()
+    g, u = x.astype(np.float64) @ wg, x.astype(np.float64) @ wu
+    h = g / (1 + np.exp(-g)) * u
+    want = h @ wd
+    # |d silu(g)/dg| <= 1.1 and the relative errors above
+    bound = (4 * 2.0 ** -8) * ((np.abs(h) + np.abs(g * u)) @ np.abs(wd)) + 2.0 ** -8 * np.abs(want) + 1e-6
+    assert np.all(np.abs(got - want) <= bound)
