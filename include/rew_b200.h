@@ -476,9 +476,9 @@ int rewb200_lane_admit(rewb200_session* s, int lane, const int32_t* ids, int S, 
  * cannot cover the growth of every active lane ("out of free blocks"). */
 int rewb200_lanes_step(rewb200_session* s, int n_steps, int32_t* out_ids);
 /* One step over unequal portions: entry e appends counts[e] tokens (ids: all entries' tokens one after the other) to
- * lane lanes[e], which is admitted by its first portion.  Prompt portions and single decoded tokens mix freely; a
- * layered model runs all entries as one batch, a grouped-query model one entry after the other.  want (optional,
- * n_want places in the concatenated tokens, ascending) asks for those positions' logits, host f32 [n_want, vocab].
+ * lane lanes[e], which is admitted by its first portion.  Prompt portions and single decoded tokens mix freely
+ * and run as one batch.  want (optional, n_want places in the concatenated tokens, ascending) asks for those positions'
+ * logits, host f32 [n_want, vocab].
  * next_ids (optional, host int32 [n_entries]) asks for the token after every entry with sample[e] != 0 (sample NULL:
  * all), chosen as rewb200_lanes_step would; it becomes the lane's next input there.  seeds as rewb200_lane_admit,
  * one per entry, or NULL.  Fails without side effects when the pool cannot hold the step. */

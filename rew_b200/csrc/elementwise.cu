@@ -460,6 +460,72 @@ __global__ void __launch_bounds__(NORMV_THREADS) residual_norm_vec_kernel(NormAr
   }
 }
 
+// residual_norm of a large step in its plain form (one slab, the residual, an RMS norm): a stream of 20 bytes an element with a
+// bf16 slab, so what matters is that loads never stop.  Two CTAs an SM stay for all rows: the next row's loads are in flight
+// while this one's squares are summed (one barrier a row), the norm's weights and the bias stay in registers.  16 384 rows of
+// 4096: 125 us, 6.4 TB/s; a CTA a row waits for its slab, its residual and its weights in turn, 259 us.
+template <bool BF16P, int NCH>
+__global__ void __launch_bounds__(NORMV_THREADS, 2) residual_norm_rows_kernel(NormArgs a, int64_t rows) {
+  __shared__ float red[2][NORMV_THREADS / 32];
+  pdl_launch_dependents();
+  const int64_t d = a.d;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int at[NCH];
+  bool in[NCH];
+  float4 g[NCH], b[NCH];
+#pragma unroll
+  for (int c = 0; c < NCH; ++c) {
+    at[c] = (c * NORMV_THREADS + threadIdx.x) * 4;
+    in[c] = at[c] < d;
+    g[c] = in[c] ? *reinterpret_cast<const float4*>(a.gamma + at[c]) : make_float4(0.f, 0.f, 0.f, 0.f);
+    b[c] = in[c] && a.bias ? *reinterpret_cast<const float4*>(a.bias + at[c]) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  pdl_wait();
+  using Part = typename std::conditional<BF16P, uint2, float4>::type;
+  using PartT = typename std::conditional<BF16P, bf16, float>::type;
+  const PartT* const part = reinterpret_cast<const PartT*>(a.partial);
+  float4 nx[NCH] = {};
+  Part np[NCH] = {};
+  auto request = [&](int64_t row) {
+#pragma unroll
+    for (int c = 0; c < NCH; ++c)
+      if (in[c]) {
+        nx[c] = *reinterpret_cast<const float4*>(a.x_res + row * d + at[c]);
+        np[c] = *reinterpret_cast<const Part*>(part + row * d + at[c]);
+      }
+  };
+  int64_t row = blockIdx.x;
+  if (row < rows) request(row);
+  for (int buf = 0; row < rows; row += gridDim.x, buf ^= 1) {
+    float4 v[NCH];
+    float ss = 0.f;
+#pragma unroll
+    for (int c = 0; c < NCH; ++c) {
+      float4 p;
+      if constexpr (BF16P) p = make_float4(__uint_as_float(np[c].x << 16), __uint_as_float(np[c].x & 0xFFFF0000u), __uint_as_float(np[c].y << 16), __uint_as_float(np[c].y & 0xFFFF0000u));
+      else p = np[c];
+      v[c] = make_float4(nx[c].x + (p.x + b[c].x), nx[c].y + (p.y + b[c].y), nx[c].z + (p.z + b[c].z), nx[c].w + (p.w + b[c].w));
+    }
+    if (row + gridDim.x < rows) request(row + gridDim.x);
+#pragma unroll
+    for (int c = 0; c < NCH; ++c)
+      if (in[c]) {
+        *reinterpret_cast<float4*>(a.x_res + row * d + at[c]) = v[c];
+        ss += v[c].x * v[c].x + v[c].y * v[c].y + v[c].z * v[c].z + v[c].w * v[c].w;
+      }
+    ss = warp_sum(ss);
+    if (lane == 0) red[buf][warp] = ss;
+    __syncthreads();   // the other buffer's readers have all passed here
+    ss = warp_sum(lane < NORMV_THREADS / 32 ? red[buf][lane] : 0.f);
+    const float scale = sqrtf(ss / (float)(a.d_mean > 0 ? a.d_mean : d) + a.eps);
+#pragma unroll
+    for (int c = 0; c < NCH; ++c)
+      if (in[c])
+        *reinterpret_cast<uint2*>(reinterpret_cast<bf16*>(a.out) + row * d + at[c]) =
+            make_uint2(pack_bf16(g[c].x * (v[c].x / scale), g[c].y * (v[c].y / scale)), pack_bf16(g[c].z * (v[c].z / scale), g[c].w * (v[c].w / scale)));
+  }
+}
+
 // Sublayers normed on the way back (OutputNormArgs): x += gamma * y / rms(y), y the sum of the slabs.  CL CTAs of a
 // cluster share a row (decode-size steps), their sums of squares meet through distributed shared memory.
 template <typename T, int CL, int NCH>
@@ -700,23 +766,16 @@ __device__ __forceinline__ void store8<bf16>(bf16* dst, const float* r) {
 }
 
 // Same work as qkv_post_kernel, eight consecutive columns (four RoPE pairs) per thread with 16-byte
-// accesses; needs head_dim % 8 == 0.  Prefill-size launches are bandwidth-bound on the f32 partials.
+// accesses; needs head_dim % 8 == 0.  Prefill-size launches are bound by the f32 partials and the latency in front of
+// them: requested ahead of the row's position and page, 16 384 rows of 6144 take 161 us (179 us behind them).
 template <typename TA>
 __global__ void __launch_bounds__(256) qkv_post_vec_kernel(QkvPostArgs a) {
   pdl_launch_dependents();
   pdl_wait();
   const int64_t row = blockIdx.x;
-  const int b = a.row_seq ? a.row_seq[row] : (int)(row / a.S), s = a.row_seq ? (int)row - a.seq[b].x : (int)(row % a.S);
-  const int pos = a.pos0[b] + s;
-  const int hd = a.hd;
-  const int nq = a.nh * hd, nkv = a.kvh * hd, ntot = nq + 2 * nkv;
-  const int rpos = pos + a.rope_shift;
-  if (pos < 0 || pos >= a.kv_capacity || rpos < 0 || rpos >= a.max_seq) {
-    if (threadIdx.x == 0) atomicExch(a.status, KS_BAD_INDEX);
-    return;
-  }
-  const int col = 8 * (blockIdx.y * blockDim.x + threadIdx.x);
+  const int ntot = (a.nh + 2 * a.kvh) * a.hd, col = 8 * (blockIdx.y * blockDim.x + threadIdx.x);
   if (col >= ntot) return;
+  // the slabs first: they are the bytes, and the position and page of the row are two loads in turn
   float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   const float* pp = a.partial + row * ntot + col;
   for (int sp = 0; sp < a.nsplit; ++sp) {
@@ -724,6 +783,15 @@ __global__ void __launch_bounds__(256) qkv_post_vec_kernel(QkvPostArgs a) {
     const float4 t1 = *reinterpret_cast<const float4*>(pp + sp * a.split_stride + 4);
     v[0] += t0.x; v[1] += t0.y; v[2] += t0.z; v[3] += t0.w;
     v[4] += t1.x; v[5] += t1.y; v[6] += t1.z; v[7] += t1.w;
+  }
+  const int b = a.row_seq ? a.row_seq[row] : (int)(row / a.S), s = a.row_seq ? (int)row - a.seq[b].x : (int)(row % a.S);
+  const int pos = a.pos0[b] + s;
+  const int hd = a.hd;
+  const int nq = a.nh * hd, nkv = a.kvh * hd;
+  const int rpos = pos + a.rope_shift;
+  if (pos < 0 || pos >= a.kv_capacity || rpos < 0 || rpos >= a.max_seq) {
+    if (threadIdx.x == 0) atomicExch(a.status, KS_BAD_INDEX);
+    return;
   }
   if (a.bias) {
     const float4 b0 = *reinterpret_cast<const float4*>(a.bias + col), b1 = *reinterpret_cast<const float4*>(a.bias + col + 4);
@@ -1241,6 +1309,20 @@ int residual_norm_launch(Ctx* c, const NormArgs& a, int64_t rows) {
               : launch_k(residual_norm_cluster_kernel<TE, 4>, g, b, 0, c->stream, c->use_pdl, a))
     e = e16 ? RB_NORMC(bf16) : RB_NORMC(float);
 #undef RB_NORMC
+    RB_CUDA(e);
+    ++g_launch_total;
+    return REWB200_OK;
+  }
+  // Above 256 rows, where a step's row-parallel Linears leave one slab, the plain form streams; wider rows than 4096 would not
+  // keep a row ahead in registers.
+  if (rows > 256 && a.d % 4 == 0 && a.d <= 2 * 4 * NORMV_THREADS && o16 && a.norm_kind == 0 && a.partial && a.nsplit == 1 && a.nsplit2 == 0 &&
+      a.nsplit3 == 0 && !a.embed && !a.add_vec && !a.gamma2 && a.x_res && a.n_peers == 0 && a.wait_n == 0) {
+    const dim3 g((unsigned)std::min<int64_t>(rows, 2 * (int64_t)c->sm_count)), b(NORMV_THREADS);
+    const bool one = a.d <= 4 * NORMV_THREADS;
+    e = a.partial_bf16 ? (one ? launch_k(residual_norm_rows_kernel<true, 1>, g, b, 0, c->stream, c->use_pdl, a, rows)
+                              : launch_k(residual_norm_rows_kernel<true, 2>, g, b, 0, c->stream, c->use_pdl, a, rows))
+                       : (one ? launch_k(residual_norm_rows_kernel<false, 1>, g, b, 0, c->stream, c->use_pdl, a, rows)
+                              : launch_k(residual_norm_rows_kernel<false, 2>, g, b, 0, c->stream, c->use_pdl, a, rows));
     RB_CUDA(e);
     ++g_launch_total;
     return REWB200_OK;

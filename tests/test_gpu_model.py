@@ -367,3 +367,17 @@ def test_decode_splitk_policy_switches_agree(rb, orc, key, other, default):
         seq = np.concatenate([prompt, nxt[:, None], ids[:, :2]], 1)
         want = orc.model_forward(cfg, t, seq, 0, True)[:, -1]
         assert rel_l2(last, want) <= 2e-2
+
+
+@pytest.mark.parametrize("d,heads,routed,S", [(136, 4, 0, 257), (2048, 16, 0, 300), (2056, 4, 0, 601), (136, 4, 8, 290)])
+def test_bf16_norms_of_large_steps(rb, orc, d, heads, routed, S):
+    """Steps above 256 rows, whose norms keep a row ahead in registers: widths that fill one float4 a thread, two, or neither, rows
+    that do not divide among the CTAs, and the f32 slab a routed model leaves instead of the bf16 one."""
+    from rew_b200 import _lib
+    cfg = W.ModelConfig(vocab=128, d_model=d, n_layers=1, n_heads=heads, n_kv_heads=2, head_dim=64, ffn=256, max_seq=640, theta=500000.0,
+                        dtype=_lib.BF16, mask_kind=1, n_routed=routed, n_shared=1 if routed else 0, top_k=routed, moe_ffn=64 if routed else 0)
+    t = [orc.bf16_round(a) if a.ndim == 2 else a for a in W.init_weights(cfg, seed=8, std=0.04, trivial_affine=False)]
+    prompt = np.random.default_rng(S).integers(0, cfg.vocab, size=(1, S)).astype(np.int32)
+    logits = rb.CausalLM(cfg).load(t).session(1, S).forward_all(prompt)
+    want = orc.model_forward(cfg, t, prompt, 0, True)
+    assert rel_l2(logits, want) <= 2e-2
