@@ -1019,6 +1019,7 @@ int enqueue_forward(rewb200_session* s, const FwdOpts& o) {
   const int64_t d = m->dp;
   int* const pos = s->d_pos + b0;
   const bool lists = o.out_rows != nullptr;
+  if (!o.seq) s->route_order.clear();
   // where the logits of lanes [b0, b0 + nb) go: behind those of the wanted rows, or at their lane index
   float* const logits = o.all_logits ? s->logits : s->logits + (size_t)(lists ? o.n_want : b0) * m->vocab_l;
   int* const next = s->d_next + b0;
@@ -1828,6 +1829,7 @@ static int decode_core(rewb200_session* s, int n_steps, int32_t* out_ids, float*
     cudaGraphExecDestroy(s->graph);
     s->graph = nullptr;
   }
+  s->route_order.clear();
   if (use_graph && !s->graph && n_steps > 0) {
     s->graph_epoch = c->option_epoch;
     cudaGraph_t g;
@@ -2193,6 +2195,12 @@ int rewb200_lanes_feed(rewb200_session* s, int n_entries, const int32_t* lanes, 
     o.seq_pos = s->feed_dev + at_pos;
     o.seq_pages = s->feed_dev + at_pages;
     o.row_seq = s->feed_dev + at_row_seq;
+    s->route_order.clear();
+    if (s->route_rec) {
+      s->route_order.resize(rows);
+      for (const StepEntry& e : entries)
+        for (int j = 0; j < e.n; ++j) s->route_order[e.src + j] = e.row0 + j;
+    }
   }
   RB_TRY(enqueue_forward(s, o));
   if (n_want > 0)
@@ -2371,8 +2379,15 @@ int rewb200_session_routing(rewb200_session* s, int moe_layer, int32_t* topi_out
   Ctx* c = s->m->c;
   RB_CUDA(cudaSetDevice(c->device));
   RB_CUDA(cudaStreamSynchronize(c->stream));
-  RB_CUDA(cudaMemcpy(topi_out, s->route_rec + (size_t)moe_layer * s->rows_cap * s->m->max_topk,
-                     (size_t)rows * s->m->max_topk * sizeof(int), cudaMemcpyDeviceToHost));
+  const size_t k = (size_t)s->m->max_topk;
+  const int* rec = s->route_rec + (size_t)moe_layer * s->rows_cap * k;
+  if ((int64_t)s->route_order.size() != rows) {
+    RB_CUDA(cudaMemcpy(topi_out, rec, (size_t)rows * k * sizeof(int), cudaMemcpyDeviceToHost));
+    return REWB200_OK;
+  }
+  std::vector<int32_t> by_row((size_t)rows * k);
+  RB_CUDA(cudaMemcpy(by_row.data(), rec, by_row.size() * sizeof(int), cudaMemcpyDeviceToHost));
+  for (int64_t i = 0; i < rows; ++i) memcpy(topi_out + i * k, by_row.data() + s->route_order[i] * k, k * sizeof(int));
   return REWB200_OK;
 }
 

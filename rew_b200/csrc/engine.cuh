@@ -270,6 +270,7 @@ struct rewb200_session {
   int* feed_dev = nullptr;             // ids and row lists of a rewb200_lanes_feed step
   size_t feed_cap = 0;
   int64_t route_rows = 0;              // rows of the forward recorded last
+  std::vector<int> route_order;        // ... and the row of every token, where a step's rows do not stand in the caller's order
   cudaGraphExec_t graph = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   float prefill_ms = 0.f, decode_ms = 0.f;

@@ -147,3 +147,29 @@ def test_feed_of_unequal_portions_in_any_order(rb, orc, dtype, hd, mask, tol):
                 assert nxt[i] == int(np.argmax(logits[want.index(ends[i])]))
     sess.reset()
     assert sess.free_blocks() == 59 and all(sess.lane_length(l) == -1 for l in range(lanes))
+
+
+def test_routing_of_a_step_of_portions_in_the_callers_order(rb):
+    """The recorded expert choices of a step whose rows were put in the order of their portions' kinds come back in the order the
+    tokens were given in: those of every portion fed alone."""
+    cfg = W.ModelConfig(vocab=64, d_model=64, n_layers=2, n_heads=2, n_kv_heads=1, head_dim=32, ffn=64, max_seq=256, theta=10000.0, mask_kind=1,
+                        n_routed=8, n_shared=1, top_k=2, moe_ffn=32)
+    rb.set_option("record_routing", "1")
+    try:
+        model = rb.CausalLM(cfg).load(W.init_weights(cfg, seed=2, std=0.3))
+        rng = np.random.default_rng(4)
+        portions = [(l, rng.integers(0, cfg.vocab, n).astype(np.int32)) for l, n in ((1, 1), (3, 40), (0, 130), (2, 1))]
+        sess = model.paged_session(4, 200, 20)
+        sess.feed(portions)
+        rows = sum(len(t) for _, t in portions)
+        got = [sess.routing(layer, rows) for layer in range(2)]
+        alone = [[], []]
+        for l, t in portions:
+            sess.reset()
+            sess.feed([(l, t)])
+            for layer in range(2):
+                alone[layer].append(sess.routing(layer, len(t)))
+        for layer in range(2):
+            assert np.array_equal(got[layer], np.concatenate(alone[layer]))
+    finally:
+        rb.set_option("record_routing", "0")
