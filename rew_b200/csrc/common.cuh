@@ -204,7 +204,7 @@ enum Epilogue : int {
 struct LinearBf16Plan {
   CUtensorMap tmW;       // W [K rows][N cols] bf16 (reference layout [in,out]); 3D when groups > 1
   int64_t K = 0, N = 0;
-  bool early_w = false;  // no kernel of a step writes W: a launch may request it ahead of its stream dependency
+  bool early_w = false;  // no kernel of a step writes W: every Linear kernel may request it ahead of its stream dependency, and only then
   int groups = 0;        // 0: one matrix; >= 1: that many stacked matrices (experts), 3-D tensor map
 };
 // y = x @ W (+bias); x [M,K] bf16 row-major (ldx elements), W as planned.

@@ -8,7 +8,8 @@
 //   - 4 consumer warps (32 columns each) read the swizzled boxes with
 //     ldmatrix(.trans for W) and accumulate in f32 with mma.sync m16n8k16.
 //   - The weight loads of the first STAGES stages are issued BEFORE
-//     griddepcontrol.wait, so under programmatic dependent launch the ramp-up of
+//     griddepcontrol.wait where no kernel of a step writes the weights
+//     (LinearBf16Plan::early_w), so under programmatic dependent launch the ramp-up of
 //     this kernel overlaps the tail of the previous one; only the activation
 //     loads and the epilogue wait for the producer kernel.
 //   - Split-K partials (f32) go to scratch and are summed by the consumer
@@ -52,6 +53,7 @@ struct LinArgs {
   const float* bias;
   const int* row_offsets;  // grouped: rows of group g = [row_offsets[g], row_offsets[g+1])
   int grouped;
+  int early_w;             // LinearBf16Plan::early_w
   int* status;
 };
 
@@ -106,6 +108,7 @@ __global__ void __launch_bounds__(160) linear_bf16_kernel(const __grid_constant_
       const uint64_t pol_w = policy_evict_first();
       const uint64_t pol_x = policy_evict_last();
       const int pre = min(C::STAGES, nkb);
+      if (!a.early_w) pdl_wait();  // the launch before may be the one that writes the weights
       for (int kb = 0; kb < pre; ++kb) {
         uint8_t* st = smem + kb * C::STAGE_BYTES;
         mbar_expect_tx(&full[kb], C::STAGE_BYTES);
@@ -347,6 +350,7 @@ int linear_bf16_launch(Ctx* c, const LinearBf16Plan& plan, const bf16* x, int64_
   a.bias = bias;
   a.row_offsets = row_offsets;
   a.grouped = grouped ? 1 : 0;
+  a.early_w = plan.early_w;
   a.status = c->d_status;
   dim3 grid((unsigned)((plan.N + BN - 1) / BN), (unsigned)((rows_for_tile + ROWS - 1) / ROWS),
             (unsigned)(grouped ? plan.groups : ksplit));

@@ -11,7 +11,8 @@
 // Roles inside the CTA (320 threads):
 //   warp 0   TMA producer: cp.async.bulk.tensor boxes of W (64 k x 64 features,
 //            two per stage) and x (64 k x TN tokens), 128-byte swizzle, into a
-//            multi-stage mbarrier ring; W loads are issued before
+//            multi-stage mbarrier ring; W loads of weights that no kernel
+//            of a step writes (TcArgs::early_w) are issued before
 //            griddepcontrol.wait so the ramp overlaps the previous kernel.
 //   warp 1   allocates TMEM, then one elected thread issues four
 //            tcgen05.mma.kind::f16 (K = 16 each) per stage from shared-memory
@@ -47,7 +48,7 @@ struct TcArgs {
   int groups;
   int tn, stages;          // launches that choose their tile and ring
   int ksplit;              // persistent kernel: pieces of a tile along K
-  int early_w;             // ... the weights are final before any step: they may be requested ahead of the stream dependency
+  int early_w;             // the weights are final before any step: they may be requested ahead of the stream dependency
   int fuse_qkv;       // cluster kernel: finish q|k|v in the epilogue (bias, RoPE, cache write) instead of one f32 slab
   QkvPostArgs qp;     // what qkv_post_kernel would have been given (partial / nsplit unused)
 };
@@ -364,6 +365,7 @@ __global__ void __launch_bounds__(TC_THREADS) linear_tc_kernel(const __grid_cons
       const uint64_t pol_w = policy_evict_first();
       const uint64_t pol_x = policy_evict_last();
       const int pre = min(stages, nkb);
+      if (!a.early_w) pdl_wait();  // the launch before may be the one that writes them
       for (int kb = 0; kb < pre; ++kb) {
         uint8_t* st = smem + kb * stage_bytes;
         mbar_expect_tx(&full[kb], stage_bytes);
@@ -946,6 +948,7 @@ int linear_tc_cluster_launch(Ctx* c, const LinearBf16Plan& plan, const bf16* x, 
   a.split_stride = 0;
   a.bias = nullptr;
   a.status = c->d_status;
+  a.early_w = plan.early_w;
   if (fuse_qkv) {
     RB_REQUIRE(fuse_qkv->act_dtype == REWB200_BF16 && fuse_qkv->hd % 2 == 0 &&
                    (int64_t)(fuse_qkv->nh + 2 * fuse_qkv->kvh) * fuse_qkv->hd == plan.N,
@@ -1041,6 +1044,7 @@ int linear_tc_launch(Ctx* c, const LinearBf16Plan& plan, const bf16* x, int64_t 
   a.bias = bias;
   a.status = c->d_status;
   a.ksplit = ksplit;
+  a.early_w = plan.early_w;
   a.tn = TN;
   dim3 grid((unsigned)((plan.N + BM - 1) / BM), (unsigned)((M + TN - 1) / TN), (unsigned)ksplit);
   // Pairs of CTAs where a launch runs long enough for the power cap to set the pace (six layers of the 8B shape, 16 384 tokens:
@@ -1070,7 +1074,6 @@ int linear_tc_launch(Ctx* c, const LinearBf16Plan& plan, const bf16* x, int64_t 
   // (4096 x 28672: 135 tokens 42 us, 48 in the persistent kernel, 300 tokens 70 and 92).  Otherwise the persistent kernel.
   const bool two = TN <= 160 && (int64_t)grid.x * grid.y * grid.z > c->sm_count;
   if (c->prefill_persistent && !two) {
-    a.early_w = plan.early_w;
     static bool attr_set = false;
     if (!attr_set) {
       RB_CUDA(cudaFuncSetAttribute(linear_tc_persist_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));

@@ -75,6 +75,27 @@ def test_linear_tiles_of_the_steps_own_size(rb_tc, M, K, N):
     assert np.all(np.abs(got - want) <= bound)
 
 
+@pytest.mark.parametrize("linear", ["tc", "mma"])
+@pytest.mark.parametrize("M", [1, 33, 64, 100, 300])
+@pytest.mark.parametrize("N", [264, 18968, 37888])
+def test_weights_that_the_launch_before_writes(rb_tc, M, N, linear):
+    """x @ (A @ B): the weights of a Linear are the output of the Linear just before it, on both sides of one feature tile an SM.
+    The same bits as with the weights brought from the host: no launch may request them before they are written."""
+    from rew_b200 import _lib
+    K, r = 520, 48
+    rng = np.random.default_rng(M + N)
+    bf = lambda *s: rb_tc.Tensor.from_host(W.bf16_round(rng.normal(size=s).astype(np.float32)), _lib.BF16)
+    lin = lambda w: rb_tc.Linear(w, None)
+    rb_tc.set_option("linear", linear)
+    x = bf(M, K)
+    for _ in range(3):
+        a, b = bf(r, K), bf(r, N)   # other weights every time: what an early request would find are the last ones
+        w = lin(b).forward(rb_tc.Tensor.from_host(np.ascontiguousarray(a.to_host().T), _lib.BF16))
+        got = lin(w).forward(x).to_host()
+        want = lin(rb_tc.Tensor.from_host(w.to_host(), _lib.BF16)).forward(x).to_host()
+        assert np.array_equal(got, want)
+
+
 @pytest.mark.parametrize("B,S", [(13, 5), (2, 80), (1, 250)])
 def test_split_steps_match_the_oracle(rb_tc, orc, B, S):
     """Steps of 65 to 256 rows whose Linears are cut along K into the count of slabs that costs least (here 2 to 4 of 18 blocks)."""
