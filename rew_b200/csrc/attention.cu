@@ -886,9 +886,8 @@ __global__ void __launch_bounds__(fa::THREADS, 2) attn_prefill_tc_kernel(const _
     mbar_init(p_full, 8);   // the eight softmax warps
     mbar_init(o_done, 1);
     fence_barrier_init();
-    pdl_launch_dependents();
   }
-  if (warp == 1) tc::alloc(tmem_slot, 256);
+  if (warp == 1) tc::alloc_then_launch_dependents(tmem_slot, 256);
   tc::fence_before();
   __syncthreads();
   tc::fence_after();
@@ -1040,9 +1039,8 @@ __global__ void __launch_bounds__(fa2::THREADS, 1) attn_prefill_tc2_kernel(const
       mbar_init(o_done + i, 1);
     }
     fence_barrier_init();
-    pdl_launch_dependents();
   }
-  if (warp == 1) tc::alloc(tmem_slot, 512);
+  if (warp == 1) tc::alloc_then_launch_dependents(tmem_slot, 512);
   tc::fence_before();
   __syncthreads();
   tc::fence_after();

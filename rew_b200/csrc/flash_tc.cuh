@@ -210,9 +210,8 @@ __global__ void __launch_bounds__(64 + QT * 256, 1) flash_tc_kernel(const __grid
       mbar_init(o_done + i, 1);
     }
     fence_barrier_init();
-    pdl_launch_dependents();
   }
-  if (warp == 1) tc::alloc(tmem_slot, TM_COLS);
+  if (warp == 1) tc::alloc_then_launch_dependents(tmem_slot, TM_COLS);
   tc::fence_before();
   __syncthreads();
   tc::fence_after();

@@ -153,9 +153,8 @@ __global__ void __launch_bounds__(64 + 512, 1) mix_stats_kernel(const __grid_con
     }
     mbar_init(q_full, 1);
     fence_barrier_init();
-    pdl_launch_dependents();
   }
-  if (warp == 1) tc::alloc(tmem_slot, 512);
+  if (warp == 1) tc::alloc_then_launch_dependents(tmem_slot, 512);
   tc::fence_before();
   __syncthreads();
   tc::fence_after();
@@ -305,9 +304,8 @@ __global__ void __launch_bounds__(64 + 128 * warpgroups(HP), 1) mix_attn_kernel(
     mbar_init(g_full, 1);
     mbar_init(o_full, 1);
     fence_barrier_init();
-    pdl_launch_dependents();
   }
-  if (warp == 1) tc::alloc(tmem_slot, 512);
+  if (warp == 1) tc::alloc_then_launch_dependents(tmem_slot, 512);
   tc::fence_before();
   __syncthreads();
   tc::fence_after();

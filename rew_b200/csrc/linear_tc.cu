@@ -335,27 +335,12 @@ __global__ void __launch_bounds__(TC_THREADS) linear_tc_kernel(const __grid_cons
     }
     mbar_init(tmem_full, 1);
     fence_barrier_init();
-    pdl_launch_dependents();
   }
-  // Large accumulators take their tensor memory after the stream dependency: a launch that held it while it waits could
-  // keep it from a CTA of the launch it waits for.
-  constexpr bool LATE = TN == 0;
-  if (LATE) {
-    __syncthreads();
-    if (warp != 0) {
-      pdl_wait();
-      if (warp == 1) tc::alloc(tmem_slot, C::tmem_cols(a));
-      tc::fence_before();
-      asm volatile("bar.sync 2, %0;" ::"n"(TC_THREADS - 32) : "memory");
-      tc::fence_after();
-    }
-  } else {
-    if (warp == 1) tc::alloc(tmem_slot, C::tmem_cols(a));
-    tc::fence_before();
-    __syncthreads();
-    tc::fence_after();
-  }
-  const uint32_t tmem_base = LATE && warp == 0 ? 0u : *tmem_slot;
+  if (warp == 1) tc::alloc_then_launch_dependents(tmem_slot, C::tmem_cols(a));
+  tc::fence_before();
+  __syncthreads();
+  tc::fence_after();
+  const uint32_t tmem_base = *tmem_slot;
 
   bool epi_ok = true;
   if (warp == 0) {
@@ -580,11 +565,8 @@ __global__ void __launch_bounds__(TC_THREADS) linear_tc_persist_kernel(const __g
       mbar_init(&tmem_empty[b], 1);
     }
     fence_barrier_init();
-    pdl_launch_dependents();
   }
-  if (warp == 1) {
-    tc::alloc(tmem_slot, (uint32_t)C::TMEM_COLS);
-  }
+  if (warp == 1) tc::alloc_then_launch_dependents(tmem_slot, (uint32_t)C::TMEM_COLS);
   tc::fence_before();
   __syncthreads();
   tc::fence_after();
@@ -797,12 +779,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS) linear_t
       mbar_init(&tmem_empty[b], 2);  // the epilogues of both CTAs
     }
     fence_barrier_init();
-    pdl_launch_dependents();
   }
-  if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"((uint32_t)C::TMEM_COLS) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-  }
+  if (warp == 1) tc::alloc_then_launch_dependents<2>(tmem_slot, (uint32_t)C::TMEM_COLS);
   tc::fence_before();
   cluster_sync_all();  // both CTAs' barriers are initialised before any remote arrival, and both allocations are done
   tc::fence_after();

@@ -213,9 +213,8 @@ __global__ void __launch_bounds__(NT_THREADS) nf4_tc_kernel(const __grid_constan
     }
     mbar_init(d_full, 1);
     fence_barrier_init();
-    pdl_launch_dependents();
   }
-  if (warp == 1) tc::alloc(tmem_slot, NT_TMEM_COLS);
+  if (warp == 1) tc::alloc_then_launch_dependents(tmem_slot, NT_TMEM_COLS);
   // pair table: entry e = (level[e & 15], level[e >> 4]) as bf16x2, one copy per lane (bank = lane)
   for (int idx = threadIdx.x; idx < 256 * 8; idx += NT_THREADS) {
     const int e = idx >> 3;

@@ -67,9 +67,22 @@ __device__ __forceinline__ void commit(uint64_t* bar) {
 }
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void alloc(uint32_t* slot_in_smem, uint32_t cols) {
-  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot_in_smem)), "r"(cols) : "memory");
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+// Takes `cols` columns of tensor memory for the CTA (GROUP = 2: for a pair of CTAs), by one whole warp, and then lets the stream's
+// next launch start.  Always in this order, which is why no kernel that takes tensor memory calls pdl_launch_dependents itself:
+// tcgen05.alloc waits without limit for columns that other CTAs of the SM hold.  Were a CTA to let later launches start first, one
+// of them could take the columns it still needs and hold them while it waits for this launch to end: neither would.  In this order
+// a launch starts only when every CTA of the launch ahead has its columns or has left, so whoever holds columns waits for launches
+// that need no more of them, and they end.
+template <int GROUP = 1>
+__device__ __forceinline__ void alloc_then_launch_dependents(uint32_t* slot_in_smem, uint32_t cols) {
+  if constexpr (GROUP == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot_in_smem)), "r"(cols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  } else {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot_in_smem)), "r"(cols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  pdl_launch_dependents();
 }
 __device__ __forceinline__ void dealloc(uint32_t base, uint32_t cols) {
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(cols) : "memory");

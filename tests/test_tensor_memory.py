@@ -1,0 +1,40 @@
+"""Rules of the kernels that take tensor memory, held on their source: what breaks them can stop a GPU, so no run shows it."""
+import os
+import re
+
+CSRC = os.path.join(os.path.dirname(os.path.abspath(__file__)), "..", "rew_b200", "csrc")
+
+
+def _kernels():
+    """(name, body) of every __global__ function, with `//` comments taken out."""
+    for f in sorted(os.listdir(CSRC)):
+        if not f.endswith((".cu", ".cuh")):
+            continue
+        text = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, f)).read())
+        for m in re.finditer(r"__global__\s+(?:void\s+|__\w+__\s*\([^)]*\)\s*)+(\w+)\s*\(", text):
+            start = text.index("{", m.end())
+            depth = 0
+            for i in range(start, len(text)):
+                depth += {"{": 1, "}": -1}.get(text[i], 0)
+                if depth == 0:
+                    break
+            yield f + ":" + m.group(1), text[start:i + 1]
+
+
+def test_tensor_memory_is_taken_before_later_launches_may_start():
+    """A CTA that let the next launch start before it had its columns could wait for columns which that launch holds while it
+    waits for this one to end.  One helper does both in the safe order; nothing else may do either."""
+    bodies = dict(_kernels())
+    takers = {k for k, b in bodies.items() if "alloc_then_launch_dependents" in b}
+    assert len(takers) >= 8 and any("linear_tc_pair" in k for k in takers) and any("flash_tc" in k for k in takers), takers
+    for k in takers:
+        assert "pdl_launch_dependents" not in bodies[k], k
+    for k, b in bodies.items():
+        assert "tcgen05.alloc" not in b, k
+    helper = open(os.path.join(CSRC, "tc.cuh")).read()
+    at = helper.index("void alloc_then_launch_dependents")
+    body = helper[at:helper.index("\n}\n", at)]
+    assert body.rindex("tcgen05.alloc") < body.index("pdl_launch_dependents();")
+    for f in os.listdir(CSRC):
+        if f.endswith((".cu", ".cuh")) and f != "tc.cuh":
+            assert "tcgen05.alloc" not in open(os.path.join(CSRC, f)).read(), f
