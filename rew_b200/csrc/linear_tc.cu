@@ -19,8 +19,10 @@
 //            descriptors and releases the stage with tcgen05.commit.
 //   warps 2-9 epilogue: tcgen05.ld the accumulator (a warp owns 32 lanes),
 //            apply bias / SwiGLU, store.
-// All waits are bounded; on a timeout the roles fall through to the common
-// exit, where TMEM is released.
+// All waits on barriers are bounded; on a timeout the roles fall through to the
+// common exit, where TMEM is released.  tcgen05.alloc, the cluster barriers and
+// the stream dependency have no limit of their own: see
+// alloc_then_launch_dependents (tc.cuh) and kAllSmem for what ends them.
 #include <string.h>
 
 #include "act.cuh"
@@ -34,6 +36,9 @@ namespace {
 constexpr int BM = 128;  // output features per CTA
 constexpr int BK = 64;
 constexpr int A_BYTES = 2 * BK * 64 * 2;  // two 64x64 boxes
+// All the shared memory of an SM.  The kernels that take all of its tensor memory ask for all of this too, whatever their ring
+// needs: no CTA of a launch that starts early sits beside them.
+constexpr int kAllSmem = 227 * 1024;
 
 struct TcArgs {
   int64_t M, N, K;
@@ -469,10 +474,10 @@ struct PersistCfg {
   static constexpr int TMEM_COLS = 512;
   static constexpr int stage_bytes(int tn) { return A_BYTES + tn * 128; }
   static constexpr int stages(int tn) {
-    const int n = (227 * 1024 - FIXED) / stage_bytes(tn);
+    const int n = (SMEM - FIXED) / stage_bytes(tn);
     return n < MAX_STAGES ? n : MAX_STAGES;
   }
-  static constexpr int smem(int tn) { return stages(tn) * stage_bytes(tn) + FIXED; }
+  static constexpr int SMEM = kAllSmem;
 };
 
 // GROUPED: the weights are `groups` stacked matrices (3-D tensor map, third coordinate = group, e.g. the
@@ -709,7 +714,7 @@ struct PairCfg {
   static constexpr int STAGES = 6;
   static constexpr int B_BYTES = (TN / 2) * 128;          // this CTA's 128 tokens x 64 k
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;   // 32 KB
-  static constexpr int SMEM = 227 * 1024;                 // all of it: no CTA of another launch beside a pair's
+  static constexpr int SMEM = kAllSmem;
   static constexpr int TMEM_COLS = 512;
 };
 
@@ -976,14 +981,14 @@ int linear_tc_grouped_launch(Ctx* c, const LinearBf16Plan& plan, const bf16* x, 
   a.tn = PersistCfg::TN;
   static bool attr_set = false;
   if (!attr_set) {
-    RB_CUDA(cudaFuncSetAttribute(linear_tc_persist_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    RB_CUDA(cudaFuncSetAttribute(linear_tc_persist_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PersistCfg::SMEM));
     attr_set = true;
   }
   const int tiles_n = (int)((plan.N + BM - 1) / BM);
   // at most ceil(M / TN) + groups token tiles exist; one CTA per SM walks them
   const int64_t max_tiles = (int64_t)tiles_n * ((M + PersistCfg::TN - 1) / PersistCfg::TN + plan.groups);
   const int ctas = (int)std::min<int64_t>(std::min<int64_t>(max_tiles, c->sm_count), kMaxPersistCtas);
-  RB_CUDA(launch_k(linear_tc_persist_kernel<true>, dim3((unsigned)ctas), dim3(TC_THREADS), (size_t)PersistCfg::smem(a.tn), c->stream, c->use_pdl,
+  RB_CUDA(launch_k(linear_tc_persist_kernel<true>, dim3((unsigned)ctas), dim3(TC_THREADS), (size_t)PersistCfg::SMEM, c->stream, c->use_pdl,
                    plan.tmW, tmX, a, tiles_n, 0));
   ++g_launch_total;
   return REWB200_OK;
@@ -1054,20 +1059,20 @@ int linear_tc_launch(Ctx* c, const LinearBf16Plan& plan, const bf16* x, int64_t 
   if (c->prefill_persistent && !two) {
     static bool attr_set = false;
     if (!attr_set) {
-      RB_CUDA(cudaFuncSetAttribute(linear_tc_persist_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+      RB_CUDA(cudaFuncSetAttribute(linear_tc_persist_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, PersistCfg::SMEM));
       attr_set = true;
     }
     const int ctas = (int)std::min<int64_t>((int64_t)grid.x * grid.y * grid.z, c->sm_count);
-    RB_CUDA(launch_k(linear_tc_persist_kernel<false>, dim3((unsigned)ctas), dim3(TC_THREADS), (size_t)PersistCfg::smem(a.tn), c->stream, c->use_pdl, plan.tmW,
+    RB_CUDA(launch_k(linear_tc_persist_kernel<false>, dim3((unsigned)ctas), dim3(TC_THREADS), (size_t)PersistCfg::SMEM, c->stream, c->use_pdl, plan.tmW,
                      tmX, a, (int)grid.x, (int)grid.y));
     ++g_launch_total;
     return REWB200_OK;
   }
   using C = TcCfg<0>;
-  a.stages = std::min((int)C::MAX_STAGES, ((TN <= 160 ? 113 : 227) * 1024 - C::FIXED) / C::stage_bytes(TN));
+  a.stages = std::min((int)C::MAX_STAGES, ((TN <= 160 ? 113 * 1024 : kAllSmem) - C::FIXED) / C::stage_bytes(TN));
   static bool attr_set = false;
   if (!attr_set) {
-    RB_CUDA(cudaFuncSetAttribute(linear_tc_kernel<0, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    RB_CUDA(cudaFuncSetAttribute(linear_tc_kernel<0, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAllSmem));
     attr_set = true;
   }
   RB_CUDA(launch_k(linear_tc_kernel<0, 0>, grid, dim3(TC_THREADS), (size_t)(a.stages * C::stage_bytes(TN) + C::FIXED), c->stream, c->use_pdl, plan.tmW, tmX, a));

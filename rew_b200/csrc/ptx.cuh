@@ -1,7 +1,8 @@
 // Thin inline-PTX wrappers for sm_100a: mbarrier, TMA (cp.async.bulk.tensor,
 // never with cluster multicast), ldmatrix, mma.sync, programmatic dependent
-// launch.  Every wait is bounded: after kSpinLimit polls the waiter records an
-// error code in a status word and gives up, so a kernel can never hang the GPU.
+// launch.  Every wait on an mbarrier or a flag is bounded: after kSpinLimit polls
+// the waiter records an error code in a status word and gives up.  (The stream
+// dependency, cluster barriers and tcgen05.alloc have no limit of their own.)
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>

@@ -5,12 +5,17 @@ import re
 CSRC = os.path.join(os.path.dirname(os.path.abspath(__file__)), "..", "rew_b200", "csrc")
 
 
+def _source(f):
+    return re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, f)).read())
+
+
+FILES = sorted(f for f in os.listdir(CSRC) if f.endswith((".cu", ".cuh")))
+
+
 def _kernels():
-    """(name, body) of every __global__ function, with `//` comments taken out."""
-    for f in sorted(os.listdir(CSRC)):
-        if not f.endswith((".cu", ".cuh")):
-            continue
-        text = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, f)).read())
+    """(name, body) of every __global__ function."""
+    for f in FILES:
+        text = _source(f)
         for m in re.finditer(r"__global__\s+(?:void\s+|__\w+__\s*\([^)]*\)\s*)+(\w+)\s*\(", text):
             start = text.index("{", m.end())
             depth = 0
@@ -31,10 +36,23 @@ def test_tensor_memory_is_taken_before_later_launches_may_start():
         assert "pdl_launch_dependents" not in bodies[k], k
     for k, b in bodies.items():
         assert "tcgen05.alloc" not in b, k
-    helper = open(os.path.join(CSRC, "tc.cuh")).read()
+    helper = _source("tc.cuh")
     at = helper.index("void alloc_then_launch_dependents")
     body = helper[at:helper.index("\n}\n", at)]
     assert body.rindex("tcgen05.alloc") < body.index("pdl_launch_dependents();")
-    for f in os.listdir(CSRC):
-        if f.endswith((".cu", ".cuh")) and f != "tc.cuh":
-            assert "tcgen05.alloc" not in open(os.path.join(CSRC, f)).read(), f
+    for f in FILES:
+        assert f == "tc.cuh" or "tcgen05.alloc" not in _source(f), f
+
+
+def test_kernels_with_all_tensor_memory_of_an_sm_take_its_shared_memory_too():
+    """The persistent and the pair Linear hold 512 columns for a whole launch: no CTA that starts early may sit beside them."""
+    text = _source("linear_tc.cu")
+    assert re.search(r"kAllSmem = 227 \* 1024;", text)
+    cfgs = re.findall(r"struct (\w+Cfg) \{(.*?)\n\};", text, re.S)
+    wide = {n for n, body in cfgs if re.search(r"TMEM_COLS = 512;", body)}
+    assert wide == {"PersistCfg", "PairCfg"}
+    for n, body in cfgs:
+        if n in wide:
+            assert re.search(r"int SMEM = kAllSmem;", body), n
+    for call in re.findall(r"launch_k\((linear_tc_(?:persist|pair)_kernel.*?)\)\);", text, re.S):
+        assert re.search(r"\(size_t\)P\w+Cfg::SMEM,", call), call
