@@ -90,6 +90,7 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
   return r;
 }
 __device__ __forceinline__ void cluster_sync_all() {
+  __syncwarp();  // one arrival a warp: its lanes may come from different branches
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // address of the same shared-memory location in CTA `rank` of this cluster
@@ -408,13 +409,12 @@ __global__ void __launch_bounds__(TC_THREADS) linear_tc_kernel(const __grid_cons
     const int q = warp & 3, half = (warp - 2) >> 2;
     bool ok = true;
     if (nkb > 0) {
-      ok = mbar_wait(tmem_full, 0, a.status);
+      ok = mbar_wait_warp(tmem_full, 0, a.status);
       tc::fence_after();
     }
     pdl_wait();
     if constexpr (CL == 1) {
       // own partial tile -> shared memory as [token][feature] f32 (the pipeline stages are free by now)
-      ok = __all_sync(0xffffffffu, ok);  // the tensor-memory load below is warp-collective
       if (half == 0) {
         uint32_t r[32];
         if (ok && nkb > 0) {
@@ -675,7 +675,7 @@ __global__ void __launch_bounds__(TC_THREADS) linear_tc_persist_kernel(const __g
       k_range(t, kb0, nkb);
       const int col0 = tile_n * BM;
       const int buf = j & 1;
-      if (ok) ok = mbar_wait(&tmem_full[buf], (j >> 1) & 1, a.status);
+      if (ok) ok = mbar_wait_warp(&tmem_full[buf], (j >> 1) & 1, a.status);
       tc::fence_after();
       // grouped launches keep one bias row per group: [groups][N]
       void* const out = reinterpret_cast<uint8_t*>(a.out) + (GROUPED || a.epi != EPI_PARTIAL_F32 ? 0 : (size_t)(t / plane) * a.split_stride * 4);
@@ -870,7 +870,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS) linear_t
       const int col0 = tile_n * 256 + (int)rank * BM, row0 = tile_m * TN;
       const int rows_valid = (int)min((int64_t)TN, a.M - row0);
       const int buf = j & 1;
-      if (ok) ok = mbar_wait(&tmem_full[buf], (j >> 1) & 1, a.status);
+      if (ok) ok = mbar_wait_warp(&tmem_full[buf], (j >> 1) & 1, a.status);
       tc::fence_after();
       if (ok)
         store_tile(a, tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * TN), a.out, (int64_t)col0 + q * 32, lane, half,

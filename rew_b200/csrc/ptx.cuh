@@ -73,6 +73,12 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* s
   return false;
 }
 
+// The same by a whole warp, ahead of warp-collective instructions (tensor-memory loads, shuffles): its lanes leave together and agree.
+// A lane that gave up by itself would leave the others in a collective load without it, which has no limit.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, int* status) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, status));
+}
+
 __device__ __forceinline__ void tma_prefetch_desc(const void* tmap) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(tmap)) : "memory");
 }

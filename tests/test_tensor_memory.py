@@ -56,3 +56,12 @@ def test_kernels_with_all_tensor_memory_of_an_sm_take_its_shared_memory_too():
             assert re.search(r"int SMEM = kAllSmem;", body), n
     for call in re.findall(r"launch_k\((linear_tc_(?:persist|pair)_kernel.*?)\)\);", text, re.S):
         assert re.search(r"\(size_t\)P\w+Cfg::SMEM,", call), call
+
+
+def test_accumulators_are_waited_for_by_whole_warps():
+    """The way out of an accumulator reads tensor memory and trades values between lanes, both collective over the warp: its wait
+    ends with a vote, so that lanes which gave up cannot leave the others in there."""
+    text = _source("linear_tc.cu")
+    waits = re.findall(r"(\w+)\(&?tmem_full\b", text)
+    assert [w for w in waits if w.startswith("mbar_wait")] == ["mbar_wait_warp"] * 3, waits
+    assert re.search(r"bool mbar_wait_warp\([^)]*\) \{\s*return __all_sync\(0xffffffffu, mbar_wait\(", _source("ptx.cuh"))
