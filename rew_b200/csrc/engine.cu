@@ -673,8 +673,9 @@ int fetch_logits(rewb200_session* s, int64_t rows, float* host) {
   return REWB200_OK;
 }
 
-// Portions that share an attention launch: the choice of kernel follows a portion's own length, as if it stood alone
-// (128 tokens and more: tcgen05; fewer: mma.sync; one: split-KV decode), so its numbers do not depend on its neighbours.
+// Portions that share an attention launch: the choice of its kernel follows a portion's own length, as if it stood alone
+// (128 tokens and more: tcgen05; fewer: mma.sync; one: split-KV decode).  What follows the step instead: the pieces a Linear is
+// cut into along K (up to 256 rows of the step) and the KV splits of single tokens, both f32 sums in another order.
 enum PortionKind : int { PORTION_LONG = 0, PORTION_SHORT, PORTION_SINGLE };
 PortionKind portion_kind(int n) { return n >= 128 ? PORTION_LONG : n > 1 ? PORTION_SHORT : PORTION_SINGLE; }
 
@@ -710,7 +711,11 @@ int gqa_blocks(rewb200_session* s, const FwdOpts& o, const NormArgs& na, int64_t
                        (size_t)rows * d * dtype_size(dt) * 2 <= pi->buf_bytes && pi->world == cf.tp_size;
   // (steps above 256 rows never split K, so a bf16 model's o / down projections write one bf16 slab there on one GPU
   // too: half the bytes between the GEMM and the residual+norm kernel, rounded where the reference's bf16 Linear rounds)
-  const bool tp_bf16_slab = (cf.tp_size > 1 ? rows > 64 : (rows > 256 && cf.n_routed == 0)) && !oneshot && dt == REWB200_BF16 && d % 4 == 0;  // smaller steps keep split-K slabs
+  // ... a portion of up to 256 rows keeps the f32 slab it has alone, whatever the step's other portions bring
+  int64_t alone = rows;
+  if (portions)
+    for (const StepEntry& e : *o.entries) alone = std::min<int64_t>(alone, e.n);
+  const bool tp_bf16_slab = (cf.tp_size > 1 ? rows > 64 : (alone > 256 && cf.n_routed == 0)) && !oneshot && dt == REWB200_BF16 && d % 4 == 0;  // smaller steps keep split-K slabs
   // ... and when the heap's bulk region holds a scatter and a gather buffer of the step, the sum itself runs
   // over the heap too (two-shot: reduce-scatter and all-gather by peer stores) instead of through NCCL
   const size_t pay = dtype_size(dt);

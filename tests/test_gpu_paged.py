@@ -173,3 +173,31 @@ def test_routing_of_a_step_of_portions_in_the_callers_order(rb):
             assert np.array_equal(got[layer], np.concatenate(alone[layer]))
     finally:
         rb.set_option("record_routing", "0")
+
+
+def test_short_portions_keep_f32_sums_beside_long_ones(rb, orc):
+    """The outputs of o and down reach the residual unrounded for every portion of up to 256 tokens, also when its neighbours bring the
+    step above that.  A model made to tell: embeddings of +-64, zero queries, keys and feed-forward, values that pass the
+    normed token on and an output matrix of -64 on its diagonal, so that a first token's residual is only what the small rest of
+    that matrix adds: multiples of 2^-6 below 2, exact in f32, lost to a bf16 spacing of 2^-2 at 64."""
+    from rew_b200 import _lib
+    d = 128
+    cfg = W.ModelConfig(vocab=64, d_model=d, n_layers=1, n_heads=2, n_kv_heads=2, head_dim=64, ffn=64, max_seq=512, dtype=_lib.BF16, mask_kind=1)
+    rng = np.random.default_rng(0)
+    sign = lambda *s: np.where(rng.random(s) < 0.5, -1.0, 1.0).astype(np.float32)
+    zero, layer = np.zeros((d, d), np.float32), "model.layers.0."
+    off = (1 - np.eye(d, dtype=np.float32)) * sign(d, d)
+    made = {"model.embedTokens.weight": 64 * sign(cfg.vocab, d), layer + "mlp.downProj.weight": np.zeros((cfg.ffn, d), np.float32),
+            layer + "selfAttn.qProj.weight": zero, layer + "selfAttn.kProj.weight": zero, layer + "selfAttn.vProj.weight": np.eye(d, dtype=np.float32),
+            layer + "selfAttn.outProj.weight": off / 64 - 64 * np.eye(d, dtype=np.float32)}
+    t = [made.pop(name, a) for (name, _), a in zip(W.tensor_specs(cfg), W.init_weights(cfg, seed=1, std=0.1))]
+    assert not made
+    t = [orc.bf16_round(a) if a.ndim == 2 else a for a in t]
+    sess = rb.CausalLM(cfg).load(t).paged_session(5, 400, 40)
+    portions = [(l, rng.integers(0, cfg.vocab, n).astype(np.int32)) for l, n in ((2, 1), (0, 300), (4, 1), (1, 1), (3, 257))]
+    ends = np.cumsum([len(ids) for _, ids in portions]) - 1
+    singles = [i for i, (_, ids) in enumerate(portions) if len(ids) == 1]
+    logits, _ = sess.feed(portions, want=[int(ends[i]) for i in singles])
+    for got, i in zip(logits, singles):
+        want = orc.model_forward(cfg, t, portions[i][1][None], 0, True)[0, -1]
+        assert np.linalg.norm(got - want) <= 2e-2 * np.linalg.norm(want)
