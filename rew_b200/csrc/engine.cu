@@ -2118,7 +2118,10 @@ int rewb200_lanes_feed(rewb200_session* s, int n_entries, const int32_t* lanes, 
       act[lanes[e]] = 1;
       any_sample = true;
     }
-  // A grouped-query step runs its portions in the order of their kinds; a layered one in the caller's.
+  // A grouped-query step runs its portions in the order of their kinds; a layered one in the caller's.  One portion alone
+  // needs no tables: it runs as an admitted prompt does, with q, k and v finished in the Linear or the attention where
+  // those can, and one row for the lm_head.
+  const bool alone = !m->layered && n_entries == 1;
   if (!m->layered) {
     std::stable_sort(entries.begin(), entries.end(), [](const StepEntry& x, const StepEntry& y) { return portion_kind(x.n) < portion_kind(y.n); });
     int row = 0;
@@ -2128,7 +2131,7 @@ int rewb200_lanes_feed(rewb200_session* s, int n_entries, const int32_t* lanes, 
       row += e.n;
     }
   }
-  // one upload: ids | rows of the lm_head (wanted places, then every lane's last row) | sampled lanes | portions and their pages |
+  // one upload: ids | rows of the lm_head (wanted places, then every lane's last row, or the one portion's) | sampled lanes | portions and their pages |
   // and for grouped-query models the rows and positions of the portions
   const size_t at_rows = (size_t)rows, at_act = at_rows + n_want + s->B, at_port = (at_act + s->B + 3) / 4 * 4,
                at_seq = at_port + 4 * (size_t)n_entries, at_pos = at_seq + 2 * (size_t)n_entries, at_pages = at_pos + n_entries,
@@ -2140,7 +2143,7 @@ int rewb200_lanes_feed(rewb200_session* s, int n_entries, const int32_t* lanes, 
     memcpy(up.data() + e.row0, ids + e.src, (size_t)e.n * sizeof(int));
     for (int i = 0; i < n_want; ++i)
       if (want[i] >= e.src && want[i] < e.src + e.n) up[at_rows + i] = e.row0 + want[i] - e.src;
-    up[at_rows + n_want + e.lane] = e.row0 + e.n - 1;
+    up[at_rows + n_want + (alone ? 0 : e.lane)] = e.row0 + e.n - 1;
     const int port[4] = {e.lane, e.pos0, e.n, 0}, seq[2] = {e.row0, e.n};
     memcpy(up.data() + at_port + 4 * k, port, sizeof(port));
     memcpy(up.data() + at_seq + 2 * k, seq, sizeof(seq));
@@ -2185,17 +2188,23 @@ int rewb200_lanes_feed(rewb200_session* s, int n_entries, const int32_t* lanes, 
   }
   RB_CUDA(cudaEventRecord(s->ev0, c->stream));
   FwdOpts o;
-  o.entries = &entries;
   o.ids_src = s->feed_dev;
   o.record_out = false;
   o.out_rows = s->feed_dev + at_rows;
   o.n_want = n_want;
   o.sample = any_sample;
-  o.sample_active = s->feed_dev + at_act;
   o.advance = 0;
+  if (alone) {
+    o.S = entries[0].n;
+    o.b0 = entries[0].lane;
+    o.nb = 1;
+  } else {
+    o.entries = &entries;
+    o.sample_active = s->feed_dev + at_act;
+  }
   if (m->layered) {
     RB_TRY(layered_prepare(s, o, rows));
-  } else {
+  } else if (!alone) {
     o.seq = reinterpret_cast<const int2*>(s->feed_dev + at_seq);
     o.seq_pos = s->feed_dev + at_pos;
     o.seq_pages = s->feed_dev + at_pages;

@@ -201,3 +201,23 @@ def test_short_portions_keep_f32_sums_beside_long_ones(rb, orc):
     for got, i in zip(logits, singles):
         want = orc.model_forward(cfg, t, portions[i][1][None], 0, True)[0, -1]
         assert np.linalg.norm(got - want) <= 2e-2 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("S", [1, 20, 64, 300])
+def test_feed_of_one_portion_costs_what_a_plain_step_does(rb, S):
+    """A step of one portion on a grouped-query model: the bits and the launches of a plain session's step of the same tokens, besides the
+    lane tables ahead of it and behind it and the row gathered for the lm_head; then the same for one more token."""
+    from rew_b200 import _lib
+    cfg = W.ModelConfig(vocab=128, d_model=256, n_layers=5, n_heads=4, n_kv_heads=2, head_dim=64, ffn=512, max_seq=512, dtype=_lib.BF16, mask_kind=1)
+    model = rb.CausalLM(cfg).load(W.init_weights(cfg, seed=5, std=0.08))
+    plain, paged = model.session(1, 400), model.paged_session(9, 400, 20)
+    launches = lambda: _lib.lib().rewb200_launch_count(0)
+    paged.feed([(l, np.arange(3, dtype=np.int32)) for l in (2, 8)])
+    for ids in (np.random.default_rng(S).integers(0, cfg.vocab, S).astype(np.int32), np.array([7], np.int32)):
+        n0 = launches()
+        nxt, want = plain.forward(ids[None], want_logits=True)
+        n1 = launches()
+        logits, got = paged.feed([(5, ids)], want=[len(ids) - 1], sample=True)
+        n2 = launches()
+        assert np.array_equal(logits, want) and got[0] == nxt[0]
+        assert n2 - n1 <= n1 - n0 + 3
