@@ -1305,11 +1305,13 @@ int attn_launch(Ctx* c, const AttnArgs& h) {
       dim3 pgrid((unsigned)((h.S + fa2::BQ - 1) / fa2::BQ), (unsigned)h.nh, (unsigned)h.B);
       RB_CUDA(launch_k(attn_prefill_tc2_kernel, pgrid, dim3(fa2::THREADS), (size_t)fa2::SMEM, c->stream, c->use_pdl, *h.tmK, *h.tmV, a));
       ++g_launch_total;
+      ++g_route_launches[ROUTE_ATTENTION_TC2];
       return REWB200_OK;
     }
     dim3 tgrid((unsigned)((h.S + fa::BQ - 1) / fa::BQ), (unsigned)h.nh, (unsigned)h.B);
     RB_CUDA(launch_k(attn_prefill_tc_kernel, tgrid, dim3(fa::THREADS), (size_t)fa::SMEM, c->stream, c->use_pdl, *h.tmK, *h.tmV, a));
     ++g_launch_total;
+    ++g_route_launches[ROUTE_ATTENTION_TC];
     return REWB200_OK;
   }
   dim3 grid((unsigned)((h.S + 63) / 64), (unsigned)h.nh, (unsigned)h.B);

@@ -22,6 +22,7 @@ namespace cg = cooperative_groups;
 namespace rewb {
 
 int64_t g_launch_total = 0;
+int64_t g_route_launches[N_ROUTES] = {};
 
 namespace {
 

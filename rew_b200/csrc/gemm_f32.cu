@@ -132,6 +132,7 @@ int launch_rows(Ctx* c, const float* A, int64_t lda, const float* B, int64_t ldb
     const dim3 grid((unsigned)((N + COLS - 1) / COLS), (unsigned)((M + mr - 1) / mr));
     RB_CUDA(launch_k(kernel, grid, dim3(256), 0, c->stream, c->use_pdl, A, B, bias, C, M, K, N, lda, ldb, ldc));
     ++g_launch_total;
+    ++g_route_launches[ROUTE_F32_ROWS];
     return REWB200_OK;
   };
   if (M == 1) return go(gemm_f32_rows_kernel<1, COLS>, 1);
@@ -157,6 +158,7 @@ int gemm_f32_ld_launch(Ctx* c, const float* A, int64_t lda, const float* B, int6
   dim3 grid((unsigned)((N + TN - 1) / TN), (unsigned)((M + TM - 1) / TM));
   RB_CUDA(launch_k(gemm_f32_kernel, grid, dim3(256), 0, c->stream, c->use_pdl, A, B, bias, C, M, K, N, lda, ldb, ldc));
   ++g_launch_total;
+  ++g_route_launches[ROUTE_F32_TILES];
   return REWB200_OK;
 }
 

@@ -901,6 +901,7 @@ int launch_tn(Ctx* c, const LinearBf16Plan& plan, const CUtensorMap& tmX, const 
   }
   RB_CUDA(launch_k(linear_tc_kernel<TN, 0>, grid, dim3(TC_THREADS), (size_t)C::SMEM, c->stream, c->use_pdl, plan.tmW, tmX, a));
   ++g_launch_total;
+  ++g_route_launches[ROUTE_LINEAR_TILE];
   return REWB200_OK;
 }
 
@@ -1047,6 +1048,7 @@ int linear_tc_launch(Ctx* c, const LinearBf16Plan& plan, const bf16* x, int64_t 
     RB_CUDA(launch_k(linear_tc_pair_kernel, dim3((unsigned)(ctas & ~1)), dim3(TC_THREADS), (size_t)PairCfg::SMEM, c->stream, c->use_pdl,
                      plan.tmW, tmXh, a, tiles_n, tiles_m));
     ++g_launch_total;
+    ++g_route_launches[ROUTE_LINEAR_PAIR];
     return REWB200_OK;
   }
   CUtensorMap tmX;
@@ -1066,6 +1068,7 @@ int linear_tc_launch(Ctx* c, const LinearBf16Plan& plan, const bf16* x, int64_t 
     RB_CUDA(launch_k(linear_tc_persist_kernel<false>, dim3((unsigned)ctas), dim3(TC_THREADS), (size_t)PersistCfg::SMEM, c->stream, c->use_pdl, plan.tmW,
                      tmX, a, (int)grid.x, (int)grid.y));
     ++g_launch_total;
+    ++g_route_launches[ROUTE_LINEAR_PERSISTENT];
     return REWB200_OK;
   }
   using C = TcCfg<0>;
@@ -1077,6 +1080,7 @@ int linear_tc_launch(Ctx* c, const LinearBf16Plan& plan, const bf16* x, int64_t 
   }
   RB_CUDA(launch_k(linear_tc_kernel<0, 0>, grid, dim3(TC_THREADS), (size_t)(a.stages * C::stage_bytes(TN) + C::FIXED), c->stream, c->use_pdl, plan.tmW, tmX, a));
   ++g_launch_total;
+  ++g_route_launches[ROUTE_LINEAR_TILE];
   return REWB200_OK;
 }
 

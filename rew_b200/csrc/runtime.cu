@@ -348,6 +348,13 @@ int64_t rewb200_launch_count(int slot) {
   return g_launch_total;
 }
 
+int64_t rewb200_kernel_launches(const char* kernel) {
+  static const char* const names[N_ROUTES] = {"linear_tile", "linear_persistent", "linear_pair", "f32_rows", "f32_tiles", "attention_tc", "attention_tc2"};
+  for (int i = 0; kernel && i < N_ROUTES; ++i)
+    if (!strcmp(kernel, names[i])) return g_route_launches[i];
+  return -1;
+}
+
 int rewb200_buffer_alloc(int slot, int dtype, const int64_t* dims, int ndims, rewb200_buffer** out) {
   Ctx* c = ctx_get(slot);
   if (!c) return REWB200_ERR;

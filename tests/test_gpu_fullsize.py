@@ -152,14 +152,14 @@ def test_full_size_moe_prefill_grouped_gemm_kernels_agree(rb):
 
 
 def test_full_size_prefill_kernel_variants_return_the_same_bits(rb):
-    """Llama-3-8B shape, 8 x 512-token prompts: the prefill with the two-CTA Linear (default), the one-CTA persistent
+    """Llama-3-8B shape, 16 x 512-token prompts: the prefill with the two-CTA Linear (default), the one-CTA persistent
     Linear and the one-tile Linear, and with one or two query tiles per CTA in the attention kernel.  All variants
     issue the same products in the same order and share their epilogue and softmax arithmetic: identical logits."""
     cfg = W.llama3_8b()
     cfg.max_seq = 640
     model = rb.CausalLM(cfg).init_random(seed=25, std=0.02)
     try:
-        B, S = 8, 512
+        B, S = 16, 512
         prompt = np.random.default_rng(9).integers(0, cfg.vocab, size=(B, S)).astype(np.int32)
 
         def run(**opts):
@@ -174,10 +174,16 @@ def test_full_size_prefill_kernel_variants_return_the_same_bits(rb):
                 rb.set_option("prefill", "pair")
                 rb.set_option("attention", "tc")
 
+        from rew_b200 import _lib
+        count = lambda kernel: _lib.lib().rewb200_kernel_launches(kernel.encode())
+        before = count("linear_pair")
         base = run()
-        assert np.isfinite(base).all()
-        for opts in ({"prefill": "persistent"}, {"prefill": "tile"}, {"attention": "tc2"}, {"attention": "tc1"}):
+        assert np.isfinite(base).all() and count("linear_pair") - before == 4 * cfg.n_layers
+        for opts, kernel in (({"prefill": "persistent"}, "linear_persistent"), ({"prefill": "tile"}, "linear_tile"),
+                             ({"attention": "tc2"}, "attention_tc2"), ({"attention": "tc1"}, "attention_tc")):
+            before = count(kernel)
             assert np.array_equal(run(**opts), base), opts
+            assert count(kernel) - before >= cfg.n_layers, opts
     finally:
         model.free()
 

@@ -130,12 +130,19 @@ def test_persistent_prefill_linear_matches_oracle(rb_tc, orc):
     assert np.array_equal(got, again)   # same MMA order, same rounding: the two kernels agree bit for bit
 
 
-@pytest.mark.parametrize("M,K,N,epi_bias", [(4100, 320, 2560, True), (8192, 1024, 1024, False), (5000, 64, 512, True)])
-def test_pair_prefill_linear_matches_oracle_and_the_one_cta_kernels(rb_tc, orc, M, K, N, epi_bias):
-    """Widths that are multiples of 256 with at least two 256-token tiles per SM run on pairs of CTAs
-    (tcgen05 cta_group::2, 256 x 256 tiles, each CTA staging half of either operand).  Ragged last token tile,
-    a single 64-row k block, more tiles than pairs: against the oracle, and bit for bit against the one-CTA
-    persistent kernel and the one-tile kernel (the same k order and the same rounding)."""
+def _launches():
+    from rew_b200 import _lib
+    return {k: _lib.lib().rewb200_kernel_launches(("linear_" + k).encode()) for k in ("tile", "persistent", "pair")}
+
+
+@pytest.mark.parametrize("M,K,N,epi_bias,pair", [(4100, 320, 2560, True, False), (8192, 1024, 1024, False, False), (5000, 64, 512, True, False),
+                                                 (8200, 320, 2560, True, True), (8449, 64, 2304, True, True), (9000, 1024, 2304, False, True)])
+def test_pair_prefill_linear_matches_oracle_and_the_one_cta_kernels(rb_tc, orc, M, K, N, epi_bias, pair):
+    """Large launches of widths that are multiples of 256 run on pairs of CTAs
+    (tcgen05 cta_group::2, 256 x 256 tiles, each CTA staging half of either operand).  Ragged last token tile
+    (8 rows and one), a single 64-row k block, more tiles than pairs: against the oracle, and bit for bit against the one-CTA
+    persistent kernel and the one-tile kernel (the same k order and the same rounding).  Smaller launches the same way,
+    on the kernel that they run on."""
     from rew_b200 import _lib
     rng = np.random.default_rng(M + N)
     x = orc.bf16_round(rng.normal(size=(M, K)))
@@ -144,14 +151,18 @@ def test_pair_prefill_linear_matches_oracle_and_the_one_cta_kernels(rb_tc, orc, 
     want = orc.linear(x, w, b)
     T = rb_tc.Tensor.from_host
     lin = rb_tc.Linear(T(w, _lib.BF16), T(b))
+    before = _launches()
     got = lin.forward(T(x, _lib.BF16)).to_host()
+    assert _launches()["pair"] - before["pair"] == pair
     assert rel_l2(got, want) < 5e-3
     assert max(rel_l2(got[r], want[r]) for r in (0, 127, 128, 255, 256, M // 2, M - 1)) < 2e-2
     others = {}
     for how in ("persistent", "tile"):
         rb_tc.set_option("prefill", how)
         try:
+            before = _launches()
             others[how] = lin.forward(T(x, _lib.BF16)).to_host()
+            assert _launches()[how] == before[how] + 1
         finally:
             rb_tc.set_option("prefill", "pair")
     assert np.array_equal(others["persistent"], others["tile"])
