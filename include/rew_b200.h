@@ -65,7 +65,7 @@ int rewb200_sync(int slot, int timeout_ms);
  *                                            rows, or on tcgen05 always   (REW_B200_LINEAR)
  *   "pdl"    = "0" | "1"                     programmatic dependent launch (REW_B200_PDL)
  *   "prefill" = "pair" | "persistent" | "tile"   Linear launches of 256-token tiles: persistent CTA pairs on 256 x 256 tiles
- *                                            (tcgen05 cta_group::2; default, widths that are multiples of 256), one
+ *                                            (tcgen05 cta_group::2; default, large launches of widths that are multiples of 256), one
  *                                            persistent CTA per SM with the epilogue overlapped, or one CTA per tile
  *   "profile_linears" = "1".."31"            which launches rewb200_session_profile_linears times: bit 0 q|k|v, 1 o,
  *                                            2 gate|up, 3 down, 4 lm_head (default 31, all)

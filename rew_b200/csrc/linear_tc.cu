@@ -1031,10 +1031,12 @@ int linear_tc_launch(Ctx* c, const LinearBf16Plan& plan, const bf16* x, int64_t 
   a.early_w = plan.early_w;
   a.tn = TN;
   dim3 grid((unsigned)((plan.N + BM - 1) / BM), (unsigned)((M + TN - 1) / TN), (unsigned)ksplit);
-  // Pairs of CTAs where a launch runs long enough for the power cap to set the pace (six layers of the 8B shape, 16 384 tokens:
-  // 42.6 against 45.0 ms); below that one CTA a tile is ahead (4096 x 28672: 4096 tokens 638 against 674 us, 512 97 against 103).
-  if (M >= 8192 && ksplit == 1 && c->prefill_persistent && c->prefill_pair && plan.N % 256 == 0 && c->sm_count % 2 == 0 &&
-      (int64_t)grid.x * token_tiles >= 2 * (int64_t)c->sm_count) {
+  // Pairs of CTAs from four tiles an SM on, where their half of the shared-memory traffic counts: 1 to 4 per cent ahead of one CTA
+  // a tile (us, pairs / one CTA: 4096 x 28672, 1024 rows 200 / 204; 2048 x 11264, 3072 rows 119 / 122; 14336 x 4096, 6144 rows
+  // 616 / 638; 5632 x 2048, 12 288 rows 240 / 249).  With fewer tiles the last wave decides, which is coarser in pairs (4096 x 6144,
+  // 2048 rows, 384 tiles 102 / 99; 2048 x 3072, 4096 rows, 384 tiles 57 / 55).  Below 1024 rows tiles of the step's own size win.
+  if (M >= 1024 && ksplit == 1 && c->prefill_persistent && c->prefill_pair && plan.N % 256 == 0 && c->sm_count % 2 == 0 &&
+      (int64_t)grid.x * token_tiles >= 4 * (int64_t)c->sm_count) {
     // two-CTA tiles: 256 features x 256 tokens per pair of SMs
     CUtensorMap tmXh;
     RB_TRY(make_tmap_2d_bf16(&tmXh, x, (uint64_t)plan.K, (uint64_t)M, (uint64_t)ldx * 2, 64, PairCfg::TN / 2));

@@ -136,7 +136,7 @@ def _launches():
 
 
 @pytest.mark.parametrize("M,K,N,epi_bias,pair", [(4100, 320, 2560, True, False), (8192, 1024, 1024, False, False), (5000, 64, 512, True, False),
-                                                 (8200, 320, 2560, True, True), (8449, 64, 2304, True, True), (9000, 1024, 2304, False, True)])
+                                                 (1025, 200, 15360, True, True), (4100, 320, 4608, True, True), (8200, 320, 2560, True, True), (8449, 64, 2304, True, True), (9000, 1024, 2304, False, True)])
 def test_pair_prefill_linear_matches_oracle_and_the_one_cta_kernels(rb_tc, orc, M, K, N, epi_bias, pair):
     """Large launches of widths that are multiples of 256 run on pairs of CTAs
     (tcgen05 cta_group::2, 256 x 256 tiles, each CTA staging half of either operand).  Ragged last token tile
@@ -170,8 +170,8 @@ def test_pair_prefill_linear_matches_oracle_and_the_one_cta_kernels(rb_tc, orc, 
 
 
 def test_persistent_prefill_model_equals_tile_kernel(rb_tc):
-    """A 20 480-token prefill puts every decoder Linear (f32 partial, SwiGLU and bf16 epilogues) on the
-    persistent kernel; the logits must equal those of the one-tile-per-CTA kernel exactly."""
+    """A 20 480-token prefill puts the decoder Linears (f32 partial and bf16 epilogues) on the persistent kernel and gate and up
+    (SwiGLU) on the pair kernel; the logits must equal those of the one-tile-per-CTA kernel exactly."""
     from rew_b200 import _lib
     cfg = W.ModelConfig(vocab=512, d_model=512, n_layers=2, n_heads=8, n_kv_heads=2, head_dim=64, ffn=1408, max_seq=640,
                         theta=500000.0, dtype=_lib.BF16, mask_kind=1)
@@ -179,7 +179,10 @@ def test_persistent_prefill_model_equals_tile_kernel(rb_tc):
     B, S = 40, 512
     prompt = np.random.default_rng(1).integers(0, cfg.vocab, size=(B, S)).astype(np.int32)
     sess = model.session(B, S + 8)
+    before = _launches()
     _, a = sess.forward(prompt, want_logits=True)
+    ran = {k: n - before[k] for k, n in _launches().items()}
+    assert ran["persistent"] == 3 * cfg.n_layers and ran["pair"] == cfg.n_layers, ran
     rb_tc.set_option("prefill", "tile")
     try:
         sess.reset()
