@@ -147,8 +147,11 @@ int launch_rows(Ctx* c, const float* A, int64_t lda, const float* B, int64_t ldb
 int gemm_f32_ld_launch(Ctx* c, const float* A, int64_t lda, const float* B, int64_t ldb, const float* bias, float* C, int64_t ldc,
                        int64_t M, int64_t K, int64_t N) {
   if (M == 0 || N == 0) return REWB200_OK;
-  // Up to 512 rows: at 1024 the tiles have caught up (768 x 4128: 444 us here, 453 us there; 512 rows 233 and 417 us).
-  if (M <= 512) {
+  // Up to 512 rows, unless 64x64 tiles give every SM eleven or more, which hide one another's barriers: us, rows / tiles,
+  // 1024 x 16384: 384 rows (1536 tiles) 855 / 885, 512 rows (2048) 1129 / 1030; 512 rows of 768 x 4128 (520) 232 / 415, of
+  // 2048 x 6144 (768) 815 / 1153, of 4096 x 4096 (512) 1216 / 2209, of 64 x 96 (16) 6 / 14.  Above 512 rows 768 x 4128 is even at 1024
+  // (444 / 453).
+  if (M <= 512 && ((M + TM - 1) / TM) * ((N + TN - 1) / TN) < 11 * (int64_t)c->sm_count) {
     const int64_t groups = (M + 15) / 16, strips = (N + 31) / 32;
     // Narrow strips while one group of rows, or fewer wide strips than two thirds of the SMs, would leave the chip idle:
     // 4096 x 4096, 1 row 57 against 161 us; 2064 x 768, 64 rows 61 against 106 us; 256 x 1376, 33 rows (129 strips) 8.9 against 6.9 us.

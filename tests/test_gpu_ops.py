@@ -293,6 +293,20 @@ def test_attention_bf16_prefill_tcgen05(rb, orc, B, nh, kvh, S, L, mode):
     assert np.array_equal(got, two_tiles)
 
 
+@pytest.mark.parametrize("M,N,kernel", [(512, 12928, "f32_rows"), (512, 16384, "f32_tiles"), (448, 16384, "f32_tiles"), (384, 16384, "f32_rows"), (513, 64, "f32_tiles")])
+def test_f32_linear_of_many_tiles(rb, M, N, kernel):
+    """Rows and columns enough for eleven 64x64 tiles an SM leave the row kernel.  Bound as below."""
+    from rew_b200 import _lib
+    K, rng = 67, np.random.default_rng(M)
+    x, w, b = rng.normal(size=(M, K)).astype(np.float32), rng.normal(size=(K, N)).astype(np.float32), rng.normal(size=N).astype(np.float32)
+    lin, tx = rb.Linear(T(rb, w), T(rb, b)), T(rb, x)
+    before = _lib.lib().rewb200_kernel_launches(kernel.encode())
+    y = lin.forward(tx).to_host()
+    assert _lib.lib().rewb200_kernel_launches(kernel.encode()) == before + 1
+    want = x.astype(np.float64) @ w + b
+    assert np.all(np.abs(y - want) <= (K + 1) * 2.0 ** -24 * (np.abs(x).astype(np.float64) @ np.abs(w) + np.abs(b)))
+
+
 @pytest.mark.parametrize("M,K,N", [(1, 1, 1), (2, 3, 7), (3, 4, 8), (5, 511, 9), (8, 512, 33), (9, 513, 31), (16, 1025, 100), (17, 515, 1376),
                                    (64, 96, 1024), (512, 70, 65), (513, 70, 65)])
 def test_f32_linear_row_groups_and_strips(rb, M, K, N):
