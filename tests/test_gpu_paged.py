@@ -221,3 +221,57 @@ def test_feed_of_one_portion_costs_what_a_plain_step_does(rb, S):
         n2 = launches()
         assert np.array_equal(logits, want) and got[0] == nxt[0]
         assert n2 - n1 <= n1 - n0 + 3
+
+
+def test_feed_with_sampling_and_seeds_in_any_order(rb, orc):
+    """Portions on a grouped-query model, sorted by kind inside the step, each lane with a seed of its own: the tokens of the oracle's
+    sampled generation of every lane alone, whatever order the lanes are given in and however a prompt is cut."""
+    cfg = W.tiny_llama(norm_kind=0, mask_kind=1)
+    t = W.init_weights(cfg, seed=23)
+    kw = dict(temperature=1.1, top_k=0, top_p=0.9, repetition_penalty=1.1)
+    rng = np.random.default_rng(6)
+    prompts = [rng.integers(0, cfg.vocab, n).astype(np.int32) for n in (40, 1, 65, 9)]
+    seeds = [900, 31, 7, 4000]
+    sess = rb.CausalLM(cfg).load(t).paged_session(4, 112, 12)
+    sess.set_sampling(**kw)
+    n_new, out = 8, [[] for _ in prompts]
+    # the first step: lanes 2, 1, 3 and 0, of which lane 0 brings only a part of its prompt and lane 3 only its first token
+    first = [(2, prompts[2]), (1, prompts[1]), (3, prompts[3][:1]), (0, prompts[0][:30])]
+    _, nxt = sess.feed(first, sample=[True, True, False, False], seeds=[seeds[l] for l, _ in first])
+    assert nxt[2] == -1 and nxt[3] == -1
+    out[2].append(int(nxt[0])), out[1].append(int(nxt[1]))
+    step = 0
+    while any(len(o) < n_new for o in out):
+        portions = [(l, np.array([out[l][-1]], np.int32) if out[l] else (prompts[0][30:] if l == 0 else prompts[3][1:]))
+                    for l in rng.permutation(4) if len(out[l]) < n_new]
+        _, nxt = sess.feed(portions, sample=True, seeds=[55 + step] * len(portions))   # seeds count only for a lane's first portion
+        for (l, _), tok in zip(portions, nxt):
+            out[l].append(int(tok))
+        step += 1
+    for l, p in enumerate(prompts):
+        want, _ = orc.generate_sampled(cfg, t, p[None], n_new, seeds=[seeds[l]], **kw)
+        assert out[l] == want[0].tolist(), l
+
+
+def test_feed_of_long_portions_with_two_query_tiles_a_cta(rb):
+    """Portions of unequal length through the attention kernel of two query tiles a CTA (one to three tiles of 256, full and ragged):
+    the bits of the kernel with one, in one step and on top of contexts of different lengths."""
+    from rew_b200 import _lib
+    cfg = W.ModelConfig(vocab=128, d_model=256, n_layers=2, n_heads=4, n_kv_heads=2, head_dim=128, ffn=256, max_seq=1024, theta=10000.0,
+                        dtype=_lib.BF16, mask_kind=1)
+    model = rb.CausalLM(cfg).load(W.init_weights(cfg, seed=3, std=0.08))
+    rng = np.random.default_rng(12)
+    steps = [[(l, rng.integers(0, cfg.vocab, n).astype(np.int32)) for l, n in step]
+             for step in (((2, 600), (0, 128), (3, 257), (1, 1), (4, 512)), ((1, 300), (3, 129), (4, 2), (0, 256)))]
+    runs = {}
+    for how, kernel in (("tc1", "attention_tc"), ("tc2", "attention_tc2")):
+        rb.set_option("attention", how)
+        try:
+            sess = model.paged_session(5, 1000, 60)
+            before = _lib.lib().rewb200_kernel_launches(kernel.encode())
+            runs[how] = [sess.feed(p, want=range(0, sum(len(ids) for _, ids in p), 7), sample=True) for p in steps]
+            assert _lib.lib().rewb200_kernel_launches(kernel.encode()) - before == 2 * cfg.n_layers
+        finally:
+            rb.set_option("attention", "tc")
+    for (a, x), (b, y) in zip(runs["tc1"], runs["tc2"]):
+        assert np.isfinite(a).all() and np.array_equal(a, b) and np.array_equal(x, y)
