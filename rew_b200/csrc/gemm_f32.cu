@@ -62,8 +62,9 @@ __global__ void __launch_bounds__(256) gemm_f32_kernel(const float* __restrict__
 // columns; its 256 threads are COLS columns x KL = 256 / COLS places along K, so that a strip 256 deep is in flight at once
 // where the 64x64 tile walks K sixteen at a time behind two barriers.  The rows of A are staged KC at a time and read four
 // k at a time by broadcast.  Partial sums meet in shared memory and are added pairwise in a fixed order, which also leaves
-// less rounding than one long chain (2048 deep: 1.6e-7 relative against 8e-7 of the tiles).  256 x 384, 1 row: 2.9 us
-// (91 us in 64x64 tiles), 768 x 4128, 8 rows: 10.7 us (381 us).
+// less rounding than one long chain (2048 deep: 1.6e-7 relative against 8e-7 of the tiles).  The order is that of the strip's
+// width, 8 or 32 columns, and so follows the rows of the call.  256 x 384, 1 row: 2.9 us (91 us in 64x64 tiles), 768 x 4128,
+// 8 rows: 10.7 us (381 us).
 constexpr int KC = 512;
 
 template <int MR, int COLS>
