@@ -918,7 +918,7 @@ __global__ void __launch_bounds__(fa::THREADS, 2) attn_prefill_tc_kernel(const _
   __syncthreads();
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (tc::elect_one()) {
       tma_prefetch_desc(&tmK);
       tma_prefetch_desc(&tmV);
       bool ok = true;
@@ -944,31 +944,28 @@ __global__ void __launch_bounds__(fa::THREADS, 2) attn_prefill_tc_kernel(const _
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (tc::elect_one()) {
       // D f32, A/B bf16, M = 128, N = 128; QK^T: both K-major; PV: A from TMEM (K-major), B = V MN-major
       const uint32_t idesc_qk = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(128 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
       const uint32_t idesc_pv = idesc_qk | (1u << 16);
-      const uint32_t q_addr = smem_u32(sQ), k_addr = smem_u32(sK), v_addr = smem_u32(sV);
+      constexpr uint32_t hi = tc::desc_hi(1024);
+      const uint32_t q_lo = tc::desc_lo(smem_u32(sQ), 16), k_lo = tc::desc_lo(smem_u32(sK), 16), v_lo = tc::desc_lo(smem_u32(sV), TILE_BYTES / 2);
       bool ok = true;
       for (int j = 0; j < ntiles && ok; ++j) {
         ok = mbar_wait(k_full, j & 1, a.status);
         if (!ok) break;
         tc::fence_after();
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {  // head_dim in steps of 16: two 64-element halves of four steps
-          const uint32_t off = (kk >> 2) * (TILE_BYTES / 2) + (kk & 3) * 32;
-          tc::umma_bf16_ss(tmem_base, tc::smem_desc(q_addr + off, 16, 1024), tc::smem_desc(k_addr + off, 16, 1024), idesc_qk,
-                           kk > 0 ? 1u : 0u);
-        }
+        for (uint32_t h = 0; h < 2; ++h)  // two 64-element halves of head_dim
+          tc::umma4_bf16_ss<tc::K_MAJOR, tc::K_MAJOR>(tmem_base, q_lo + h * (TILE_BYTES / 2 >> 4), k_lo + h * (TILE_BYTES / 2 >> 4), hi, idesc_qk, h);
         tc::commit(s_full);
         tc::commit(k_empty);
         ok = mbar_wait(p_full, j & 1, a.status) && mbar_wait(v_full, j & 1, a.status);
         if (!ok) break;
         tc::fence_after();
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk)  // keys in steps of 16 = two 8-row swizzle atoms
-          tc::umma_bf16_ta(tmem_base + 128, tmem_base + kk * 8, tc::smem_desc(v_addr + kk * 2048, TILE_BYTES / 2, 1024), idesc_pv,
-                           (j > 0 || kk > 0) ? 1u : 0u);
+        for (uint32_t h = 0; h < 2; ++h)  // 64 keys each
+          tc::umma4_bf16_ts<tc::MN_MAJOR>(tmem_base + 128, tmem_base + h * 32, v_lo + h * 4 * tc::MN_MAJOR, hi, idesc_pv, j > 0 || h > 0);
         tc::commit(o_done);
         tc::commit(v_empty);
       }
@@ -1078,7 +1075,7 @@ __global__ void __launch_bounds__(fa2::THREADS, 1) attn_prefill_tc2_kernel(const
   __syncthreads();
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (tc::elect_one()) {
       tma_prefetch_desc(&tmK);
       tma_prefetch_desc(&tmV);
       bool ok = true;
@@ -1105,7 +1102,7 @@ __global__ void __launch_bounds__(fa2::THREADS, 1) attn_prefill_tc2_kernel(const
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (tc::elect_one()) {
       const uint32_t idesc_qk = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(128 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
       const uint32_t idesc_pv = idesc_qk | (1u << 16);
       const uint32_t q_addr = smem_u32(sQ), k_addr = smem_u32(sK), v_addr = smem_u32(sV);
@@ -1118,11 +1115,8 @@ __global__ void __launch_bounds__(fa2::THREADS, 1) attn_prefill_tc2_kernel(const
         const uint32_t qa = q_lo + t * (TILE_BYTES >> 4), ka = k_lo + (j & 1) * (TILE_BYTES >> 4);
         const uint32_t d = tmem_base + t * 128;
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {  // head_dim in steps of 16: two 64-element halves of four steps
-          constexpr uint32_t half_step = (TILE_BYTES / 2) >> 4;
-          const uint32_t off = (kk >> 2) * half_step + (kk & 3) * 2;
-          tc::umma_bf16_ss_lh(d, qa + off, ka + off, hi, idesc_qk, kk > 0 ? 1u : 0u);
-        }
+        for (uint32_t h = 0; h < 2; ++h)  // two 64-element halves of head_dim
+          tc::umma4_bf16_ss<tc::K_MAJOR, tc::K_MAJOR>(d, qa + h * (TILE_BYTES / 2 >> 4), ka + h * (TILE_BYTES / 2 >> 4), hi, idesc_qk, h);
         tc::commit(s_full + t);
       };
       if (nt_max > 0) {
@@ -1147,8 +1141,8 @@ __global__ void __launch_bounds__(fa2::THREADS, 1) attn_prefill_tc2_kernel(const
             const uint32_t pa = tmem_base + t * 128, od = tmem_base + 256 + t * 128;
             const uint32_t acc0 = j > 0 ? 1u : 0u;
 #pragma unroll
-            for (int kk = 0; kk < 8; ++kk)  // keys in steps of 16 = two 8-row swizzle atoms
-              tc::umma_bf16_ta_lh(od, pa + kk * 8, va + kk * (2048 >> 4), hi, idesc_pv, kk > 0 ? 1u : acc0);
+            for (uint32_t h = 0; h < 2; ++h)  // 64 keys each
+              tc::umma4_bf16_ts<tc::MN_MAJOR>(od, pa + h * 32, va + h * 4 * tc::MN_MAJOR, hi, idesc_pv, h > 0 ? 1u : acc0);
             tc::commit(o_done + t);
           }
           if (j + 1 < nt[t]) {

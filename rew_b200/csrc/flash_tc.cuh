@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(64 + QT * 256, 1) flash_tc_kernel(const __grid
   __syncthreads();
 
   if (warp == 0) {
-    if (lane == 0 && n > 0) {
+    if (n > 0 && tc::elect_one()) {
       tma_prefetch_desc(&tm_a);
       tma_prefetch_desc(&tm_b);
       bool ok = true;
@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(64 + QT * 256, 1) flash_tc_kernel(const __grid
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && n > 0) {
+    if (n > 0 && tc::elect_one()) {
       const uint32_t idesc_qk = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(128 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
       const uint32_t idesc_pv = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(cf.nb_v * 8) << 17) | ((uint32_t)(128 >> 4) << 24);
       constexpr uint32_t hi = tc::desc_hi(1024);
@@ -274,11 +274,7 @@ __global__ void __launch_bounds__(64 + QT * 256, 1) flash_tc_kernel(const __grid
       auto issue_qk = [&](int t) {
         const uint32_t qa = q_lo + t * (q_bytes >> 4);
         for (int b = 0; b < nb; ++b)
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk) {
-            const uint32_t off = b * (BOX_BYTES >> 4) + kk * 2;
-            tc::umma_bf16_ss_lh(tmem_base + t * 128, qa + off, k_lo + off, hi, idesc_qk, (b > 0 || kk > 0) ? 1u : 0u);
-          }
+          tc::umma4_bf16_ss<tc::K_MAJOR, tc::K_MAJOR>(tmem_base + t * 128, qa + b * (BOX_BYTES >> 4), k_lo + b * (BOX_BYTES >> 4), hi, idesc_qk, b > 0);
         tc::commit(s_full + t);
       };
       bool ok = mbar_wait(k_full, 0, a.status);
@@ -303,9 +299,9 @@ __global__ void __launch_bounds__(64 + QT * 256, 1) flash_tc_kernel(const __grid
             const uint32_t va = v_lo + st * (v_bytes >> 4);
             const uint32_t acc0 = j > jlo[t] ? 1u : 0u;
 #pragma unroll
-            for (int kk = 0; kk < 8; ++kk)
-              tc::umma_bf16_ta_lh(tmem_base + QT * 128 + t * 128, tmem_base + t * 128 + kk * 8, va + kk * (2048 >> 4), hi, idesc_pv,
-                                  kk > 0 ? 1u : acc0);
+            for (uint32_t h = 0; h < 2; ++h)
+              tc::umma4_bf16_ts<tc::MN_MAJOR>(tmem_base + QT * 128 + t * 128, tmem_base + t * 128 + h * 32, va + h * 4 * tc::MN_MAJOR, hi, idesc_pv,
+                                              h > 0 ? 1u : acc0);
             tc::commit(o_done + t);
           }
           if (active(t, j + 1)) {

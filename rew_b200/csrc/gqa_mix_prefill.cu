@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(64 + 512, 1) mix_stats_kernel(const __grid_con
   const int nt = et.n > 128 ? 2 : 1;                    // query tiles
   float m = -INFINITY, l = 0.f;
   if (warp == 0) {
-    if (lane == 0) {
+    if (tc::elect_one()) {
       bool ok = true;
       mbar_expect_tx(q_full, nt * tb);
       for (int t = 0; t < nt; ++t)
@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(64 + 512, 1) mix_stats_kernel(const __grid_con
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (tc::elect_one()) {
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TILE >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
       constexpr uint32_t hi = tc::desc_hi(1024);
       const uint32_t q_lo = tc::desc_lo(smem_u32(sQ), 16), k_lo = tc::desc_lo(smem_u32(ring), 16);
@@ -193,12 +193,10 @@ __global__ void __launch_bounds__(64 + 512, 1) mix_stats_kernel(const __grid_con
           if (turn > 0) ok = mbar_wait(s_free + 2 * t + buf, (turn - 1) & 1, a.status);
           if (!ok) break;
           tc::fence_after();
-          for (int b = 0; b < nb; ++b)
-#pragma unroll
-            for (int kk = 0; kk < 4; ++kk) {
-              const uint32_t off = b * (BOX >> 4) + kk * 2;
-              tc::umma_bf16_ss_lh(tmem + t * 256 + buf * 128, q_lo + t * (tb >> 4) + off, k_lo + s * (tb >> 4) + off, hi, idesc, (b > 0 || kk > 0) ? 1u : 0u);
-            }
+          for (int b = 0; b < nb; ++b) {
+            const uint32_t off = b * (BOX >> 4);
+            tc::umma4_bf16_ss<tc::K_MAJOR, tc::K_MAJOR>(tmem + t * 256 + buf * 128, q_lo + t * (tb >> 4) + off, k_lo + s * (tb >> 4) + off, hi, idesc, b > 0);
+          }
           tc::commit(s_full + 2 * t + buf);
         }
         if (ok) tc::commit(k_empty + s);
@@ -335,7 +333,7 @@ __global__ void __launch_bounds__(64 + 128 * warpgroups(HP), 1) mix_attn_kernel(
   }
 
   if (warp == 0) {
-    if (lane == 0 && n > 0) {
+    if (n > 0 && tc::elect_one()) {
       bool ok = true;
       int cnt = 0;
       // column q * G2 + hh of kv head c: G2 heads from its first one on (those behind its last are never weighed)
@@ -361,7 +359,7 @@ __global__ void __launch_bounds__(64 + 128 * warpgroups(HP), 1) mix_attn_kernel(
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && n > 0) {
+    if (n > 0 && tc::elect_one()) {
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(nc >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
       const uint32_t idesc_pv = idesc | (1u << 15) | (1u << 16);          // both operands with the contracted index outermost
       constexpr uint32_t hi = tc::desc_hi(1024);
@@ -377,10 +375,8 @@ __global__ void __launch_bounds__(64 + 128 * warpgroups(HP), 1) mix_attn_kernel(
           if (!ok) break;
           tc::fence_after();
           for (int b = 0; b < nbk; ++b)
-#pragma unroll
-            for (int kk = 0; kk < 4; ++kk)
-              tc::umma_bf16_ss_lh(tmem + c * nc, k_lo + s * (st_bytes >> 4) + b * (BOX >> 4) + kk * 2, q_lo + c * (q_bytes >> 4) + b * (nc * 128 >> 4) + kk * 2, hi, idesc,
-                                  (b > 0 || kk > 0) ? 1u : 0u);
+            tc::umma4_bf16_ss<tc::K_MAJOR, tc::K_MAJOR>(tmem + c * nc, k_lo + s * (st_bytes >> 4) + b * (BOX >> 4),
+                                                        q_lo + c * (q_bytes >> 4) + b * (nc * 128 >> 4), hi, idesc, b > 0);
           tc::commit(empty + s);
         }
         if (ok) tc::commit(s_full);
@@ -396,8 +392,9 @@ __global__ void __launch_bounds__(64 + 128 * warpgroups(HP), 1) mix_attn_kernel(
           tc::fence_after();
           const uint32_t pb = p_lo + (col >> 6) * (BOX >> 4) + ((col & 63) * 2 >> 4);
 #pragma unroll
-          for (int kk = 0; kk < 8; ++kk)
-            tc::umma_bf16_ss_lh(tmem + 256 + col, v_lo + s * (st_bytes >> 4) + kk * (2048 >> 4), pb + kk * (2048 >> 4), hi, idesc_pv, (j > 0 || kk > 0) ? 1u : 0u);
+          for (uint32_t h = 0; h < 2; ++h)
+            tc::umma4_bf16_ss<tc::MN_MAJOR, tc::MN_MAJOR>(tmem + 256 + col, v_lo + s * (st_bytes >> 4) + h * 4 * tc::MN_MAJOR, pb + h * 4 * tc::MN_MAJOR, hi,
+                                                          idesc_pv, j > 0 || h > 0);
           tc::commit(empty + s);
         }
         if (ok) tc::commit(j + 1 < kt.n ? p_free : o_full);

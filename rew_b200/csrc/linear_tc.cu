@@ -14,9 +14,10 @@
 //            multi-stage mbarrier ring; W loads of weights that no kernel
 //            of a step writes (TcArgs::early_w) are issued before
 //            griddepcontrol.wait so the ramp overlaps the previous kernel.
-//   warp 1   allocates TMEM, then one elected thread issues four
-//            tcgen05.mma.kind::f16 (K = 16 each) per stage from shared-memory
-//            descriptors and releases the stage with tcgen05.commit.
+//   warp 1   allocates TMEM, then one elected thread (elect.sync: see elect_one
+//            in tc.cuh) issues four tcgen05.mma.kind::f16 (K = 16 each) per stage
+//            from shared-memory descriptors in one block of code and releases the
+//            stage with tcgen05.commit.
 //   warps 2-9 epilogue: tcgen05.ld the accumulator (a warp owns 32 lanes),
 //            apply bias / SwiGLU, store.
 // All waits on barriers are bounded; on a timeout the roles fall through to the
@@ -350,7 +351,7 @@ __global__ void __launch_bounds__(TC_THREADS) linear_tc_kernel(const __grid_cons
 
   bool epi_ok = true;
   if (warp == 0) {
-    if (lane == 0) {
+    if (tc::elect_one()) {
       tma_prefetch_desc(&tmW);
       tma_prefetch_desc(&tmX);
       const uint64_t pol_w = policy_evict_first();
@@ -379,7 +380,7 @@ __global__ void __launch_bounds__(TC_THREADS) linear_tc_kernel(const __grid_cons
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && nkb > 0) {
+    if (nkb > 0 && tc::elect_one()) {
       // instruction descriptor: D f32, A/B bf16, A MN-major, B K-major, N = tn, M = 128
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | ((uint32_t)(tn >> 3) << 17) |
                              ((uint32_t)(BM >> 4) << 24);
@@ -391,14 +392,9 @@ __global__ void __launch_bounds__(TC_THREADS) linear_tc_kernel(const __grid_cons
         tc::fence_after();
         const uint32_t sa = smem_base + s * stage_bytes;
         const uint32_t sb = sa + A_BYTES;
-#pragma unroll
-        for (int kk = 0; kk < BK / 16; ++kk) {
-          // A: 16 k-rows of 128 bytes = two 8-row swizzle atoms 1024 B apart (SBO); the second
-          //    64-feature box is 8192 B further (LBO).  B: rows of 128 B, 8-row atoms 1024 B apart.
-          const uint64_t da = tc::smem_desc(sa + kk * 2048, A_BYTES / 2, 1024);
-          const uint64_t db = tc::smem_desc(sb + kk * 32, 16, 1024);
-          tc::umma_bf16_ss(tmem_base, da, db, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
-        }
+        // A: 16 k-rows of 128 bytes = two 8-row swizzle atoms 1024 B apart (SBO); the second
+        //    64-feature box is 8192 B further (LBO).  B: rows of 128 B, 8-row atoms 1024 B apart.
+        tc::umma4_bf16_ss<tc::MN_MAJOR, tc::K_MAJOR>(tmem_base, tc::desc_lo(sa, A_BYTES / 2), tc::desc_lo(sb, 16), tc::desc_hi(1024), idesc, kb > 0);
         tc::commit(&empty[s]);  // stage is free once these MMAs have read it
         if (++s == stages) s = 0, ++lap;
       }
@@ -461,12 +457,11 @@ __global__ void __launch_bounds__(TC_THREADS) linear_tc_kernel(const __grid_cons
 // One CTA per SM walks its share of the output tiles (or of their pieces along K).  The accumulator is
 // double-buffered in TMEM (2 x 256 columns), so the epilogue warps drain tile j while the MMA warp
 // already accumulates tile j + 1 and the TMA ring keeps running across tile boundaries; the per-tile
-// cost becomes max(main loop, epilogue) instead of their sum.  What bounds it: the tensor core takes
-// 0.27 us for the 128 x 64 block of weights of a stage whatever the tokens of the tile (the weights are
-// an MN-major operand), so a step of up to 256 tokens is fast when every SM has equal work and slow
-// when 32 of them do: hence the pieces along K, and tiles of the step's own size (a multiple of 16
-// tokens), which leave room for a deep ring.  135 tokens of 4096 x 28672: 42 us (67 us in one-tile CTAs
-// of 256 tokens), of which 35 us are the weights' time out of HBM.
+// cost becomes max(main loop, epilogue) instead of their sum.  What bounds it: up to 256 tokens the
+// weights' way from HBM, at equal work of all SMs, so a step is slow when 32 of them have all of it: hence
+// the pieces along K, and tiles of the step's own size (a multiple of 16 tokens), which leave room for a deep
+// ring.  135 tokens of 4096 x 28672: 42 us (67 us in one-tile CTAs of 256 tokens), of which 35 us are the
+// weights' time out of HBM.
 struct PersistCfg {
   static constexpr int TN = 256;                          // most tokens of a tile
   static constexpr int MAX_STAGES = 8;
@@ -578,7 +573,7 @@ __global__ void __launch_bounds__(TC_THREADS) linear_tc_persist_kernel(const __g
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (tc::elect_one()) {
       tma_prefetch_desc(&tmW);
       tma_prefetch_desc(&tmX);
       const uint64_t pol_w = policy_evict_first();
@@ -629,7 +624,7 @@ __global__ void __launch_bounds__(TC_THREADS) linear_tc_persist_kernel(const __g
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (tc::elect_one()) {
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | ((uint32_t)(TN >> 3) << 17) |
                              ((uint32_t)(BM >> 4) << 24);
       const uint32_t smem_base = smem_u32(smem);
@@ -651,12 +646,7 @@ __global__ void __launch_bounds__(TC_THREADS) linear_tc_persist_kernel(const __g
           tc::fence_after();
           const uint32_t sa = smem_base + s * stage_bytes;
           const uint32_t sb = sa + A_BYTES;
-#pragma unroll
-          for (int kk = 0; kk < BK / 16; ++kk) {
-            const uint64_t da = tc::smem_desc(sa + kk * 2048, A_BYTES / 2, 1024);
-            const uint64_t db = tc::smem_desc(sb + kk * 32, 16, 1024);
-            tc::umma_bf16_ss(d_tmem, da, db, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
-          }
+          tc::umma4_bf16_ss<tc::MN_MAJOR, tc::K_MAJOR>(d_tmem, tc::desc_lo(sa, A_BYTES / 2), tc::desc_lo(sb, 16), tc::desc_hi(1024), idesc, kb > 0);
           tc::commit(&empty[s]);
           if (++s == STAGES) s = 0, ++lap;
         }
@@ -728,14 +718,6 @@ __device__ __forceinline__ void tma_load_2d_pair(void* dst, const void* tmap, ui
       "l"(policy)
       : "memory");
 }
-__device__ __forceinline__ void umma_bf16_ss_pair(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n\t}"
-      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0u)
-      : "memory");
-}
 // arrives on the barrier at shared::cluster address `bar_cluster_addr` once every tcgen05 operation this thread
 // has issued so far is complete
 __device__ __forceinline__ void commit_pair(uint32_t bar_cluster_addr) {
@@ -792,7 +774,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS) linear_t
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (tc::elect_one()) {
       tma_prefetch_desc(&tmW);
       tma_prefetch_desc(&tmX);
       const uint64_t pol_w = policy_evict_first();
@@ -820,7 +802,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS) linear_t
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && tc::elect_one()) {
       // D f32, A/B bf16, A MN-major, B K-major, N = 256 tokens, M = 256 features over the pair
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
       const uint32_t smem_base = smem_u32(smem);
@@ -841,12 +823,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS) linear_t
           tc::fence_after();
           const uint32_t sa = smem_base + s * C::STAGE_BYTES;
           const uint32_t sb = sa + A_BYTES;
-#pragma unroll
-          for (int kk = 0; kk < BK / 16; ++kk) {
-            const uint64_t da = tc::smem_desc(sa + kk * 2048, A_BYTES / 2, 1024);
-            const uint64_t db = tc::smem_desc(sb + kk * 32, 16, 1024);
-            umma_bf16_ss_pair(d_tmem, da, db, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
-          }
+          tc::umma4_bf16_ss<tc::MN_MAJOR, tc::K_MAJOR, 2>(d_tmem, tc::desc_lo(sa, A_BYTES / 2), tc::desc_lo(sb, 16), tc::desc_hi(1024), idesc, kb > 0);
           // the stage is free in BOTH CTAs once these MMAs have read it
           commit_pair(smem_u32(&empty[s]));
           commit_pair(dsmem_addr(smem_u32(&empty[s]), 1));

@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(NT_THREADS) nf4_tc_kernel(const __grid_constan
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (tc::elect_one()) {
       tma_prefetch_desc(&tmX);
       const uint64_t pol_x = policy_evict_last();
       // Two rings.  Codes (4 KB per block, plain bulk copy) and the scale pairs of the tile's two
@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(NT_THREADS) nf4_tc_kernel(const __grid_constan
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && nkb > 0) {
+    if (nkb > 0 && tc::elect_one()) {
       // instruction descriptor: D f32, A and B bf16, both K-major (A lives in tensor memory), N = 32, M = 128
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(32 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
       const uint32_t xs_addr = smem_u32(xs);
@@ -278,11 +278,7 @@ __global__ void __launch_bounds__(NT_THREADS) nf4_tc_kernel(const __grid_constan
         ok = mbar_wait(&a_full[p], (kb / NT_ABUF) & 1, status) && mbar_wait(&x_full[s], (kb / NT_XST) & 1, status);
         if (!ok) break;
         tc::fence_after();
-#pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {
-          const uint64_t db = tc::smem_desc(xs_addr + s * NT_XBYTES + kk * 32, 16, 1024);
-          tc::umma_bf16_ta(tmem_base, tmem_base + 32 + p * 32 + kk * 8, db, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
-        }
+        tc::umma4_bf16_ts<tc::K_MAJOR>(tmem_base, tmem_base + 32 + p * 32, tc::desc_lo(xs_addr + s * NT_XBYTES, 16), tc::desc_hi(1024), idesc, kb > 0);
         tc::commit(&x_empty[s]);
         tc::commit(&a_empty[p]);
       }

@@ -8,58 +8,66 @@
 namespace rewb {
 namespace tc {
 
-// shared-memory matrix descriptor: start address, leading / stride byte offsets in 16-byte units,
-// descriptor version 1, 128-byte swizzle
-__device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
-  return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)(lbo_bytes >> 4) << 16) | ((uint64_t)(sbo_bytes >> 4) << 32) |
-         (1ull << 46) | (2ull << 61);
+// One lane of a converged warp, the same one every time.  tcgen05 and bulk-copy instructions take uniform operands.  Behind a
+// branch on the lane's number the compiler does not know that one lane is left and guards every one of them with a loop over
+// the lanes; behind elect.sync it does.  Together with issuing the four products of a 64-deep stage in one block of code
+// (below) this is the price of a product: 148 CTAs, M = 128, cycles a product of 16 k: N = 16 to 128 lane test 90 (144 with
+// descriptors built at run time), elected 49 to 64, elected and in fours 40 to 64; N = 256 128 in every form, which is the
+// tensor core's own rate (N = 128: 64).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
 }
-// D[tmem] (+)= A[tmem] * B[smem descriptor]
-__device__ __forceinline__ void umma_bf16_ta(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// D[tmem] (+)= A[smem descriptor] * B[smem descriptor]
-__device__ __forceinline__ void umma_bf16_ss(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// Descriptor halves for a lean issue loop: the high word is the same for every operand of a kernel with one
-// stride-byte-offset, the low word is (address >> 4) | (leading byte offset >> 4) << 16, so stepping an operand
-// by `bytes` (a multiple of 16, inside the 256 KB window) is one 32-bit add of bytes >> 4.
+
+// Shared-memory operands as the two words of a descriptor.  The high word is the same for every operand of a kernel with one
+// stride-byte-offset, the low word is (address >> 4) | (leading byte offset >> 4) << 16, so stepping an operand by `bytes` (a
+// multiple of 16, inside the 256 KB window) is one 32-bit add of bytes >> 4.
 __device__ __forceinline__ uint32_t desc_lo(uint32_t saddr, uint32_t lbo_bytes) {
   return ((saddr & 0x3FFFFu) >> 4) | ((lbo_bytes >> 4) << 16);
 }
 __device__ __forceinline__ constexpr uint32_t desc_hi(uint32_t sbo_bytes) { return (sbo_bytes >> 4) | (1u << 14) | (2u << 29); }
-// D[tmem] (+)= A[smem] * B[smem], descriptors given as (low, shared high) words
-__device__ __forceinline__ void umma_bf16_ss_lh(uint32_t d_tmem, uint32_t alo, uint32_t blo, uint32_t hi, uint32_t idesc,
-                                                uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
-      "setp.ne.b32 p, %5, 0;\n\t"
-      "mov.b64 da, {%1, %3};\n\t"
-      "mov.b64 db, {%2, %3};\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n\t}"
-      ::"r"(d_tmem), "r"(alo), "r"(blo), "r"(hi), "r"(idesc), "r"(accumulate)
-      : "memory");
+
+// Descriptor steps from one product of 16 k to the next inside a 128-byte swizzled tile, in units of 16 bytes
+constexpr int K_MAJOR = 32 >> 4;      // k runs along the 128-byte rows
+constexpr int MN_MAJOR = 2048 >> 4;   // k runs across them: two atoms of eight rows
+
+// Four products in a row: D[tmem] (+)= A[smem] * B[smem] over 64 k; `accumulate` is about the first.  GROUP = 2: a pair of CTAs.
+template <int A_STEP, int B_STEP, int GROUP = 1>
+__device__ __forceinline__ void umma4_bf16_ss(uint32_t d_tmem, uint32_t alo, uint32_t blo, uint32_t hi, uint32_t idesc, uint32_t accumulate) {
+#define REWB_UMMA4_SS(INSTR, MASK)                                                                                         \
+  asm volatile(                                                                                                            \
+      "{\n\t.reg .pred p, q;\n\t.reg .b32 u, v;\n\t.reg .b64 a0, a1, a2, a3, b0, b1, b2, b3;\n\t"                            \
+      "setp.ne.b32 p, %5, 0;\n\tsetp.eq.b32 q, 0, 0;\n\t"                                                                 \
+      "mov.b64 a0, {%1, %3};\n\tmov.b64 b0, {%2, %3};\n\t"                                                                \
+      "add.u32 u, %1, %6;\n\tadd.u32 v, %2, %7;\n\tmov.b64 a1, {u, %3};\n\tmov.b64 b1, {v, %3};\n\t"                      \
+      "add.u32 u, %1, 2 * %6;\n\tadd.u32 v, %2, 2 * %7;\n\tmov.b64 a2, {u, %3};\n\tmov.b64 b2, {v, %3};\n\t"              \
+      "add.u32 u, %1, 3 * %6;\n\tadd.u32 v, %2, 3 * %7;\n\tmov.b64 a3, {u, %3};\n\tmov.b64 b3, {v, %3};\n\t" INSTR        \
+      " [%0], a0, b0, %4, " MASK "p;\n\t" INSTR " [%0], a1, b1, %4, " MASK "q;\n\t" INSTR " [%0], a2, b2, %4, " MASK       \
+      "q;\n\t" INSTR " [%0], a3, b3, %4, " MASK "q;\n\t}" ::"r"(d_tmem),                                                   \
+      "r"(alo), "r"(blo), "r"(hi), "r"(idesc), "r"(accumulate), "n"(A_STEP), "n"(B_STEP), "r"(0u)                           \
+      : "memory")
+  if constexpr (GROUP == 1)
+    REWB_UMMA4_SS("tcgen05.mma.cta_group::1.kind::f16", "");
+  else
+    REWB_UMMA4_SS("tcgen05.mma.cta_group::2.kind::f16", "{%8, %8, %8, %8, %8, %8, %8, %8}, ");
+#undef REWB_UMMA4_SS
 }
-// D[tmem] (+)= A[tmem] * B[smem]
-__device__ __forceinline__ void umma_bf16_ta_lh(uint32_t d_tmem, uint32_t a_tmem, uint32_t blo, uint32_t hi, uint32_t idesc,
-                                                uint32_t accumulate) {
+// The same with A in tensor memory (8 columns for 16 k)
+template <int B_STEP>
+__device__ __forceinline__ void umma4_bf16_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t blo, uint32_t hi, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
-      "setp.ne.b32 p, %5, 0;\n\t"
-      "mov.b64 db, {%2, %3};\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "r"(blo), "r"(hi), "r"(idesc), "r"(accumulate)
+      "{\n\t.reg .pred p, q;\n\t.reg .b32 v, a1, a2, a3;\n\t.reg .b64 b0, b1, b2, b3;\n\t"
+      "setp.ne.b32 p, %5, 0;\n\tsetp.eq.b32 q, 0, 0;\n\t"
+      "mov.b64 b0, {%2, %3};\n\t"
+      "add.u32 v, %2, %6;\n\tmov.b64 b1, {v, %3};\n\tadd.u32 a1, %1, 8;\n\t"
+      "add.u32 v, %2, 2 * %6;\n\tmov.b64 b2, {v, %3};\n\tadd.u32 a2, %1, 16;\n\t"
+      "add.u32 v, %2, 3 * %6;\n\tmov.b64 b3, {v, %3};\n\tadd.u32 a3, %1, 24;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b0, %4, p;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], b1, %4, q;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [a2], b2, %4, q;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [a3], b3, %4, q;\n\t}" ::"r"(d_tmem),
+      "r"(a_tmem), "r"(blo), "r"(hi), "r"(idesc), "r"(accumulate), "n"(B_STEP)
       : "memory");
 }
 __device__ __forceinline__ void commit(uint64_t* bar) {
