@@ -700,12 +700,16 @@ __global__ void __launch_bounds__(TC_THREADS) linear_tc_persist_kernel(const __g
 // accumulators are announced to both CTAs' epilogue warps the same way; the leader reuses an accumulator
 // buffer once the epilogues of both CTAs have arrived on its `tmem_empty` barrier.
 struct PairCfg {
-  static constexpr int TN = 256;                          // tokens per tile (both CTAs together)
-  static constexpr int STAGES = 6;
-  static constexpr int B_BYTES = (TN / 2) * 128;          // this CTA's 128 tokens x 64 k
-  static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;   // 32 KB
+  static constexpr int TN = 256;                          // most tokens per tile (both CTAs together), a multiple of 32
+  static constexpr int MAX_STAGES = 10;
+  static constexpr int FIXED = 1024 + 256;
   static constexpr int SMEM = kAllSmem;
   static constexpr int TMEM_COLS = 512;
+  static constexpr int stage_bytes(int tn) { return A_BYTES + tn * 64; }   // this CTA's tn / 2 tokens x 64 k: 32 KB in all at 256 tokens
+  static constexpr int stages(int tn) {
+    const int n = (SMEM - FIXED) / stage_bytes(tn);
+    return n < MAX_STAGES ? n : MAX_STAGES;
+  }
 };
 
 constexpr uint32_t kPeerBitMask = 0xFEFFFFFFu;  // clears the bit that tells the two CTAs of a pair apart in a shared::cluster address
@@ -731,19 +735,19 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS) linear_t
                                                                                         const __grid_constant__ CUtensorMap tmX,
                                                                                         TcArgs a, int tiles_n, int tiles_m) {
   using C = PairCfg;
-  constexpr int TN = C::TN;
+  const int TN = a.tn, STAGES = C::stages(TN), stage_bytes = C::stage_bytes(TN);
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + C::STAGES * C::STAGE_BYTES);
-  uint64_t* empty = full + C::STAGES;
-  uint64_t* tmem_full = empty + C::STAGES;   // [2]
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES * stage_bytes);
+  uint64_t* empty = full + STAGES;
+  uint64_t* tmem_full = empty + STAGES;   // [2]
   uint64_t* tmem_empty = tmem_full + 2;      // [2]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();   // 0: leader
   const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
-  const int total_tiles = tiles_n * tiles_m;  // tiles of 256 features x 256 tokens
+  const int total_tiles = tiles_n * tiles_m;  // tiles of 256 features x TN tokens
   const int nkb = (int)((a.K + BK - 1) / BK);
   auto tile_coords = [&](int lin, int& tile_n, int& tile_m) {
     constexpr int GROUP_M = 8;
@@ -757,7 +761,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS) linear_t
   };
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < C::STAGES; ++s) {
+    for (int s = 0; s < STAGES; ++s) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
@@ -779,34 +783,51 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS) linear_t
       tma_prefetch_desc(&tmX);
       const uint64_t pol_w = policy_evict_first();
       const uint64_t pol_x = policy_evict_last();
+      // stages whose weights are requested ahead of the stream dependency (no kernel of a step writes them)
+      int early = 0;
+      if (a.early_w && pair < total_tiles) {
+        int tile_n, tile_m;
+        tile_coords(pair, tile_n, tile_m);
+        early = min(STAGES, nkb);
+        for (int i = 0; i < early; ++i) {
+          uint8_t* st = smem + i * stage_bytes;
+          if (rank == 0) mbar_expect_tx(&full[i], 2 * stage_bytes);
+          tma_load_2d_pair(st, &tmW, &full[i], tile_n * 256 + (int)rank * BM, i * BK, pol_w);
+          tma_load_2d_pair(st + A_BYTES / 2, &tmW, &full[i], tile_n * 256 + (int)rank * BM + 64, i * BK, pol_w);
+        }
+      }
       pdl_wait();  // the activations come from the previous kernel
-      int it = 0;
+      int s = 0, lap = 0;
       bool ok = true;
       for (int t = pair; t < total_tiles && ok; t += n_pairs) {
         int tile_n, tile_m;
         tile_coords(t, tile_n, tile_m);
         const int col0 = tile_n * 256 + (int)rank * BM, row0 = tile_m * TN + (int)rank * (TN / 2);
-        for (int kb = 0; kb < nkb; ++kb, ++it) {
-          const int s = it % C::STAGES;
-          if (it >= C::STAGES && !mbar_wait(&empty[s], ((it / C::STAGES) - 1) & 1, a.status)) {
+        for (int kb = 0; kb < nkb; ++kb) {
+          if (lap > 0 && !mbar_wait(&empty[s], (lap - 1) & 1, a.status)) {
             ok = false;
             break;
           }
-          uint8_t* st = smem + s * C::STAGE_BYTES;
-          if (rank == 0) mbar_expect_tx(&full[s], 2 * C::STAGE_BYTES);  // this CTA's stage and the peer's
+          uint8_t* st = smem + s * stage_bytes;
           const int k = kb * BK;
-          tma_load_2d_pair(st, &tmW, &full[s], col0, k, pol_w);
-          tma_load_2d_pair(st + A_BYTES / 2, &tmW, &full[s], col0 + 64, k, pol_w);
+          if (early > 0) {
+            --early;
+          } else {
+            if (rank == 0) mbar_expect_tx(&full[s], 2 * stage_bytes);  // this CTA's stage and the peer's
+            tma_load_2d_pair(st, &tmW, &full[s], col0, k, pol_w);
+            tma_load_2d_pair(st + A_BYTES / 2, &tmW, &full[s], col0 + 64, k, pol_w);
+          }
           tma_load_2d_pair(st + A_BYTES, &tmX, &full[s], k, row0, pol_x);
+          if (++s == STAGES) s = 0, ++lap;
         }
       }
     }
   } else if (warp == 1) {
     if (rank == 0 && tc::elect_one()) {
-      // D f32, A/B bf16, A MN-major, B K-major, N = 256 tokens, M = 256 features over the pair
+      // D f32, A/B bf16, A MN-major, B K-major, N = TN tokens, M = 256 features over the pair
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
       const uint32_t smem_base = smem_u32(smem);
-      int it = 0, j = 0;
+      int s = 0, lap = 0, j = 0;
       bool ok = true;
       for (int t = pair; t < total_tiles && ok; t += n_pairs, ++j) {
         const int buf = j & 1;
@@ -815,18 +836,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS) linear_t
           if (!ok) break;
           tc::fence_after();
         }
-        const uint32_t d_tmem = tmem_base + (uint32_t)(buf * TN);
-        for (int kb = 0; kb < nkb; ++kb, ++it) {
-          const int s = it % C::STAGES;
-          ok = mbar_wait(&full[s], (it / C::STAGES) & 1, a.status);
+        const uint32_t d_tmem = tmem_base + (uint32_t)(buf * C::TN);
+        for (int kb = 0; kb < nkb; ++kb) {
+          ok = mbar_wait(&full[s], lap & 1, a.status);
           if (!ok) break;
           tc::fence_after();
-          const uint32_t sa = smem_base + s * C::STAGE_BYTES;
+          const uint32_t sa = smem_base + s * stage_bytes;
           const uint32_t sb = sa + A_BYTES;
           tc::umma4_bf16_ss<tc::MN_MAJOR, tc::K_MAJOR, 2>(d_tmem, tc::desc_lo(sa, A_BYTES / 2), tc::desc_lo(sb, 16), tc::desc_hi(1024), idesc, kb > 0);
           // the stage is free in BOTH CTAs once these MMAs have read it
           commit_pair(smem_u32(&empty[s]));
           commit_pair(dsmem_addr(smem_u32(&empty[s]), 1));
+          if (++s == STAGES) s = 0, ++lap;
         }
         if (ok) {
           commit_pair(smem_u32(&tmem_full[buf]));
@@ -850,7 +871,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS) linear_t
       if (ok) ok = mbar_wait_warp(&tmem_full[buf], (j >> 1) & 1, a.status);
       tc::fence_after();
       if (ok)
-        store_tile(a, tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * TN), a.out, (int64_t)col0 + q * 32, lane, half,
+        store_tile(a, tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * C::TN), a.out, (int64_t)col0 + q * 32, lane, half,
                    a.bias, row0, rows_valid, true);
       // every epilogue warp of this CTA has read its part of the accumulator: tell the leader
       tc::fence_before();
@@ -981,6 +1002,34 @@ int linear_tc_preload() {
   return REWB200_OK;
 }
 
+// More tiles of up to 160 tokens than SMs: two CTAs an SM, since those of a second wave start as the first ones leave
+// (4096 x 28672: 135 tokens 42 us, 48 in the persistent kernel).  Otherwise the persistent kernel.
+static bool tc_two_per_sm(Ctx* c, int tn, int64_t tiles) { return tn <= 160 && tiles > c->sm_count; }
+
+// Token tiles of a step of 65 to 1023 rows whose K is not cut: of one CTA (*tn tokens) or of a pair (*pair_tn, else 0).  More tiles
+// than the rows need fill SMs that a launch would leave empty and even out its last wave.  What a tile of one, or of a pair, costs
+// a block of 64 k: what arrives at an SM (weights and tokens; a pair shares the tokens), 0.2 us from its latency up; measured over
+// 4096 x 28672, 4096 x 6144, 4096 x 4096, 14336 x 4096, 2048 x 11264 and 2048 x 2048 at 100 to 900 rows.  Us a launch, before (as few tiles
+// of one CTA as hold the rows) / now: 14336 x 4096 at 333 rows 56.4 / 45.5, 512 rows 74.4 / 51.4; 4096 x 4096 at 333 rows 20.1 / 16.0; 4096 x 6144 at
+// 333 rows 21.2 / 17.4, 900 rows 45.6 / 34.9; 4096 x 28672 at 256 rows 55.7 / 51.9, 512 rows 103 / 94; 2048 x 11264 at 512 rows 28.1 / 21.1.
+static void choose_tiles(Ctx* c, int64_t M, int64_t N, bool pairs, int* tn, int* pair_tn) {
+  const int64_t fewest = (M + 255) / 256, cols = (N + BM - 1) / BM, sms = c->sm_count;
+  auto waves = [](int64_t n, int64_t at_once) { return (double)((n + at_once - 1) / at_once); };
+  double best = 0;
+  for (int64_t t = fewest; t <= fewest + 4; ++t) {
+    const int64_t rows = (M + t - 1) / t;
+    const int one = (int)((rows + 15) / 16 * 16), two = (int)((rows + 31) / 32 * 32);
+    if (t > fewest && one < 64) break;
+    const int64_t tiles_one = cols * ((M + one - 1) / one);
+    const double us = 0.18 + 0.0002 * std::min(one, 144) + 0.0014 * std::max(one - 144, 0);
+    const double cost = us * (tc_two_per_sm(c, one, tiles_one) ? 2 * waves(tiles_one, 2 * sms) : waves(tiles_one, sms));
+    if (best == 0 || cost < best) best = cost, *tn = one, *pair_tn = 0;
+    if (!pairs) continue;
+    const double pair_cost = (0.178 + 0.0002 * std::min(two, 128) + 0.00075 * std::max(two - 128, 0)) * waves(cols / 2 * ((M + two - 1) / two), sms / 2);
+    if (pair_cost < best) best = pair_cost, *pair_tn = two;
+  }
+}
+
 // Same contract as linear_bf16_launch (ungrouped).
 int linear_tc_launch(Ctx* c, const LinearBf16Plan& plan, const bf16* x, int64_t ldx, int64_t M, int epi, int ksplit,
                      void* out, int64_t ldo, const float* bias) {
@@ -989,8 +1038,18 @@ int linear_tc_launch(Ctx* c, const LinearBf16Plan& plan, const bf16* x, int64_t 
   RB_REQUIRE(ksplit >= 1 && (ksplit == 1 || epi == EPI_PARTIAL_F32), "split-K needs the partial epilogue");
   RB_REQUIRE(epi != EPI_SWIGLU_BF16 || plan.N % 16 == 0, "SwiGLU epilogue needs interleaved width % 16 == 0");
   if (M == 0) return REWB200_OK;
-  const int64_t token_tiles = M <= 64 ? 1 : (M + 255) / 256;
-  const int TN = M <= 32 ? 32 : M <= 64 ? 64 : (int)(((M + token_tiles - 1) / token_tiles + 15) / 16 * 16);
+  const bool pairs = c->prefill_persistent && c->prefill_pair && plan.N % 256 == 0 && c->sm_count % 2 == 0 && ksplit == 1;
+  const int64_t fewest = (M + 255) / 256;   // token tiles
+  int TN = M <= 32 ? 32 : M <= 64 ? 64 : (int)(((M + fewest - 1) / fewest + 15) / 16 * 16), pair_tn = 0;
+  if (M >= 1024) {
+    // Pairs of CTAs from four tiles an SM on, where their half of the shared-memory traffic counts: 1 to 4 per cent ahead of one CTA
+    // a tile (us, pairs / one CTA: 4096 x 28672, 1024 rows 200 / 204; 2048 x 11264, 3072 rows 119 / 122; 14336 x 4096, 6144 rows
+    // 616 / 638; 5632 x 2048, 12 288 rows 240 / 249).  With fewer tiles the last wave decides, which is coarser in pairs (4096 x 6144,
+    // 2048 rows, 384 tiles 102 / 99; 2048 x 3072, 4096 rows, 384 tiles 57 / 55).
+    if (pairs && (plan.N + BM - 1) / BM * fewest >= 4 * (int64_t)c->sm_count) pair_tn = PairCfg::TN;
+  } else if (M > 64 && ksplit == 1 && c->prefill_persistent) {
+    choose_tiles(c, M, plan.N, pairs, &TN, &pair_tn);
+  }
   TcArgs a;
   memset(&a, 0, sizeof(a));
   a.M = M;
@@ -1008,24 +1067,20 @@ int linear_tc_launch(Ctx* c, const LinearBf16Plan& plan, const bf16* x, int64_t 
   a.early_w = plan.early_w;
   a.tn = TN;
   dim3 grid((unsigned)((plan.N + BM - 1) / BM), (unsigned)((M + TN - 1) / TN), (unsigned)ksplit);
-  // Pairs of CTAs from four tiles an SM on, where their half of the shared-memory traffic counts: 1 to 4 per cent ahead of one CTA
-  // a tile (us, pairs / one CTA: 4096 x 28672, 1024 rows 200 / 204; 2048 x 11264, 3072 rows 119 / 122; 14336 x 4096, 6144 rows
-  // 616 / 638; 5632 x 2048, 12 288 rows 240 / 249).  With fewer tiles the last wave decides, which is coarser in pairs (4096 x 6144,
-  // 2048 rows, 384 tiles 102 / 99; 2048 x 3072, 4096 rows, 384 tiles 57 / 55).  Below 1024 rows tiles of the step's own size win.
-  if (M >= 1024 && ksplit == 1 && c->prefill_persistent && c->prefill_pair && plan.N % 256 == 0 && c->sm_count % 2 == 0 &&
-      (int64_t)grid.x * token_tiles >= 4 * (int64_t)c->sm_count) {
-    // two-CTA tiles: 256 features x 256 tokens per pair of SMs
+  if (pair_tn) {
+    // two-CTA tiles: 256 features x pair_tn tokens per pair of SMs
     CUtensorMap tmXh;
-    RB_TRY(make_tmap_2d_bf16(&tmXh, x, (uint64_t)plan.K, (uint64_t)M, (uint64_t)ldx * 2, 64, PairCfg::TN / 2));
+    RB_TRY(make_tmap_2d_bf16(&tmXh, x, (uint64_t)plan.K, (uint64_t)M, (uint64_t)ldx * 2, 64, pair_tn / 2));
     static bool pair_attr = false;
     if (!pair_attr) {
       RB_CUDA(cudaFuncSetAttribute(linear_tc_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg::SMEM));
       pair_attr = true;
     }
-    const int tiles_n = (int)(plan.N / 256), tiles_m = (int)token_tiles;
-    const int ctas = (int)std::min<int64_t>(2 * (int64_t)tiles_n * tiles_m, c->sm_count);
-    RB_CUDA(launch_k(linear_tc_pair_kernel, dim3((unsigned)(ctas & ~1)), dim3(TC_THREADS), (size_t)PairCfg::SMEM, c->stream, c->use_pdl,
-                     plan.tmW, tmXh, a, tiles_n, tiles_m));
+    a.tn = pair_tn;
+    const int tiles_n = (int)(plan.N / 256), tiles_m = (int)((M + pair_tn - 1) / pair_tn);
+    const int64_t ctas = std::min<int64_t>(2 * (int64_t)tiles_n * tiles_m, c->sm_count);
+    RB_CUDA(launch_k(linear_tc_pair_kernel, dim3((unsigned)ctas), dim3(TC_THREADS), (size_t)PairCfg::SMEM, c->stream, c->use_pdl, plan.tmW, tmXh, a,
+                     tiles_n, tiles_m));
     ++g_launch_total;
     ++g_route_launches[ROUTE_LINEAR_PAIR];
     return REWB200_OK;
@@ -1034,9 +1089,7 @@ int linear_tc_launch(Ctx* c, const LinearBf16Plan& plan, const bf16* x, int64_t 
   RB_TRY(make_tmap_2d_bf16(&tmX, x, (uint64_t)plan.K, (uint64_t)M, (uint64_t)ldx * 2, 64, TN));
   if (M <= 32) return launch_tn<32>(c, plan, tmX, a, grid);
   if (M <= 64) return launch_tn<64>(c, plan, tmX, a, grid);
-  // More tiles of up to 160 tokens than SMs: two CTAs an SM, since those of a second wave start as the first ones leave
-  // (4096 x 28672: 135 tokens 42 us, 48 in the persistent kernel, 300 tokens 70 and 92).  Otherwise the persistent kernel.
-  const bool two = TN <= 160 && (int64_t)grid.x * grid.y * grid.z > c->sm_count;
+  const bool two = tc_two_per_sm(c, TN, (int64_t)grid.x * grid.y * grid.z);
   if (c->prefill_persistent && !two) {
     static bool attr_set = false;
     if (!attr_set) {

@@ -169,6 +169,34 @@ def test_pair_prefill_linear_matches_oracle_and_the_one_cta_kernels(rb_tc, orc, 
     assert np.array_equal(got, others["persistent"])
 
 
+@pytest.mark.parametrize("M,K,N,pair", [(96, 64, 256, True), (193, 64, 1024, True), (257, 200, 1024, True), (449, 64, 4096, True), (161, 200, 28672, True),
+                                        (333, 1024, 28672, True), (385, 200, 28672, True), (511, 136, 18944, True), (900, 200, 6144, True),
+                                        (300, 200, 1152, False), (65, 64, 2048, False)])
+def test_pairs_with_tiles_of_the_steps_own_size(rb_tc, M, K, N, pair):
+    """Pair tiles of 64 to 256 tokens in steps of 32: a last tile of one token, more tiles than pairs, K that is no multiple of a
+    block, weights narrower than a wave; a width that pairs cannot take, a step that one CTA a tile suits better.  bf16
+    operands are exact in f32, so the only roundings are K + 1 of f32 sums and the bf16 output's half ulp; and the same bits
+    as the one-CTA kernels, whose products run in the same order."""
+    from rew_b200 import _lib
+    rng = np.random.default_rng(M + N)
+    x, w = W.bf16_round(rng.normal(size=(M, K))), W.bf16_round(rng.normal(size=(K, N)))
+    b = rng.normal(size=N).astype(np.float32)
+    T = rb_tc.Tensor.from_host
+    lin, xs = rb_tc.Linear(T(w, _lib.BF16), T(b)), T(x, _lib.BF16)
+    before = _launches()
+    got = lin.forward(xs).to_host()
+    assert _launches()["pair"] - before["pair"] == pair
+    want = x.astype(np.float64) @ w + b
+    bound = (K + 1) * 2.0 ** -24 * (np.abs(x).astype(np.float64) @ np.abs(w) + np.abs(b)) + 2.0 ** -8 * np.abs(want)
+    assert np.all(np.abs(got - want) <= bound)
+    for how in ("persistent", "tile"):
+        rb_tc.set_option("prefill", how)
+        try:
+            assert np.array_equal(lin.forward(xs).to_host(), got)
+        finally:
+            rb_tc.set_option("prefill", "pair")
+
+
 def test_persistent_prefill_model_equals_tile_kernel(rb_tc):
     """A 20 480-token prefill puts the decoder Linears (f32 partial and bf16 epilogues) on the persistent kernel and gate and up
     (SwiGLU) on the pair kernel; the logits must equal those of the one-tile-per-CTA kernel exactly."""
