@@ -1568,7 +1568,6 @@ int rewb200_model_finalize(rewb200_model* m) {
         RB_TRY(nf4_alloc(c, w->K, w->N, &w->nf4));
         m->allocs.push_back(w->nf4.q);
         m->allocs.push_back(w->nf4.sc);
-        m->allocs.push_back(w->nf4.sc2);
         RB_TRY(nf4_quantize_launch(c, w->w, REWB200_BF16, w->N, w->cm, w->nf4));
         RB_CUDA(cudaStreamSynchronize(c->stream));
         auto it = std::find(m->allocs.begin(), m->allocs.end(), w->w);

@@ -7,15 +7,14 @@
 // max(1e-10, absmax), code = nearest of the 16 NF4 levels (first one on a tie), value = level * scale.
 //
 // Device layout (this library's own; rewb200_nf4_unpack gives back the reference's bytes):
-//   q   [ceil(N/128)][K/64][128 features][32 bytes]  the 64 codes of one feature and one block of 64 input
-//         rows, byte j = (code of row 2j) | (code of row 2j+1) << 4; features past N hold code 7 (= 0.0)
+//   q   [ceil(N/128)][K/64] blocks of 4352 bytes: the codes of 128 features and 64 input rows as [2][128 features][16 bytes],
+//         byte j of half h = (code of row 32h + 2j) | (code of row 32h + 2j + 1) << 4, features past N code 7 (= 0.0); behind them
+//         the scales of the block's two 64-feature groups as [2][32] bf16 pairs (rows 2j, 2j + 1): what the GEMV multiplies by
 //   sc  [N/64][K] f32      the scales of one 64-feature group, contiguous along k
-//   sc2 [N/64][K/2] u32    the same scales as bf16 pairs (rows 2j, 2j+1): what the GEMV multiplies by
 // GEMV (rows <= 32) on the 5th-generation tensor core with the WEIGHT operand in tensor memory:
 //   D[128 features][32 tokens] (TMEM, f32) += A[128 features][64 k] (TMEM, bf16) * B[64 k][32 tokens] (smem)
-//   warp 0      TMA producer, two rings: 14 stages of the tile's 4 KB of codes + the scale pairs of its two
-//               groups (bulk copies out of HBM, 56 KB in flight per CTA), 4 stages of the activation tile
-//               (32 tokens x 64 k, 128-byte swizzle, out of L2)
+//   warp 0      TMA producer, two rings: 14 stages of the tile's codes with their scale pairs (one bulk copy each out of
+//               HBM, 60 KB in flight per CTA), 16 KB of activation tiles (16 or 32 tokens x 64 k, 128-byte swizzle, out of L2)
 //   warp 1      one thread issues four tcgen05.mma (K = 16 each) per block of 64 rows, A read from TMEM
 //   warps 2-9   dequantisers: a warp owns the 32 TMEM lanes (features) of its lane quarter and every
 //               other block; a lane reads its feature's 32 code bytes from the stage, turns each byte into a bf16 pair
@@ -53,15 +52,17 @@ __device__ __forceinline__ int64_t map_col(const ColMap& cm, int64_t n) {
   return (within / cm.gran) * cm.gstride + (within % cm.gran) + seg * cm.seg_off;
 }
 
+constexpr int NF4_CODES = 128 * 32;               // codes of a block: 128 features x 64 rows
+constexpr int NF4_BLOCK = NF4_CODES + 2 * 32 * 4;  // with the scale pairs of its two groups
+__device__ __forceinline__ int64_t block_byte(int64_t k, int64_t n, int64_t KB) { return ((n >> 7) * KB + (k >> 6)) * NF4_BLOCK; }
 // byte offset of the pair byte of W[k][n] inside q
 __device__ __forceinline__ int64_t code_byte(int64_t k, int64_t n, int64_t KB) {
-  return (((n >> 7) * KB + (k >> 6)) * 128 + (n & 127)) * 32 + ((k & 63) >> 1);
+  return block_byte(k, n, KB) + ((k & 63) >> 5) * 2048 + (n & 127) * 16 + ((k & 31) >> 1);
 }
 
 // grid (N/64, K/64), 64 threads: thread r quantises the 64 features of group g for input row kb*64 + r.
 template <typename T>
-__global__ void __launch_bounds__(64) nf4_quantize_kernel(const T* src, int64_t ld, ColMap cm, uint8_t* q, float* sc,
-                                                          uint32_t* sc2, int64_t K, int64_t N) {
+__global__ void __launch_bounds__(64) nf4_quantize_kernel(const T* src, int64_t ld, ColMap cm, uint8_t* q, float* sc, int64_t K, int64_t N) {
   __shared__ uint8_t codes[64][64 + 4];  // [row][feature]
   __shared__ float srow[64];
   const int g = blockIdx.x, kb = blockIdx.y, r = threadIdx.x;
@@ -105,14 +106,14 @@ __global__ void __launch_bounds__(64) nf4_quantize_kernel(const T* src, int64_t 
     }
     words[w] = u;
   }
-  uint4* dst = reinterpret_cast<uint4*>(q + code_byte((int64_t)kb * 64, n, KB));
-  dst[0] = make_uint4(words[0], words[1], words[2], words[3]);
-  dst[1] = make_uint4(words[4], words[5], words[6], words[7]);
-  if (r < 32) sc2[(int64_t)g * (K / 2) + (int64_t)kb * 32 + r] = pack_bf16(srow[2 * r], srow[2 * r + 1]);
+  *reinterpret_cast<uint4*>(q + code_byte((int64_t)kb * 64, n, KB)) = make_uint4(words[0], words[1], words[2], words[3]);
+  *reinterpret_cast<uint4*>(q + code_byte((int64_t)kb * 64 + 32, n, KB)) = make_uint4(words[4], words[5], words[6], words[7]);
+  if (r < 32)
+    reinterpret_cast<uint32_t*>(q + block_byte((int64_t)kb * 64, n, KB) + NF4_CODES)[(g & 1) * 32 + r] = pack_bf16(srow[2 * r], srow[2 * r + 1]);
 }
 
 // dst (bf16, column-mapped) = level * scale.  A stream of stores, 2 bytes a weight against half a byte of codes: a CTA takes the 64
-// input rows of a 128-feature tile (its codes are 4 KB in one piece), a thread eight features of eight rows, i.e. one word of
+// input rows of a 128-feature tile (its codes are one piece of 4 KB), a thread eight features of eight rows, i.e. one word of
 // codes per feature, and writes eight 16-byte pieces of a row each.  The four matrices of an 8B-shaped layer (218 M weights)
 // take 127 us, 4.3 TB/s of codes and stores; one element a thread and its code byte from wherever it lies, 664 us.
 __global__ void __launch_bounds__(128) nf4_expand_kernel(const uint8_t* q, const float* sc, int64_t K, int64_t N, bf16* dst, int64_t ld, ColMap cm) {
@@ -130,7 +131,7 @@ __global__ void __launch_bounds__(128) nf4_expand_kernel(const uint8_t* q, const
   uint32_t w[8] = {};
   if (n < N) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) w[j] = *reinterpret_cast<const uint32_t*>(q + code_byte((int64_t)kb * 64, n + j, KB) + 4 * octet);
+    for (int j = 0; j < 8; ++j) w[j] = *reinterpret_cast<const uint32_t*>(q + code_byte((int64_t)kb * 64 + 8 * octet, n + j, KB));
   }
   __syncthreads();
   if (n >= N) return;
@@ -156,18 +157,15 @@ __global__ void __launch_bounds__(128) nf4_codes_kernel(const uint8_t* q, int64_
   }
 }
 
-constexpr int NT_XST = 4;                    // activation stages: they come out of L2, a short ring is enough
-constexpr int NT_CST = 14;                   // code stages: 56 KB of packed weights in flight per CTA hide the HBM latency
-constexpr int NT_XBYTES = 32 * 128;          // activations of a block: 32 tokens x 64 k bf16 (128-byte swizzle)
-constexpr int NT_CBYTES = 128 * 32;          // codes of a block: 128 features x 32 bytes
-constexpr int NT_SBYTES = 2 * 32 * 4;        // scale pairs of a block: 2 groups x 32 pairs
-constexpr int NT_CSTAGE = NT_CBYTES + NT_SBYTES;   // code stage = codes | scale pairs
+constexpr int NT_XRING = 16 * 1024;          // activation stages: they come out of L2, a short ring is enough
+constexpr int NT_XST = NT_XRING / (16 * 128);   // at most: a stage is tn tokens x 64 k bf16 (128-byte swizzle)
+constexpr int NT_CST = 14;                   // code stages: 60 KB of packed weights in flight per CTA hide the HBM latency
 constexpr int NT_DEQ = 8;                    // dequantiser warps
 constexpr int NT_THREADS = (2 + NT_DEQ) * 32;
 constexpr int NT_ABUF = 4;                   // weight-operand buffers in tensor memory
 constexpr int NT_TMEM_COLS = 256;            // D: columns 0-31; A buffer b: columns 32 + 32 b .. +31
 constexpr int NT_LUT_BYTES = 256 * 32 * 4;
-constexpr int NT_SMEM = NT_XST * NT_XBYTES + NT_CST * NT_CSTAGE + NT_LUT_BYTES + 512 + 1024;
+constexpr int NT_SMEM = NT_XRING + NT_CST * NF4_BLOCK + NT_LUT_BYTES + 512 + 1024;
 
 __device__ __forceinline__ uint32_t hmul2_bf16(uint32_t a, uint32_t b) {
   uint32_t r;
@@ -176,13 +174,12 @@ __device__ __forceinline__ uint32_t hmul2_bf16(uint32_t a, uint32_t b) {
 }
 
 __global__ void __launch_bounds__(NT_THREADS) nf4_tc_kernel(const __grid_constant__ CUtensorMap tmX, const uint8_t* __restrict__ q,
-                                                            const uint32_t* __restrict__ sc2, int M, int64_t K, int64_t N,
-                                                            int kb_per_split, float* __restrict__ out, int* status) {
+                                                            int M, int tn, int64_t K, int64_t N, int kb_per_split, float* __restrict__ out, int* status) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* xs = smem;                                                    // [NT_XST] activation tiles
-  uint8_t* cs = smem + NT_XST * NT_XBYTES;                               // [NT_CST]{codes | scale pairs}
-  uint32_t* lut = reinterpret_cast<uint32_t*>(cs + NT_CST * NT_CSTAGE);  // [256 byte values][32 lanes]
+  uint8_t* xs = smem;                                                    // [xst] activation tiles
+  uint8_t* cs = smem + NT_XRING;                                         // [NT_CST]{codes | scale pairs}
+  uint32_t* lut = reinterpret_cast<uint32_t*>(cs + NT_CST * NF4_BLOCK);  // [256 byte values][32 lanes]
   uint64_t* x_full = reinterpret_cast<uint64_t*>(lut + 256 * 32);
   uint64_t* x_empty = x_full + NT_XST;
   uint64_t* c_full = x_empty + NT_XST;      // [NT_CST]
@@ -197,6 +194,8 @@ __global__ void __launch_bounds__(NT_THREADS) nf4_tc_kernel(const __grid_constan
   const int KB = (int)(K / 64);
   const int kb0 = split * kb_per_split;
   const int nkb = max(0, min(kb_per_split, KB - kb0));
+  const int xbytes = tn * 128, xst = NT_XRING / xbytes;   // 4 stages of 32 tokens or 8 of 16: a power of two
+  const int xsh = tn == 16 ? 3 : 2;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < NT_XST; ++s) {
@@ -230,35 +229,27 @@ __global__ void __launch_bounds__(NT_THREADS) nf4_tc_kernel(const __grid_constan
     if (tc::elect_one()) {
       tma_prefetch_desc(&tmX);
       const uint64_t pol_x = policy_evict_last();
-      // Two rings.  Codes (4 KB per block, plain bulk copy) and the scale pairs of the tile's two
-      // 64-feature groups come from HBM: 14 stages, 56 KB in flight per CTA.  The activation tile of a
-      // block (tensor copy) comes out of L2: 4 stages.  Codes and scales do not depend on the previous
-      // kernel: the first ring-full is requested before waiting for it.
-      const int64_t g0 = ((int64_t)tile * 128) >> 6, G = N >> 6;
+      // Two rings.  The codes of a block with its scale pairs are one bulk copy out of HBM, the activation tile of a block (tensor
+      // copy) comes out of L2.  Codes do not depend on the previous kernel: the first ring-full is requested before waiting for it.
       auto load_codes = [&](int kb) {
         const int s = kb % NT_CST;
-        uint8_t* st = cs + s * NT_CSTAGE;
-        mbar_expect_tx(&c_full[s], NT_CSTAGE);
-        bulk_load_1d(st, q + ((int64_t)tile * KB + kb0 + kb) * NT_CBYTES, NT_CBYTES, &c_full[s]);
-        for (int h = 0; h < 2; ++h) {
-          const int64_t g = min(g0 + h, G - 1);  // a half tile past N re-reads the last group (its lanes are never stored)
-          bulk_load_1d(st + NT_CBYTES + h * 128, sc2 + g * (K / 2) + (int64_t)(kb0 + kb) * 32, 128, &c_full[s]);
-        }
+        mbar_expect_tx(&c_full[s], NF4_BLOCK);
+        bulk_load_1d(cs + s * NF4_BLOCK, q + ((int64_t)tile * KB + kb0 + kb) * NF4_BLOCK, NF4_BLOCK, &c_full[s]);
       };
       auto load_x = [&](int kb) {
-        const int s = kb % NT_XST;
-        mbar_expect_tx(&x_full[s], NT_XBYTES);
-        tma_load_2d_hint(xs + s * NT_XBYTES, &tmX, &x_full[s], (kb0 + kb) * 64, 0, pol_x);
+        const int s = kb & (xst - 1);
+        mbar_expect_tx(&x_full[s], xbytes);
+        tma_load_2d_hint(xs + s * xbytes, &tmX, &x_full[s], (kb0 + kb) * 64, 0, pol_x);
       };
       for (int kb = 0; kb < min(NT_CST, nkb); ++kb) load_codes(kb);
       pdl_wait();  // the activations come from the previous kernel
-      for (int kb = 0; kb < min(NT_XST, nkb); ++kb) load_x(kb);
-      // block t, once consumed, frees the activation slot of block t + NT_XST and the code slot of t + NT_CST
+      for (int kb = 0; kb < min(xst, nkb); ++kb) load_x(kb);
+      // block t, once consumed, frees the activation slot of block t + xst and the code slot of t + NT_CST
       for (int t = 0; t < nkb; ++t) {
-        const int xk = t + NT_XST, ck = t + NT_CST;
+        const int xk = t + xst, ck = t + NT_CST;
         if (xk >= nkb && ck >= nkb) break;
         if (xk < nkb) {
-          if (!mbar_wait(&x_empty[xk % NT_XST], ((xk / NT_XST) - 1) & 1, status)) break;
+          if (!mbar_wait(&x_empty[xk & (xst - 1)], ((xk >> xsh) - 1) & 1, status)) break;
           load_x(xk);
         }
         if (ck < nkb) {
@@ -269,16 +260,16 @@ __global__ void __launch_bounds__(NT_THREADS) nf4_tc_kernel(const __grid_constan
     }
   } else if (warp == 1) {
     if (nkb > 0 && tc::elect_one()) {
-      // instruction descriptor: D f32, A and B bf16, both K-major (A lives in tensor memory), N = 32, M = 128
-      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(32 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+      // instruction descriptor: D f32, A and B bf16, both K-major (A lives in tensor memory), N = tn, M = 128
+      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(tn >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
       const uint32_t xs_addr = smem_u32(xs);
       bool ok = true;
       for (int kb = 0; kb < nkb && ok; ++kb) {
-        const int p = kb % NT_ABUF, s = kb % NT_XST;
-        ok = mbar_wait(&a_full[p], (kb / NT_ABUF) & 1, status) && mbar_wait(&x_full[s], (kb / NT_XST) & 1, status);
+        const int p = kb % NT_ABUF, s = kb & (xst - 1);
+        ok = mbar_wait(&a_full[p], (kb / NT_ABUF) & 1, status) && mbar_wait(&x_full[s], (kb >> xsh) & 1, status);
         if (!ok) break;
         tc::fence_after();
-        tc::umma4_bf16_ts<tc::K_MAJOR>(tmem_base, tmem_base + 32 + p * 32, tc::desc_lo(xs_addr + s * NT_XBYTES, 16), tc::desc_hi(1024), idesc, kb > 0);
+        tc::umma4_bf16_ts<tc::K_MAJOR>(tmem_base, tmem_base + 32 + p * 32, tc::desc_lo(xs_addr + s * xbytes, 16), tc::desc_hi(1024), idesc, kb > 0);
         tc::commit(&x_empty[s]);
         tc::commit(&a_empty[p]);
       }
@@ -296,10 +287,10 @@ __global__ void __launch_bounds__(NT_THREADS) nf4_tc_kernel(const __grid_constan
     for (int kb = p; kb < nkb; kb += 2) {
       const int s = kb % NT_CST, ab = kb % NT_ABUF, use = kb / NT_ABUF;
       if (ok) ok = mbar_wait(&c_full[s], (kb / NT_CST) & 1, status);
-      const uint8_t* st = cs + s * NT_CSTAGE;
-      const uint4* cp = reinterpret_cast<const uint4*>(st + (quarter * 32 + lane) * 32);
-      const uint4 qa = cp[0], qb = cp[1];
-      const uint4* sp4 = reinterpret_cast<const uint4*>(st + NT_CBYTES + (quarter >> 1) * 128);
+      const uint8_t* st = cs + s * NF4_BLOCK;
+      const uint4* cp = reinterpret_cast<const uint4*>(st) + quarter * 32 + lane;
+      const uint4 qa = cp[0], qb = cp[128];
+      const uint4* sp4 = reinterpret_cast<const uint4*>(st + NF4_CODES + (quarter >> 1) * 128);
       const uint32_t words[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
       uint32_t r[32];
 #pragma unroll
@@ -361,28 +352,26 @@ int nf4_alloc(Ctx* c, int64_t K, int64_t N, Nf4W* w) {
   w->K = K;
   w->N = N;
   const int64_t tiles = (N + 127) / 128;
-  RB_CUDA(cudaMalloc((void**)&w->q, (size_t)tiles * 128 * K / 2));
-  RB_CUDA(cudaMemset(w->q, 0x77, (size_t)tiles * 128 * K / 2));  // code 7 = 0.0 for the features past N
+  const size_t bytes = (size_t)tiles * (K / 64) * NF4_BLOCK;
+  RB_CUDA(cudaMalloc((void**)&w->q, bytes));
+  RB_CUDA(cudaMemset(w->q, 0x77, bytes));  // code 7 = 0.0 for the features past N, whose scales are finite
   RB_CUDA(cudaMalloc((void**)&w->sc, (size_t)K * (N / 64) * sizeof(float)));
-  RB_CUDA(cudaMalloc((void**)&w->sc2, (size_t)(K / 2) * (N / 64) * sizeof(uint32_t)));
   return REWB200_OK;
 }
 
 void nf4_free(Nf4W* w) {
   if (w->q) cudaFree(w->q);
   if (w->sc) cudaFree(w->sc);
-  if (w->sc2) cudaFree(w->sc2);
   w->q = nullptr;
   w->sc = nullptr;
-  w->sc2 = nullptr;
 }
 
 int nf4_quantize_launch(Ctx* c, const void* src, int src_dtype, int64_t ld, ColMap cm, const Nf4W& w) {
   const dim3 grid((unsigned)(w.N / 64), (unsigned)(w.K / 64));
   if (src_dtype == REWB200_BF16)
-    nf4_quantize_kernel<bf16><<<grid, 64, 0, c->stream>>>((const bf16*)src, ld, cm, w.q, w.sc, w.sc2, w.K, w.N);
+    nf4_quantize_kernel<bf16><<<grid, 64, 0, c->stream>>>((const bf16*)src, ld, cm, w.q, w.sc, w.K, w.N);
   else if (src_dtype == REWB200_F32)
-    nf4_quantize_kernel<float><<<grid, 64, 0, c->stream>>>((const float*)src, ld, cm, w.q, w.sc, w.sc2, w.K, w.N);
+    nf4_quantize_kernel<float><<<grid, 64, 0, c->stream>>>((const float*)src, ld, cm, w.q, w.sc, w.K, w.N);
   else
     return fail("nf4 quantise: weights must be f32 or bf16");
   RB_CUDA(cudaGetLastError());
@@ -414,7 +403,7 @@ int nf4_codes_launch(Ctx* c, const Nf4W& w, uint8_t* codes) {
 // With so few rows the tensor core has nothing to do and the kernel is a stream of codes: 0.5 byte per weight
 // against 2 for bf16, so the instruction count per code byte is what matters.  A CTA owns 128 features and a
 // range of 64-row blocks; thread t owns feature t and reads its 32 code bytes of a block with two 16-byte
-// loads (consecutive threads, consecutive 32 bytes: the tile's 4 KB are one contiguous run); the next block's
+// loads (consecutive threads, consecutive 16 bytes); the next block's
 // codes are requested before this block's are consumed.  A code byte (two weights) costs one lookup in a
 // 256-entry table of fp16 level PAIRS (eight copies side by side, so that lanes rarely share a bank) and one HFMA2 per row with the
 // matching pair of activations, which are staged once per block already multiplied by the group's scales
@@ -439,15 +428,16 @@ __global__ void __launch_bounds__(128) nf4_gemv_small_kernel(const uint8_t* __re
     tab[i] = __floats2half2_rn(kNf4[byte & 15], kNf4[byte >> 4]);
   }
   const int cp = lane & 7;
-  const uint4* qp = reinterpret_cast<const uint4*>(q) + (((int64_t)tile * KB + kb0) * 128 + t) * 2;
+  constexpr int BLOCK = NF4_BLOCK / 16;
+  const uint4* qp = reinterpret_cast<const uint4*>(q) + ((int64_t)tile * KB + kb0) * BLOCK + t;
   uint4 c0 = make_uint4(0x77777777u, 0x77777777u, 0x77777777u, 0x77777777u), c1 = c0, n0 = c0, n1 = c0, m0 = c0, m1 = c0;  // code 7 = 0.0
   if (nkb > 0) {  // the weights do not depend on the previous kernel: three blocks are requested before the wait
     c0 = __ldcs(qp);
-    c1 = __ldcs(qp + 1);
+    c1 = __ldcs(qp + 128);
   }
   if (nkb > 1) {
-    n0 = __ldcs(qp + 256);
-    n1 = __ldcs(qp + 257);
+    n0 = __ldcs(qp + BLOCK);
+    n1 = __ldcs(qp + BLOCK + 128);
   }
   pdl_wait();
   // staging: thread t prepares pair (t & 31) of group (t >> 5) & 1 for rows (t >> 6), (t >> 6) + 2
@@ -491,8 +481,8 @@ __global__ void __launch_bounds__(128) nf4_gemv_small_kernel(const uint8_t* __re
   for (int kb = 0; kb < nkb; ++kb) {
     const int buf = kb & 1;
     if (kb + 2 < nkb) {
-      m0 = __ldcs(qp + (int64_t)(kb + 2) * 256);
-      m1 = __ldcs(qp + (int64_t)(kb + 2) * 256 + 1);
+      m0 = __ldcs(qp + (int64_t)(kb + 2) * BLOCK);
+      m1 = __ldcs(qp + (int64_t)(kb + 2) * BLOCK + 128);
     }
     if (kb + 1 < nkb) put(buf ^ 1);     // block kb + 1, requested one iteration ago
     if (kb + 2 < nkb) fetch(kb + 2);
@@ -581,7 +571,8 @@ int nf4_gemv_launch(Ctx* c, const Nf4W& w, const bf16* x, int64_t ldx, int64_t M
     return REWB200_OK;
   }
   CUtensorMap tmX;
-  RB_TRY(make_tmap_2d_bf16(&tmX, x, (uint64_t)w.K, (uint64_t)M, (uint64_t)ldx * 2, 64, 32));
+  const int tn = M <= 16 ? 16 : 32;
+  RB_TRY(make_tmap_2d_bf16(&tmX, x, (uint64_t)w.K, (uint64_t)M, (uint64_t)ldx * 2, 64, tn));
   static bool attr_set = false;
   if (!attr_set) {
     RB_CUDA(cudaFuncSetAttribute(nf4_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, NT_SMEM));
@@ -589,7 +580,7 @@ int nf4_gemv_launch(Ctx* c, const Nf4W& w, const bf16* x, int64_t ldx, int64_t M
     attr_set = true;
   }
   RB_CUDA(launch_k(nf4_tc_kernel, grid, dim3(NT_THREADS), (size_t)NT_SMEM, c->stream, c->use_pdl, tmX, (const uint8_t*)w.q,
-                   (const uint32_t*)w.sc2, (int)M, w.K, w.N, per, out, c->d_status));
+                   (int)M, tn, w.K, w.N, per, out, c->d_status));
   ++g_launch_total;
   return REWB200_OK;
 }
