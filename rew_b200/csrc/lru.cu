@@ -26,10 +26,11 @@ __global__ void __launch_bounds__(NW == 1 ? 128 : 32 * NW) lru_kernel(LruArgs a)
   pdl_launch_dependents();
   const LruDims& m = a.m;
   const int warp = threadIdx.x >> 5, ln = threadIdx.x & 31, w = NW == 1 ? 0 : warp, width = m.blocks * m.n;
-  const int ch = (NW == 1 ? blockIdx.x * 4 + warp : blockIdx.x) * 32 + ln;
-  const bool on = ch < width;
-  const int b = on ? ch / m.n : 0, j = ch - b * m.n;
-  const float decay = on ? m.decay[ch] : 0.f, yb = on ? m.y_bias[ch] : 0.f;
+  const int own = (NW == 1 ? blockIdx.x * 4 + warp : blockIdx.x) * 32 + ln;
+  const bool on = own < width;
+  const int ch = on ? own : width - 1;   // lanes past the last channel read it and store nothing
+  const int b = ch / m.n, j = ch - b * m.n;
+  const float decay = m.decay[ch], yb = m.y_bias[ch];
   if (!a.early) pdl_wait();
   const GlaPortion p = portion_of(a, blockIdx.y);
   float* const st = a.state + (int64_t)p.lane * width + ch;
@@ -42,20 +43,29 @@ __global__ void __launch_bounds__(NW == 1 ? 128 : 32 * NW) lru_kernel(LruArgs a)
   for (int t0 = 0, it = 0; t0 < p.n; t0 += NW * TT, ++it) {
     const int tb = t0 + w * TT, nt = on ? min(p.n - tb, TT) : 0;
     float r[TT], i[TT], u[TT], y[TT];
+    if (tb < p.n) {   // the run has tokens
+      // All loads of the run are under way before the first is used: tokens past its end read the last one, whose values nobody
+      // uses.  (A branch a token kept every load behind the use of the one before.  3072 channels of a portion of 150
+      // tokens beside seven of one: 26.6 us, now 18.3; seven portions of 700: 176 us, now 144.)
+      T uu[TT];
 #pragma unroll
-    for (int k = 0; k < TT; ++k) {
-      r[k] = i[k] = u[k] = y[k] = 0.f;
-      if (k >= nt) continue;
-      const int64_t t = tb + k;
-      r[k] = gp[t * 2 * m.ldn];
-      i[k] = gp[t * 2 * m.ldn + m.ldn];
-      u[k] = ldf<T>(up[t * m.ldn]);
-      y[k] = yp[t * a.ld];
+      for (int k = 0; k < TT; ++k) {
+        const int64_t t = min(tb + k, p.n - 1);
+        r[k] = gp[t * 2 * m.ldn];
+        i[k] = gp[t * 2 * m.ldn + m.ldn];
+        uu[k] = up[t * m.ldn];
+        y[k] = yp[t * a.ld];
+      }
+      for (int s = 1; s < a.nsplit; ++s) {
+        float d[TT];
+#pragma unroll
+        for (int k = 0; k < TT; ++k) d[k] = yp[s * a.split_stride + (int64_t)min(tb + k, p.n - 1) * a.ld];
+#pragma unroll
+        for (int k = 0; k < TT; ++k) y[k] += d[k];
+      }
+#pragma unroll
+      for (int k = 0; k < TT; ++k) u[k] = ldf<T>(uu[k]);
     }
-    for (int s = 1; s < a.nsplit; ++s)
-#pragma unroll
-      for (int k = 0; k < TT; ++k)
-        if (k < nt) y[k] += yp[s * a.split_stride + (tb + k) * a.ld];
     // r, i become the decay and the contribution of a token; tokens past the end change nothing
 #pragma unroll
     for (int k = 0; k < TT; ++k) {
