@@ -1280,7 +1280,7 @@ int attn_launch(Ctx* c, const AttnArgs& h) {
     }
     return REWB200_OK;
   }
-  if (c->attn_tc && a.hd == 128 && h.S >= 128 && (!a.causal || a.mask_kind == 1) && h.q_ss % 8 == 0 && h.q_sh % 8 == 0 &&
+  if (c->attn_tc && a.hd == 128 && h.S >= kAttnTcRows && (!a.causal || a.mask_kind == 1) && h.q_ss % 8 == 0 && h.q_sh % 8 == 0 &&
       h.q_sb % 8 == 0 && h.o_ss % 8 == 0 && h.o_sh % 8 == 0 && h.o_sb % 8 == 0) {
     static bool tc_attr = false;
     if (!tc_attr) {

@@ -395,6 +395,10 @@ struct AttnArgs {
                                 // token from the q|k|v projection's split-K slabs itself (what qkv_post_launch would
                                 // have done in a launch of its own) and appends K / V to the cache; `q` is not read
 };
+// Queries of a sequence from which its attention runs on tcgen05 (tiles of 128 queries and 128 keys; head_dim 128) and no longer on
+// mma.sync (64 and 64): half a tile.  12 lanes of the 8B shape, one of them with portions of 100 tokens behind up to 500: 26 us a launch
+// on mma.sync, 13 on tcgen05 (the step's six layers, 10.01 / 9.74 ms); prompts of 20 to 100 tokens and portions of 6 to 12 take the same time on either.
+constexpr int kAttnTcRows = 64;
 int attn_launch(Ctx* c, const AttnArgs& a);
 int decode_splits(Ctx* c, int64_t B, int kvh);  // KV splits a decode attention launch of B sequences x kvh kv heads uses
 size_t attn_scratch_bytes(int64_t B, int nh, int hd, int max_splits);

@@ -674,10 +674,10 @@ int fetch_logits(rewb200_session* s, int64_t rows, float* host) {
 }
 
 // Portions that share an attention launch: the choice of its kernel follows a portion's own length, as if it stood alone
-// (128 tokens and more: tcgen05; fewer: mma.sync; one: split-KV decode).  What follows the step instead: the pieces a Linear is
+// (kAttnTcRows tokens and more: tcgen05 where the model can; fewer: mma.sync; one: split-KV decode).  What follows the step instead: the pieces a Linear is
 // cut into along K (up to 256 rows of the step) and the KV splits of single tokens, both f32 sums in another order.
 enum PortionKind : int { PORTION_LONG = 0, PORTION_SHORT, PORTION_SINGLE };
-PortionKind portion_kind(int n) { return n >= 128 ? PORTION_LONG : n > 1 ? PORTION_SHORT : PORTION_SINGLE; }
+PortionKind portion_kind(int n) { return n >= kAttnTcRows ? PORTION_LONG : n > 1 ? PORTION_SHORT : PORTION_SINGLE; }
 
 // The decoder blocks of a grouped-query model (llama.nim:106-129, deepseek.nim:198-220) over rows = nb*S tokens: embedding
 // and first norm, then every layer; leaves the final norm's output in s->xn.
