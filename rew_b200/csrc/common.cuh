@@ -7,6 +7,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -83,6 +84,10 @@ struct Ctx {
   int option_epoch = 0;      // bumped by rewb200_set_option; captured graphs from older epochs are rebuilt
   void* pinned = nullptr;    // pinned host staging for H2D/D2H of buffers
   size_t pinned_bytes = 0;
+  static constexpr size_t kHomeHalf = 512 * 1024;
+  char* home = nullptr;      // pinned, two halves of kHomeHalf behind `pinned`: results of steps on their way to the host (bring_home)
+  cudaEvent_t ev_home[2] = {};   // a half has arrived
+  std::mutex home_mutex;     // one step's results at a time
 };
 Ctx* ctx_get(int slot);       // nullptr + error when not initialised
 Ctx* ctx_current();           // slot 0

@@ -650,17 +650,63 @@ int moe_routed(rewb200_session* s, MoeDev& X, const void* x, int64_t d, int64_t 
 
 namespace {
 
+struct Piece {
+  const void* dev;
+  void* host;      // NULL: not wanted
+  size_t bytes;
+};
+
+// The results of a step into the caller's memory, behind everything enqueued; returns once they and the device's status word are
+// there (ctx_status).  A copy into pageable memory goes at 4 GB/s (6.5 MB of logits: 1.6 ms); here one half of the slot's pinned ring
+// is emptied while the other one fills.  A second thread that comes for results meanwhile has them copied the other way.
+int bring_home(rewb200_session* s, std::initializer_list<Piece> pieces) {
+  Ctx* c = s->m->c;
+  std::unique_lock<std::mutex> ring(c->home_mutex, std::try_to_lock);
+  Piece on_way[2];
+  auto land = [&](int half) -> int {
+    RB_CUDA(cudaEventSynchronize(c->ev_home[half]));
+    memcpy(on_way[half].host, c->home + half * Ctx::kHomeHalf, on_way[half].bytes);
+    return REWB200_OK;
+  };
+  int sent = 0;
+  for (const Piece& p : pieces) {
+    if (!p.host || p.bytes == 0) continue;
+    if (!ring) {
+      RB_CUDA(cudaMemcpyAsync(p.host, p.dev, p.bytes, cudaMemcpyDeviceToHost, c->stream));
+      continue;
+    }
+    for (size_t at = 0; at < p.bytes; ++sent) {
+      const int half = sent & 1;
+      const size_t n = std::min(Ctx::kHomeHalf, p.bytes - at);
+      if (sent >= 2) RB_TRY(land(half));
+      RB_CUDA(cudaMemcpyAsync(c->home + half * Ctx::kHomeHalf, (const char*)p.dev + at, n, cudaMemcpyDeviceToHost, c->stream));
+      RB_CUDA(cudaEventRecord(c->ev_home[half], c->stream));
+      on_way[half] = {nullptr, (char*)p.host + at, n};
+      at += n;
+    }
+  }
+  RB_CUDA(cudaMemcpyAsync(c->h_status, c->d_status, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  for (int i = std::max(0, sent - 2); i < sent; ++i) RB_TRY(land(i & 1));
+  RB_CUDA(cudaStreamSynchronize(c->stream));
+  return REWB200_OK;
+}
+
+// While the GPU works: has the system find the pages that results will be copied into (their contents stay).  A page of fresh memory
+// costs its first writer more than the copy does.
+void expect_home(void* host, size_t bytes) {
+  if (!host || bytes < 16 * 1024) return;
+  volatile char* p = (volatile char*)host;
+  for (size_t at = 0; at < bytes; at += 4096) p[at] = p[at];
+  p[bytes - 1] = p[bytes - 1];
+}
+
 // Copies the last-position logits [B, vocab] to the host; under tensor parallelism the
 // vocabulary slices are all-gathered first and re-interleaved on the host.
 int fetch_logits(rewb200_session* s, int64_t rows, float* host) {
   rewb200_model* m = s->m;
   Ctx* c = m->c;
   const int tp = m->cfg.tp_size;
-  if (tp == 1) {
-    RB_CUDA(cudaMemcpyAsync(host, s->logits, (size_t)rows * m->cfg.vocab * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
-    RB_CUDA(cudaStreamSynchronize(c->stream));
-    return REWB200_OK;
-  }
+  if (tp == 1) return bring_home(s, {{s->logits, host, (size_t)rows * m->cfg.vocab * sizeof(float)}});
   const size_t per = (size_t)rows * m->vocab_l * sizeof(float);
   RB_REQUIRE(per * tp <= s->gather_bytes, "logit gather buffer too small for this many rows");
   RB_TRY(comm_allgather_bytes(c, m->slot, s->logits, s->gather_scratch, per));
@@ -1804,14 +1850,15 @@ int rewb200_session_forward(rewb200_session* s, const int32_t* ids, int S, int32
   }
   RB_TRY(enqueue_forward(s, o));
   RB_CUDA(cudaEventRecord(s->ev1, c->stream));
-  if (next_ids)
-    RB_CUDA(cudaMemcpyAsync(next_ids, s->d_next, s->B * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-  if (logits_out) RB_TRY(fetch_logits(s, s->B, logits_out));
-  RB_CUDA(cudaStreamSynchronize(c->stream));
+  const size_t logits_bytes = (size_t)s->B * m->cfg.vocab * sizeof(float);
+  expect_home(logits_out, logits_bytes);
+  const bool whole = m->cfg.tp_size == 1;   // a slice of the vocabulary is gathered first
+  if (logits_out && !whole) RB_TRY(fetch_logits(s, s->B, logits_out));
+  RB_TRY(bring_home(s, {{s->d_next, next_ids, s->B * sizeof(int)}, {s->logits, whole ? logits_out : nullptr, logits_bytes}}));
   RB_CUDA(cudaEventElapsedTime(&s->prefill_ms, s->ev0, s->ev1));
   s->host_pos += S;
   if (m->cfg.tp_size > 1 || m->cfg.ep_size > 1) RB_TRY(comm_check_async(m->slot));
-  return ctx_check_status(c);
+  return ctx_status(c);
 }
 
 // n_steps decode steps for every lane of the session (captured once into a CUDA graph, then replayed).
@@ -1861,19 +1908,18 @@ static int decode_core(rewb200_session* s, int n_steps, int32_t* out_ids, float*
     }
   }
   RB_CUDA(cudaEventRecord(s->ev1, c->stream));
-  if (out_ids && n_steps > 0) {
-    // device layout [step][B] -> host [B][n_steps]
-    std::vector<int32_t> tmp((size_t)n_steps * s->B);
-    RB_CUDA(cudaMemcpyAsync(tmp.data(), s->d_out, tmp.size() * sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
-    RB_CUDA(cudaStreamSynchronize(c->stream));
+  const size_t logits_bytes = (size_t)s->B * m->cfg.vocab * sizeof(float);
+  expect_home(last_logits, logits_bytes);
+  const bool whole = m->cfg.tp_size == 1;   // a slice of the vocabulary is gathered first
+  if (last_logits && !whole) RB_TRY(fetch_logits(s, s->B, last_logits));
+  std::vector<int32_t> tmp(out_ids ? (size_t)n_steps * s->B : 0);
+  RB_TRY(bring_home(s, {{s->d_out, tmp.data(), tmp.size() * sizeof(int32_t)}, {s->logits, whole ? last_logits : nullptr, logits_bytes}}));
+  if (out_ids)   // device layout [step][B] -> host [B][n_steps]
     for (int st = 0; st < n_steps; ++st)
       for (int b = 0; b < s->B; ++b) out_ids[(size_t)b * n_steps + st] = tmp[(size_t)st * s->B + b];
-  }
-  if (last_logits) RB_TRY(fetch_logits(s, s->B, last_logits));
-  RB_CUDA(cudaStreamSynchronize(c->stream));
   RB_CUDA(cudaEventElapsedTime(&s->decode_ms, s->ev0, s->ev1));
   if (m->cfg.tp_size > 1 || m->cfg.ep_size > 1) RB_TRY(comm_check_async(m->slot));
-  return ctx_check_status(c);
+  return ctx_status(c);
 }
 
 int rewb200_session_decode(rewb200_session* s, int n_steps, int32_t* out_ids, float* last_logits) {
@@ -2216,20 +2262,19 @@ int rewb200_lanes_feed(rewb200_session* s, int n_entries, const int32_t* lanes, 
     }
   }
   RB_TRY(enqueue_forward(s, o));
-  if (n_want > 0)
-    RB_CUDA(cudaMemcpyAsync(logits_out, s->logits, (size_t)n_want * m->cfg.vocab * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
   feed_lanes_kernel<<<(unsigned)n_entries, 64, 0, c->stream>>>(d_port, nullptr, s->max_pages, s->d_pos, s->d_active, s->block_table);
   RB_CUDA(cudaGetLastError());
   ++g_launch_total;
   RB_CUDA(cudaEventRecord(s->ev1, c->stream));
   std::vector<int> next(s->B, -1);
-  if (any_sample) RB_CUDA(cudaMemcpyAsync(next.data(), s->d_next, s->B * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-  RB_CUDA(cudaStreamSynchronize(c->stream));
+  const size_t logits_bytes = (size_t)n_want * m->cfg.vocab * sizeof(float);
+  expect_home(logits_out, logits_bytes);
+  RB_TRY(bring_home(s, {{s->d_next, any_sample ? next.data() : nullptr, s->B * sizeof(int)}, {s->logits, logits_out, logits_bytes}}));
   RB_CUDA(cudaEventElapsedTime(&s->prefill_ms, s->ev0, s->ev1));
   for (const StepEntry& e : entries) s->lane_len[e.lane] = e.pos0 + e.n;
   if (next_ids)
     for (int e = 0; e < n_entries; ++e) next_ids[e] = act[lanes[e]] ? next[lanes[e]] : -1;
-  return ctx_check_status(c);
+  return ctx_status(c);
 }
 
 int rewb200_lane_release(rewb200_session* s, int lane) {

@@ -188,7 +188,9 @@ int rewb200_init(const int* device_ordinals, int n) {
     RB_CUDA(cudaMemset(c->d_tickets, 0, Ctx::kTickets * sizeof(int)));
     RB_CUDA(cudaMallocHost(&c->h_status, 256));
     c->pinned_bytes = 64u << 20;
-    RB_CUDA(cudaMallocHost(&c->pinned, c->pinned_bytes));
+    RB_CUDA(cudaMallocHost(&c->pinned, c->pinned_bytes + 2 * Ctx::kHomeHalf));
+    c->home = (char*)c->pinned + c->pinned_bytes;
+    for (cudaEvent_t& e : c->ev_home) RB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     cudaMemPool_t pool;
     RB_CUDA(cudaDeviceGetDefaultMemPool(&pool, dev));
     uint64_t thresh = UINT64_MAX;  // keep freed blocks cached in the pool
@@ -218,6 +220,7 @@ int rewb200_shutdown(void) {
     cudaStreamDestroy(c->side);
     cudaEventDestroy(c->ev_fork);
     cudaEventDestroy(c->ev_join);
+    for (cudaEvent_t e : c->ev_home) cudaEventDestroy(e);
     delete c;
   }
   g_ctx.clear();
