@@ -156,7 +156,24 @@ template <> struct Vec4<bf16> {
   }
 };
 
+__device__ __forceinline__ void add4(float4& v, const float4 w) { v.x += w.x; v.y += w.y; v.z += w.z; v.w += w.w; }
+// v += the slabs at p, in order.  G loads are under way together whatever their number: what is left over of an unrolled loop has them
+// wait for one another, half a microsecond each.
+template <int G>
+__device__ __forceinline__ void sum_slabs(float4& v, const float* p, int n, int64_t stride) {
+  for (int s = 0; s < n; s += G) {
+    float4 t[G];
+#pragma unroll
+    for (int j = 0; j < G; ++j)
+      if (s + j < n) t[j] = *reinterpret_cast<const float4*>(p + (s + j) * stride);
+#pragma unroll
+    for (int j = 0; j < G; ++j)
+      if (s + j < n) add4(v, t[j]);
+  }
+}
+
 // Sum of the split-K slabs at element offset `idx` (a multiple of 4), in slab order.
+template <int G = 4>   // above 64 rows there are four slabs at most
 __device__ __forceinline__ float4 partial_sum4(const NormArgs& a, int64_t idx) {
   float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
   if (a.partial_bf16) {
@@ -170,27 +187,12 @@ __device__ __forceinline__ float4 partial_sum4(const NormArgs& a, int64_t idx) {
   }
   const float* pp = a.partial + idx;
   if (a.wait_n > 0) return __ldcg(reinterpret_cast<const float4*>(pp));  // one slab, written by the peers
-  int s = 0;
-  for (; s + 4 <= a.nsplit; s += 4) {
-    const float4 p0 = *reinterpret_cast<const float4*>(pp + (s + 0) * a.split_stride);
-    const float4 p1 = *reinterpret_cast<const float4*>(pp + (s + 1) * a.split_stride);
-    const float4 p2 = *reinterpret_cast<const float4*>(pp + (s + 2) * a.split_stride);
-    const float4 p3 = *reinterpret_cast<const float4*>(pp + (s + 3) * a.split_stride);
-    p.x += p0.x; p.y += p0.y; p.z += p0.z; p.w += p0.w;
-    p.x += p1.x; p.y += p1.y; p.z += p1.z; p.w += p1.w;
-    p.x += p2.x; p.y += p2.y; p.z += p2.z; p.w += p2.w;
-    p.x += p3.x; p.y += p3.y; p.z += p3.z; p.w += p3.w;
-  }
-  for (; s < a.nsplit; ++s) {
-    const float4 p0 = *reinterpret_cast<const float4*>(pp + s * a.split_stride);
-    p.x += p0.x; p.y += p0.y; p.z += p0.z; p.w += p0.w;
-  }
+  sum_slabs<G>(p, pp, a.nsplit, a.split_stride);
   return p;
 }
 
 // What a block with several branches, or a stack that runs layers several times, adds on top (NormArgs::partial2, partial3,
 // add_embed, add_vec) at column i of a row; idx = row * d + i.
-__device__ __forceinline__ void add4(float4& v, const float4 w) { v.x += w.x; v.y += w.y; v.z += w.z; v.w += w.w; }
 __device__ __forceinline__ float4 partial2_sum4(const NormArgs& a, int64_t idx) {
   float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 4
@@ -356,9 +358,10 @@ __device__ __forceinline__ void tp_exchange4_two(const NormArgs& a, float4 (&p)[
 }
 
 template <typename TE, typename TO, int NCH>
-__global__ void __launch_bounds__(NORMV_THREADS) residual_norm_vec_kernel(NormArgs a) {
+__global__ void __launch_bounds__(NORMV_THREADS, NCH <= 2 ? 2 : 1) residual_norm_vec_kernel(NormArgs a) {
   __shared__ float red[33];
   pdl_launch_dependents();
+  if (a.norm_kind >= 0) prefetch_floats(a.gamma, (int)a.d);   // depends on no earlier kernel
   pdl_wait();
   if (a.wait_n > 0) peer_flags_wait(a.wait_cells, 1, a.wait_n, -1, *a.wait_epoch + a.wait_offset, a.status);
   const int64_t row = blockIdx.x;
@@ -376,8 +379,15 @@ __global__ void __launch_bounds__(NORMV_THREADS) residual_norm_vec_kernel(NormAr
     }
     erow = reinterpret_cast<const TE*>(a.embed) + id * d;
   }
-  float4 vals[NCH];
+  float4 vals[NCH], xin[NCH];
   const bool summed = a.partial != nullptr;
+  // the residual (or embedding) row is requested ahead of the slabs
+#pragma unroll
+  for (int c = 0; c < NCH; ++c) {
+    const int64_t i = ((int64_t)c * NORMV_THREADS + threadIdx.x) * 4;
+    xin[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (i < d) xin[c] = erow && !a.add_embed ? Vec4<TE>::load(erow + i) : *reinterpret_cast<const float4*>(xr + i);
+  }
   if (summed) {
     int64_t idx[NCH];
 #pragma unroll
@@ -396,7 +406,7 @@ __global__ void __launch_bounds__(NORMV_THREADS) residual_norm_vec_kernel(NormAr
     const int64_t i = ((int64_t)c * NORMV_THREADS + threadIdx.x) * 4;
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     if (i < d) {
-      v = erow && !a.add_embed ? Vec4<TE>::load(erow + i) : *reinterpret_cast<const float4*>(xr + i);
+      v = xin[c];
       if (summed) {
         float4 p = vals[c];
         if (a.nsplit2 > 0) add4(p, partial2_sum4(a, row * d + i));
@@ -530,7 +540,7 @@ __global__ void __launch_bounds__(NORMV_THREADS, 2) residual_norm_rows_kernel(No
 // Sublayers normed on the way back (OutputNormArgs): x += gamma * y / rms(y), y the sum of the slabs.  CL CTAs of a
 // cluster share a row (decode-size steps), their sums of squares meet through distributed shared memory.
 template <typename T, int CL, int NCH>
-__global__ void __launch_bounds__(CL == 1 ? 512 : 256) output_norm_kernel(OutputNormArgs a) {
+__global__ void __launch_bounds__(CL == 1 ? 512 : 256, NCH <= 2 ? 2 : 1) output_norm_kernel(OutputNormArgs a) {
   constexpr int THREADS = CL == 1 ? 512 : 256;
   __shared__ float red[33];
   __shared__ float part[2];
@@ -579,12 +589,14 @@ __global__ void __launch_bounds__(CL == 1 ? 512 : 256) output_norm_kernel(Output
     } else if (!a.replace) {
       x[c] = *reinterpret_cast<const float4*>(xr + i);
     }
-    const int64_t at = row * d + col0 + i;
     if (a.bias) y[c] = *reinterpret_cast<const float4*>(a.bias + col0 + i);
-#pragma unroll 8
-    for (int s = 0; s < a.nsplit; ++s) add4(y[c], *reinterpret_cast<const float4*>(a.partial + s * a.split_stride + at));
-#pragma unroll 4
-    for (int s = 0; s < a.nsplit2; ++s) add4(y[c], *reinterpret_cast<const float4*>(a.partial2 + s * a.split_stride + at));
+  }
+#pragma unroll
+  for (int c = 0; c < NCH; ++c) {
+    const int64_t i = ((int64_t)c * THREADS + threadIdx.x) * 4, at = row * d + col0 + i;
+    if (i >= dq) continue;
+    sum_slabs<CL == 1 ? 4 : 8>(y[c], a.partial + at, a.nsplit, a.split_stride);
+    sum_slabs<4>(y[c], a.partial2 + at, a.nsplit2, a.split_stride);
     ss += y[c].x * y[c].x + y[c].y * y[c].y + y[c].z * y[c].z + y[c].w * y[c].w;
   }
   if (a.replace) {
@@ -639,6 +651,7 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(256) residual_norm_c
   const int64_t d = a.d, dq = d >> 2, col0 = (int64_t)rank * dq;
   float* xr = a.x_res + row * d;
   float4 vals[NCH];
+  prefetch_floats(a.gamma + col0, (int)dq);   // depends on no earlier kernel
   pdl_wait();
   const TE* erow = nullptr;
   if (a.embed) {
@@ -655,11 +668,13 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(256) residual_norm_c
   const bool summed = a.partial != nullptr;
   // the residual (or embedding) row is requested first, so that its latency runs under the slab loads and,
   // with tensor parallelism, under the exchange
-  float4 xin[NCH];
+  float4 xin[NCH], gamma[NCH], bias[NCH];
 #pragma unroll
   for (int c = 0; c < NCH; ++c) {
     const int64_t off = ((int64_t)c * 256 + threadIdx.x) * 4;
-    xin[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+    xin[c] = gamma[c] = bias[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (off < dq) gamma[c] = *reinterpret_cast<const float4*>(a.gamma + col0 + off);
+    if (off < dq && summed && a.bias) bias[c] = *reinterpret_cast<const float4*>(a.bias + col0 + off);
     if (off < dq) xin[c] = erow && !a.add_embed ? Vec4<TE>::load(erow + col0 + off) : *reinterpret_cast<const float4*>(xr + col0 + off);
   }
   if (summed) {
@@ -668,7 +683,7 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(256) residual_norm_c
     for (int c = 0; c < NCH; ++c) {
       const int64_t off = ((int64_t)c * 256 + threadIdx.x) * 4;
       idx[c] = off < dq ? row * d + col0 + off : -1;
-      vals[c] = off < dq ? partial_sum4(a, idx[c]) : make_float4(0.f, 0.f, 0.f, 0.f);
+      vals[c] = off < dq ? partial_sum4<8>(a, idx[c]) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     if (a.n_peers > 0) {
       if (a.two_shot) tp_exchange4_two<NCH>(a, vals, idx);
@@ -686,10 +701,7 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(256) residual_norm_c
         float4 p = vals[c];
         if (a.nsplit2 > 0) add4(p, partial2_sum4(a, row * d + i));
         if (a.nsplit3 > 0) add4(p, partial3_sum4(a, row, row * d + i));
-        if (a.bias) {
-          const float4 b = *reinterpret_cast<const float4*>(a.bias + i);
-          p.x += b.x; p.y += b.y; p.z += b.z; p.w += b.w;
-        }
+        if (a.bias) add4(p, bias[c]);
         v.x += p.x; v.y += p.y; v.z += p.z; v.w += p.w;
       }
       if (erow && a.add_embed) add4(v, Vec4<TE>::load(erow + i));
@@ -735,7 +747,7 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(256) residual_norm_c
     const int64_t off = ((int64_t)c * 256 + threadIdx.x) * 4;
     if (off >= dq) continue;
     const int64_t i = col0 + off;
-    const float4 g = *reinterpret_cast<const float4*>(a.gamma + i);
+    const float4 g = gamma[c];
     float4 o;
     if (a.norm_kind == 0) {
       const float4 u = make_float4(vals[c].x / scale, vals[c].y / scale, vals[c].z / scale, vals[c].w / scale);
@@ -779,12 +791,18 @@ __global__ void __launch_bounds__(256) qkv_post_vec_kernel(QkvPostArgs a) {
   // the slabs first: they are the bytes, and the position and page of the row are two loads in turn
   float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   const float* pp = a.partial + row * ntot + col;
-  for (int sp = 0; sp < a.nsplit; ++sp) {
-    const float4 t0 = *reinterpret_cast<const float4*>(pp + sp * a.split_stride);
-    const float4 t1 = *reinterpret_cast<const float4*>(pp + sp * a.split_stride + 4);
-    v[0] += t0.x; v[1] += t0.y; v[2] += t0.z; v[3] += t0.w;
-    v[4] += t1.x; v[5] += t1.y; v[6] += t1.z; v[7] += t1.w;
+  float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
+  for (int sp = 0; sp < a.nsplit; sp += 4) {
+    float4 t[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (sp + j / 2 < a.nsplit) t[j] = *reinterpret_cast<const float4*>(pp + (sp + j / 2) * a.split_stride + 4 * (j & 1));
+#pragma unroll
+    for (int j = 0; j < 8; j += 2)
+      if (sp + j / 2 < a.nsplit) add4(lo, t[j]), add4(hi, t[j + 1]);
   }
+  v[0] = lo.x; v[1] = lo.y; v[2] = lo.z; v[3] = lo.w;
+  v[4] = hi.x; v[5] = hi.y; v[6] = hi.z; v[7] = hi.w;
   const int b = a.row_seq ? a.row_seq[row] : (int)(row / a.S), s = a.row_seq ? (int)row - a.seq[b].x : (int)(row % a.S);
   const int pos = a.pos0[b] + s;
   const int hd = a.hd;
