@@ -280,9 +280,14 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(const __grid_constant_
   const int tps = (ntiles + a.nsplit - 1) / a.nsplit;
   const int t0 = split * tps, t1 = min(ntiles, t0 + tps);
   const int nt_local = max(0, t1 - t0);
+  // The CTA with a sequence's last tile finishes the newest K / V row itself (below).  It asks for that tile early as well, as long
+  // as it is among the first, and puts the row into its copy: through memory and a bulk copy behind the row's stores, the
+  // tile arrived 1.5 us later.
+  const bool owns_last = ntiles > 0 && t0 <= ntiles - 1 && ntiles - 1 < t1;
+  const bool patch = a.f_partial && a.early_kv && owns_last && nt_local <= ATT_STAGES - 1;
   int early = 0;
   if (threadIdx.x == 0 && a.early_kv)
-    for (; early < min(ATT_STAGES - 1, nt_local) && t0 + early < ntiles - 1; ++early)
+    for (; early < min(ATT_STAGES - 1, nt_local) && (t0 + early < ntiles - 1 || patch); ++early)
       load_tile<HD>(smem + early * T::STAGE_BYTES, &full[early], &tmK, &tmV, tile_row0(a, b, hk, t0 + early));
   pdl_wait();
 
@@ -295,39 +300,64 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(const __grid_constant_
     const float* cr = a.f_cos + (int64_t)(pos_ok ? rpos : 0) * HD;
     const float* sr = a.f_sin + (int64_t)(pos_ok ? rpos : 0) * HD;
     const int nq = a.nh * HD, nkv = a.kvh * HD;
-    auto pair_at = [&](int col, bool rope, int e) -> uint32_t {  // e: element index of the pair inside its head
-      float v0 = 0.f, v1 = 0.f;
-      for (int sp = 0; sp < a.f_ks; ++sp) {
-        const float2 p2 = *reinterpret_cast<const float2*>(pr + sp * a.f_stride + col);
-        v0 += p2.x;
-        v1 += p2.y;
+    const int q_pairs = a.group * (HD / 2), pairs = q_pairs + (owns_last && pos_ok ? HD : 0);   // q, then HD / 2 of k and of v
+    const int64_t crow = owns_last && pos_ok ? kv_row(a, b, hk, pos) * HD : 0;
+    const uint32_t tile_k = smem_u32(smem) + (nt_local - 1) * T::STAGE_BYTES;
+    if (patch && pos_ok) mbar_wait(&full[nt_local - 1], 0, a.status);
+    // Three pairs a thread at a time (all of them with four query heads a group), and all that they need requested before any of
+    // it is used: pair by pair, slab by slab, then bias, then angle, this stretch took 3 us of a launch's 9.
+    constexpr int U = 3;
+    for (int p0 = threadIdx.x; p0 < pairs; p0 += U * 128) {
+      float2 v[U], bias[U];
+      float c[U], s[U];
+      int col[U], e[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int p = min(p0 + u * 128, pairs - 1), k = p - q_pairs;
+        e[u] = 2 * (k < 0 ? p % (HD / 2) : k % (HD / 2));
+        col[u] = k < 0 ? (hk * a.group + p / (HD / 2)) * HD + e[u] : (k < HD / 2 ? nq : nq + nkv) + hk * HD + e[u];
+        v[u] = bias[u] = make_float2(0.f, 0.f);
+        if (a.f_bias) bias[u] = *reinterpret_cast<const float2*>(a.f_bias + col[u]);
+        c[u] = cr[e[u]];
+        s[u] = sr[e[u]];
       }
-      if (a.f_bias) {
-        v0 += a.f_bias[col];
-        v1 += a.f_bias[col + 1];
+      for (int sp = 0; sp < a.f_ks; sp += 4) {
+        float2 x[U][4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+          for (int u = 0; u < U; ++u)
+            if (sp + j < a.f_ks) x[u][j] = *reinterpret_cast<const float2*>(pr + (sp + j) * a.f_stride + col[u]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+          for (int u = 0; u < U; ++u)
+            if (sp + j < a.f_ks) {
+              v[u].x += x[u][j].x;
+              v[u].y += x[u][j].y;
+            }
       }
-      if (rope) {
-        const float c0 = cr[e], s0 = sr[e];
-        const float r0 = rope_even(c0, s0, v0, v1), r1 = rope_odd(c0, s0, v0, v1);
-        v0 = r0;
-        v1 = r1;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int p = p0 + u * 128, k = p - q_pairs;
+        if (p >= pairs) break;
+        if (a.f_bias) {
+          v[u].x += bias[u].x;
+          v[u].y += bias[u].y;
+        }
+        const uint32_t rot = pack_bf16(rope_even(c[u], s[u], v[u].x, v[u].y), rope_odd(c[u], s[u], v[u].x, v[u].y));
+        if (k < 0) {
+          sQ[p] = rot;
+          continue;
+        }
+        const bool is_k = k < HD / 2;
+        const uint32_t word = is_k ? rot : pack_bf16(v[u].x, v[u].y);
+        *reinterpret_cast<uint32_t*>(reinterpret_cast<bf16*>(const_cast<void*>(is_k ? a.k : a.v)) + crow + e[u]) = word;
+        if (patch)
+          asm volatile("st.shared.b32 [%0], %1;" ::"r"(kv_addr<HD>(tile_k + (is_k ? 0 : T::KV_BYTES), pos % TILE, e[u] / 8) + (e[u] % 8) * 2), "r"(word) : "memory");
       }
-      return pack_bf16(v0, v1);
-    };
-    for (int p = threadIdx.x; p < a.group * (HD / 2); p += blockDim.x) {
-      const int row = p / (HD / 2), e = 2 * (p % (HD / 2));
-      sQ[p] = pair_at((hk * a.group + row) * HD + e, true, e);
     }
-    const bool owns_last = ntiles > 0 && t0 <= ntiles - 1 && ntiles - 1 < t1;
-    if (owns_last && pos_ok) {
-      const int64_t crow = kv_row(a, b, hk, pos) * HD;
-      for (int p = threadIdx.x; p < HD; p += blockDim.x) {  // HD / 2 pairs of k, then HD / 2 pairs of v
-        const bool is_k = p < HD / 2;
-        const int e = 2 * (is_k ? p : p - HD / 2);
-        const uint32_t pk = pair_at((is_k ? nq : nq + nkv) + hk * HD + e, is_k, e);
-        bf16* dst = reinterpret_cast<bf16*>(const_cast<void*>(is_k ? a.k : a.v)) + crow + e;
-        *reinterpret_cast<uint32_t*>(dst) = pk;
-      }
+    if (owns_last && pos_ok && !patch) {
       // the row is read back by the bulk tensor copy of the last tile (async proxy): order the stores before it
       __threadfence();
       asm volatile("fence.proxy.async.global;" ::: "memory");
