@@ -1350,15 +1350,21 @@ int gla_mixer(rewb200_session* s, const FwdOpts& o, const StepLists& t, size_t r
   ga.dtype = m->cfg.dtype;
   ga.early = in_graph ? 1 : 0;
   ga.status = c->d_status;
-  RB_TRY(gla_recurrent_launch(c, ga));
-  if (!t.uniform && s->plan_gla_large > 0) {
-    ga.list = t.gla_large;
-    ga.count = s->plan_gla_large;
-    ga.chunks = t.gla_chunks;
-    ga.n_chunks = s->plan_gla_chunks;
-    ga.work = s->gla_work;
-    RB_TRY(gla_chunk_launch(c, ga));
+  // single tokens run beside the walk over the portions' chunks: 16 heads, 15 single tokens and a portion of 61, 34 us behind
+  // the portion's preparation one after the other, 30 together
+  GlaArgs large = ga;
+  const bool portions = !t.uniform && s->plan_gla_large > 0;
+  if (portions) {
+    ga.beside = large.beside = ga.count > 0 ? 1 : 0;
+    large.list = t.gla_large;
+    large.count = s->plan_gla_large;
+    large.chunks = t.gla_chunks;
+    large.n_chunks = s->plan_gla_chunks;
+    large.work = s->gla_work;
+    RB_TRY(gla_prepare_launch(c, large));
   }
+  RB_TRY(gla_recurrent_launch(c, ga));
+  if (portions) RB_TRY(gla_scan_launch(c, large));
   if (o.trace) RB_TRY(o.trace->mark(TC_ATTN));
   return REWB200_OK;
 }
@@ -1514,15 +1520,20 @@ int delta_mixer(rewb200_session* s, const FwdOpts& o, const StepLists& t, size_t
   da.dtype = m->cfg.dtype;
   da.early = in_graph ? 1 : 0;
   da.status = c->d_status;
-  RB_TRY(delta_recurrent_launch(c, da));
-  if (!t.uniform && s->plan_delta_large > 0) {
-    da.list = t.delta_large;
-    da.count = s->plan_delta_large;
-    da.chunks = t.delta_chunks;
-    da.n_chunks = s->plan_delta_chunks;
-    da.work = s->gla_work;
-    RB_TRY(delta_chunk_launch(c, da));
+  // as in gla_mixer: single tokens beside the walk over the portions' chunks
+  DeltaArgs large = da;
+  const bool portions = !t.uniform && s->plan_delta_large > 0;
+  if (portions) {
+    da.beside = large.beside = da.count > 0 ? 1 : 0;
+    large.list = t.delta_large;
+    large.count = s->plan_delta_large;
+    large.chunks = t.delta_chunks;
+    large.n_chunks = s->plan_delta_chunks;
+    large.work = s->gla_work;
+    RB_TRY(delta_prepare_launch(c, large));
   }
+  RB_TRY(delta_recurrent_launch(c, da));
+  if (portions) RB_TRY(delta_scan_launch(c, large));
   if (o.trace) RB_TRY(o.trace->mark(TC_ATTN));
   return REWB200_OK;
 }

@@ -39,6 +39,8 @@ struct DeltaArgs {
   int64_t ldo;
   int dtype;
   int early;               // captured decode step: state and positions predate the step
+  int beside;              // single tokens and portions of a step at the same time: the launch of single tokens lets the next one start once it has passed
+                           // its own wait (what it reads is then there for both), and the walk over portions waits for it at its end
   int* status;
 };
 int delta_recurrent_launch(Ctx* c, const DeltaArgs& a);
@@ -47,6 +49,7 @@ bool delta_chunk_ok(const DeltaDims& m);
 int delta_chunks(int n);                                  // chunks of a portion of n tokens
 int2 delta_chunk_rows(const GlaPortion& p, int i);        // first row and tokens of its i-th chunk
 size_t delta_chunk_bytes(const DeltaDims& m);             // scratch of one chunk, all heads
-int delta_chunk_launch(Ctx* c, const DeltaArgs& a);
+int delta_prepare_launch(Ctx* c, const DeltaArgs& a);
+int delta_scan_launch(Ctx* c, const DeltaArgs& a);
 
 }  // namespace rewb

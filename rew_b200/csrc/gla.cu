@@ -117,7 +117,7 @@ template <typename T, int NT, int KI>
 __global__ void __launch_bounds__(NT, NT == 128 ? (KI <= 16 ? 4 : 3) : KI <= 8 ? 2 : 1) gla_recurrent_kernel(GlaArgs a, int slices) {
   extern __shared__ __align__(16) float sm[];
   __shared__ float red[NT / 32];
-  pdl_launch_dependents();
+  if (!a.beside) pdl_launch_dependents();
   const GlaDims& m = a.m;
   const int h = blockIdx.x, K = m.dim, V = m.vdim, vq = a.ldv / 4;
   // weights depend on no earlier kernel
@@ -137,6 +137,7 @@ __global__ void __launch_bounds__(NT, NT == 128 ? (KI <= 16 ? 4 : 3) : KI <= 8 ?
 #pragma unroll
   for (int i = 0; i < KI; ++i) S[i] = i < held ? *reinterpret_cast<const float4*>(st + i * step) : make_float4(0.f, 0.f, 0.f, 0.f);
   if (a.early) pdl_wait();
+  if (a.beside) pdl_launch_dependents();
   if (threadIdx.x < (unsigned)(a.ldv - V)) s.v[V + threadIdx.x] = 0.f;
   for (int t = 0; t < p.n; ++t) {
     load_token<NT>(a, s, h, p.row0 + t);
@@ -179,8 +180,9 @@ template <typename T, int NT>
 __global__ void __launch_bounds__(NT) gla_plain_kernel(GlaArgs a) {
   extern __shared__ __align__(16) float sm[];
   __shared__ float red[NT / 32];
-  pdl_launch_dependents();
+  if (!a.beside) pdl_launch_dependents();
   pdl_wait();
+  if (a.beside) pdl_launch_dependents();
   const GlaDims& m = a.m;
   const int h = blockIdx.x, K = m.dim, V = m.vdim;
   const GlaPortion p = portion_of(a, blockIdx.y);

@@ -40,6 +40,8 @@ struct GlaArgs {
   int64_t ldo;
   int dtype;
   int early;               // captured decode step: state and positions predate the step
+  int beside;              // single tokens and portions of a step at the same time: the launch of single tokens lets the next one start once it has passed
+                           // its own wait (what it reads is then there for both), and the walk over portions waits for it at its end
   int* status;
 };
 int64_t gla_state_ld(int vdim);
@@ -48,6 +50,7 @@ bool gla_chunk_ok(const GlaDims& m);
 int gla_chunks(int n);                                  // chunks of a portion of n tokens
 int2 gla_chunk_rows(const GlaPortion& p, int i);        // first row and tokens of its i-th chunk
 size_t gla_chunk_bytes(const GlaDims& m);               // scratch of one chunk, all heads
-int gla_chunk_launch(Ctx* c, const GlaArgs& a);
+int gla_prepare_launch(Ctx* c, const GlaArgs& a);
+int gla_scan_launch(Ctx* c, const GlaArgs& a);
 
 }  // namespace rewb

@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(CLUSTER ? NT / 2 : NT, CLUSTER ? 3 : 2) gla_sc
   }
   pdl_launch_dependents();
   __syncthreads();
-  pdl_wait();
+  if (!a.beside) pdl_wait();
   const GlaPortion p = a.list[blockIdx.z];
   const int chunks = (p.n + C - 1) / C;
   auto load = [&](int c) {
@@ -523,6 +523,7 @@ __global__ void __launch_bounds__(CLUSTER ? NT / 2 : NT, CLUSTER ? 3 : 2) gla_sc
       }
   }
   if constexpr (CLUSTER) cg::this_cluster().sync();   // a peer may still read this CTA's sums
+  if (a.beside) pdl_wait();                           // whoever waits for this launch means the single tokens too
 }
 
 }  // namespace
@@ -532,7 +533,7 @@ int gla_chunks(int n) { return (n + C - 1) / C; }
 int2 gla_chunk_rows(const GlaPortion& p, int i) { return make_int2(p.row0 + i * C, std::min(C, p.n - i * C)); }
 size_t gla_chunk_bytes(const GlaDims& m) { return (size_t)m.heads * layout_of(m).bytes; }
 
-int gla_chunk_launch(Ctx* c, const GlaArgs& a) {
+int gla_prepare_launch(Ctx* c, const GlaArgs& a) {
   if (a.count == 0) return REWB200_OK;
   RB_REQUIRE(gla_chunk_ok(a.m) && a.dtype == REWB200_BF16 && a.list && a.chunks && a.work, "gated linear attention: sizes without a chunk kernel");
   const ChunkLayout cl = layout_of(a.m);
@@ -540,6 +541,12 @@ int gla_chunk_launch(Ctx* c, const GlaArgs& a) {
   RB_CUDA(cudaFuncSetAttribute(gla_prepare_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, prep_smem));
   RB_CUDA(launch_k(gla_prepare_kernel, dim3((unsigned)a.m.heads, (unsigned)a.n_chunks), dim3(NT), prep_smem, c->stream, c->use_pdl, a, cl));
   ++g_launch_total;
+  return REWB200_OK;
+}
+
+int gla_scan_launch(Ctx* c, const GlaArgs& a) {
+  if (a.count == 0) return REWB200_OK;
+  const ChunkLayout cl = layout_of(a.m);
   // few portions: a cluster of CTAs shares a head's value columns
   int nv = 1;
   while (nv < 4 && cl.vp % (nv * 2 * 16) == 0 && (int64_t)nv * a.m.heads * a.count < c->sm_count) nv *= 2;
