@@ -124,16 +124,33 @@ __global__ void __launch_bounds__(128) attn_f32_kernel(AttnDev a) {
   const float* V = reinterpret_cast<const float*>(a.v);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
 
-  for (int j = warp; j < kv_len; j += nw) {
-    const float* kr = K + kv_row(a, b, hk, j) * hd;
-    float d = 0.f;
-    for (int e = lane; e < hd; e += 32) d += q[e] * kr[e];
-    d = warp_sum(d);
-    if (lane == 0) {
-      float s = d * a.scale;
-      if (a.causal) s = s + (visible(a, i, j, ctx) ? 0.0f : -1e9f);
-      scores[j] = s;
+  // four keys of a warp are under way together: the row of a key, the key and its sum each wait for the last (a launch over 20 keys, one
+  // query of 8 heads of 32: 5.0 us, now 4.6)
+  constexpr int AT_ONCE = 4;
+  for (int j0 = warp; j0 < kv_len; j0 += AT_ONCE * nw) {
+    const float* kr[AT_ONCE];
+    float d[AT_ONCE];
+#pragma unroll
+    for (int u = 0; u < AT_ONCE; ++u) {
+      kr[u] = K + kv_row(a, b, hk, min(j0 + u * nw, kv_len - 1)) * hd;
+      d[u] = 0.f;
     }
+    for (int e = lane; e < hd; e += 32) {
+      const float qe = q[e];
+#pragma unroll
+      for (int u = 0; u < AT_ONCE; ++u) d[u] += qe * kr[u][e];
+    }
+#pragma unroll
+    for (int u = 0; u < AT_ONCE; ++u) d[u] = warp_sum(d[u]);
+    if (lane == 0)
+#pragma unroll
+      for (int u = 0; u < AT_ONCE; ++u) {
+        const int j = j0 + u * nw;
+        if (j >= kv_len) break;
+        float s = d[u] * a.scale;
+        if (a.causal) s = s + (visible(a, i, j, ctx) ? 0.0f : -1e9f);
+        scores[j] = s;
+      }
   }
   __syncthreads();
   float mx = -INFINITY;
@@ -166,6 +183,7 @@ __global__ void __launch_bounds__(128) attn_f32_kernel(AttnDev a) {
     const int grp = threadIdx.x / min(hd, (int)blockDim.x);
     float acc = 0.f;
     if (d < hd && grp < ngroups)
+#pragma unroll 4
       for (int j = grp; j < kv_len; j += ngroups) acc += scores[j] * V[kv_row(a, b, hk, j) * hd + d];
     red[threadIdx.x] = acc;
     __syncthreads();

@@ -53,9 +53,11 @@ __global__ void scatter_cols_f32_kernel(const float* src, int64_t src_ld, int64_
 
 // f32 path: out[r][c] = silu(gu[r][c]) * gu[r][f + c]   (src/rew/nn/gated_ffn.nim:55-59)
 __global__ void swiglu_rows_f32_kernel(const float* gu, float* out, int64_t rows, int64_t f) {
+  pdl_launch_dependents();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= rows * f) return;
   const int64_t r = i / f, c = i % f;
+  pdl_wait();
+  if (i >= rows * f) return;
   const float x = gu[r * 2 * f + c];
   const float sig = 1.0f / (1.0f + expf(-x));
   out[i] = (x * sig) * gu[r * 2 * f + f + c];
@@ -293,8 +295,7 @@ int acts_alloc(Ctx* c, T** p, size_t bytes) {
 
 int swiglu_rows_f32_launch(Ctx* c, const float* gu, float* out, int64_t rows, int64_t f) {
   const int64_t n = rows * f;
-  swiglu_rows_f32_kernel<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(gu, out, rows, f);
-  RB_CUDA(cudaGetLastError());
+  RB_CUDA(launch_k(swiglu_rows_f32_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, c->stream, c->use_pdl, gu, out, rows, f));
   ++g_launch_total;
   return REWB200_OK;
 }
@@ -991,10 +992,7 @@ int gqa_blocks(rewb200_session* s, const FwdOpts& o, const NormArgs& na, int64_t
         RB_TRY(run_linear(s, L.gu, s->xn, d, rows, false, EPI_SWIGLU_BF16, s->h, L.ffn_local, nullptr));
       } else {
         RB_TRY(run_linear(s, L.gu, s->xn, d, rows, false, EPI_BIAS_F32, s->gu32, 2 * L.ffn_local, nullptr));
-        const int64_t n = rows * L.ffn_local;
-        swiglu_rows_f32_kernel<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(s->gu32, (float*)s->h, rows, L.ffn_local);
-        RB_CUDA(cudaGetLastError());
-        ++g_launch_total;
+        RB_TRY(swiglu_rows_f32_launch(c, s->gu32, (float*)s->h, rows, L.ffn_local));
       }
       if (o.trace) RB_TRY(o.trace->mark(TC_GATE_UP));
       RB_TRY(run_row_parallel(L.down, s->h, L.ffn_local, &ks));
