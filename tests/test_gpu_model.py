@@ -381,3 +381,23 @@ def test_bf16_norms_of_large_steps(rb, orc, d, heads, routed, S):
     logits = rb.CausalLM(cfg).load(t).session(1, S).forward_all(prompt)
     want = orc.model_forward(cfg, t, prompt, 0, True)
     assert rel_l2(logits, want) <= 2e-2
+
+
+@pytest.mark.parametrize("B,vocab", [(1, 131072), (2, 65537), (5, 120011)])
+def test_logits_of_any_size_come_home_whole(rb, orc, B, vocab):
+    """Results travel in pieces of 512 KB: exactly one, one and a few bytes, several with a ragged end; behind a prompt, behind decode
+    steps and from a step of portions.  f32 sums of d products against the oracle."""
+    cfg = W.ModelConfig(vocab=vocab, d_model=64, n_layers=1, n_heads=2, n_kv_heads=1, head_dim=32, ffn=64, max_seq=32, theta=10000.0, mask_kind=1)
+    t = W.init_weights(cfg, seed=3)
+    prompt = np.random.default_rng(B).integers(0, vocab, size=(B, 5)).astype(np.int32)
+    model = rb.CausalLM(cfg).load(t)
+    sess = model.session(B, 16)
+    nxt, logits = sess.forward(prompt, want_logits=True)
+    want = orc.model_forward(cfg, t, prompt, 0, True)[:, -1]
+    assert rel_l2(logits, want) <= 1e-5 and np.array_equal(nxt, logits.argmax(1))
+    ids, last = sess.decode(2, want_logits=True)
+    seq = np.concatenate([prompt, nxt[:, None], ids[:, :1]], 1)
+    want = orc.model_forward(cfg, t, seq, 0, True)[:, -1]
+    assert rel_l2(last, want) <= 1e-5 and np.array_equal(ids[:, 1], last.argmax(1))
+    fed = model.paged_session(B, 16, B + 2).feed([(b, prompt[b]) for b in range(B)], want=[5 * b + 4 for b in range(B)], sample=True)
+    assert rel_l2(fed[0], logits) <= 1e-5 and np.array_equal(fed[1], nxt)
