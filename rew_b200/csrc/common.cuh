@@ -123,7 +123,6 @@ void nf4_free(Nf4W* w);
 int nf4_quantize_launch(Ctx* c, const void* src, int src_dtype, int64_t ld, ColMap cm, const Nf4W& w);
 int nf4_dequant_launch(Ctx* c, const Nf4W& w, bf16* dst, int64_t ld, ColMap cm);
 int nf4_codes_launch(Ctx* c, const Nf4W& w, uint8_t* codes);
-int nf4_pick_ksplit(Ctx* c, int64_t K, int64_t N);
 int nf4_pick_ksplit(Ctx* c, int64_t K, int64_t N, int64_t M);  // rows of the step: up to four run on the CUDA-core GEMV
 // out: [ksplit][M][N] f32 partial sums of x[M,K] @ W (no bias); 1 <= M <= 32
 int nf4_gemv_launch(Ctx* c, const Nf4W& w, const bf16* x, int64_t ldx, int64_t M, int ksplit, float* out);

@@ -163,7 +163,8 @@ constexpr int NT_CST = 14;                   // code stages: 60 KB of packed wei
 constexpr int NT_DEQ = 8;                    // dequantiser warps
 constexpr int NT_THREADS = (2 + NT_DEQ) * 32;
 constexpr int NT_ABUF = 4;                   // weight-operand buffers in tensor memory
-constexpr int NT_TMEM_COLS = 256;            // D: columns 0-31; A buffer b: columns 32 + 32 b .. +31
+constexpr int NT_TMEM_COLS = 256;            // D: columns 0-31 and 160-191; A buffer b: columns 32 + 32 b .. +31
+constexpr int NT_D1 = 160;
 constexpr int NT_LUT_BYTES = 256 * 32 * 4;
 constexpr int NT_SMEM = NT_XRING + NT_CST * NF4_BLOCK + NT_LUT_BYTES + 512 + 1024;
 
@@ -174,7 +175,8 @@ __device__ __forceinline__ uint32_t hmul2_bf16(uint32_t a, uint32_t b) {
 }
 
 __global__ void __launch_bounds__(NT_THREADS) nf4_tc_kernel(const __grid_constant__ CUtensorMap tmX, const uint8_t* __restrict__ q,
-                                                            int M, int tn, int64_t K, int64_t N, int kb_per_split, float* __restrict__ out, int* status) {
+                                                            int M, int tn, int64_t K, int64_t N, int kb_per_split, int span, int slabs,
+                                                            float* __restrict__ out, int* status) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* xs = smem;                                                    // [xst] activation tiles
@@ -186,14 +188,16 @@ __global__ void __launch_bounds__(NT_THREADS) nf4_tc_kernel(const __grid_constan
   uint64_t* c_empty = c_full + NT_CST;      // [NT_CST]
   uint64_t* a_full = c_empty + NT_CST;      // [NT_ABUF]
   uint64_t* a_empty = a_full + NT_ABUF;     // [NT_ABUF]
-  uint64_t* d_full = a_empty + NT_ABUF;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(d_full + 1);
+  uint64_t* d_full = a_empty + NT_ABUF;     // [2]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(d_full + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tile = blockIdx.x, split = blockIdx.y;
-  const int KB = (int)(K / 64);
-  const int kb0 = split * kb_per_split;
-  const int nkb = max(0, min(kb_per_split, KB - kb0));
+  // This CTA's blocks, in the order of memory (a tile's blocks along k, then the next tile's): kb_per_split of one tile, or `span` that
+  // may end one tile and begin the next, with an accumulator for either (see nf4_span).
+  const int KB = (int)(K / 64), total = (int)((N + 127) / 128) * KB;
+  const int first = span > 0 ? (int)blockIdx.x * span : (int)blockIdx.x * KB + min((int)blockIdx.y * kb_per_split, KB);
+  const int nkb = span > 0 ? min(span, total - first) : max(0, min(kb_per_split, KB - (int)blockIdx.y * kb_per_split));
+  const int tile0 = span > 0 ? first / KB : (int)blockIdx.x, k0 = first % KB, here = min(nkb, KB - k0);   // here: blocks of the first tile
   const int xbytes = tn * 128, xst = NT_XRING / xbytes;   // 4 stages of 32 tokens or 8 of 16: a power of two
   const int xsh = tn == 16 ? 3 : 2;
 
@@ -211,6 +215,7 @@ __global__ void __launch_bounds__(NT_THREADS) nf4_tc_kernel(const __grid_constan
       mbar_init(&a_empty[b], 1);
     }
     mbar_init(d_full, 1);
+    mbar_init(d_full + 1, 1);
     fence_barrier_init();
   }
   if (warp == 1) tc::alloc_then_launch_dependents(tmem_slot, NT_TMEM_COLS);
@@ -234,12 +239,12 @@ __global__ void __launch_bounds__(NT_THREADS) nf4_tc_kernel(const __grid_constan
       auto load_codes = [&](int kb) {
         const int s = kb % NT_CST;
         mbar_expect_tx(&c_full[s], NF4_BLOCK);
-        bulk_load_1d(cs + s * NF4_BLOCK, q + ((int64_t)tile * KB + kb0 + kb) * NF4_BLOCK, NF4_BLOCK, &c_full[s]);
+        bulk_load_1d(cs + s * NF4_BLOCK, q + (int64_t)(first + kb) * NF4_BLOCK, NF4_BLOCK, &c_full[s]);
       };
       auto load_x = [&](int kb) {
         const int s = kb & (xst - 1);
         mbar_expect_tx(&x_full[s], xbytes);
-        tma_load_2d_hint(xs + s * xbytes, &tmX, &x_full[s], (kb0 + kb) * 64, 0, pol_x);
+        tma_load_2d_hint(xs + s * xbytes, &tmX, &x_full[s], (kb < here ? k0 + kb : kb - here) * 64, 0, pol_x);
       };
       for (int kb = 0; kb < min(NT_CST, nkb); ++kb) load_codes(kb);
       pdl_wait();  // the activations come from the previous kernel
@@ -269,17 +274,16 @@ __global__ void __launch_bounds__(NT_THREADS) nf4_tc_kernel(const __grid_constan
         ok = mbar_wait(&a_full[p], (kb / NT_ABUF) & 1, status) && mbar_wait(&x_full[s], (kb >> xsh) & 1, status);
         if (!ok) break;
         tc::fence_after();
-        tc::umma4_bf16_ts<tc::K_MAJOR>(tmem_base, tmem_base + 32 + p * 32, tc::desc_lo(xs_addr + s * xbytes, 16), tc::desc_hi(1024), idesc, kb > 0);
+        tc::umma4_bf16_ts<tc::K_MAJOR>(tmem_base + (kb < here ? 0 : NT_D1), tmem_base + 32 + p * 32, tc::desc_lo(xs_addr + s * xbytes, 16), tc::desc_hi(1024), idesc,
+                                       kb > 0 && kb != here);
         tc::commit(&x_empty[s]);
         tc::commit(&a_empty[p]);
+        if (kb + 1 == here || kb + 1 == nkb) tc::commit(d_full + (kb < here ? 0 : 1));
       }
-      if (ok) tc::commit(d_full);
     }
   } else {
     // ---------------- dequantisers: lane quarter = warp % 4 (the TMEM lanes a warp may touch), parity = which blocks
     const int dw = warp - 2, p = dw >> 2, quarter = warp & 3;
-    const int64_t n_feat = (int64_t)tile * 128 + quarter * 32 + lane;
-    const bool valid = (int64_t)tile * 128 + quarter * 32 < N;  // N % 64 == 0: a quarter is all in or all out
     const uint8_t* lut_bytes = reinterpret_cast<const uint8_t*>(lut);
     const uint32_t lane4 = (uint32_t)lane * 4;
     const uint32_t a_lane = tmem_base + ((uint32_t)(quarter * 32) << 16) + 32;
@@ -311,28 +315,36 @@ __global__ void __launch_bounds__(NT_THREADS) nf4_tc_kernel(const __grid_constan
         ok = mbar_wait(&a_empty[ab], (use - 1) & 1, status);
         tc::fence_after();
       }
-      if (valid) tc::st32(a_lane + ab * 32, r);
+      tc::st32(a_lane + ab * 32, r);   // features past N: zeros
       tc::fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&a_full[ab]);
     }
     if (p == 0) {
-      // ---------------- epilogue: D[feature = lane][token = column] -> out[split][token][feature]
-      uint32_t r[32];
-#pragma unroll
-      for (int j = 0; j < 32; ++j) r[j] = 0u;
-      if (nkb > 0) {
-        ok = mbar_wait(d_full, 0, status) && ok;
-        ok = __all_sync(0xffffffffu, ok);  // the load below is warp-collective
-        tc::fence_after();
-        if (ok) tc::ld32(tmem_base + ((uint32_t)(quarter * 32) << 16), r);
-      }
+      // ---------------- epilogue: D[feature = lane][token = column] -> out[slab][token][feature]
       pdl_wait();  // the slab buffer may still be read by the previous kernel
-      if (valid && ok) {
-        float* op = out + (int64_t)split * M * N + n_feat;
+      for (int part = 0; part < (nkb > here ? 2 : 1); ++part) {
+        const int tile = tile0 + part;
+        uint32_t r[32];
+#pragma unroll
+        for (int j = 0; j < 32; ++j) r[j] = 0u;
+        if (nkb > 0) {
+          ok = mbar_wait(d_full + part, 0, status) && ok;
+          ok = __all_sync(0xffffffffu, ok);  // the load below is warp-collective
+          tc::fence_after();
+          if (ok) tc::ld32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (part ? NT_D1 : 0), r);
+        }
+        // N % 64 == 0: a quarter is all in or all out
+        if ((int64_t)tile * 128 + quarter * 32 >= N || !ok) continue;
+        // CTAs that share a tile take its slabs in turn; the last of them clears those that nobody takes
+        const int slab = span > 0 ? (int)blockIdx.x - tile * KB / span : (int)blockIdx.y;
+        const bool last = span > 0 && ((tile + 1) * KB - 1) / span == (int)blockIdx.x;
+        float* op = out + (int64_t)slab * M * N + (int64_t)tile * 128 + quarter * 32 + lane;
 #pragma unroll
         for (int j = 0; j < 32; ++j)
           if (j < M) op[(int64_t)j * N] = __uint_as_float(r[j]);
+        if (last)
+          for (int64_t j = M; j < (int64_t)(slabs - slab) * M; ++j) op[j * N] = 0.f;
       }
     }
   }
@@ -526,7 +538,22 @@ constexpr int nf4_small_smem() { return 256 * 8 * 4 + 2 * 2 * MR * 32 * 4; }
 
 constexpr int kNf4SmallRows = 4;
 
-int nf4_pick_ksplit(Ctx* c, int64_t K, int64_t N);
+// CTAs along K of one tile each
+int nf4_tile_split(Ctx* c, int64_t K, int64_t N) {
+  const int tiles = (int)((N + 127) / 128), KB = (int)(K / 64), slots = 2 * c->sm_count;
+  int ks = std::max(1, slots / tiles);
+  ks = std::min(ks, std::max(1, KB / 4));
+  return std::max(1, std::min(ks, 16));
+}
+// ... or, where those leave a fifth of the slots empty, equal shares of all blocks: a CTA's share ends one tile and begins the next.  The
+// blocks of a share, and the slabs that this takes; 0: a tile a CTA.  4096 x 28672 has 224 tiles for 296 slots: one CTA an SM works for 64
+// blocks while its neighbours' two work for 128.  Four rows 33.3 us a launch, 28.5 with shares of 49 blocks.
+int nf4_span(Ctx* c, int64_t K, int64_t N, int* slabs) {
+  const int64_t tiles = (N + 127) / 128, KB = K / 64, slots = 2 * c->sm_count, whole = tiles * nf4_tile_split(c, K, N);
+  const int64_t span = std::max<int64_t>(4, (tiles * KB + slots - 1) / slots);
+  *slabs = (int)((KB + span - 1) / span + 1);
+  return span <= KB && *slabs <= 16 && whole * 5 < slots * 4 && (tiles * KB + span - 1) / span > whole ? (int)span : 0;
+}
 
 int nf4_pick_ksplit(Ctx* c, int64_t K, int64_t N, int64_t M) {
   if (M <= kNf4SmallRows && c->nf4_small) {  // many small CTAs (8 per SM resident): about eight waves' worth keeps the stream smooth
@@ -535,23 +562,21 @@ int nf4_pick_ksplit(Ctx* c, int64_t K, int64_t N, int64_t M) {
     ks = std::min(ks, std::max(1, KB / 4));  // at least four blocks per CTA: the table and pipeline start-up are per CTA
     return std::max(1, std::min(ks, 16));
   }
-  return nf4_pick_ksplit(c, K, N);
-}
-
-int nf4_pick_ksplit(Ctx* c, int64_t K, int64_t N) {
-  const int tiles = (int)((N + 127) / 128), KB = (int)(K / 64), slots = 2 * c->sm_count;
-  int ks = std::max(1, slots / tiles);
-  ks = std::min(ks, std::max(1, KB / 4));
-  return std::max(1, std::min(ks, 16));
+  int slabs;
+  return nf4_span(c, K, N, &slabs) > 0 ? slabs : nf4_tile_split(c, K, N);
 }
 
 int nf4_gemv_launch(Ctx* c, const Nf4W& w, const bf16* x, int64_t ldx, int64_t M, int ksplit, float* out) {
   RB_REQUIRE(M >= 1 && M <= 32, "nf4 GEMV handles 1 to 32 rows");
   RB_REQUIRE(ldx % 8 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0, "nf4 GEMV needs 16-byte aligned activation rows");
   const int KB = (int)(w.K / 64);
+  int slabs;
+  const int share = nf4_span(c, w.K, w.N, &slabs);
+  const bool spans = share > 0 && ksplit == slabs && !(M <= kNf4SmallRows && c->nf4_small);   // fewer slabs: the caller had no room for them
   ksplit = std::max(1, std::min(ksplit, KB));
   const int per = (KB + ksplit - 1) / ksplit;
-  const dim3 grid((unsigned)((w.N + 127) / 128), (unsigned)ksplit);
+  const unsigned tiles = (unsigned)((w.N + 127) / 128);
+  const dim3 grid = spans ? dim3((tiles * KB + share - 1) / share) : dim3(tiles, (unsigned)ksplit);
   if (M <= kNf4SmallRows && c->nf4_small) {
     static bool small_attr = false;
     if (!small_attr) {
@@ -580,7 +605,7 @@ int nf4_gemv_launch(Ctx* c, const Nf4W& w, const bf16* x, int64_t ldx, int64_t M
     attr_set = true;
   }
   RB_CUDA(launch_k(nf4_tc_kernel, grid, dim3(NT_THREADS), (size_t)NT_SMEM, c->stream, c->use_pdl, tmX, (const uint8_t*)w.q,
-                   (int)M, tn, w.K, w.N, per, out, c->d_status));
+                   (int)M, tn, w.K, w.N, per, spans ? share : 0, slabs, out, c->d_status));
   ++g_launch_total;
   return REWB200_OK;
 }

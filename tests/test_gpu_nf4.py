@@ -63,6 +63,22 @@ def test_qlora_forward_matches_oracle(rb, orc, M, K, N):
     assert rel_l2(got.reshape(M, N), want) <= 2e-2
 
 
+@pytest.mark.parametrize("M,K,N", [(1, 1024, 19200), (4, 512, 19264), (17, 512, 25600), (33, 640, 22336)])
+def test_shares_of_blocks_that_end_one_tile_and_begin_the_next(rb, orc, M, K, N):
+    """Widths whose tiles leave a fifth of the CTA slots empty: equal shares of all blocks, tiles of two or three slabs and of one that
+    somebody clears, half a tile at the end.  bf16 levels, scales and their product (three roundings of 2^-9) against f32, tile by tile."""
+    rng = np.random.default_rng(M + N)
+    w = (rng.standard_normal((K, N)) / np.sqrt(K)).astype(np.float32)
+    x = bf16_round(rng.standard_normal((M, K)))
+    packed, scales = orc.nf4_quantize(w, 64)
+    T = rb.Tensor.from_host
+    lin = rb.QloraLinear(T(w), bias=T(np.zeros(N, np.float32)))
+    want = orc.qlora_forward(x, packed, scales, K, N, 64, bias=np.zeros(N, np.float32))
+    for _ in range(2):   # the second call finds the first one's slabs in its scratch
+        got = lin.forward(T(x, dtype=_lib.BF16)).to_host()
+        assert max(rel_l2(got[:, n:n + 64], want[:, n:n + 64]) for n in range(0, N, 64)) <= 3 * 2.0 ** -9 + 2.0 ** -8
+
+
 @pytest.mark.parametrize("M", [1, 2, 4])
 def test_small_row_gemv_agrees_with_the_tensor_core_kernel(rb, orc, M):
     """Option nf4_gemv=cuda streams the codes of steps of up to four rows through the CUDA cores (fp16 level
