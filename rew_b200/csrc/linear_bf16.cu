@@ -299,7 +299,7 @@ int linear_bf16_pick_ksplit(Ctx* c, int64_t M, int64_t K, int64_t N) {
   int split = 1;
   if (M > 64 && c->linear_impl != 0) {
     // Above 64 rows every slab costs its M rows twice through L2 (4 bytes an element there and back, about 4 TB/s), and an SM
-    // spends 0.29 us on a 128 x 64 block of weights whatever the step's rows: the count that makes both together least.
+    // spends 0.2 to 0.33 us on a 128 x 64 block of weights as the step's rows grow (0.29 here): the count that makes both together least.
     // 135 rows of 4096 x 6144 (48 tiles) take 3 slabs, of 4096 x 4096 and 14336 x 4096 (32 tiles) 4.
     double best = 0;
     for (int k = 1; k <= 4 && (k == 1 || nkb / k >= c->splitk_min_blocks); ++k) {
