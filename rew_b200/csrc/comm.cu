@@ -190,7 +190,8 @@ int rewb200_comm_peer_alloc(int slot, int64_t allreduce_bytes, int64_t alltoall_
   PeerHeap& h = g_heap[slot];
   const size_t total = kHeapHeader + 2 * (size_t)g_comm[slot].world * (size_t)allreduce_bytes + (size_t)alltoall_bytes;
   RB_CUDA(cudaMalloc(&h.local, total));
-  RB_CUDA(cudaMemset(h.local, 0, kHeapHeader + 2 * (size_t)g_comm[slot].world * (size_t)allreduce_bytes));  // flag 0 = no data yet
+  RB_CUDA(cudaMemsetAsync(h.local, 0, kHeapHeader + 2 * (size_t)g_comm[slot].world * (size_t)allreduce_bytes, c->stream));  // flag 0 = no data yet
+  RB_CUDA(cudaStreamSynchronize(c->stream));  // a peer may write as soon as it has the handle
   static_assert(sizeof(cudaIpcMemHandle_t) == 64, "CUDA IPC handles are 64 bytes");
   cudaIpcMemHandle_t ih;
   RB_CUDA(cudaIpcGetMemHandle(&ih, h.local));

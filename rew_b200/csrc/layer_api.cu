@@ -557,9 +557,10 @@ int rewb200_sampler_create(int slot, int batch, int vocab, int max_tokens, float
       k[2 * b] = (uint32_t)(seeds[b] & 0xFFFFFFFFull);
       k[2 * b + 1] = (uint32_t)(seeds[b] >> 32);
     }
-    RB_CUDA(cudaMemcpy(s->keys, k.data(), k.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
-    RB_CUDA(cudaMemset(s->steps, 0, batch * sizeof(int)));
-    RB_CUDA(cudaMemset(s->hist_len, 0, batch * sizeof(int)));
+    RB_CUDA(cudaMemcpyAsync(s->keys, k.data(), k.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, c->stream));
+    RB_CUDA(cudaMemsetAsync(s->steps, 0, batch * sizeof(int), c->stream));
+    RB_CUDA(cudaMemsetAsync(s->hist_len, 0, batch * sizeof(int), c->stream));
+    RB_CUDA(cudaStreamSynchronize(c->stream));
     return REWB200_OK;
   };
   const int st = body();
@@ -581,13 +582,14 @@ int rewb200_sampler_observe(rewb200_sampler* s, const int32_t* ids, int n_per_ro
   RB_CUDA(cudaStreamSynchronize(c->stream));
   std::vector<int> len((size_t)s->B);
   RB_CUDA(cudaMemcpy(len.data(), s->hist_len, s->B * sizeof(int), cudaMemcpyDeviceToHost));
+  for (int b = 0; b < s->B; ++b) RB_REQUIRE(len[b] + n_per_row <= s->cap, "sampler: more tokens than its budget");
   for (int b = 0; b < s->B; ++b) {
-    RB_REQUIRE(len[b] + n_per_row <= s->cap, "sampler: more tokens than its budget");
-    RB_CUDA(cudaMemcpy(s->hist + (size_t)b * s->cap + len[b], ids + (size_t)b * n_per_row, (size_t)n_per_row * sizeof(int),
-                       cudaMemcpyHostToDevice));
+    RB_CUDA(cudaMemcpyAsync(s->hist + (size_t)b * s->cap + len[b], ids + (size_t)b * n_per_row, (size_t)n_per_row * sizeof(int),
+                            cudaMemcpyHostToDevice, c->stream));
     len[b] += n_per_row;
   }
-  RB_CUDA(cudaMemcpy(s->hist_len, len.data(), s->B * sizeof(int), cudaMemcpyHostToDevice));
+  RB_CUDA(cudaMemcpyAsync(s->hist_len, len.data(), s->B * sizeof(int), cudaMemcpyHostToDevice, c->stream));
+  RB_CUDA(cudaStreamSynchronize(c->stream));
   return REWB200_OK;
 }
 

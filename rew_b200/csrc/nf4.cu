@@ -366,7 +366,7 @@ int nf4_alloc(Ctx* c, int64_t K, int64_t N, Nf4W* w) {
   const int64_t tiles = (N + 127) / 128;
   const size_t bytes = (size_t)tiles * (K / 64) * NF4_BLOCK;
   RB_CUDA(cudaMalloc((void**)&w->q, bytes));
-  RB_CUDA(cudaMemset(w->q, 0x77, bytes));  // code 7 = 0.0 for the features past N, whose scales are finite
+  RB_CUDA(cudaMemsetAsync(w->q, 0x77, bytes, c->stream));  // ahead of the quantiser; code 7 = 0.0 for the features past N, whose scales are finite
   RB_CUDA(cudaMalloc((void**)&w->sc, (size_t)K * (N / 64) * sizeof(float)));
   return REWB200_OK;
 }

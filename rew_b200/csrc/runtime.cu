@@ -183,9 +183,9 @@ int rewb200_init(const int* device_ordinals, int n) {
     RB_CUDA(cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
     RB_CUDA(cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming));
     RB_CUDA(cudaMalloc(&c->d_status, 256));
-    RB_CUDA(cudaMemset(c->d_status, 0, 256));
+    RB_CUDA(cudaMemsetAsync(c->d_status, 0, 256, c->stream));
     RB_CUDA(cudaMalloc(&c->d_tickets, Ctx::kTickets * sizeof(int)));
-    RB_CUDA(cudaMemset(c->d_tickets, 0, Ctx::kTickets * sizeof(int)));
+    RB_CUDA(cudaMemsetAsync(c->d_tickets, 0, Ctx::kTickets * sizeof(int), c->stream));
     RB_CUDA(cudaMallocHost(&c->h_status, 256));
     c->pinned_bytes = 64u << 20;
     RB_CUDA(cudaMallocHost(&c->pinned, c->pinned_bytes + 2 * Ctx::kHomeHalf));
