@@ -1326,6 +1326,12 @@ int gqa_mixer(rewb200_session* s, const FwdOpts& o, const StepLists& t, size_t r
   return REWB200_OK;
 }
 
+// Number of a launch of single tokens beside portions (GlaArgs::beside), never 0
+unsigned beside_number(Ctx* c) {
+  const unsigned n = ++c->beside_steps;
+  return n ? n : ++c->beside_steps;
+}
+
 int gla_mixer(rewb200_session* s, const FwdOpts& o, const StepLists& t, size_t r, int64_t rows, bool in_graph, int ks) {
   rewb200_model* m = s->m;
   Ctx* c = m->c;
@@ -1350,12 +1356,13 @@ int gla_mixer(rewb200_session* s, const FwdOpts& o, const StepLists& t, size_t r
   ga.dtype = m->cfg.dtype;
   ga.early = in_graph ? 1 : 0;
   ga.status = c->d_status;
+  ga.passed = c->d_passed;
   // single tokens run beside the walk over the portions' chunks: 16 heads, 15 single tokens and a portion of 61, 34 us behind
   // the portion's preparation one after the other, 30 together
   GlaArgs large = ga;
   const bool portions = !t.uniform && s->plan_gla_large > 0;
   if (portions) {
-    ga.beside = large.beside = ga.count > 0 ? 1 : 0;
+    ga.beside = large.beside = ga.count > 0 ? beside_number(c) : 0;
     large.list = t.gla_large;
     large.count = s->plan_gla_large;
     large.chunks = t.gla_chunks;
@@ -1520,11 +1527,12 @@ int delta_mixer(rewb200_session* s, const FwdOpts& o, const StepLists& t, size_t
   da.dtype = m->cfg.dtype;
   da.early = in_graph ? 1 : 0;
   da.status = c->d_status;
+  da.passed = c->d_passed;
   // as in gla_mixer: single tokens beside the walk over the portions' chunks
   DeltaArgs large = da;
   const bool portions = !t.uniform && s->plan_delta_large > 0;
   if (portions) {
-    da.beside = large.beside = da.count > 0 ? 1 : 0;
+    da.beside = large.beside = da.count > 0 ? beside_number(c) : 0;
     large.list = t.delta_large;
     large.count = s->plan_delta_large;
     large.chunks = t.delta_chunks;

@@ -7,6 +7,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -54,6 +55,8 @@ struct Ctx {
   bool attn_fused_merge = false;  // measured slower than the separate merge launch (3.20 vs 3.06 ms per step at batch 1)
   int* h_status = nullptr;   // pinned, 64 ints: [0] mirror of d_status; [16..31] / [32..47] per-peer pair counts sent /
                              // received by the expert-parallel prefix exchange
+  unsigned* d_passed = nullptr;          // behind d_status: the last step whose single tokens passed their wait (GlaArgs::beside)
+  std::atomic<unsigned> beside_steps{0};
   int sm_count = 0;
   bool use_pdl = true;
   int linear_impl = 2;       // bf16 Linear: 0 mma.sync, 1 tcgen05 when rows > 32, 2 tcgen05 always (default)

@@ -39,8 +39,10 @@ struct DeltaArgs {
   int64_t ldo;
   int dtype;
   int early;               // captured decode step: state and positions predate the step
-  int beside;              // single tokens and portions of a step at the same time: the launch of single tokens lets the next one start once it has passed
-                           // its own wait (what it reads is then there for both), and the walk over portions waits for it at its end
+  unsigned beside;         // not 0: single tokens and portions of a step at the same time.  The launch of single tokens lets the next one start once it
+                           // has passed its own wait and put this number, the step's own, into *passed; the walk over portions goes by
+                           // that (pdl_wait_beside) and waits for the single tokens at its end
+  unsigned* passed;
   int* status;
 };
 int delta_recurrent_launch(Ctx* c, const DeltaArgs& a);

@@ -310,7 +310,8 @@ __global__ void __launch_bounds__(CLUSTER ? NT / 2 : NT, CLUSTER ? 3 : 2) delta_
   }
   pdl_launch_dependents();
   __syncthreads();
-  if (!a.beside) pdl_wait();
+  if (a.beside) pdl_wait_beside(a.passed, a.beside);
+  else pdl_wait();
   const GlaPortion p = a.list[blockIdx.z];
   const int chunks = (p.n + C - 1) / C;
   auto load = [&](int c) {

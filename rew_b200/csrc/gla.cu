@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(NT, NT == 128 ? (KI <= 16 ? 4 : 3) : KI <= 8 ?
 #pragma unroll
   for (int i = 0; i < KI; ++i) S[i] = i < held ? *reinterpret_cast<const float4*>(st + i * step) : make_float4(0.f, 0.f, 0.f, 0.f);
   if (a.early) pdl_wait();
-  if (a.beside) pdl_launch_dependents();
+  if (a.beside) pdl_launch_beside(a.passed, a.beside);
   if (threadIdx.x < (unsigned)(a.ldv - V)) s.v[V + threadIdx.x] = 0.f;
   for (int t = 0; t < p.n; ++t) {
     load_token<NT>(a, s, h, p.row0 + t);
@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(NT) gla_plain_kernel(GlaArgs a) {
   __shared__ float red[NT / 32];
   if (!a.beside) pdl_launch_dependents();
   pdl_wait();
-  if (a.beside) pdl_launch_dependents();
+  if (a.beside) pdl_launch_beside(a.passed, a.beside);
   const GlaDims& m = a.m;
   const int h = blockIdx.x, K = m.dim, V = m.vdim;
   const GlaPortion p = portion_of(a, blockIdx.y);

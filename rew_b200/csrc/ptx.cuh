@@ -145,6 +145,27 @@ __device__ __forceinline__ void pdl_launch_dependents() {
 }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// A launch that runs beside the one before it (GlaArgs::beside) reads what earlier launches wrote without waiting for its neighbour.  That
+// a neighbour has passed its own wait does not make that memory visible to others, so the neighbour says so in memory: one of its threads
+// stores the step's number behind its wait (release), and what starts beside it has to see that number (acquire).  Nobody polls:
+// who does not see it takes the plain wait.
+__device__ __forceinline__ void pdl_launch_beside(unsigned* passed, unsigned number) {
+  if (threadIdx.x != 0) return;
+  if (blockIdx.x == 0 && blockIdx.y == 0) asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(passed), "r"(number) : "memory");
+  pdl_launch_dependents();
+}
+// the whole block
+__device__ __forceinline__ void pdl_wait_beside(const unsigned* passed, unsigned number) {
+  int seen = 0;
+  if (threadIdx.x == 0) {
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(passed) : "memory");
+    seen = v == number;
+  }
+  if (!__syncthreads_or(seen)) pdl_wait();
+  fence_proxy_async();   // bulk copies read that memory too
+}
+
 // ---- flags between the ranks of a node (peer heap) ------------------------------------------------
 // Writer: every thread of the CTA has issued its stores into the peer's memory; after the CTA barrier
 // the flag store (release, system scope) orders them before the flag.  Reader: polls a cell of its OWN

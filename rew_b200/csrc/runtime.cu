@@ -184,6 +184,7 @@ int rewb200_init(const int* device_ordinals, int n) {
     RB_CUDA(cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming));
     RB_CUDA(cudaMalloc(&c->d_status, 256));
     RB_CUDA(cudaMemsetAsync(c->d_status, 0, 256, c->stream));
+    c->d_passed = (unsigned*)c->d_status + 32;
     RB_CUDA(cudaMalloc(&c->d_tickets, Ctx::kTickets * sizeof(int)));
     RB_CUDA(cudaMemsetAsync(c->d_tickets, 0, Ctx::kTickets * sizeof(int), c->stream));
     RB_CUDA(cudaMallocHost(&c->h_status, 256));

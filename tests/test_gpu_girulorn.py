@@ -208,6 +208,33 @@ def test_mixed_batches_against_each_request_alone(rb, dtype):
         close(np.concatenate(got[r]), want[r], dtype)
 
 
+def test_single_tokens_beside_portions_as_one_after_the_other(rb):
+    """Single tokens that run beside a walk over portions, again and again, against the same steps with every launch behind the one
+    before it (option pdl=0): the same bits.  Portions of one chunk, of several and with a remainder, one and several of them."""
+    cfg = K.small()
+    model = build(rb, cfg, K.weights(cfg, seed=5, score_gain=1.5), "bfloat16")
+    rng = np.random.default_rng(7)
+    lanes = 6
+    steps = [[(l, int(rng.integers(2, 60))) for l in range(lanes)]]
+    for portions in ([150], [32], [33, 64], [100, 2, 41], [17], [200]):
+        order = rng.permutation(lanes)
+        steps.append([(int(l), portions[i] if i < len(portions) else 1) for i, l in enumerate(order)])
+    ids = [[(l, K.tokens(cfg, n, seed=10 * i + l)) for l, n in step] for i, step in enumerate(steps)]
+
+    def serve():
+        sess = model.paged_session(lanes, 640, 70)
+        return [sess.feed(step, want=range(sum(len(t) for _, t in step)))[0] for step in ids]
+
+    rb.set_option("pdl", "0")
+    try:
+        want = serve()
+    finally:
+        rb.set_option("pdl", "1")
+    for _ in range(8):
+        for got, w in zip(serve(), want):
+            assert np.array_equal(got, w)
+
+
 def test_long_prompt_with_many_routed_pairs(rb, dtype):
     """More (token, expert) pairs than the small-step sort takes, beside a decoding lane."""
     cfg = K.config([K.gla(K.moe(6, 4, 16)), K.attention(K.moe(6, 3, 16))])
