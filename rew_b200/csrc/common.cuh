@@ -134,7 +134,8 @@ int nf4_gemv_launch(Ctx* c, const Nf4W& w, const bf16* x, int64_t ldx, int64_t M
 // attribute (the kernel then starts early and calls griddepcontrol.wait itself).
 extern int64_t g_launch_total;  // kernels launched by this library since load
 // ... and of the kernels that a rule on sizes chooses between (rewb200_kernel_launches)
-enum KernelRoute : int { ROUTE_LINEAR_TILE = 0, ROUTE_LINEAR_PERSISTENT, ROUTE_LINEAR_PAIR, ROUTE_F32_ROWS, ROUTE_F32_TILES, ROUTE_ATTENTION_TC, ROUTE_ATTENTION_TC2, N_ROUTES };
+enum KernelRoute : int { ROUTE_LINEAR_TILE = 0, ROUTE_LINEAR_PERSISTENT, ROUTE_LINEAR_PAIR, ROUTE_F32_ROWS, ROUTE_F32_TILES, ROUTE_ATTENTION_TC, ROUTE_ATTENTION_TC2,
+                         ROUTE_RESULTS_PINNED, ROUTE_RESULTS_RING, ROUTE_RESULTS_PAGEABLE, N_ROUTES };
 extern int64_t g_route_launches[N_ROUTES];
 
 template <typename... KArgs, typename... Args>

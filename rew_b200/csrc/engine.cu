@@ -651,15 +651,32 @@ int moe_routed(rewb200_session* s, MoeDev& X, const void* x, int64_t d, int64_t 
 
 namespace {
 
+constexpr size_t kHomeSmall = 16 * 1024;   // results below this take a few microseconds either way
+
 struct Piece {
   const void* dev;
   void* host;      // NULL: not wanted
   size_t bytes;
 };
 
+// Pinned by the caller (allocated or registered so): copied into by the device itself, at the link's rate.  Small results are not asked about.
+bool pinned_home(const void* host, size_t bytes) {
+  if (!host || bytes < kHomeSmall) return false;
+  for (const char* p : {(const char*)host, (const char*)host + bytes - 1}) {
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    if (at.type != cudaMemoryTypeHost) return false;
+  }
+  return true;
+}
+
 // The results of a step into the caller's memory, behind everything enqueued; returns once they and the device's status word are
 // there (ctx_status).  A copy into pageable memory goes at 4 GB/s (6.5 MB of logits: 1.6 ms); here one half of the slot's pinned ring
-// is emptied while the other one fills.  A second thread that comes for results meanwhile has them copied the other way.
+// is emptied while the other one fills.  Into pinned memory they go straight.  A second thread that comes for results meanwhile has
+// them copied into pageable memory by the driver.
 int bring_home(rewb200_session* s, std::initializer_list<Piece> pieces) {
   Ctx* c = s->m->c;
   std::unique_lock<std::mutex> ring(c->home_mutex, std::try_to_lock);
@@ -672,7 +689,9 @@ int bring_home(rewb200_session* s, std::initializer_list<Piece> pieces) {
   int sent = 0;
   for (const Piece& p : pieces) {
     if (!p.host || p.bytes == 0) continue;
-    if (!ring) {
+    const bool direct = pinned_home(p.host, p.bytes);
+    ++g_route_launches[direct ? ROUTE_RESULTS_PINNED : ring ? ROUTE_RESULTS_RING : ROUTE_RESULTS_PAGEABLE];
+    if (direct || !ring) {
       RB_CUDA(cudaMemcpyAsync(p.host, p.dev, p.bytes, cudaMemcpyDeviceToHost, c->stream));
       continue;
     }
@@ -695,7 +714,7 @@ int bring_home(rewb200_session* s, std::initializer_list<Piece> pieces) {
 // While the GPU works: has the system find the pages that results will be copied into (their contents stay).  A page of fresh memory
 // costs its first writer more than the copy does.
 void expect_home(void* host, size_t bytes) {
-  if (!host || bytes < 16 * 1024) return;
+  if (!host || bytes < kHomeSmall || pinned_home(host, bytes)) return;
   volatile char* p = (volatile char*)host;
   for (size_t at = 0; at < bytes; at += 4096) p[at] = p[at];
   p[bytes - 1] = p[bytes - 1];
@@ -2511,6 +2530,7 @@ int rewb200_model_forward_all(rewb200_session* s, const int32_t* ids, int S, int
     RB_TRY(layered_prepare(s, o, rows));
   }
   RB_TRY(enqueue_forward(s, o));
+  expect_home(logits_out, (size_t)rows * m->cfg.vocab * sizeof(float));
   RB_TRY(fetch_logits(s, rows, logits_out));
   return ctx_check_status(c);
 }

@@ -401,3 +401,81 @@ def test_logits_of_any_size_come_home_whole(rb, orc, B, vocab):
     assert rel_l2(last, want) <= 1e-5 and np.array_equal(ids[:, 1], last.argmax(1))
     fed = model.paged_session(B, 16, B + 2).feed([(b, prompt[b]) for b in range(B)], want=[5 * b + 4 for b in range(B)], sample=True)
     assert rel_l2(fed[0], logits) <= 1e-5 and np.array_equal(fed[1], nxt)
+
+
+def _copies():
+    from rew_b200 import _lib
+    return {k: _lib.lib().rewb200_kernel_launches(("results_" + k).encode()) for k in ("pinned", "ring", "pageable")}
+
+
+@pytest.mark.parametrize("vocab", [3000, 40001, 300000])
+def test_results_into_pinned_and_pageable_memory(rb, vocab):
+    """A caller's pinned memory is copied into directly, pageable memory through the slot's ring: the same values behind a prompt, decode
+    steps, a step of portions and a whole forward.  Below 16 KB nobody asks which of them it is."""
+    import torch
+    from rew_b200 import _lib
+    cfg = W.ModelConfig(vocab=vocab, d_model=64, n_layers=1, n_heads=2, n_kv_heads=1, head_dim=32, ffn=64, max_seq=32, theta=10000.0, mask_kind=1)
+    model = rb.CausalLM(cfg).load(W.init_weights(cfg, seed=3))
+    ids = np.random.default_rng(vocab).integers(0, vocab, size=(2, 5)).astype(np.int32)
+    lib, at = _lib.lib(), lambda a, t=_lib.F32P: a.ctypes.data_as(t)
+
+    def serve(empty):
+        out = [empty((n, vocab)) for n in (2, 2, 1, 10)]
+        nxt, dec = np.empty(2, np.int32), np.empty((2, 2), np.int32)
+        sess = model.session(2, 16)
+        _lib.check(lib.rewb200_session_forward(sess._h, at(ids, _lib.I32P), 5, at(nxt, _lib.I32P), at(out[0])))
+        _lib.check(lib.rewb200_session_decode(sess._h, 2, at(dec, _lib.I32P), at(out[1])))
+        paged = model.paged_session(2, 16, 4)
+        one = lambda *v: np.array(v, np.int32)
+        lanes, counts, want = one(1, 0), one(5, 5), one(9)
+        _lib.check(lib.rewb200_lanes_feed(paged._h, 2, at(lanes, _lib.I32P), at(counts, _lib.I32P), at(ids, _lib.I32P), 1, at(want, _lib.I32P), at(out[2]),
+                                          None, None, None))
+        _lib.check(lib.rewb200_model_forward_all(sess._h, at(ids, _lib.I32P), 5, 0, 1, at(out[3])))
+        return out, nxt, dec
+
+    before = _copies()
+    out, nxt, dec = serve(lambda shape: np.full(shape, np.nan, np.float32))
+    middle = _copies()
+    pin, pin_nxt, pin_dec = serve(lambda shape: torch.full(shape, float("nan"), pin_memory=True).numpy())
+    after = _copies()
+    large = sum(4 * o.size >= 16 * 1024 for o in out)
+    assert large == (4 if vocab > 4096 else 3)
+    assert middle["pinned"] == before["pinned"] and after["pinned"] - middle["pinned"] == large
+    assert middle["ring"] - before["ring"] == 6 and after["ring"] - middle["ring"] == 6 - large   # two of them chosen ids
+    assert np.array_equal(nxt, pin_nxt) and np.array_equal(dec, pin_dec)
+    for a, b in zip(out, pin):
+        assert np.isfinite(a).all() and np.array_equal(a, b)
+
+
+def test_two_threads_that_come_for_results_together(rb):
+    """One slot, two threads with a model each: who finds the ring taken has the driver copy; both get what they get alone."""
+    import threading
+    cfg = W.ModelConfig(vocab=60000, d_model=64, n_layers=1, n_heads=2, n_kv_heads=1, head_dim=32, ffn=64, max_seq=32, theta=10000.0, mask_kind=1)
+    sessions = [rb.CausalLM(cfg).load(W.init_weights(cfg, seed=s)).session(16, 16) for s in (1, 2)]
+    ids = np.random.default_rng(0).integers(0, cfg.vocab, size=(16, 5)).astype(np.int32)
+
+    def forward(sess):
+        sess.reset()
+        return sess.forward(ids, want_logits=True)
+
+    alone = [forward(s) for s in sessions]
+    before, wrong, enough = _copies()["pageable"], [], threading.Event()
+
+    def work(i):
+        try:
+            for _ in range(300):
+                nxt, logits = forward(sessions[i])
+                if not (np.array_equal(nxt, alone[i][0]) and np.array_equal(logits, alone[i][1])):
+                    wrong.append(i)
+                if _copies()["pageable"] >= before + 6 or enough.is_set():
+                    break
+        except Exception as e:
+            wrong.append(e)
+        enough.set()
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in (0, 1)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong and _copies()["pageable"] > before
