@@ -126,9 +126,9 @@ int rewb200_set_option(int slot, const char* key, const char* value);
 /* Number of kernels this library has launched on the slot since init. */
 int64_t rewb200_launch_count(int slot);
 /* The same for one of the kernels that a rule on sizes chooses between (a captured step counts when it is captured): "linear_tile",
- * "linear_persistent" (dense), "linear_pair", "f32_rows", "f32_tiles", "attention_tc", "attention_tc2"; and of the copies that bring a
- * step's results to the host: "results_pinned" (straight into the caller's pinned memory), "results_ring" (through the slot's own),
- * "results_pageable" (while another thread has the ring); -1 for any other name. */
+ * "linear_persistent" (dense), "linear_pair", "f32_rows", "f32_tiles", "attention_tc", "attention_tc2", "nf4_tiles", "nf4_shares";
+ * and of the copies that bring a step's results to the host: "results_pinned" (straight into the caller's pinned memory),
+ * "results_ring" (through the slot's own), "results_pageable" (while another thread has the ring); -1 for any other name. */
 int64_t rewb200_kernel_launches(const char* kernel);
 
 /* ---- device buffers -------------------------------------------------------

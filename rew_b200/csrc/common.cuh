@@ -126,7 +126,8 @@ void nf4_free(Nf4W* w);
 int nf4_quantize_launch(Ctx* c, const void* src, int src_dtype, int64_t ld, ColMap cm, const Nf4W& w);
 int nf4_dequant_launch(Ctx* c, const Nf4W& w, bf16* dst, int64_t ld, ColMap cm);
 int nf4_codes_launch(Ctx* c, const Nf4W& w, uint8_t* codes);
-int nf4_pick_ksplit(Ctx* c, int64_t K, int64_t N, int64_t M);  // rows of the step: up to four run on the CUDA-core GEMV
+// slabs of a launch of M rows (up to four can run on the CUDA-core GEMV), `most` of which the caller has room for
+int nf4_pick_ksplit(Ctx* c, int64_t K, int64_t N, int64_t M, int64_t most);
 // out: [ksplit][M][N] f32 partial sums of x[M,K] @ W (no bias); 1 <= M <= 32
 int nf4_gemv_launch(Ctx* c, const Nf4W& w, const bf16* x, int64_t ldx, int64_t M, int ksplit, float* out);
 
@@ -135,7 +136,7 @@ int nf4_gemv_launch(Ctx* c, const Nf4W& w, const bf16* x, int64_t ldx, int64_t M
 extern int64_t g_launch_total;  // kernels launched by this library since load
 // ... and of the kernels that a rule on sizes chooses between (rewb200_kernel_launches)
 enum KernelRoute : int { ROUTE_LINEAR_TILE = 0, ROUTE_LINEAR_PERSISTENT, ROUTE_LINEAR_PAIR, ROUTE_F32_ROWS, ROUTE_F32_TILES, ROUTE_ATTENTION_TC, ROUTE_ATTENTION_TC2,
-                         ROUTE_RESULTS_PINNED, ROUTE_RESULTS_RING, ROUTE_RESULTS_PAGEABLE, N_ROUTES };
+                         ROUTE_RESULTS_PINNED, ROUTE_RESULTS_RING, ROUTE_RESULTS_PAGEABLE, ROUTE_NF4_TILES, ROUTE_NF4_SHARES, N_ROUTES };
 extern int64_t g_route_launches[N_ROUTES];
 
 template <typename... KArgs, typename... Args>

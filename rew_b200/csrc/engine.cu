@@ -401,8 +401,7 @@ int run_linear(rewb200_session* s, const LinW& w, const void* x, int64_t ldx, in
   if (fused) *fused = false;
   if (w.quant && rows <= 32) {
     // weight-only NF4: codes dequantised inside the GEMV, f32 split-K slabs
-    int ks = nf4_pick_ksplit(c, w.K, w.N, rows);
-    while (ks > 1 && (size_t)ks * rows * w.N * sizeof(float) > s->part_bytes) --ks;
+    const int ks = nf4_pick_ksplit(c, w.K, w.N, rows, (int64_t)(s->part_bytes / ((size_t)rows * w.N * sizeof(float))));
     RB_REQUIRE((size_t)ks * rows * w.N * sizeof(float) <= s->part_bytes, "split-K scratch too small for the quantised Linear");
     RB_TRY(nf4_gemv_launch(c, w.nf4, (const bf16*)x, ldx, rows, ks, s->part));
     if (partial) {

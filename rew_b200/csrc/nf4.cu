@@ -33,6 +33,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "nf4_split.cuh"
 #include "ptx.cuh"
 #include "tc.cuh"
 
@@ -193,7 +194,7 @@ __global__ void __launch_bounds__(NT_THREADS) nf4_tc_kernel(const __grid_constan
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // This CTA's blocks, in the order of memory (a tile's blocks along k, then the next tile's): kb_per_split of one tile, or `span` that
-  // may end one tile and begin the next, with an accumulator for either (see nf4_span).
+  // may end one tile and begin the next, with an accumulator for either (see nf4_split).
   const int KB = (int)(K / 64), total = (int)((N + 127) / 128) * KB;
   const int first = span > 0 ? (int)blockIdx.x * span : (int)blockIdx.x * KB + min((int)blockIdx.y * kb_per_split, KB);
   const int nkb = span > 0 ? min(span, total - first) : max(0, min(kb_per_split, KB - (int)blockIdx.y * kb_per_split));
@@ -538,45 +539,26 @@ constexpr int nf4_small_smem() { return 256 * 8 * 4 + 2 * 2 * MR * 32 * 4; }
 
 constexpr int kNf4SmallRows = 4;
 
-// CTAs along K of one tile each
-int nf4_tile_split(Ctx* c, int64_t K, int64_t N) {
-  const int tiles = (int)((N + 127) / 128), KB = (int)(K / 64), slots = 2 * c->sm_count;
-  int ks = std::max(1, slots / tiles);
-  ks = std::min(ks, std::max(1, KB / 4));
-  return std::max(1, std::min(ks, 16));
-}
-// ... or, where those leave a fifth of the slots empty, equal shares of all blocks: a CTA's share ends one tile and begins the next.  The
-// blocks of a share, and the slabs that this takes; 0: a tile a CTA.  4096 x 28672 has 224 tiles for 296 slots: one CTA an SM works for 64
-// blocks while its neighbours' two work for 128.  Four rows 33.3 us a launch, 28.5 with shares of 49 blocks.
-int nf4_span(Ctx* c, int64_t K, int64_t N, int* slabs) {
-  const int64_t tiles = (N + 127) / 128, KB = K / 64, slots = 2 * c->sm_count, whole = tiles * nf4_tile_split(c, K, N);
-  const int64_t span = std::max<int64_t>(4, (tiles * KB + slots - 1) / slots);
-  *slabs = (int)((KB + span - 1) / span + 1);
-  return span <= KB && *slabs <= 16 && whole * 5 < slots * 4 && (tiles * KB + span - 1) / span > whole ? (int)span : 0;
-}
-
-int nf4_pick_ksplit(Ctx* c, int64_t K, int64_t N, int64_t M) {
+int nf4_pick_ksplit(Ctx* c, int64_t K, int64_t N, int64_t M, int64_t most) {
   if (M <= kNf4SmallRows && c->nf4_small) {  // many small CTAs (8 per SM resident): about eight waves' worth keeps the stream smooth
     const int tiles = (int)((N + 127) / 128), KB = (int)(K / 64);
     int ks = std::max(1, 8 * c->sm_count / tiles);
     ks = std::min(ks, std::max(1, KB / 4));  // at least four blocks per CTA: the table and pipeline start-up are per CTA
-    return std::max(1, std::min(ks, 16));
+    return std::max(1, (int)std::min<int64_t>(std::min(ks, 16), most));
   }
-  int slabs;
-  return nf4_span(c, K, N, &slabs) > 0 ? slabs : nf4_tile_split(c, K, N);
+  return nf4_split(c->sm_count, K, N, most).slabs;
 }
 
 int nf4_gemv_launch(Ctx* c, const Nf4W& w, const bf16* x, int64_t ldx, int64_t M, int ksplit, float* out) {
   RB_REQUIRE(M >= 1 && M <= 32, "nf4 GEMV handles 1 to 32 rows");
   RB_REQUIRE(ldx % 8 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0, "nf4 GEMV needs 16-byte aligned activation rows");
   const int KB = (int)(w.K / 64);
-  int slabs;
-  const int share = nf4_span(c, w.K, w.N, &slabs);
-  const bool spans = share > 0 && ksplit == slabs && !(M <= kNf4SmallRows && c->nf4_small);   // fewer slabs: the caller had no room for them
+  const Nf4Split split = nf4_split(c->sm_count, w.K, w.N, ksplit);
+  const bool spans = split.span > 0 && split.slabs == ksplit && !(M <= kNf4SmallRows && c->nf4_small);
   ksplit = std::max(1, std::min(ksplit, KB));
   const int per = (KB + ksplit - 1) / ksplit;
   const unsigned tiles = (unsigned)((w.N + 127) / 128);
-  const dim3 grid = spans ? dim3((tiles * KB + share - 1) / share) : dim3(tiles, (unsigned)ksplit);
+  const dim3 grid = spans ? dim3((tiles * KB + split.span - 1) / split.span) : dim3(tiles, (unsigned)ksplit);
   if (M <= kNf4SmallRows && c->nf4_small) {
     static bool small_attr = false;
     if (!small_attr) {
@@ -605,8 +587,9 @@ int nf4_gemv_launch(Ctx* c, const Nf4W& w, const bf16* x, int64_t ldx, int64_t M
     attr_set = true;
   }
   RB_CUDA(launch_k(nf4_tc_kernel, grid, dim3(NT_THREADS), (size_t)NT_SMEM, c->stream, c->use_pdl, tmX, (const uint8_t*)w.q,
-                   (int)M, tn, w.K, w.N, per, spans ? share : 0, slabs, out, c->d_status));
+                   (int)M, tn, w.K, w.N, per, spans ? split.span : 0, split.slabs, out, c->d_status));
   ++g_launch_total;
+  ++g_route_launches[spans ? ROUTE_NF4_SHARES : ROUTE_NF4_TILES];
   return REWB200_OK;
 }
 
@@ -771,7 +754,7 @@ int rewb200_qlora_linear(const rewb200_buffer* x, const rewb200_nf4* h, const re
     *y = out;
     return REWB200_OK;
   }
-  const int ks = nf4_pick_ksplit(c, K, N, std::min<int64_t>(M, 32));
+  const int ks = nf4_pick_ksplit(c, K, N, std::min<int64_t>(M, 32), 16);
   float *part = nullptr, *xa = nullptr;
   cudaError_t e = cudaMalloc((void**)&part, (size_t)ks * 32 * N * sizeof(float));
   if (e == cudaSuccess && rank > 0) e = cudaMalloc((void**)&xa, (size_t)M * rank * sizeof(float));

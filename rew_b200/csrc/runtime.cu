@@ -354,7 +354,7 @@ int64_t rewb200_launch_count(int slot) {
 
 int64_t rewb200_kernel_launches(const char* kernel) {
   static const char* const names[N_ROUTES] = {"linear_tile", "linear_persistent", "linear_pair", "f32_rows", "f32_tiles", "attention_tc", "attention_tc2",
-                                              "results_pinned", "results_ring", "results_pageable"};
+                                              "results_pinned", "results_ring", "results_pageable", "nf4_tiles", "nf4_shares"};
   for (int i = 0; kernel && i < N_ROUTES; ++i)
     if (!strcmp(kernel, names[i])) return g_route_launches[i];
   return -1;

@@ -75,7 +75,9 @@ def test_shares_of_blocks_that_end_one_tile_and_begin_the_next(rb, orc, M, K, N)
     lin = rb.QloraLinear(T(w), bias=T(np.zeros(N, np.float32)))
     want = orc.qlora_forward(x, packed, scales, K, N, 64, bias=np.zeros(N, np.float32))
     for _ in range(2):   # the second call finds the first one's slabs in its scratch
+        before = _gemvs()
         got = lin.forward(T(x, dtype=_lib.BF16)).to_host()
+        assert [a - b for a, b in zip(_gemvs(), before)] == [0, (M + 31) // 32]
         assert max(rel_l2(got[:, n:n + 64], want[:, n:n + 64]) for n in range(0, N, 64)) <= 3 * 2.0 ** -9 + 2.0 ** -8
 
 
@@ -160,3 +162,25 @@ def test_nf4_model_logits_match_reference_semantics(rb, orc, B, S):
     assert rel_l2(last, want) <= 2e-2
     # and the quantisation is not a no-op: the unquantised weights give visibly different logits
     assert rel_l2(orc.model_forward(cfg, t, seq, 0, True)[:, -1], want) > 2e-2
+
+
+def _gemvs():
+    return [_lib.lib().rewb200_kernel_launches(k.encode()) for k in ("nf4_tiles", "nf4_shares")]
+
+
+@pytest.mark.parametrize("B,shares", [(24, 1), (32, 0)])
+def test_gate_and_up_without_room_for_the_slabs_of_their_shares(rb, orc, B, shares):
+    """Gate and up of 2048 x 9728 in equal shares of blocks leave five slabs; the scratch of a session holds those of 25 rows.  Above
+    that whole tiles take their place.  Tolerance of the model test above."""
+    from rew_b200 import weights as W
+    cfg = W.ModelConfig(vocab=256, d_model=2048, n_layers=1, n_heads=8, n_kv_heads=2, head_dim=128, ffn=4864, max_seq=64,
+                        theta=500000.0, dtype=_lib.BF16, mask_kind=1, weight_quant=1)
+    t = [orc.bf16_round(a) if a.ndim == 2 else a for a in W.init_weights(cfg, seed=4, std=0.02, trivial_affine=False)]
+    ids = np.random.default_rng(B).integers(0, cfg.vocab, size=(B, 1)).astype(np.int32)
+    sess = rb.CausalLM(cfg).load(t).session(B, 8)
+    before = _gemvs()
+    logits = sess.forward(ids, want_logits=True)[1]
+    tiles, shared = (a - b for a, b in zip(_gemvs(), before))
+    assert (tiles, shared) == (4 - shares, shares)
+    want = orc.model_forward(cfg, _nf4_reference_tensors(orc, cfg, t), ids, 0, True)[:, -1]
+    assert rel_l2(logits, want) <= 2e-2
