@@ -1012,21 +1012,28 @@ static bool tc_two_per_sm(Ctx* c, int tn, int64_t tiles) { return tn <= 160 && t
 // 4096 x 28672, 4096 x 6144, 4096 x 4096, 14336 x 4096, 2048 x 11264 and 2048 x 2048 at 100 to 900 rows.  Us a launch, before (as few tiles
 // of one CTA as hold the rows) / now: 14336 x 4096 at 333 rows 56.4 / 45.5, 512 rows 74.4 / 51.4; 4096 x 4096 at 333 rows 20.1 / 16.0; 4096 x 6144 at
 // 333 rows 21.2 / 17.4, 900 rows 45.6 / 34.9; 4096 x 28672 at 256 rows 55.7 / 51.9, 512 rows 103 / 94; 2048 x 11264 at 512 rows 28.1 / 21.1.
+// Two CTAs an SM (tc_two_per_sm) cost less than that in one wave or two, where the second CTA of an SM fills the pauses of the first, and
+// more than that in three, where every wave begins and ends by itself.  So pairs must be ahead of them by 1.3 % (us, pairs / two an SM:
+// 4096 x 28672 at 81 to 96 rows 44.4 / 39.8, at 113 to 128 44.8 / 41.0; 2048 x 11264 at 257 to 288 rows 20.4 / 19.6; 4096 x 5120 at 785 to 896
+// rows 35.0 / 32.6), and steps that fewer tiles hold don't go there for a third wave (2048 x 21888, two an SM / tiles of one CTA: 640
+// rows 56.5 / 52.3, 700 rows 59.5 / 55.6, 800 rows 62.2 / 60.0).
 static void choose_tiles(Ctx* c, int64_t M, int64_t N, bool pairs, int* tn, int* pair_tn) {
   const int64_t fewest = (M + 255) / 256, cols = (N + BM - 1) / BM, sms = c->sm_count;
   auto waves = [](int64_t n, int64_t at_once) { return (double)((n + at_once - 1) / at_once); };
   double best = 0;
+  bool best_shared = false;
   for (int64_t t = fewest; t <= fewest + 4; ++t) {
     const int64_t rows = (M + t - 1) / t;
     const int one = (int)((rows + 15) / 16 * 16), two = (int)((rows + 31) / 32 * 32);
     if (t > fewest && one < 64) break;
     const int64_t tiles_one = cols * ((M + one - 1) / one);
+    const bool shared = tc_two_per_sm(c, one, tiles_one);   // SMs, by two CTAs each
     const double us = 0.18 + 0.0002 * std::min(one, 144) + 0.0014 * std::max(one - 144, 0);
-    const double cost = us * (tc_two_per_sm(c, one, tiles_one) ? 2 * waves(tiles_one, 2 * sms) : waves(tiles_one, sms));
-    if (best == 0 || cost < best) best = cost, *tn = one, *pair_tn = 0;
+    const double cost = us * (shared ? 2 * waves(tiles_one, 2 * sms) : waves(tiles_one, sms));
+    if (best == 0 || (cost < best && !(shared && tiles_one > 4 * sms))) best = cost, *tn = one, *pair_tn = 0, best_shared = shared;
     if (!pairs) continue;
     const double pair_cost = (0.178 + 0.0002 * std::min(two, 128) + 0.00075 * std::max(two - 128, 0)) * waves(cols / 2 * ((M + two - 1) / two), sms / 2);
-    if (pair_cost < best) best = pair_cost, *pair_tn = two;
+    if (pair_cost * (best_shared ? 1.013 : 1) < best) best = pair_cost, *pair_tn = two, best_shared = false;
   }
 }
 

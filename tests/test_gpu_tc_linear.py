@@ -197,6 +197,25 @@ def test_pairs_with_tiles_of_the_steps_own_size(rb_tc, M, K, N, pair):
             rb_tc.set_option("prefill", "pair")
 
 
+@pytest.mark.parametrize("M,N,kernel", [(96, 28672, "tile"), (112, 28672, "tile"), (128, 28672, "tile"), (272, 11264, "tile"), (360, 11264, "tile"), (833, 5120, "tile"),
+                                        (300, 21888, "tile"), (640, 21888, "persistent"), (700, 21888, "persistent"), (800, 21888, "persistent"),
+                                        (192, 28672, "pair"), (128, 11264, "pair")])
+def test_near_ties_of_the_tile_rule_go_to_the_faster_kernel(rb_tc, M, N, kernel):
+    """Steps whose estimates lie within a few per cent of one another, by the kernel that is faster there (the rule's comment has the times);
+    bound of the test above."""
+    from rew_b200 import _lib
+    K, rng = 64, np.random.default_rng(M + N)
+    x, w = W.bf16_round(rng.normal(size=(M, K))), W.bf16_round(rng.normal(size=(K, N)))
+    T = rb_tc.Tensor.from_host
+    lin, xs = rb_tc.Linear(T(w, _lib.BF16), T(np.zeros(N, np.float32))), T(x, _lib.BF16)
+    before = _launches()
+    got = lin.forward(xs).to_host()
+    after = _launches()
+    assert {k: after[k] - before[k] for k in after} == {k: int(k == kernel) for k in after}
+    bound = (K + 1) * 2.0 ** -24 * (np.abs(x) @ np.abs(w)).astype(np.float64) + 2.0 ** -8 * np.abs(x.astype(np.float64) @ w)
+    assert np.all(np.abs(got - x.astype(np.float64) @ w) <= bound)
+
+
 def test_persistent_prefill_model_equals_tile_kernel(rb_tc):
     """A 20 480-token prefill puts the decoder Linears (f32 partial and bf16 epilogues) on the persistent kernel and gate and up
     (SwiGLU) on the pair kernel; the logits must equal those of the one-tile-per-CTA kernel exactly."""
