@@ -157,6 +157,15 @@ template <> struct Vec4<bf16> {
 };
 
 __device__ __forceinline__ void add4(float4& v, const float4 w) { v.x += w.x; v.y += w.y; v.z += w.z; v.w += w.w; }
+// Slabs of a row requested together by the kernels that give a row (or a part of it) a CTA.  Up to 256 rows there are up to four, and few
+// rows to hide a load's wait behind.  Above that there is one slab, the rows hide it, and the registers of three more, or of a bound on
+// CTAs other than the compiler's own choice, only cost CTAs an SM.  Us a launch, one / four at once: RoPE and cache append of 16 384 rows
+// of 6144 133 / 197, of 4096 rows of 1536 12.6 / 17.3; norm on the way back, 1600 rows of 4096 21.9 / 27.2, 600 rows of 2048 7.5 / 8.7; first norm of
+// 4096 rows of 1024 26.7 / 33.4; norm on the way back of 90 rows of 2048, their Linear cut along K, 6.1 / 4.6.
+constexpr int slabs_at_once(int nsplit, int64_t rows) { return nsplit > 1 || rows <= 256 ? 4 : 1; }
+// ... and CTAs of 512 threads an SM, NCH groups of four columns a thread; 0: not said
+constexpr int norm_ctas(int nch, int at_once) { return at_once == 1 ? 0 : nch <= 2 ? 2 : 1; }
+
 // v += the slabs at p, in order.  G loads are under way together whatever their number: what is left over of an unrolled loop has them
 // wait for one another, half a microsecond each.
 template <int G>
@@ -173,7 +182,7 @@ __device__ __forceinline__ void sum_slabs(float4& v, const float* p, int n, int6
 }
 
 // Sum of the split-K slabs at element offset `idx` (a multiple of 4), in slab order.
-template <int G = 4>   // above 64 rows there are four slabs at most
+template <int G>
 __device__ __forceinline__ float4 partial_sum4(const NormArgs& a, int64_t idx) {
   float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
   if (a.partial_bf16) {
@@ -357,11 +366,12 @@ __device__ __forceinline__ void tp_exchange4_two(const NormArgs& a, float4 (&p)[
   }
 }
 
-template <typename TE, typename TO, int NCH>
-__global__ void __launch_bounds__(NORMV_THREADS, NCH <= 2 ? 2 : 1) residual_norm_vec_kernel(NormArgs a) {
+template <typename TE, typename TO, int NCH, int G>
+__global__ void __launch_bounds__(NORMV_THREADS, norm_ctas(NCH, G)) residual_norm_vec_kernel(NormArgs a) {
   __shared__ float red[33];
+  constexpr bool AHEAD = G > 1;
   pdl_launch_dependents();
-  if (a.norm_kind >= 0) prefetch_floats(a.gamma, (int)a.d);   // depends on no earlier kernel
+  if (AHEAD && a.norm_kind >= 0) prefetch_floats(a.gamma, (int)a.d);   // depends on no earlier kernel
   pdl_wait();
   if (a.wait_n > 0) peer_flags_wait(a.wait_cells, 1, a.wait_n, -1, *a.wait_epoch + a.wait_offset, a.status);
   const int64_t row = blockIdx.x;
@@ -379,14 +389,15 @@ __global__ void __launch_bounds__(NORMV_THREADS, NCH <= 2 ? 2 : 1) residual_norm
     }
     erow = reinterpret_cast<const TE*>(a.embed) + id * d;
   }
-  float4 vals[NCH], xin[NCH];
+  auto row_in = [&](int64_t i) { return erow && !a.add_embed ? Vec4<TE>::load(erow + i) : *reinterpret_cast<const float4*>(xr + i); };
+  float4 vals[NCH], xin[AHEAD ? NCH : 1];
   const bool summed = a.partial != nullptr;
-  // the residual (or embedding) row is requested ahead of the slabs
+  if constexpr (AHEAD) {   // the residual (or embedding) row is requested ahead of the slabs
 #pragma unroll
-  for (int c = 0; c < NCH; ++c) {
-    const int64_t i = ((int64_t)c * NORMV_THREADS + threadIdx.x) * 4;
-    xin[c] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (i < d) xin[c] = erow && !a.add_embed ? Vec4<TE>::load(erow + i) : *reinterpret_cast<const float4*>(xr + i);
+    for (int c = 0; c < NCH; ++c) {
+      const int64_t i = ((int64_t)c * NORMV_THREADS + threadIdx.x) * 4;
+      xin[c] = i < d ? row_in(i) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
   }
   if (summed) {
     int64_t idx[NCH];
@@ -394,7 +405,7 @@ __global__ void __launch_bounds__(NORMV_THREADS, NCH <= 2 ? 2 : 1) residual_norm
     for (int c = 0; c < NCH; ++c) {
       const int64_t i = ((int64_t)c * NORMV_THREADS + threadIdx.x) * 4;
       idx[c] = i < d ? row * d + i : -1;
-      vals[c] = i < d ? partial_sum4(a, idx[c]) : make_float4(0.f, 0.f, 0.f, 0.f);
+      vals[c] = i < d ? partial_sum4<G>(a, idx[c]) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     if (a.n_peers > 0) {
       if (a.two_shot) tp_exchange4_two<NCH>(a, vals, idx);
@@ -406,7 +417,7 @@ __global__ void __launch_bounds__(NORMV_THREADS, NCH <= 2 ? 2 : 1) residual_norm
     const int64_t i = ((int64_t)c * NORMV_THREADS + threadIdx.x) * 4;
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     if (i < d) {
-      v = xin[c];
+      v = AHEAD ? xin[AHEAD ? c : 0] : row_in(i);
       if (summed) {
         float4 p = vals[c];
         if (a.nsplit2 > 0) add4(p, partial2_sum4(a, row * d + i));
@@ -539,8 +550,8 @@ __global__ void __launch_bounds__(NORMV_THREADS, 2) residual_norm_rows_kernel(No
 
 // Sublayers normed on the way back (OutputNormArgs): x += gamma * y / rms(y), y the sum of the slabs.  CL CTAs of a
 // cluster share a row (decode-size steps), their sums of squares meet through distributed shared memory.
-template <typename T, int CL, int NCH>
-__global__ void __launch_bounds__(CL == 1 ? 512 : 256, NCH <= 2 ? 2 : 1) output_norm_kernel(OutputNormArgs a) {
+template <typename T, int CL, int NCH, int G>
+__global__ void __launch_bounds__(CL == 1 ? 512 : 256, CL == 1 ? norm_ctas(NCH, G) : NCH <= 2 ? 2 : 1) output_norm_kernel(OutputNormArgs a) {
   constexpr int THREADS = CL == 1 ? 512 : 256;
   __shared__ float red[33];
   __shared__ float part[2];
@@ -595,8 +606,8 @@ __global__ void __launch_bounds__(CL == 1 ? 512 : 256, NCH <= 2 ? 2 : 1) output_
   for (int c = 0; c < NCH; ++c) {
     const int64_t i = ((int64_t)c * THREADS + threadIdx.x) * 4, at = row * d + col0 + i;
     if (i >= dq) continue;
-    sum_slabs<CL == 1 ? 4 : 8>(y[c], a.partial + at, a.nsplit, a.split_stride);
-    sum_slabs<4>(y[c], a.partial2 + at, a.nsplit2, a.split_stride);
+    sum_slabs<G>(y[c], a.partial + at, a.nsplit, a.split_stride);
+    sum_slabs<G < 4 ? G : 4>(y[c], a.partial2 + at, a.nsplit2, a.split_stride);
     ss += y[c].x * y[c].x + y[c].y * y[c].y + y[c].z * y[c].z + y[c].w * y[c].w;
   }
   if (a.replace) {
@@ -780,8 +791,8 @@ __device__ __forceinline__ void store8<bf16>(bf16* dst, const float* r) {
 
 // Same work as qkv_post_kernel, eight consecutive columns (four RoPE pairs) per thread with 16-byte
 // accesses; needs head_dim % 8 == 0.  Prefill-size launches are bound by the f32 partials and the latency in front of
-// them: requested ahead of the row's position and page, 16 384 rows of 6144 take 161 us (179 us behind them).
-template <typename TA>
+// them: requested ahead of the row's position and page, 16 384 rows of 6144 take 133 us.
+template <typename TA, int G>
 __global__ void __launch_bounds__(256) qkv_post_vec_kernel(QkvPostArgs a) {
   pdl_launch_dependents();
   pdl_wait();
@@ -792,13 +803,13 @@ __global__ void __launch_bounds__(256) qkv_post_vec_kernel(QkvPostArgs a) {
   float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   const float* pp = a.partial + row * ntot + col;
   float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
-  for (int sp = 0; sp < a.nsplit; sp += 4) {
-    float4 t[8];
+  for (int sp = 0; sp < a.nsplit; sp += G) {
+    float4 t[2 * G];
 #pragma unroll
-    for (int j = 0; j < 8; ++j)
+    for (int j = 0; j < 2 * G; ++j)
       if (sp + j / 2 < a.nsplit) t[j] = *reinterpret_cast<const float4*>(pp + (sp + j / 2) * a.split_stride + 4 * (j & 1));
 #pragma unroll
-    for (int j = 0; j < 8; j += 2)
+    for (int j = 0; j < 2 * G; j += 2)
       if (sp + j / 2 < a.nsplit) add4(lo, t[j]), add4(hi, t[j + 1]);
   }
   v[0] = lo.x; v[1] = lo.y; v[2] = lo.z; v[3] = lo.w;
@@ -1236,15 +1247,16 @@ int output_norm_launch(Ctx* c, const OutputNormArgs& a, int64_t rows) {
     ++g_launch_total;
     return REWB200_OK;
   };
-#define RB_ONORM(T, CL)                                                                                         \
-  (nch <= 1 ? go(output_norm_kernel<T, CL, 1>, CL) : nch <= 2 ? go(output_norm_kernel<T, CL, 2>, CL)            \
-   : nch <= 4 ? go(output_norm_kernel<T, CL, 4>, CL) : go(output_norm_kernel<T, CL, 8>, CL))
+#define RB_ONORM(T, CL, G)                                                                                      \
+  (nch <= 1 ? go(output_norm_kernel<T, CL, 1, G>, CL) : nch <= 2 ? go(output_norm_kernel<T, CL, 2, G>, CL)      \
+   : nch <= 4 ? go(output_norm_kernel<T, CL, 4, G>, CL) : go(output_norm_kernel<T, CL, 8, G>, CL))
   if (cluster) {
     const int nch = (int)((a.d / 16 + 255) / 256);
-    return bf ? RB_ONORM(bf16, 4) : RB_ONORM(float, 4);
+    return bf ? RB_ONORM(bf16, 4, 8) : RB_ONORM(float, 4, 8);
   }
   const int nch = (int)((a.d / 4 + 511) / 512);
-  return bf ? RB_ONORM(bf16, 1) : RB_ONORM(float, 1);
+  if (slabs_at_once(std::max(a.nsplit, a.nsplit2), rows) == 1) return bf ? RB_ONORM(bf16, 1, 1) : RB_ONORM(float, 1, 1);
+  return bf ? RB_ONORM(bf16, 1, 4) : RB_ONORM(float, 1, 4);
 #undef RB_ONORM
 }
 
@@ -1349,16 +1361,18 @@ int residual_norm_launch(Ctx* c, const NormArgs& a, int64_t rows) {
   if (a.d % 4 == 0) {
     const int nch = (int)((a.d / 4 + NORMV_THREADS - 1) / NORMV_THREADS);
     dim3 g((unsigned)rows), b(NORMV_THREADS);
-#define RB_NORMV(TE, TO)                                                                                   \
-  (nch <= 1   ? launch_k(residual_norm_vec_kernel<TE, TO, 1>, g, b, 0, c->stream, c->use_pdl, a)             \
-   : nch <= 2 ? launch_k(residual_norm_vec_kernel<TE, TO, 2>, g, b, 0, c->stream, c->use_pdl, a)             \
-   : nch <= 4 ? launch_k(residual_norm_vec_kernel<TE, TO, 4>, g, b, 0, c->stream, c->use_pdl, a)             \
-              : launch_k(residual_norm_vec_kernel<TE, TO, 8>, g, b, 0, c->stream, c->use_pdl, a))
+#define RB_NORMV_G(TE, TO, G)                                                                               \
+  (nch <= 1   ? launch_k(residual_norm_vec_kernel<TE, TO, 1, G>, g, b, 0, c->stream, c->use_pdl, a)          \
+   : nch <= 2 ? launch_k(residual_norm_vec_kernel<TE, TO, 2, G>, g, b, 0, c->stream, c->use_pdl, a)          \
+   : nch <= 4 ? launch_k(residual_norm_vec_kernel<TE, TO, 4, G>, g, b, 0, c->stream, c->use_pdl, a)          \
+              : launch_k(residual_norm_vec_kernel<TE, TO, 8, G>, g, b, 0, c->stream, c->use_pdl, a))
+#define RB_NORMV(TE, TO) (slabs_at_once(a.nsplit, rows) == 1 ? RB_NORMV_G(TE, TO, 1) : RB_NORMV_G(TE, TO, 4))
     if (e16 && o16) e = RB_NORMV(bf16, bf16);
     else if (e16) e = RB_NORMV(bf16, float);
     else if (o16) e = RB_NORMV(float, bf16);
     else e = RB_NORMV(float, float);
 #undef RB_NORMV
+#undef RB_NORMV_G
     RB_CUDA(e);
     ++g_launch_total;
     return REWB200_OK;
@@ -1382,10 +1396,13 @@ int qkv_post_launch(Ctx* c, const QkvPostArgs& a, int64_t B) {
   if (a.hd % 8 == 0 && rows > 64) {  // prefill sizes: eight columns per thread
     const int nchunk = (a.nh + 2 * a.kvh) * a.hd / 8;
     dim3 vgrid((unsigned)rows, (unsigned)((nchunk + 255) / 256));
+    const bool one = slabs_at_once(a.nsplit, rows) == 1;
     if (a.act_dtype == REWB200_BF16)
-      e = launch_k(qkv_post_vec_kernel<bf16>, vgrid, dim3(256), 0, c->stream, c->use_pdl, a);
+      e = one ? launch_k(qkv_post_vec_kernel<bf16, 1>, vgrid, dim3(256), 0, c->stream, c->use_pdl, a)
+              : launch_k(qkv_post_vec_kernel<bf16, 4>, vgrid, dim3(256), 0, c->stream, c->use_pdl, a);
     else
-      e = launch_k(qkv_post_vec_kernel<float>, vgrid, dim3(256), 0, c->stream, c->use_pdl, a);
+      e = one ? launch_k(qkv_post_vec_kernel<float, 1>, vgrid, dim3(256), 0, c->stream, c->use_pdl, a)
+              : launch_k(qkv_post_vec_kernel<float, 4>, vgrid, dim3(256), 0, c->stream, c->use_pdl, a);
     RB_CUDA(e);
     ++g_launch_total;
     return REWB200_OK;

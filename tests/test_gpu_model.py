@@ -383,6 +383,19 @@ def test_bf16_norms_of_large_steps(rb, orc, d, heads, routed, S):
     assert rel_l2(logits, want) <= 2e-2
 
 
+@pytest.mark.parametrize("dtype,tol", [("f32", 1e-5), ("bf16", 2e-2)])
+@pytest.mark.parametrize("S", [65, 255, 256, 257])
+def test_norms_and_rotations_of_steps_around_256_rows(rb, orc, S, dtype, tol):
+    """Up to 256 rows the slabs of a row are requested together, above that there is one."""
+    from rew_b200 import _lib
+    cfg = W.ModelConfig(vocab=128, d_model=1032, n_layers=2, n_heads=6, n_kv_heads=2, head_dim=64, ffn=520, max_seq=300, theta=10000.0,
+                        dtype=_lib.BF16 if dtype == "bf16" else _lib.F32, mask_kind=1)
+    t = [orc.bf16_round(a) if a.ndim == 2 else a for a in W.init_weights(cfg, seed=9, std=0.04, trivial_affine=False)]
+    prompt = np.random.default_rng(S).integers(0, cfg.vocab, size=(1, S)).astype(np.int32)
+    logits = rb.CausalLM(cfg).load(t).session(1, S).forward_all(prompt)
+    assert rel_l2(logits, orc.model_forward(cfg, t, prompt, 0, True)) <= tol
+
+
 @pytest.mark.parametrize("B,vocab", [(1, 131072), (2, 65537), (5, 120011)])
 def test_logits_of_any_size_come_home_whole(rb, orc, B, vocab):
     """Results travel in pieces of 512 KB: exactly one, one and a few bytes, several with a ragged end; behind a prompt, behind decode

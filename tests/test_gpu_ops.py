@@ -121,6 +121,19 @@ def test_norms(rb, orc, rows, d):
     assert rel_l2(rb.rmsNorm(T(rb, xb, _lib.BF16), T(rb, g), 1e-5).to_host(), orc.rmsnorm(xb, g, 1e-5)) < 5e-3
 
 
+@pytest.mark.parametrize("d", [1024, 2052, 8192, 16384])
+def test_norms_on_either_side_of_256_rows(rb, orc, d):
+    """Kernels of steps up to 256 rows and of larger ones, at every number of columns a thread can have: the rows they share come out
+    with the same bits, and within the tolerances above."""
+    from rew_b200 import _lib
+    rng = np.random.default_rng(d)
+    x = rng.normal(size=(257, d)).astype(np.float32) * 3
+    g = (1 + 0.1 * rng.normal(size=d)).astype(np.float32)
+    for a, kind, tol in ((x, _lib.F32, F32_TOL), (orc.bf16_round(x), _lib.BF16, 5e-3)):
+        few, many = (rb.rmsNorm(T(rb, a[:n], kind), T(rb, g), 1e-5).to_host() for n in (256, 257))
+        assert rel_l2(many, orc.rmsnorm(a, g, 1e-5)) < tol and np.array_equal(few, many[:256])
+
+
 def test_rope_bf16_and_errors(rb, orc):
     from rew_b200 import _lib
     from rew_b200._lib import RewB200Error
