@@ -57,7 +57,7 @@ struct AttnDev {
   // Decode only (S == 1), optional: q, k and v of the new token are not read from memory but finished here from
   // the f32 split-K slabs of the q|k|v projection (sum in slab order, bias, interleaved-pair RoPE, bf16), exactly
   // as qkv_post_kernel would have done one launch earlier; the CTA whose tile range ends the sequence also writes
-  // the new K / V row into the cache before it requests that tile.
+  // the new K / V row into the cache: ahead of its request for that tile, or, if it has asked for the tile early, into the tile's copy as well.
   const float* f_partial;  // [f_ks][B][f_ntot]; nullptr: q comes from `q`, the cache is complete
   int f_ks;
   int64_t f_stride;
@@ -291,7 +291,8 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(const __grid_constant_
   // Inside the engine's step, sequence lengths and block tables were written at least two kernels back
   // in the stream (every kernel of the chain waits on its predecessor before it ends), and the kernel
   // just before this one writes only the newest cache row, which lies in the last tile.  Then (early_kv)
-  // every other K/V tile can be requested before griddepcontrol.wait, while that predecessor still runs.
+  // every other K/V tile can be requested before griddepcontrol.wait, while that predecessor still runs, and the last one too
+  // where this kernel finishes the newest row itself (`patch`).
   if (!a.early_kv) pdl_wait();
   const int kv_len = kv_len_of(a, b);
   const int ntiles = (kv_len + TILE - 1) / TILE;
@@ -299,8 +300,8 @@ __global__ void __launch_bounds__(128) attn_decode_kernel(const __grid_constant_
   const int t0 = split * tps, t1 = min(ntiles, t0 + tps);
   const int nt_local = max(0, t1 - t0);
   // The CTA with a sequence's last tile finishes the newest K / V row itself (below).  It asks for that tile early as well, as long
-  // as it is among the first, and puts the row into its copy: through memory and a bulk copy behind the row's stores, the
-  // tile arrived 1.5 us later.
+  // as it is among the first (two tiles of 64 tokens: a context of up to 128 where sequences are not split, longer where they are), and
+  // puts the row into its copy: through memory and a bulk copy behind the row's stores, the tile arrived 1.5 us later.
   const bool owns_last = ntiles > 0 && t0 <= ntiles - 1 && ntiles - 1 < t1;
   const bool patch = a.f_partial && a.early_kv && owns_last && nt_local <= ATT_STAGES - 1;
   int early = 0;

@@ -405,8 +405,10 @@ struct AttnArgs {
                                 // have done in a launch of its own) and appends K / V to the cache; `q` is not read
 };
 // Queries of a sequence from which its attention runs on tcgen05 (tiles of 128 queries and 128 keys; head_dim 128) and no longer on
-// mma.sync (64 and 64): half a tile.  12 lanes of the 8B shape, one of them with portions of 100 tokens behind up to 500: 26 us a launch
-// on mma.sync, 13 on tcgen05 (the step's six layers, 10.01 / 9.74 ms); prompts of 20 to 100 tokens and portions of 6 to 12 take the same time on either.
+// mma.sync (64 and 64): half a tile.  Us a layer that tcgen05 saves, 8B shape: a portion of 64 tokens beside eleven single ones, behind 0 / 300 /
+// 700 tokens, 5 / 14 / 34; of 100 tokens 11 / 16 / 45; 8 prompts of 100 tokens 32, 32 of them 50; prompts of 64 tokens, 1, 8 or 32 of
+// them, the same time on either.  The error against 64 bits is that of a prompt of 128 tokens and more: 0.3 % above mma.sync's, because
+// wider key tiles have fewer keys that set a new maximum, whose weight is exactly one.
 constexpr int kAttnTcRows = 64;
 int attn_launch(Ctx* c, const AttnArgs& a);
 int decode_splits(Ctx* c, int64_t B, int kvh);  // KV splits a decode attention launch of B sequences x kvh kv heads uses

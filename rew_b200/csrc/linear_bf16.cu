@@ -299,8 +299,10 @@ int linear_bf16_pick_ksplit(Ctx* c, int64_t M, int64_t K, int64_t N) {
   int split = 1;
   if (M > 64 && c->linear_impl != 0) {
     // Above 64 rows every slab costs its M rows twice through L2 (4 bytes an element there and back, about 4 TB/s), and an SM
-    // spends 0.2 to 0.33 us on a 128 x 64 block of weights as the step's rows grow (0.29 here): the count that makes both together least.
-    // 135 rows of 4096 x 6144 (48 tiles) take 3 slabs, of 4096 x 4096 and 14336 x 4096 (32 tiles) 4.
+    // some time on a 128 x 64 block of weights: the count that makes both together least.  135 rows of 4096 x 6144 (48 tiles) take 3
+    // slabs, of 4096 x 4096 and 14336 x 4096 (32 tiles) 4.  The 0.29 us are what these counts were measured with; today a block takes
+    // 0.2 to 0.36 us (choose_tiles in linear_tc.cu), which gives the same counts but above 212 rows of 4096 x 4096 and 2048 x 2048 (4, here
+    // 3), above 236 of 4096 x 6144 and 2048 x 3072 (3, here 2) and at 98 to 141 of 2048 x 3072 (3, here 4).
     double best = 0;
     for (int k = 1; k <= 4 && (k == 1 || nkb / k >= c->splitk_min_blocks); ++k) {
       const double us = 0.29 * ((tiles * k + c->sm_count - 1) / c->sm_count) * ((nkb + k - 1) / k) + 8e-6 * k * M * N / 4;

@@ -12,7 +12,7 @@
 //         the scales of the block's two 64-feature groups as [2][32] bf16 pairs (rows 2j, 2j + 1): what the GEMV multiplies by
 //   sc  [N/64][K] f32      the scales of one 64-feature group, contiguous along k
 // GEMV (rows <= 32) on the 5th-generation tensor core with the WEIGHT operand in tensor memory:
-//   D[128 features][32 tokens] (TMEM, f32) += A[128 features][64 k] (TMEM, bf16) * B[64 k][32 tokens] (smem)
+//   D[128 features][16 or 32 tokens] (TMEM, f32) += A[128 features][64 k] (TMEM, bf16) * B[64 k][16 or 32 tokens] (smem)
 //   warp 0      TMA producer, two rings: 14 stages of the tile's codes with their scale pairs (one bulk copy each out of
 //               HBM, 60 KB in flight per CTA), 16 KB of activation tiles (16 or 32 tokens x 64 k, 128-byte swizzle, out of L2)
 //   warp 1      one thread issues four tcgen05.mma (K = 16 each) per block of 64 rows, A read from TMEM
@@ -578,7 +578,7 @@ int nf4_gemv_launch(Ctx* c, const Nf4W& w, const bf16* x, int64_t ldx, int64_t M
     return REWB200_OK;
   }
   CUtensorMap tmX;
-  const int tn = M <= 16 ? 16 : 32;
+  const int tn = M <= 16 ? 16 : 32;   // a decode step of six 8B layers, us, 32 / 16: 1 row 497.0 / 496.5, 4 rows 530.6 / 528.6, 8 rows 553 / 549.5
   RB_TRY(make_tmap_2d_bf16(&tmX, x, (uint64_t)w.K, (uint64_t)M, (uint64_t)ldx * 2, 64, tn));
   static bool attr_set = false;
   if (!attr_set) {

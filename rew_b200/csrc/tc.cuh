@@ -8,12 +8,11 @@
 namespace rewb {
 namespace tc {
 
-// One lane of a converged warp, the same one every time.  tcgen05 and bulk-copy instructions take uniform operands.  Behind a
-// branch on the lane's number the compiler does not know that one lane is left and guards every one of them with a loop over
-// the lanes; behind elect.sync it does.  Together with issuing the four products of a 64-deep stage in one block of code
-// (below) this is the price of a product: 148 CTAs, M = 128, cycles a product of 16 k: N = 16 to 128 lane test 90 (144 with
-// descriptors built at run time), elected 49 to 64, elected and in fours 40 to 64; N = 256 128 in every form, which is the
-// tensor core's own rate (N = 128: 64).
+// One lane of a converged warp, the same one every time, for roles of a single thread.  Measured against a branch on the lane's number, and
+// together with issuing the four products of a 64-deep stage in one block of code (below): 148 CTAs, M = 128, cycles a product of 16 k,
+// N = 16 to 128 lane test 90 (144 with descriptors built at run time), elected 49 to 64, elected and in fours 40 to 64; N = 256 128 in
+// every form, which is the tensor core's own rate (N = 128: 64).  Likely cause: elect.sync tells the compiler that one lane is left, as a
+// test of the lane's number does not, and these instructions take operands that are the same for a whole warp.
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));

@@ -131,7 +131,7 @@ def test_launch_counter_moves(rb):
 
 
 def test_bf16_prefill_attention_kernels_agree_and_chunked_prefill(rb):
-    """head_dim 128 and prompts of 128+ tokens put prefill attention on the tcgen05 kernel: its logits match
+    """head_dim 128 and prompts of 64 tokens and more put prefill attention on the tcgen05 kernel: its logits match
     the mma.sync kernel's, and a prompt fed in two chunks (the second attends to a 150-token context through
     the paged cache) matches the same prompt fed at once."""
     from rew_b200 import _lib

@@ -278,10 +278,11 @@ def test_swiglu_and_embedding(rb, orc):
 
 
 @pytest.mark.parametrize("B,nh,kvh,S,L", [(2, 8, 2, 512, 512), (1, 4, 4, 300, 300), (1, 8, 1, 130, 400), (3, 4, 2, 128, 128),
-                                          (1, 2, 2, 1000, 1000), (2, 4, 2, 256, 256), (1, 4, 1, 384, 700)])
+                                          (1, 2, 2, 1000, 1000), (2, 4, 2, 256, 256), (1, 4, 1, 384, 700),
+                                          (2, 4, 2, 64, 64), (1, 8, 2, 65, 300), (3, 4, 4, 127, 127), (1, 4, 1, 100, 800)])
 @pytest.mark.parametrize("mode", ["plain", "standard"])
 def test_attention_bf16_prefill_tcgen05(rb, orc, B, nh, kvh, S, L, mode):
-    """head_dim 128 and at least 128 queries: the tcgen05 kernel (S and O in tensor memory).  Ragged last
+    """head_dim 128 and at least 64 queries: the tcgen05 kernel (S and O in tensor memory).  Ragged last
     tiles, grouped heads, and a context longer than the query block (keys j <= i + L - S visible)."""
     from rew_b200 import _lib
     rng = np.random.default_rng(S + L)

@@ -110,7 +110,7 @@ def test_pool_exhaustion_and_lane_errors(rb):
 
 @pytest.mark.parametrize("dtype,hd,mask,tol", [("f32", 32, 0, 1e-5), ("f32", 32, 1, 1e-5), ("bf16", 64, 1, 2e-2), ("bf16", 128, 1, 2e-2), ("bf16", 128, 0, 2e-2)])
 def test_feed_of_unequal_portions_in_any_order(rb, orc, dtype, hd, mask, tol):
-    """Every kind of portion (one token, below 128, 128 and more) in one step, several of each, in scrambled order and on lanes
+    """Every kind of portion (one token, below 64, 64 and more) in one step, several of each, in scrambled order and on lanes
     whose contexts differ: wanted rows equal the oracle's forward of each lane's whole text.  A conventional mask only lets
     later portions see earlier ones; the mask as written is checked on first portions, where it needs no context."""
     from rew_b200 import _lib
@@ -251,6 +251,39 @@ def test_feed_with_sampling_and_seeds_in_any_order(rb, orc):
     for l, p in enumerate(prompts):
         want, _ = orc.generate_sampled(cfg, t, p[None], n_new, seeds=[seeds[l]], **kw)
         assert out[l] == want[0].tolist(), l
+
+
+@pytest.mark.parametrize("first", [0, 64, 130])
+def test_feed_of_portions_on_either_side_of_64_queries(rb, orc, first):
+    """Head size 128: portions of 3 to 63 tokens attend on mma.sync, those of 64 and more on tcgen05, one launch a layer for all of a kind,
+    behind nothing, a whole page and pages and a half.  Every row of the step against the oracle."""
+    from rew_b200 import _lib
+    cfg = W.ModelConfig(vocab=128, d_model=256, n_layers=2, n_heads=4, n_kv_heads=2, head_dim=128, ffn=192, max_seq=512, theta=10000.0,
+                        dtype=_lib.BF16, mask_kind=1)
+    t = [orc.bf16_round(a) if a.ndim == 2 else a for a in W.init_weights(cfg, seed=3, std=0.08, trivial_affine=False)]
+    rng = np.random.default_rng(first)
+    sizes = {5: 64, 1: 3, 0: 63, 6: 1, 2: 40, 4: 65, 3: 127}
+    texts = {l: rng.integers(0, cfg.vocab, first + l + n).astype(np.int32) for l, n in sizes.items()}   # contexts of unequal length
+    at = {l: len(texts[l]) - n for l, n in sizes.items()}
+    sess = rb.CausalLM(cfg).load(t).paged_session(7, 300, 40)
+    before_it = [(l, texts[l][:at[l]]) for l in sizes if at[l]]
+    if before_it:
+        sess.feed(before_it)
+    count = lambda: [_lib.lib().rewb200_kernel_launches(k.encode()) for k in ("attention_tc", "attention_tc2")]
+    before = count()
+    logits, _ = sess.feed([(l, texts[l][at[l]:]) for l in sizes], want=range(sum(sizes.values())))
+    assert [a - b for a, b in zip(count(), before)] == [cfg.n_layers, 0]
+    row = 0
+    for l, n in sizes.items():
+        want = orc.model_forward(cfg, t, texts[l][None], 0, True)[0, at[l]:]
+        err = np.linalg.norm(logits[row:row + n] - want, axis=1) / np.linalg.norm(want, axis=1)
+        assert err.max() <= 3e-2, (l, n, err.argmax(), err.max())     # as the test above: rows one by one
+        row += n
+    # without a portion of 64 or more nothing runs on tcgen05
+    sess.reset()
+    before = count()
+    sess.feed([(l, texts[l][:n]) for l, n in ((0, 63), (1, 3), (2, 40), (6, 1))])
+    assert count() == before
 
 
 def test_feed_of_long_portions_with_two_query_tiles_a_cta(rb):
