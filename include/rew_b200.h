@@ -444,7 +444,8 @@ void rewb200_session_free(rewb200_session* s);
 int rewb200_session_reset(rewb200_session* s);
 /* Feeds `S` new tokens per sequence (host int32 [batch,S]) at the current
  * offset, appends K/V, returns greedy next ids (host int32 [batch]) and, when
- * logits_out != NULL, the last-position logits (host f32 [batch,vocab]). */
+ * logits_out != NULL, the last-position logits (host f32 [batch,vocab]).
+ * Here and below, logits in pinned memory are copied into by the device itself. */
 int rewb200_session_forward(rewb200_session* s, const int32_t* ids, int S, int32_t* next_ids, float* logits_out);
 /* `n_steps` greedy decode steps entirely on the device starting from the ids
  * the last forward produced; host out_ids [batch,n_steps]. */
