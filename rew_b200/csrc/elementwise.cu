@@ -1252,6 +1252,11 @@ int output_norm_launch(Ctx* c, const OutputNormArgs& a, int64_t rows) {
    : nch <= 4 ? go(output_norm_kernel<T, CL, 4, G>, CL) : go(output_norm_kernel<T, CL, 8, G>, CL))
   if (cluster) {
     const int nch = (int)((a.d / 16 + 255) / 256);
+    // Eight slabs of a row under way together take registers, and where two of these CTAs share an SM their registers keep the next Linear's
+    // CTA, which starts early for its weights, from joining them.  With a sixth more CTAs than SMs that costs more than two slabs at a time
+    // (us a decode step, eight / two: musavik, 8 layers, 38 sequences 1009 / 1018, 44 1038 / 1026, 48 1072 / 1054, 64 1147 / 1136; girulorn, 6
+    // layers, 40 528 / 534, 44 538 / 534, 48 544 / 541).
+    if (rows * 24 > (int64_t)c->sm_count * 7) return bf ? RB_ONORM(bf16, 4, 2) : RB_ONORM(float, 4, 2);
     return bf ? RB_ONORM(bf16, 4, 8) : RB_ONORM(float, 4, 8);
   }
   const int nch = (int)((a.d / 4 + 511) / 512);

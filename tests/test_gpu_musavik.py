@@ -607,6 +607,18 @@ def test_bf16_decode_step_matches_the_fed_step(rb):
     assert err(lg[-1:], logits) < 1e-2
 
 
+@pytest.mark.parametrize("lanes", [43, 44, 64])
+def test_norms_on_the_way_back_where_two_ctas_share_an_sm(rb, lanes):
+    """From 44 rows on the norms on clusters take two slabs at a time: feed-forwards long enough that their way out is cut along K."""
+    cfg = K.config([K.rglru(K.dense(2080)), K.rglru(K.dense(4160))])
+    t = K.weights(cfg, seed=17)
+    ps = build(rb, cfg, t, "bfloat16", max_seq=64).paged_session(lanes, 64, lanes + 1)
+    reqs = [K.tokens(cfg, 6 + i % 5, seed=300 + i) for i in range(lanes)]
+    ps.feed([(i, r[:-1]) for i, r in enumerate(reqs)])
+    lg, _ = ps.feed([(i, r[-1:]) for i, r in enumerate(reqs)], want=range(lanes))
+    close(lg, np.concatenate([G.forward(cfg, t, r)[-1:] for r in reqs]), "bfloat16")
+
+
 def test_wide_batches_of_decoding_lanes(rb):
     """More lanes than a small step has rows, each at its own length."""
     cfg = K.config([K.parallel(K.dense(), heads=4, kv_heads=4, dim=64, vdim=64, rot=64, size=30, keep=3), K.rglru(K.dense())])
